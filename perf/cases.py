@@ -132,6 +132,24 @@ def _lognormal(g, rows, cols, dtype):
     return torch.where((u > 0.495) & (u < 0.505), torch.zeros((), device=DEVICE), mag).to(dtype)
 
 
+def _train_inputs(g, case):
+    t, k, n = case["tokens"], case["k"], case["n"]
+    return _normal(g, t, k), _normal(g, n, k) * k ** -0.5, _normal(g, t, n)
+
+
+def _linear_inputs(g, case):
+    tokens, k, n = case["tokens"], case["k"], case["n"]
+    x = _normal(g, tokens, k, outliers=1e-3)
+    w = _normal(g, n, k) * k ** -0.5
+    if case["kind"] == "rowwise":
+        x *= torch.pow(10.0, torch.rand(tokens, 1, generator=g, device=DEVICE) * 2.0 - 1.0).to(torch.bfloat16)
+    return x, w
+
+
+def _bias(g, case):
+    return torch.randn(case["n"], generator=g, device=DEVICE).to(torch.bfloat16) if case["bias"] else None
+
+
 def prepare(case, seed):
     g = _gen(seed)
     kind = case["kind"]
@@ -152,18 +170,13 @@ def prepare(case, seed):
         s["x"] = _normal(g, case["rows"], case["cols"], outliers=1e-4, factor=1000.0)
         s["quantizer"] = dtq.ShardedQuantizer()
     elif kind == "mx8_train":
-        s["x"] = _normal(g, case["tokens"], case["k"])
-        s["w"] = _normal(g, case["n"], case["k"]) * case["k"] ** -0.5
-        s["grad"] = _normal(g, case["tokens"], case["n"])
+        s["x"], s["w"], s["grad"] = _train_inputs(g, case)
     else:
-        tokens, k, n = case["tokens"], case["k"], case["n"]
-        s["x"] = _normal(g, tokens, k, outliers=1e-3)
-        w = _normal(g, n, k) * k ** -0.5
+        s["x"], w = _linear_inputs(g, case)
         if kind == "rowwise":
-            s["x"] *= torch.pow(10.0, torch.rand(tokens, 1, generator=g, device=DEVICE) * 2.0 - 1.0).to(torch.bfloat16)
             payload, _, scale = dtq.dynamic_scaled_quant_rowwise(w, torch.float8_e4m3fn)
             s["w"], s["w_scale"] = payload.t(), scale.reciprocal().t()
-            s["bias"] = torch.randn(n, generator=g, device=DEVICE).to(torch.bfloat16) if case["bias"] else None
+            s["bias"] = _bias(g, case)
         elif kind == "mx8":
             payload, s["w_scale"] = dtq.mx_fp8_quantize_blocked(w)
             s["w"] = payload.t()
@@ -207,6 +220,52 @@ def run(s):
     dw = dtq.mx_fp8_bf16(pgt, pxt.t(), sgt, sxt)
     return y, dx, dw
 
+
+# ---- the same in 64 bits ------------------------------------------------------------------------------------------
+
+def _rowwise64(x):
+    """Row-wise e4m3: the payload, and the fp32 factor that undoes its scale, both as fp64."""
+    sd = 448.0 / (x.abs().amax(1, keepdim=True).double() + 1e-12)
+    payload = (x.double() * sd).float().clamp(-448.0, 448.0).to(torch.float8_e4m3fn).double()
+    return payload, sd.float().reciprocal().double()
+
+
+def _mx64(x, fp4=False):
+    """The values that the MX blocks of 32 along the last dimension stand for, as fp64."""
+    rows, cols = x.shape
+    v = x.reshape(rows, cols // 32, 32)
+    mag = (v.contiguous().view(torch.int16).to(torch.int32) & 0x7FFF).amax(2, keepdim=True)
+    exponent = (((mag + 0x7F) >> 7) - (2 if fp4 else 8)).clamp_min(0) - 127  # ceil(log2) less the format's largest exponent
+    scale = torch.exp2(exponent.double())
+    v = v.double() / scale
+    if fp4:
+        a = v.abs()
+        step = torch.where(a < 2.0, 0.5, torch.where(a < 4.0, 1.0, 2.0))  # of e2m1: 0 .5 1 1.5 2 3 4 6
+        v = (torch.round(v / step) * step).clamp(-6.0, 6.0)
+    else:
+        v = v.float().clamp(-448.0, 448.0).to(torch.float8_e4m3fn).double()
+    return (v * scale).reshape(rows, cols)
+
+
+def exact(case, seed):
+    """The products of the quantized operands in fp64; the casts are bit patterns and have no such value."""
+    kind = case["kind"]
+    if kind not in ("rowwise", "mx8", "mx4", "mx8_train"):
+        return None
+    g = _gen(seed)
+    if kind == "mx8_train":
+        x, w, grad = _train_inputs(g, case)
+        return (_mx64(x) @ _mx64(w).t(), _mx64(grad) @ _mx64(w.t()).t(), _mx64(grad.t()) @ _mx64(x.t()).t())
+    x, w = _linear_inputs(g, case)
+    if kind != "rowwise":
+        return _mx64(x, kind == "mx4") @ _mx64(w, kind == "mx4").t()
+    bias = _bias(g, case)
+    (px, fx), (pw, fw) = _rowwise64(x), _rowwise64(w)
+    y = (px @ pw.t()).mul_(fx).mul_(fw.t())
+    return y if bias is None else y.add_(bias.double())
+
+
+# ---- what a pass cannot do without, and how far two correct ones may differ ---------------------------------------
 
 def work(case):
     """Bytes: inputs read once, outputs written once (what lies between two calls is not counted); flops: the products'."""
