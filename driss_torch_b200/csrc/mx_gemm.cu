@@ -310,7 +310,37 @@ __device__ __forceinline__ void tmem_load_32(uint32_t (&v)[32], uint32_t taddr) 
       : "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tmem_load_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// Waits for this thread's tensor-memory loads.  The registers pass through the statement, so that no use of them can
+// be scheduled before it.
+__device__ __forceinline__ void tmem_load_wait(uint32_t (&v)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]),
+                 "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]), "+r"(v[16]),
+                 "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]), "+r"(v[24]),
+                 "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])
+               :
+               : "memory");
+}
+
+// 32 bf16 of one output row (64 bytes at `dst`), of which the first `live` columns exist (a multiple of 8).  A lane owns
+// a row, so a warp-wide store of 16 bytes per lane touches 32 half sectors and L2 sees every sector twice; where the
+// row pitch allows it (`wide`: output and pitch 32-byte aligned) a lane stores whole 32-byte sectors.  Streaming: the
+// output must not push the operands out of L2.
+__device__ __forceinline__ void store_row_32(uint16_t *dst, const uint32_t (&p)[16], int64_t live, bool wide) {
+  if (wide) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      if (q * 16 < live)  // N % 16 == 0 here
+        asm volatile("st.global.cs.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + q * 16), "r"(p[8 * q]),
+                     "r"(p[8 * q + 1]), "r"(p[8 * q + 2]), "r"(p[8 * q + 3]), "r"(p[8 * q + 4]), "r"(p[8 * q + 5]),
+                     "r"(p[8 * q + 6]), "r"(p[8 * q + 7])
+                     : "memory");
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (q * 8 < live) stg_stream(dst + q * 8, make_uint4(p[4 * q], p[4 * q + 1], p[4 * q + 2], p[4 * q + 3]));
+  }
+}
 
 struct GemmParams {
   RowwiseEpilogue rowwise;
@@ -491,7 +521,8 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const uint32_t taddr = tmem + (uint32_t(quad * 32) << 16) + uint32_t(acc * kBN + half * kHalfCols + c * 32);
         tmem_load_32(v[0], taddr);
         tmem_load_32(v[1], taddr + 32);
-        tmem_load_wait();
+        tmem_load_wait(v[0]);
+        tmem_load_wait(v[1]);
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           if constexpr (MODE == kRowwise) apply_rowwise(v[u], rw.xs, rw.cs[c + u], rw.bs[c + u], rw.has_bias);
@@ -548,12 +579,29 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 //     [512 bytes]), so that a missing atom is simply filled with zeros; every CTA needs its own A atom and
 //     both B atoms (its accumulator spans all 256 columns);
 //   * the leader's MMA thread copies the scales (tcgen05.cp.cta_group::2: each CTA's shared memory into that
-//     CTA's tensor memory), issues the MMAs, and commits twice per barrier, once for each CTA's copy of it;
-//   * the peer's epilogue warps arrive on the leader's `tmem_empty` barrier through the cluster address space.
+//     CTA's tensor memory), issues the MMAs, and commits to both CTAs' copies of a barrier at once;
+//   * two accumulators alternate, so that the tensor cores work on the next tile while the epilogue empties this one
+//     (see PairTmem); the peer's epilogue warps arrive on the leader's `tmem_empty` barriers through the cluster
+//     address space.
 // Every wait is bounded as above; an abort is forwarded to the other CTA, and both always meet at the cluster
 // barrier before tensor memory is freed.
 constexpr int kPairStages = 6;
 constexpr int kPairBN = 256;  // tile columns; each CTA holds kPairBN / 2 rows of B
+
+// Tensor memory of the pair kernel: two accumulators of 256 columns.  Without block scales they fill the 512 columns
+// exactly.  With block scales 24 columns are needed beside them, so the second accumulator starts 32 columns early and
+// shares columns 224..255 with the first: the MMAs of a tile may start as soon as the epilogue has taken those 32
+// columns of the tile BEFORE it (which it reads first) and all of the tile before that.
+// With one accumulator the tensor cores stood still for about 3 us per tile, from the last MMA of a tile until all of it
+// had been read.  Measured (one against two, B200, steady state): MXFP4 2000 x 12288 x 4096 with its cast 65.6 -> 59.6 us,
+// row-wise 32768 x 4096 x 4096 with its quantization 587 -> 547 us; an MXFP8 training step at 8192^3 stays at 1.57-1.59 ms,
+// because the board's power limit sets its clock and busier tensor cores run at a lower one.
+template <int MODE>
+struct PairTmem {
+  static constexpr bool kShared = Format<MODE>::kScaled;
+  static constexpr int kAcc1 = kShared ? 224 : 256;  // first column of the second accumulator
+  static constexpr int kSfa = 480, kSfb = 488;       // scales: A 4 columns per atom along K, B 8
+};
 
 template <int MODE>
 struct __align__(1024) PairSmem {
@@ -563,8 +611,8 @@ struct __align__(1024) PairSmem {
   uint8_t sfb[kPairStages][2 * Format<MODE>::kKAtoms * 512];  // scales of all 256 rows of B: [128 columns][atom along K]
   uint64_t full[kPairStages];                    // used in the leader CTA only
   uint64_t empty[kPairStages];
-  uint64_t tmem_full;
-  uint64_t tmem_empty;                           // used in the leader CTA only
+  uint64_t tmem_full[2];                         // one per accumulator
+  uint64_t tmem_empty[2];                        // used in the leader CTA only
   uint32_t tmem_base;
   int abort;
 };
@@ -605,8 +653,12 @@ __device__ __forceinline__ void tma_pair_load_3d(void *dst, const CUtensorMap *m
       "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr) : "memory");
+// All MMAs issued so far, once done, arrive on the barrier at this offset in BOTH CTAs of the pair.
+__device__ __forceinline__ void umma_commit_pair(uint64_t *bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                   smem_addr(bar)),
+               "h"(static_cast<uint16_t>(3))
+               : "memory");
 }
 
 struct PairParams {
@@ -614,6 +666,7 @@ struct PairParams {
   uint16_t *out;  // bf16 [M, N]
   int M, N;
   int m_pairs, n_tiles, k_stages;  // 256-row tile rows, 256-column tile columns, 128-byte K stages
+  bool wide_stores;                // rows of the output start on 32-byte boundaries
   int *status;
 };
 
@@ -638,8 +691,10 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       mbar_init(&sm.full[s], 1);   // the leader's producer arrives once, expecting both CTAs' bytes
       mbar_init(&sm.empty[s], 1);  // one commit of the leader's MMA thread per CTA
     }
-    mbar_init(&sm.tmem_full, 1);
-    mbar_init(&sm.tmem_empty, 2 * kEpilogueWarps);  // the epilogue warps of both CTAs
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&sm.tmem_full[i], 1);
+      mbar_init(&sm.tmem_empty[i], 2 * kEpilogueWarps);  // the epilogue warps of both CTAs
+    }
     sm.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -699,13 +754,17 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       uint32_t stage = 0, phase = 0;
       int local_tile = 0;
       bool ok = true;
-      const uint32_t peer_full = map_to_cta(smem_addr(&sm.tmem_full), 1);
       for (int tile = cluster_id; tile < total_tiles && ok; tile += n_clusters, ++local_tile) {
-        if (local_tile > 0 && !mbar_wait_warp(&sm.tmem_empty, (local_tile - 1) & 1u, abort)) {
+        // shared columns: wait for the previous tile's (its epilogue has then also emptied the accumulator used here, two
+        // tiles ago); separate accumulators: for the tile two before this one
+        constexpr int kBack = PairTmem<MODE>::kShared ? 1 : 2;
+        const int before = local_tile - kBack;
+        if (before >= 0 && !mbar_wait_warp(&sm.tmem_empty[before & 1], (before >> 1) & 1u, abort)) {
           ok = false;
           break;
         }
         tmem_fence_after();
+        const uint32_t d_tmem = tmem + ((local_tile & 1) ? PairTmem<MODE>::kAcc1 : 0);
         for (int ks = 0; ks < p.k_stages; ++ks) {
           if (!mbar_wait_warp(&sm.full[stage], phase, abort)) {
             ok = false;
@@ -716,10 +775,11 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if constexpr (Format<MODE>::kScaled) {
 #pragma unroll
               for (int j = 0; j < kKAtoms; ++j) {  // each CTA's shared memory -> that CTA's tensor memory, columns as above
-                copy_scale_atom<true>(tmem + kSfaCol + 4 * j, smem_addr(sm.sfa[stage] + j * 512));
+                copy_scale_atom<true>(tmem + PairTmem<MODE>::kSfa + 4 * j, smem_addr(sm.sfa[stage] + j * 512));
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
-                  copy_scale_atom<true>(tmem + kSfbCol + j * 8 + 4 * h, smem_addr(sm.sfb[stage] + (h * kKAtoms + j) * 512));
+                  copy_scale_atom<true>(tmem + PairTmem<MODE>::kSfb + j * 8 + 4 * h,
+                                        smem_addr(sm.sfb[stage] + (h * kKAtoms + j) * 512));
               }
             }
             const uint32_t a_addr = smem_addr(sm.a[stage]), b_addr = smem_addr(sm.b[stage]);
@@ -727,14 +787,12 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             for (uint32_t k = 0; k < 4; ++k) {
               const uint32_t accumulate = (ks > 0 || k > 0) ? 1u : 0u;
               const uint32_t j = Format<MODE>::k_atom(k), id = Format<MODE>::sf_id(k);
-              issue_mma<MODE, true>(tmem, operand_desc(a_addr + k * 32), operand_desc(b_addr + k * 32),
+              issue_mma<MODE, true>(d_tmem, operand_desc(a_addr + k * 32), operand_desc(b_addr + k * 32),
                                    instr_desc(id, kPairBN, 256, Format<MODE>::kFormatBits | p.rowwise.operand_format_bits),
-                                   accumulate, (tmem + kSfaCol + 4 * j) | (id << 30), (tmem + kSfbCol + j * 8) | (id << 30));
+                                   accumulate, (tmem + PairTmem<MODE>::kSfa + 4 * j) | (id << 30),
+                                   (tmem + PairTmem<MODE>::kSfb + j * 8) | (id << 30));
             }
-            // the stage is free in both CTAs once these MMAs have read it
-            const uint32_t empty_bar = smem_addr(&sm.empty[stage]);
-            umma_commit_pair(empty_bar);
-            umma_commit_pair(map_to_cta(empty_bar, 1));
+            umma_commit_pair(&sm.empty[stage]);  // the stage is free in both CTAs once these MMAs have read it
           }
           __syncwarp();
           if (++stage == kPairStages) {
@@ -742,10 +800,8 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             phase ^= 1u;
           }
         }
-        if (ok && elect_one()) {  // both CTAs' halves of the accumulator are complete once all MMAs so far have finished
-          umma_commit_pair(smem_addr(&sm.tmem_full));
-          umma_commit_pair(peer_full);
-        }
+        // both CTAs' halves of the accumulator are complete once all MMAs so far have finished
+        if (ok && elect_one()) umma_commit_pair(&sm.tmem_full[local_tile & 1]);
         __syncwarp();
       }
       if (!ok && lane == 0) {
@@ -756,16 +812,21 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
   } else {
     // ---- epilogue: this CTA's 128 rows of the tile, 8 warps as in the single-CTA kernel --------------------
+    // A warp's 128 columns go 32 at a time, the next 32 on their way from tensor memory while these are converted and
+    // stored.  The half that holds the shared columns starts with them: half 1 at its end (columns 255..224 of the first
+    // accumulator), half 0 at its beginning (columns 0..31 of the second, the same columns of tensor memory).
     const int quad = warp & 3, half = (warp - 2) >> 2;
-    const uint32_t leader_empty = map_to_cta(smem_addr(&sm.tmem_empty), 0);
+    const uint32_t leader_empty[2] = {map_to_cta(smem_addr(&sm.tmem_empty[0]), 0), map_to_cta(smem_addr(&sm.tmem_empty[1]), 0)};
     int local_tile = 0;
     for (int tile = cluster_id; tile < total_tiles; tile += n_clusters, ++local_tile) {
       int mp, nt;
       tile_coords(tile, p.m_pairs, p.n_tiles, &mp, &nt);
       const int64_t row = int64_t(mp) * 256 + int64_t(rank) * kBM + quad * 32 + lane;
+      const int64_t col0 = int64_t(nt) * kPairBN + half * 128;
+      const int acc = local_tile & 1;
       RowwiseRegs<4> rw;
-      if constexpr (MODE == kRowwise) load_rowwise<4>(rw, p.rowwise, row, int64_t(nt) * kPairBN + half * 128, lane, p.M, p.N);
-      if (!mbar_wait(&sm.tmem_full, local_tile & 1u, abort)) {
+      if constexpr (MODE == kRowwise) load_rowwise<4>(rw, p.rowwise, row, col0, lane, p.M, p.N);
+      if (!mbar_wait(&sm.tmem_full[acc], (local_tile >> 1) & 1u, abort)) {
         if (lane == 0) {
           atomicExch(p.status, DTQ_ERR_TIMEOUT);
           *abort = 1;
@@ -774,36 +835,31 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         break;
       }
       tmem_fence_after();
-      uint32_t packed[4][16];
+      const uint32_t taddr = tmem + (uint32_t(quad * 32) << 16) + uint32_t((acc ? PairTmem<MODE>::kAcc1 : 0) + half * 128);
+      uint16_t *dst = p.out + row * p.N + col0;
+      // the i-th 32 columns of this warp in the order it takes them
+      auto chunk_at = [&](int i) { return PairTmem<MODE>::kShared && half ? 3 - i : i; };
+      // handed back after the shared columns (the other half has none to wait for) or after everything
+      const int release_after = PairTmem<MODE>::kShared ? (half == acc ? -1 : 0) : 3;
+      auto hand_back = [&] {
+        tmem_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(acc ? leader_empty[1] : leader_empty[0]);
+      };
+      if (release_after < 0) hand_back();
+      uint32_t v[2][32];
+      tmem_load_32(v[0], taddr + chunk_at(0) * 32);
 #pragma unroll
-      for (int c = 0; c < 4; c += 2) {  // two loads in flight per wait
-        uint32_t v[2][32];
-        const uint32_t taddr = tmem + (uint32_t(quad * 32) << 16) + uint32_t(half * 128 + c * 32);
-        tmem_load_32(v[0], taddr);
-        tmem_load_32(v[1], taddr + 32);
-        tmem_load_wait();
+      for (int i = 0; i < 4; ++i) {
+        tmem_load_wait(v[i & 1]);
+        if (i == release_after) hand_back();
+        if (i < 3) tmem_load_32(v[(i + 1) & 1], taddr + chunk_at(i + 1) * 32);
+        const int c = chunk_at(i);
+        if constexpr (MODE == kRowwise) apply_rowwise(v[i & 1], rw.xs, rw.cs[i], rw.bs[i], rw.has_bias);  // c == i
+        uint32_t packed[16];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          if constexpr (MODE == kRowwise) apply_rowwise(v[u], rw.xs, rw.cs[c + u], rw.bs[c + u], rw.has_bias);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) packed[c + u][i] = pack_bf16(v[u][2 * i], v[u][2 * i + 1]);
-        }
-      }
-      tmem_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(leader_empty);
-      if (row < p.M) {
-        uint16_t *dst = p.out + row * p.N + int64_t(nt) * kPairBN + half * 128;
-        const int64_t col0 = int64_t(nt) * kPairBN + half * 128;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            if (col0 + c * 32 + q * 8 < p.N)
-              stg_stream(dst + c * 32 + q * 8,
-                         make_uint4(packed[c][4 * q], packed[c][4 * q + 1], packed[c][4 * q + 2], packed[c][4 * q + 3]));
-          }
-        }
+        for (int j = 0; j < 16; ++j) packed[j] = pack_bf16(v[i & 1][2 * j], v[i & 1][2 * j + 1]);
+        if (row < p.M) store_row_32(dst + c * 32, packed, p.N - (col0 + c * 32), p.wide_stores);
       }
     }
   }
@@ -952,6 +1008,7 @@ int launch_pair(const GemmCall &c, int max_clusters) {
   p.out = static_cast<uint16_t *>(c.out);
   p.M = static_cast<int>(c.m);
   p.N = static_cast<int>(c.n);
+  p.wide_stores = c.n % 16 == 0 && aligned_to(c.out, 32);
   p.m_pairs = static_cast<int>(ceil_div64(c.m, 256));
   p.n_tiles = static_cast<int>(ceil_div64(c.n, kPairBN));
   p.k_stages = static_cast<int>(ceil_div64(c.k_bytes, kBK));

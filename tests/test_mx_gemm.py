@@ -261,3 +261,35 @@ def test_fp4_reference_size_grid_sqnr(size):
     _, s_rm = dt.mx_fp4_quantize(a)
     assert torch.equal(as_bytes(a_scale), qo.to_blocked(s_rm.cpu(), m, k // 32))
     dt.check_device_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["mx8", "mx4", "rowwise"])
+@pytest.mark.parametrize("m,n,k", [(4864, 4096, 160),   # 19 x 16 pair tiles: each accumulator used more than twice, 2 stages per tile
+                                   (4700, 4104, 96)])   # the same with ragged last tiles and 16-byte stores
+def test_pair_kernel_alternating_accumulators(m, n, k, mode):
+    # exactly summable inputs, so fp64 on the device gives the same bits
+    from driss_torch_b200 import _cabi
+
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = torch.randint(-3, 4, (m, k), generator=g, device="cuda").float()
+    b = torch.randint(-3, 4, (n, k), generator=g, device="cuda").float()
+    if mode == "rowwise":
+        xs = torch.exp2(torch.randint(-3, 3, (m,), generator=g, device="cuda").float())
+        ws = torch.exp2(torch.randint(-3, 3, (n,), generator=g, device="cuda").float())
+        got = _cabi.rowwise_fp8_bf16(a.to(E4M3), b.to(E4M3), xs, ws, kernel="pair")
+        want = (a.double() @ b.double().t()) * xs[:, None] * ws[None, :]
+    else:
+        sa = torch.randint(125, 130, (m, k // 32), generator=g, device="cuda")
+        sb = torch.randint(125, 130, (n, k // 32), generator=g, device="cuda")
+        sab, sbb = (qo.to_blocked(s.cpu().to(torch.uint8), s.shape[0], k // 32).cuda() for s in (sa, sb))
+        full = [(v.double().view(-1, k // 32, 32) * torch.exp2(s.double() - 127).unsqueeze(2)).view(-1, k) for v, s in ((a, sa), (b, sb))]
+        want = full[0] @ full[1].t()
+        if mode == "mx8":
+            got = _cabi.mx_fp8_bf16(a.to(E4M3), b.to(E4M3), sab, sbb, kernel="pair")
+        else:
+            code = torch.tensor([13, 12, 10, 0, 2, 4, 5], dtype=torch.uint8, device="cuda")  # e2m1 of -3 .. 3
+            pa, pb = (code[(v + 3).long()] for v in (a, b))
+            got = _cabi.mx_fp4_bf16(pa[:, ::2] | (pa[:, 1::2] << 4), pb[:, ::2] | (pb[:, 1::2] << 4), sab, sbb, kernel="pair")
+    assert torch.equal(got.view(torch.int16), want.to(torch.bfloat16).view(torch.int16))
+    assert _cabi.workspace_status(_cabi.workspace(torch.device("cuda", torch.cuda.current_device()))) == 0
