@@ -7,10 +7,10 @@
 // the same source, mx_fp4_bf16 (:243-271) and the row-wise scaled GEMM behind sweep_mm (src/sweep_mm.cu,
 // src/scaled_mm_kernels/f8f8bf16_rowwise_kernel.h:151-175), see Format below.
 //
-// Hand-written for sm_100a.  Three kernels from one source (chosen per call by a measured cost model, see
-// launch_gemm): an SM pair on a 256 x 256 tile (tcgen05.mma.cta_group::2, further down), and one CTA per SM on a
-// 128 x 256 or a 128 x 128 tile (this kernel).  Common to all:
-//   * persistent CTAs of 320 threads walk the output tiles; K advances in stages of 128 bytes;
+// Hand-written for sm_100a.  Four kernels from one source (chosen per call by a measured cost model, see
+// launch_gemm): an SM pair on a 256 x 256 tile (tcgen05.mma.cta_group::2, further down), one CTA per SM on a
+// 128 x 256 or a 128 x 128 tile (this kernel), and for few tiles a cluster that splits K (last).  Common to all:
+//   * persistent CTAs of 320 threads walk the output tiles (the split kernel: 192, one tile); K advances in stages of 128 bytes;
 //   * warp 0 is the producer: per stage tiled TMA loads of the operands (boxes of 128 bytes of K, 128-byte
 //     swizzle, rows and columns past the edges filled with zeros) and of the stage's scale atoms (a 3-D tensor
 //     map over the blocked scale array, an atom past the end arrives as zeros), all counted on the stage's `full`
@@ -881,6 +881,262 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   }
 }
 
+// ---- few output tiles: weights as the M operand, K split over a cluster ------------------------------------
+// A decode step multiplies a handful of token rows with all the weights: bound by reading B once.  The kernels above
+// give it one CTA per 128 or 256 rows of B (64 CTAs for 8192 outputs, less than half of the SMs, 64 stages of K one after
+// the other).  Here
+//   * the roles are swapped: 128 rows of B are the MMA's M operand and the tokens its N operand (32, 64 or 128 wide), so
+//     a stage carries 16 KB of weights and only as many token rows as there are;
+//   * the CTAs of a cluster (1, 2, 4 or 8) take consecutive ranges of the K stages of one tile; two CTAs fit an SM, with
+//     up to 160 KB of weights on their way per SM;
+//   * partial sums (fp32) go to each CTA's own shared memory, and after a cluster barrier every CTA adds up all CTAs'
+//     partials of its share of the tokens through distributed shared memory, in the order of K;
+//   * while the kernel before this one drains, the first stages of weights are already asked into L2: that is where this
+//     GPU's memory is coherent, so it does not matter whether that kernel still writes them.
+// Measured (B200, back to back, weights not in L2; 128 x 128 kernel -> this one; reading the weights alone at the measured
+// copy rate): 8 x 8192 x 8192 MXFP8 27.9 -> 13.6 us (10.3), 16 x 8192 x 4096 row-wise 15.4 -> 8.5 (5.1),
+// 16 x 256 x 8192 16.5 -> 5.0, 300 x 2048 x 8192 19.4 -> 14.3.
+constexpr int kSplitThreads = 192;   // producer warp, MMA warp, 4 warps that empty tensor memory; all six add up and store
+constexpr int kSplitWarps = kSplitThreads / 32;
+constexpr int kMaxSplits = 8;        // portable cluster size
+constexpr int kSplitPrefetch = 8;    // stages of weights asked into L2 ahead of the dependency
+
+template <int BN, int STAGES, int MODE>
+struct __align__(1024) SplitSmem {
+  uint8_t w[STAGES][kBM * kBK];  // 128 rows of weights; with x, reused for the fp32 partial sums [token][128]
+  uint8_t x[STAGES][BN * kBK];   // the tile's tokens
+  uint8_t sfw[STAGES][Format<MODE>::kKAtoms * 512];
+  uint8_t sfx[STAGES][Format<MODE>::kKAtoms * 512];
+  uint64_t full[STAGES];
+  uint64_t empty[STAGES];
+  uint64_t tmem_full;
+  uint32_t tmem_base;
+  int abort;
+};
+
+struct SplitParams {
+  RowwiseEpilogue rowwise;
+  uint16_t *out;  // bf16 [M, N]
+  int M, N;
+  int n_tiles, k_stages, splits;  // 128-column tiles of the output, 128-byte K stages, CTAs per cluster
+  int *status;
+};
+
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap *map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y)
+               : "memory");
+}
+
+template <int BN, int STAGES, int MODE>
+__global__ void __launch_bounds__(kSplitThreads, 2)
+mx_gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                     const __grid_constant__ CUtensorMap map_sfw, const __grid_constant__ CUtensorMap map_sfx, SplitParams p) {
+  using Smem = SplitSmem<BN, STAGES, MODE>;
+  static_assert(BN * kBM * 4 <= STAGES * (kBM + BN) * kBK, "partial sums fit the stage buffers");
+  constexpr int kKAtoms = Format<MODE>::kKAtoms;
+  constexpr uint32_t kSfw = BN, kSfx = BN + 8;             // tensor-memory columns of the scales (4 per atom)
+  constexpr uint32_t kCols = BN == 32 ? 64 : 2 * BN;       // two CTAs' columns fit an SM's 512
+  extern __shared__ unsigned char smem_raw[];
+  Smem &sm = *reinterpret_cast<Smem *>(smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u));
+  const int warp = int(warp_uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
+  const int rank = int(warp_uniform(cluster_ctarank()));
+  volatile int *abort = &sm.abort;
+  const int tile = blockIdx.x / p.splits;
+  const int nt = tile % p.n_tiles, tt = tile / p.n_tiles;
+  const int k0 = int(int64_t(p.k_stages) * rank / p.splits), k1 = int(int64_t(p.k_stages) * (rank + 1) / p.splits);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&sm.full[s], 1);
+      mbar_init(&sm.empty[s], 1);
+    }
+    mbar_init(&sm.tmem_full, 1);
+    sm.abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int ks = k0; ks < k1 && ks < k0 + kSplitPrefetch; ++ks) tma_prefetch_2d(&map_w, ks * kBK, nt * kBM);
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&sm.tmem_base)), "r"(kCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tmem_fence_before();
+  __syncthreads();
+  tmem_fence_after();
+  // only now that this CTA has its tensor memory may a dependent's CTA become resident beside it and take some
+  pdl_launch_dependents();
+  pdl_wait();
+  const uint32_t tmem = warp_uniform(sm.tmem_base);
+
+  if (warp == 0) {
+    // ---- producer ------------------------------------------------------------------------------------------
+    uint32_t stage = 0, phase = 0;
+    bool first_pass = true, ok = true;
+    for (int ks = k0; ks < k1; ++ks) {
+      if (!first_pass && !mbar_wait_warp(&sm.empty[stage], phase ^ 1u, abort)) {
+        ok = false;
+        break;
+      }
+      if (elect_one()) {
+        mbar_expect_tx(&sm.full[stage], kBM * kBK + BN * kBK + (Format<MODE>::kScaled ? 2 * kKAtoms * 512 : 0));
+        tma_load_2d(sm.w[stage], &map_w, ks * kBK, nt * kBM, &sm.full[stage]);
+        tma_load_2d(sm.x[stage], &map_x, ks * kBK, tt * BN, &sm.full[stage]);
+        if constexpr (Format<MODE>::kScaled) {
+          tma_load_3d(sm.sfw[stage], &map_sfw, 0, ks * kKAtoms, nt, &sm.full[stage]);
+          tma_load_3d(sm.sfx[stage], &map_sfx, 0, ks * kKAtoms, tt, &sm.full[stage]);  // tt > 0 only with BN = 128
+        }
+      }
+      __syncwarp();
+      if (++stage == STAGES) {
+        stage = 0;
+        phase ^= 1u;
+        first_pass = false;
+      }
+    }
+    if (!ok && lane == 0) {  // as in the single-CTA kernel: no copies left on their way when the CTA leaves
+      atomicExch(p.status, DTQ_ERR_TIMEOUT);
+      *abort = 1;
+      for (uint32_t j = 0; j < uint32_t(STAGES); ++j) {
+        if (j < stage) mbar_wait(&sm.full[j], phase, nullptr);
+        else if (!first_pass) mbar_wait(&sm.full[j], phase ^ 1u, nullptr);
+      }
+    }
+  } else if (warp == 1) {
+    // ---- MMA issuer ------------------------------------------------------------------------------------------
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int ks = k0; ks < k1; ++ks) {
+      if (!mbar_wait_warp(&sm.full[stage], phase, abort)) {
+        ok = false;
+        break;
+      }
+      tmem_fence_after();
+      if (elect_one()) {
+        if constexpr (Format<MODE>::kScaled) {
+#pragma unroll
+          for (int j = 0; j < kKAtoms; ++j) {
+            copy_scale_atom<false>(tmem + kSfw + 4 * j, smem_addr(sm.sfw[stage] + j * 512));
+            copy_scale_atom<false>(tmem + kSfx + 4 * j, smem_addr(sm.sfx[stage] + j * 512));
+          }
+        }
+        const uint32_t w_addr = smem_addr(sm.w[stage]), x_addr = smem_addr(sm.x[stage]);
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+          const uint32_t accumulate = (ks > k0 || k > 0) ? 1u : 0u;
+          const uint32_t j = Format<MODE>::k_atom(k), id = Format<MODE>::sf_id(k);
+          issue_mma<MODE, false>(tmem, operand_desc(w_addr + k * 32), operand_desc(x_addr + k * 32),
+                                 instr_desc(id, BN, kBM, Format<MODE>::kFormatBits | p.rowwise.operand_format_bits), accumulate,
+                                 (tmem + kSfw + 4 * j) | (id << 30), (tmem + kSfx + 4 * j) | (id << 30));
+        }
+        umma_commit(&sm.empty[stage]);
+      }
+      __syncwarp();
+      if (++stage == STAGES) {
+        stage = 0;
+        phase ^= 1u;
+      }
+    }
+    if (ok && elect_one()) umma_commit(&sm.tmem_full);
+    __syncwarp();
+    if (!ok && lane == 0) {
+      atomicExch(p.status, DTQ_ERR_TIMEOUT);
+      *abort = 1;
+    }
+  }
+
+  // ---- partial sums: tensor memory -> this CTA's shared memory [token][128 outputs] -------------------------
+  float *partial = reinterpret_cast<float *>(sm.w);
+  const int live = min(BN, p.M - tt * BN);  // tokens of this tile
+  const int64_t n0 = int64_t(nt) * kBM + lane * 4;  // this lane's four outputs in the sum below; N % 8 == 0
+  const bool n_live = n0 < p.N;
+  float4 cs = make_float4(0.0f, 0.0f, 0.0f, 0.0f), bs = cs;
+  if constexpr (MODE == kRowwise) {
+    if (n_live) {  // fetched before the wait below
+      const float *c = p.rowwise.col_scale + n0;
+      cs = make_float4(__ldg(c), __ldg(c + 1), __ldg(c + 2), __ldg(c + 3));
+      if (p.rowwise.bias) {
+        if (p.rowwise.bias_is_bf16) {
+          const uint16_t *b = static_cast<const uint16_t *>(p.rowwise.bias) + n0;
+          bs = make_float4(bf16_lo(__ldg(b)), bf16_lo(__ldg(b + 1)), bf16_lo(__ldg(b + 2)), bf16_lo(__ldg(b + 3)));
+        } else {
+          const float *b = static_cast<const float *>(p.rowwise.bias) + n0;
+          bs = make_float4(__ldg(b), __ldg(b + 1), __ldg(b + 2), __ldg(b + 3));
+        }
+      }
+    }
+  }
+  if (warp >= 2) {
+    const int quad = warp & 3;  // the quarter of tensor memory that this warp can read
+    // the barrier completes when all MMAs have, so nothing reads the stage buffers any more
+    if (!mbar_wait(&sm.tmem_full, 0u, abort)) {
+      if (lane == 0) {
+        atomicExch(p.status, DTQ_ERR_TIMEOUT);
+        *abort = 1;
+      }
+    } else {
+      tmem_fence_after();
+#pragma unroll
+      for (int c = 0; c < BN / 32; ++c) {
+        if (c * 32 < live) {
+          uint32_t v[32];
+          tmem_load_32(v, tmem + (uint32_t(quad * 32) << 16) + uint32_t(c * 32));
+          tmem_load_wait(v);
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (c * 32 + i < live) partial[(c * 32 + i) * kBM + quad * 32 + lane] = __uint_as_float(v[i]);
+        }
+      }
+      tmem_fence_before();
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();
+
+  // ---- sum over the cluster: token t by CTA t % splits, a warp per token, four outputs per lane --------------
+  if (!*abort) {
+    for (int t = rank + p.splits * warp; t < live; t += p.splits * kSplitWarps) {
+      const uint32_t mine = smem_addr(partial + t * kBM + lane * 4);
+      float4 part[kMaxSplits];
+#pragma unroll
+      for (int j = 0; j < kMaxSplits; ++j)
+        if (j < p.splits) part[j] = ld_cluster_f4(map_to_cta(mine, j));
+      float4 f = part[0];
+#pragma unroll
+      for (int j = 1; j < kMaxSplits; ++j)
+        if (j < p.splits) f = make_float4(f.x + part[j].x, f.y + part[j].y, f.z + part[j].z, f.w + part[j].w);
+      const int64_t row = int64_t(tt) * BN + t;
+      if constexpr (MODE == kRowwise) {  // the same steps as apply_rowwise
+        const float xs = __ldg(p.rowwise.row_scale + row);
+        f = make_float4(__fmul_rn(__fmul_rn(f.x, xs), cs.x), __fmul_rn(__fmul_rn(f.y, xs), cs.y), __fmul_rn(__fmul_rn(f.z, xs), cs.z),
+                        __fmul_rn(__fmul_rn(f.w, xs), cs.w));
+        if (p.rowwise.bias)
+          f = make_float4(__fadd_rn(f.x, bs.x), __fadd_rn(f.y, bs.y), __fadd_rn(f.z, bs.z), __fadd_rn(f.w, bs.w));
+      }
+      if (n_live)
+        stg_stream(p.out + row * p.N + n0,
+                   make_uint2(pack_bf16(__float_as_uint(f.x), __float_as_uint(f.y)), pack_bf16(__float_as_uint(f.z), __float_as_uint(f.w))));
+    }
+  }
+  __syncwarp();
+  if (warp == 1 && *abort && elect_one()) {  // MMAs may still be in flight: wait (bounded) for them, as in the single-CTA kernel
+    mbar_init(&sm.tmem_full, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    umma_commit(&sm.tmem_full);
+    mbar_wait(&sm.tmem_full, 0u, nullptr);
+  }
+  __syncwarp();
+  cluster_sync_all();  // nobody leaves while another CTA may still read its partial sums
+  if (warp == 1) {
+    tmem_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
+  }
+}
+
 // ---- host side --------------------------------------------------------------------------------------------
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -934,15 +1190,16 @@ int make_scale_map(CUtensorMap *map, const void *base, int64_t atom_rows, int64_
 
 constexpr int kMaxGemmDevices = 64;
 
-// Clusters of two, launched as a programmatic dependent of what is before it on the stream (attr: room for two).
-void cluster_launch_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, int grid, size_t smem, cudaStream_t st) {
+// Clusters of `cluster` CTAs, launched as a programmatic dependent of what is before it on the stream (attr: room for two).
+void cluster_launch_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, int grid, int threads, int cluster, size_t smem,
+                           cudaStream_t st) {
   *cfg = cudaLaunchConfig_t{};
   cfg->gridDim = dim3(grid);
-  cfg->blockDim = dim3(kGemmThreads);
+  cfg->blockDim = dim3(threads);
   cfg->dynamicSmemBytes = smem;
   cfg->stream = st;
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.x = cluster;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -967,7 +1224,7 @@ int pair_cluster_capacity(int dev_id, int *max_clusters) {
       if (cudaFuncSetAttribute(mx_gemm_pair_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess) {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[2];
-        cluster_launch_config(&cfg, attr, 2, smem, nullptr);
+        cluster_launch_config(&cfg, attr, 2, kGemmThreads, 2, smem, nullptr);
         cfg.numAttrs = 1;  // the occupancy query wants the cluster shape only
         if (cudaOccupancyMaxActiveClusters(&n, mx_gemm_pair_kernel<MODE>, &cfg) != cudaSuccess) n = 0;
       }
@@ -1017,7 +1274,7 @@ int launch_pair(const GemmCall &c, int max_clusters) {
   const int clusters = static_cast<int>(tiles < max_clusters ? tiles : max_clusters);
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
-  cluster_launch_config(&cfg, attr, 2 * clusters, sizeof(PairSmem<MODE>) + 1024, c.st);
+  cluster_launch_config(&cfg, attr, 2 * clusters, kGemmThreads, 2, sizeof(PairSmem<MODE>) + 1024, c.st);
   return cuda_status(cudaLaunchKernelEx(&cfg, mx_gemm_pair_kernel<MODE>, map_a, map_b, map_sfa, map_sfb, p));
 }
 
@@ -1059,6 +1316,57 @@ int launch_shape(const GemmCall &c, const DeviceInfo &dev) {
                                              map_b, map_sfa, map_sfb, p));
 }
 
+// Token rows per tile of the split kernel.
+int split_tokens(int64_t m) { return m <= 32 ? 32 : (m <= 64 ? 64 : 128); }
+
+// CTAs per tile of the split kernel: as many (1, 2, 4, 8) as fill the device's two CTAs per SM, with at least eight K
+// stages each.
+int split_count(int64_t tiles, int64_t stages, const DeviceInfo &dev) {
+  int splits = 1;
+  while (splits < kMaxSplits && tiles * splits * 2 <= 2 * dev.sm_count && stages >= 16 * splits) splits *= 2;
+  return splits;
+}
+
+template <int BN, int STAGES, int MODE>
+int launch_split(const GemmCall &c, const DeviceInfo &dev) {
+  static std::atomic<int> configured[kMaxGemmDevices];
+  int dev_id = 0;
+  DTQ_CUDA_TRY(cudaGetDevice(&dev_id));
+  if (dev_id < 0 || dev_id >= kMaxGemmDevices) return DTQ_ERR_INVALID_ARGUMENT;
+  const int smem = static_cast<int>(sizeof(SplitSmem<BN, STAGES, MODE>)) + 1024;
+  if (!configured[dev_id].load(std::memory_order_acquire)) {  // setting the attribute twice is harmless
+    DTQ_CUDA_TRY(cudaFuncSetAttribute(mx_gemm_split_kernel<BN, STAGES, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    configured[dev_id].store(1, std::memory_order_release);
+  }
+  CUtensorMap map_w, map_x, map_sfw, map_sfx;
+  if (int e = make_operand_map(&map_w, c.b, c.n, c.k_bytes, kBM)) return e;
+  if (int e = make_operand_map(&map_x, c.a, c.m, c.k_bytes, BN)) return e;
+  if constexpr (Format<MODE>::kScaled) {
+    if (int e = make_scale_map(&map_sfw, c.sfb, ceil_div64(c.n, 128), c.katoms, 1, Format<MODE>::kKAtoms)) return e;
+    if (int e = make_scale_map(&map_sfx, c.sfa, ceil_div64(c.m, 128), c.katoms, 1, Format<MODE>::kKAtoms)) return e;
+  } else {  // never dereferenced by the kernel
+    map_sfw = map_w;
+    map_sfx = map_w;
+  }
+  SplitParams p;
+  p.rowwise = c.rowwise;
+  p.rowwise.operand_format_bits = c.rowwise.operand_format_bits << 3;  // the caller's A is the MMA's B here, and its B is e4m3 (0)
+  p.out = static_cast<uint16_t *>(c.out);
+  p.M = static_cast<int>(c.m);
+  p.N = static_cast<int>(c.n);
+  p.n_tiles = static_cast<int>(ceil_div64(c.n, kBM));
+  p.k_stages = static_cast<int>(ceil_div64(c.k_bytes, kBK));
+  p.status = c.status;
+  const int64_t tiles = int64_t(p.n_tiles) * ceil_div64(c.m, BN);
+  p.splits = split_count(tiles, p.k_stages, dev);
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[2];
+  cluster_launch_config(&cfg, attr, static_cast<int>(tiles * p.splits), kSplitThreads, p.splits, smem, c.st);
+  return cuda_status(cudaLaunchKernelEx(&cfg, mx_gemm_split_kernel<BN, STAGES, MODE>, map_w, map_x, map_sfw, map_sfx, p));
+}
+
+constexpr int kGemmSplit = DTQ_GEMM_NARROW + 1;  // only launch_gemm itself chooses it
+
 template <int MODE>
 int launch_gemm(const GemmCall &c, int kernel, const DeviceInfo &dev) {
   // Which kernel: estimated time = a fixed part (launch, set-up, filling the pipeline, the last epilogue) plus
@@ -1079,8 +1387,24 @@ int launch_gemm(const GemmCall &c, int kernel, const DeviceInfo &dev) {
           ? 10.0 + static_cast<double>(ceil_div64(ceil_div64(c.m, 256) * ceil_div64(c.n, 256), max_clusters)) * stages * 0.36
           : 1e30;
   if (kernel == DTQ_GEMM_PAIR && max_clusters <= 0) return DTQ_ERR_CUDA_BASE + static_cast<int>(cudaErrorNotSupported);
+  // Few tiles and a long K: the split kernel, once it gets four CTAs per tile, or two where a tile is only 32 tokens wide.
+  // Measured split against the best of the others, us: four CTAs, row-wise 64 x 8192 x 4096 9.9 / 12.1, 128 x 4096 x 4096
+  // 10.3 / 12.4, 300 x 2048 x 8192 14.3 / 19.4, MXFP4 512 x 1024 x 8192 10.3 / 12.0; two CTAs, 16 x 16384 x 8192 24.0 / 27.0,
+  // MXFP4 16 x 8192 x 4096 6.7 / 9.2, but 512 x 4096 x 4096 14.3 / 13.4 and MXFP4 64 x 8192 x 4096 8.1 / 8.0; one CTA,
+  // 32 x 1024 x 1024 6.1 / 4.9.
+  if (kernel == DTQ_GEMM_AUTO) {
+    const int64_t tiles = ceil_div64(c.n, 128) * ceil_div64(c.m, split_tokens(c.m));
+    if (split_count(tiles, ceil_div64(c.k_bytes, kBK), dev) >= (c.m <= 32 ? 2 : 4)) kernel = kGemmSplit;
+  }
   if (kernel == DTQ_GEMM_AUTO)
     kernel = (pair <= wide && pair <= narrow) ? DTQ_GEMM_PAIR : (narrow < wide ? DTQ_GEMM_NARROW : DTQ_GEMM_WIDE);
+  if (kernel == kGemmSplit) {
+    switch (split_tokens(c.m)) {
+      case 32: return launch_split<32, 5, MODE>(c, dev);
+      case 64: return launch_split<64, 4, MODE>(c, dev);
+      default: return launch_split<128, 3, MODE>(c, dev);
+    }
+  }
   if (kernel == DTQ_GEMM_PAIR) return launch_pair<MODE>(c, max_clusters);
   if (kernel == DTQ_GEMM_NARROW) return launch_shape<NarrowShape, MODE>(c, dev);
   return launch_shape<WideShape, MODE>(c, dev);

@@ -354,12 +354,14 @@ int dtq_mx_fp4_bf16(const void *a, const void *b, const void *a_scales_blocked, 
 
 /*
  * Both GEMMs with the element format (DTQ_E4M3 or DTQ_E2M1) and the kernel named instead of chosen from the
- * problem size (for benchmarks, and for tests that run every kernel on every size; the results of the kernels are
- * bit-identical):
+ * problem size (for benchmarks, and for tests that run every kernel on every size; the results of the named kernels
+ * are bit-identical):
  *   DTQ_GEMM_PAIR    two CTAs of a cluster (an SM pair) per 256 x 256 tile, tcgen05.mma.cta_group::2: least
  *                    operand traffic per SM, what large problems use;
  *   DTQ_GEMM_WIDE    one CTA per 128 x 256 tile;
- *   DTQ_GEMM_NARROW  one CTA per 128 x 128 tile, two accumulators (epilogue under the next tile's MMAs).
+ *   DTQ_GEMM_NARROW  one CTA per 128 x 128 tile, two accumulators (epilogue under the next tile's MMAs);
+ *   DTQ_GEMM_AUTO    one of these, or for few output tiles and operand rows of at least 2 KB a cluster per tile whose CTAs
+ *                    take a part of K each (fp32 partial sums added in the order of K, so the last bit may differ).
  * No reference counterpart (the reference fixes one CUTLASS tile shape, src/mx_fp8_bf16.cu:231-233).
  */
 #define DTQ_GEMM_AUTO 0

@@ -263,12 +263,8 @@ def test_fp4_reference_size_grid_sqnr(size):
     dt.check_device_status()
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("mode", ["mx8", "mx4", "rowwise"])
-@pytest.mark.parametrize("m,n,k", [(4864, 4096, 160),   # 19 x 16 pair tiles: each accumulator used more than twice, 2 stages per tile
-                                   (4700, 4104, 96)])   # the same with ragged last tiles and 16-byte stores
-def test_pair_kernel_alternating_accumulators(m, n, k, mode):
-    # exactly summable inputs, so fp64 on the device gives the same bits
+def _check_exact_on_device(mode, m, n, k, kernel, a_dtype=E4M3, bias=None):
+    # exactly summable inputs, so that fp64 on the device gives the same bits whatever the order of the sums
     from driss_torch_b200 import _cabi
 
     g = torch.Generator(device="cuda").manual_seed(m + n + k)
@@ -277,8 +273,9 @@ def test_pair_kernel_alternating_accumulators(m, n, k, mode):
     if mode == "rowwise":
         xs = torch.exp2(torch.randint(-3, 3, (m,), generator=g, device="cuda").float())
         ws = torch.exp2(torch.randint(-3, 3, (n,), generator=g, device="cuda").float())
-        got = _cabi.rowwise_fp8_bf16(a.to(E4M3), b.to(E4M3), xs, ws, kernel="pair")
-        want = (a.double() @ b.double().t()) * xs[:, None] * ws[None, :]
+        bias_d = None if bias is None else (torch.randint(-8, 9, (n,), generator=g, device="cuda") * 0.5).to(bias)
+        got = _cabi.rowwise_fp8_bf16(a.to(a_dtype), b.to(E4M3), xs, ws, bias=bias_d, kernel=kernel)
+        want = (a.double() @ b.double().t()) * xs[:, None] * ws[None, :] + (0.0 if bias is None else bias_d.double())
     else:
         sa = torch.randint(125, 130, (m, k // 32), generator=g, device="cuda")
         sb = torch.randint(125, 130, (n, k // 32), generator=g, device="cuda")
@@ -286,10 +283,32 @@ def test_pair_kernel_alternating_accumulators(m, n, k, mode):
         full = [(v.double().view(-1, k // 32, 32) * torch.exp2(s.double() - 127).unsqueeze(2)).view(-1, k) for v, s in ((a, sa), (b, sb))]
         want = full[0] @ full[1].t()
         if mode == "mx8":
-            got = _cabi.mx_fp8_bf16(a.to(E4M3), b.to(E4M3), sab, sbb, kernel="pair")
+            got = _cabi.mx_fp8_bf16(a.to(E4M3), b.to(E4M3), sab, sbb, kernel=kernel)
         else:
             code = torch.tensor([13, 12, 10, 0, 2, 4, 5], dtype=torch.uint8, device="cuda")  # e2m1 of -3 .. 3
             pa, pb = (code[(v + 3).long()] for v in (a, b))
-            got = _cabi.mx_fp4_bf16(pa[:, ::2] | (pa[:, 1::2] << 4), pb[:, ::2] | (pb[:, 1::2] << 4), sab, sbb, kernel="pair")
+            got = _cabi.mx_fp4_bf16(pa[:, ::2] | (pa[:, 1::2] << 4), pb[:, ::2] | (pb[:, 1::2] << 4), sab, sbb, kernel=kernel)
     assert torch.equal(got.view(torch.int16), want.to(torch.bfloat16).view(torch.int16))
     assert _cabi.workspace_status(_cabi.workspace(torch.device("cuda", torch.cuda.current_device()))) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["mx8", "mx4", "rowwise"])
+@pytest.mark.parametrize("m,n,k", [(4864, 4096, 160),   # 19 x 16 pair tiles: each accumulator used more than twice, 2 stages per tile
+                                   (4700, 4104, 96)])   # the same with ragged last tiles and 16-byte stores
+def test_pair_kernel_alternating_accumulators(m, n, k, mode):
+    _check_exact_on_device(mode, m, n, k, "pair")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["mx8", "mx4", "rowwise"])
+@pytest.mark.parametrize("tokens,n,kb", [(1, 8, 2048), (32, 136, 2064), (31, 9600, 4080),              # 32-token tiles, 2 CTAs per tile
+                                         (33, 264, 4096), (64, 1000, 8192), (65, 520, 4208),           # 64 and 128 tokens, 4 to 8 CTAs
+                                         (128, 4096, 8176), (129, 136, 8192), (300, 2056, 4096),       # several token tiles
+                                         (16, 8192, 16384), (33, 264, 2048), (8, 19200, 4096)])        # the last two just outside the rule
+def test_few_tiles_split_along_k(tokens, n, kb, mode):
+    # `kb` bytes per operand row; K stages that do not divide evenly, a last stage that is partly past the end
+    if mode != "rowwise":
+        kb = kb // 32 * 32
+    _check_exact_on_device(mode, tokens, n, kb * 2 if mode == "mx4" else kb, "auto",
+                           a_dtype=torch.float8_e5m2 if tokens % 2 else E4M3, bias=[None, torch.float32, torch.bfloat16][tokens % 3])
