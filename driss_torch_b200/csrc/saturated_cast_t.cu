@@ -12,14 +12,19 @@
 // double precision, src/dynamic_scaled_quant.cu:111-117), bit for bit.  The casts are elementwise,
 // so out_t is the transpose of out: every element is converted ONCE.
 //
-// Fast path (rows % 16 == 0, 16-byte rows of input, aligned pointers): a CTA owns a tile of 128
+// Fast path (16-byte rows of input; rows % 16 == 0 and aligned outputs): a CTA owns a tile of 128
 // rows x 256 input bytes (128 bf16 or 64 fp32 columns).  Rows enter with 16-byte loads (a full
 // 256-byte segment per row); each lane casts its chunk, stores the bytes to `out` if wanted, and
 // parks them in shared memory (128 x 128 bytes; 4-word groups XOR-swizzled by the 16-row group, so
 // both phases are free of bank conflicts).  Then a lane takes a word column (four byte columns) of
 // 16 rows, transposes its 4 x 4 byte blocks with byte permutes, and stores 16 contiguous bytes to
 // each of four rows of out_t; the eight lanes of a word column cover full 128-byte lines.
-// Any other shape or alignment: a 32 x 32 byte-tile kernel, one element per thread.
+// Any other number of rows (or alignment of out_t): the rows of out_t start at every byte offset, so no 16-byte store
+// fits.  The transposed tile goes through shared memory once more, and a warp writes one row segment of out_t (up to 128
+// bytes) at a time: each lane one aligned 4-byte word, cut out of two words of shared memory by a funnel shift, and up to
+// six single bytes for the ends.  That costs a quarter more than aligned rows, by the issue of those
+// stores (16 row segments per warp); launch_transposed has the figures.
+// Rows of input that are not 16-byte aligned: a 32 x 32 byte-tile kernel, one element per thread.
 #include "dtq_device.cuh"
 #include "dtq_host.h"
 
@@ -110,7 +115,8 @@ struct DynCast<DTQ_F32, OUT> {
 };
 
 // FULL: the tile lies inside the matrix, no access is predicated.  BOTH: also write the row-major output.
-template <typename C, bool BOTH, bool FULL>
+// RAGGED: rows of out_t start at any byte.
+template <typename C, bool BOTH, bool RAGGED, bool FULL>
 __device__ __forceinline__ void transposed_tile(uint32_t (&tile)[kTileRows][kTileWords], const uint4 *__restrict__ in,
                                                 uint8_t *__restrict__ out, uint8_t *__restrict__ out_t,
                                                 const typename C::Scale &s, int64_t rows, int64_t cols,
@@ -146,7 +152,7 @@ __device__ __forceinline__ void transposed_tile(uint32_t (&tile)[kTileRows][kTil
   // ---- columns: lane = 8 * q + g: 16-row group g of the tile, word column 4 * warp + q (four byte columns)
   const int g = lane & 7, q = lane >> 3;
   const int word = warp * 4 + q;
-  if (word >= kRowWords) return;  // fp32 input: half as many byte columns per tile
+  if (!RAGGED && word >= kRowWords) return;  // fp32 input: half as many byte columns per tile
   const int64_t r_first = row0 + g * 16;
   const int64_t col = col0 + word * 4;
   uint32_t w[16];
@@ -163,6 +169,32 @@ __device__ __forceinline__ void transposed_tile(uint32_t (&tile)[kTileRows][kTil
     t[2][k] = __byte_perm(a1, b1, 0x5410);
     t[3][k] = __byte_perm(a1, b1, 0x7632);
   }
+  if constexpr (RAGGED) {
+    // the tile again, now as [byte column][row]: 32 words of rows per column
+    uint32_t *tile_t = &tile[0][0];
+    __syncthreads();
+    if (word < kRowWords) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<uint4 *>(tile_t + (word * 4 + j) * kTileWords + g * 4) = make_uint4(t[j][0], t[j][1], t[j][2], t[j][3]);
+    }
+    __syncthreads();
+    const int len = FULL ? kTileRows : static_cast<int>(min(rows - row0, int64_t(kTileRows)));
+    const int ncols = FULL ? 4 * kRowWords : static_cast<int>(min(cols - col0, int64_t(4 * kRowWords)));
+    for (int cc = warp; cc < ncols; cc += kThreadsT / 32) {
+      uint8_t *dst = out_t + (col0 + cc) * rows + row0;
+      const uint32_t *src = tile_t + cc * kTileWords;
+      const int head = min(static_cast<int>(-reinterpret_cast<uintptr_t>(dst) & 3), len);  // bytes before the first aligned word
+      const int words = (len - head) >> 2, tail = (len - head) & 3;
+      if (lane < words)
+        *reinterpret_cast<uint32_t *>(dst + head + 4 * lane) = __funnelshift_r(src[lane], src[(lane + 1) & 31], 8 * head);
+      if (lane < head + tail) {
+        const int i = lane < head ? lane : len - tail + lane - head;
+        dst[i] = reinterpret_cast<const uint8_t *>(src)[i];
+      }
+    }
+    return;
+  }
   // rows % 16 == 0: a 16-row group is inside or outside as a whole; cols % 4 == 0 likewise for a word column
   if (FULL || (r_first < rows && col < cols)) {
     uint8_t *dst = out_t + col * rows + r_first;
@@ -174,7 +206,7 @@ __device__ __forceinline__ void transposed_tile(uint32_t (&tile)[kTileRows][kTil
 // `scale` points to the scale (Cast) or to the amax (DynCast); scale_out, if given, receives the fp32 scale
 // a DynCast derived from the amax, amax_out the amax it used (the given one, clamped at zero).
 constexpr int kTransposedMinBlocks = 4;
-template <typename C, bool BOTH>
+template <typename C, bool BOTH, bool RAGGED>
 __global__ void __launch_bounds__(kThreadsT, kTransposedMinBlocks)
 cast_transposed_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, uint8_t *__restrict__ out_t,
                        const float *__restrict__ scale, float *__restrict__ scale_out, float *__restrict__ amax_out,
@@ -193,9 +225,9 @@ cast_transposed_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, 
   const int64_t row0 = (t / col_tiles) * kTileRows;
   const int64_t col0 = (t % col_tiles) * kTileCols;
   if (row0 + kTileRows <= rows && col0 + kTileCols <= cols)
-    transposed_tile<C, BOTH, true>(tile, in, out, out_t, s, rows, cols, row0, col0);
+    transposed_tile<C, BOTH, RAGGED, true>(tile, in, out, out_t, s, rows, cols, row0, col0);
   else
-    transposed_tile<C, BOTH, false>(tile, in, out, out_t, s, rows, cols, row0, col0);
+    transposed_tile<C, BOTH, RAGGED, false>(tile, in, out, out_t, s, rows, cols, row0, col0);
 }
 
 // Any shape and alignment: 32 x 32 tiles of fp8 bytes, block (32, 8), one element per thread per step.
@@ -235,12 +267,17 @@ template <typename C, bool BOTH>
 int launch_transposed(const void *in, void *out, void *out_t, const float *scale, float *scale_out, float *amax_out,
                       int64_t rows, int64_t cols, cudaStream_t st) {
   constexpr int kTileCols = 16 * C::kChunkElems;
-  const bool fast = rows % 16 == 0 && cols % C::kChunkElems == 0 && aligned_to(in, 16) && aligned_to(out_t, 16) &&
-                    (!BOTH || aligned_to(out, 8));
-  if (fast) {
+  // Tiles wherever the input's rows can be read 16 bytes at a time; 16-byte stores of the transposed output where all its
+  // rows start on 16 bytes, else the byte-shifted ones.  Measured, both orientations from bf16: 5003 x 4096 39.1 us with the
+  // byte-tile kernel, 15.7 us (5.2 TB/s) with shifted rows; 16383 x 8192 112 us with shifted rows, 16384 x 8192 with
+  // aligned ones 88 us.
+  const bool tiles = cols % C::kChunkElems == 0 && aligned_to(in, 16) && (!BOTH || aligned_to(out, 8));
+  const bool aligned_rows = rows % 16 == 0 && aligned_to(out_t, 16);
+  auto kernel = aligned_rows ? cast_transposed_kernel<C, BOTH, false> : cast_transposed_kernel<C, BOTH, true>;
+  if (tiles) {
     const int64_t row_tiles = ceil_div64(rows, kTileRows), col_tiles = ceil_div64(cols, kTileCols);
     if (row_tiles > 0x7FFFFFFFLL / col_tiles) return DTQ_ERR_TOO_LARGE;
-    return cuda_status(launch_after_dependency(cast_transposed_kernel<C, BOTH>, dim3(static_cast<unsigned>(row_tiles * col_tiles)),
+    return cuda_status(launch_after_dependency(kernel, dim3(static_cast<unsigned>(row_tiles * col_tiles)),
                                                dim3(kThreadsT), 0, st, static_cast<const uint4 *>(in),
                                                static_cast<uint8_t *>(out), static_cast<uint8_t *>(out_t), scale, scale_out,
                                                amax_out, rows, cols, col_tiles));

@@ -231,3 +231,25 @@ def test_transposed_on_every_bf16_pattern():
             out, out_t = dt.saturated_cast_dual(bits.cuda(), scale.cuda(), fp8_dtype)
             assert_fp8_equal(out, want, fp8_dtype, "row-major")
             assert_fp8_equal(out_t, want.t().contiguous(), fp8_dtype, "transposed")
+
+
+@pytest.mark.parametrize("rows", [1, 3, 31, 127, 128, 129, 272, 1003])  # remainders of the 128-row tile and of a 16-byte row
+@pytest.mark.parametrize("cols", [8, 72, 136, 1000])                    # multiples of a 16-byte chunk, not of the tile
+@pytest.mark.parametrize("in_dtype", IN_DTYPES)
+@pytest.mark.parametrize("offset", [0, 5])                              # byte offset of the transposed output
+def test_transposed_rows_at_any_byte(rows, cols, in_dtype, offset):
+    from driss_torch_b200 import _cabi
+
+    fp8_dtype = FP8_DTYPES[rows % 2]
+    a = _input(rows, cols, in_dtype, seed=rows * 31 + cols)
+    scale = workloads.tensor_scale(a, fp8_dtype)
+    want = qo.saturated_cast(a, scale.item(), fp8_dtype)
+    for both in (False, True):
+        room = torch.full((rows * cols + 64,), 0x55, dtype=torch.uint8, device="cuda")
+        out_t = room[16 + offset:16 + offset + rows * cols].view(fp8_dtype).view(cols, rows)
+        got = _cabi.saturated_cast_transposed(a.cuda(), scale.cuda(), fp8_dtype, out_t=out_t, both=both)
+        assert_fp8_equal(out_t, want.t().contiguous(), fp8_dtype, "transposed")
+        if both:
+            assert_fp8_equal(got[0], want, fp8_dtype, "row-major")
+        edge = torch.cat([room[:16 + offset], room[16 + offset + rows * cols:]])
+        assert (edge == 0x55).all(), "bytes outside the output were written"
