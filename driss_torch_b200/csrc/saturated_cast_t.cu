@@ -24,7 +24,7 @@
 // bytes) at a time: each lane one aligned 4-byte word, cut out of two words of shared memory by a funnel shift, and up to
 // six single bytes for the ends.  That costs a quarter more than aligned rows, by the issue of those
 // stores (16 row segments per warp); launch_transposed has the figures.
-// Rows of input that are not 16-byte aligned: a 32 x 32 byte-tile kernel, one element per thread.
+// Rows of input that are not 16-byte aligned, or few tiles of ragged rows: a 32 x 32 byte-tile kernel, one element per thread.
 #include "dtq_device.cuh"
 #include "dtq_host.h"
 
@@ -267,12 +267,16 @@ template <typename C, bool BOTH>
 int launch_transposed(const void *in, void *out, void *out_t, const float *scale, float *scale_out, float *amax_out,
                       int64_t rows, int64_t cols, cudaStream_t st) {
   constexpr int kTileCols = 16 * C::kChunkElems;
-  // Tiles wherever the input's rows can be read 16 bytes at a time; 16-byte stores of the transposed output where all its
-  // rows start on 16 bytes, else the byte-shifted ones.  Measured, both orientations from bf16: 5003 x 4096 39.1 us with the
-  // byte-tile kernel, 15.7 us (5.2 TB/s) with shifted rows; 16383 x 8192 112 us with shifted rows, 16384 x 8192 with
-  // aligned ones 88 us.
-  const bool tiles = cols % C::kChunkElems == 0 && aligned_to(in, 16) && (!BOTH || aligned_to(out, 8));
+  // Tiles where the input's rows can be read 16 bytes at a time; 16-byte stores of the transposed output where all its
+  // rows start on 16 bytes, else the byte-shifted ones, unless there are fewer tiles than SMs: then the smaller tiles of
+  // the byte kernel are quicker.  Measured, both orientations from bf16, byte tiles / shifted rows: 33 x 256 (2 tiles)
+  // 1.7 / 3.2 us, 333 x 1000 (24) 2.9 / 4.1, 40 x 8192 (64) 3.0 / 3.4, 1001 x 4096 (256) 8.8 / 7.3, 5003 x 4096
+  // (1280) 37.0 / 15.7, 16383 x 8192 232 / 112; 16384 x 8192 with aligned rows 88.
+  const bool readable = cols % C::kChunkElems == 0 && aligned_to(in, 16) && (!BOTH || aligned_to(out, 8));
   const bool aligned_rows = rows % 16 == 0 && aligned_to(out_t, 16);
+  DeviceInfo dev;
+  if (int e = current_device_info(&dev)) return e;
+  const bool tiles = readable && (aligned_rows || ceil_div64(rows, kTileRows) * ceil_div64(cols, kTileCols) >= dev.sm_count);
   auto kernel = aligned_rows ? cast_transposed_kernel<C, BOTH, false> : cast_transposed_kernel<C, BOTH, true>;
   if (tiles) {
     const int64_t row_tiles = ceil_div64(rows, kTileRows), col_tiles = ceil_div64(cols, kTileCols);

@@ -233,8 +233,9 @@ def test_transposed_on_every_bf16_pattern():
             assert_fp8_equal(out_t, want.t().contiguous(), fp8_dtype, "transposed")
 
 
-@pytest.mark.parametrize("rows", [1, 3, 31, 127, 128, 129, 272, 1003])  # remainders of the 128-row tile and of a 16-byte row
-@pytest.mark.parametrize("cols", [8, 72, 136, 1000])                    # multiples of a 16-byte chunk, not of the tile
+@pytest.mark.parametrize("rows,cols", [(1, 19080), (3, 19080), (127, 19080), (128, 19080), (129, 9592), (1003, 2504), (2500, 1000),
+                                       (19001, 72),                    # enough tiles: remainders of the tile both ways
+                                       (1, 8), (31, 72), (333, 1000)])  # the byte-tile kernel
 @pytest.mark.parametrize("in_dtype", IN_DTYPES)
 @pytest.mark.parametrize("offset", [0, 5])                              # byte offset of the transposed output
 def test_transposed_rows_at_any_byte(rows, cols, in_dtype, offset):
