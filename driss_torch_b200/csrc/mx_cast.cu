@@ -30,13 +30,19 @@ constexpr int kUnroll = 4;  // tied to the scale-byte mapping below: lane&3 pick
 template <bool BLOCKED>
 __global__ void __launch_bounds__(kThreads, 2048 / kThreads)
 mx_stream_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, uint8_t *__restrict__ scales,
-                 int64_t nchunks, int64_t kblocks, int64_t katoms) {
+                 int64_t nchunks, int64_t kblocks, int64_t katoms, int64_t rows, unsigned pad_blocks) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int64_t kTile = int64_t(kThreads) * kUnroll;
   // may have become resident under the tail of the kernel before it on the stream: wait for that kernel
   pdl_launch_dependents();
   pdl_wait();
-  for (int64_t tile = blockIdx.x; tile * kTile < nchunks; tile += gridDim.x) {
+  if constexpr (BLOCKED) {  // the first blocks of the grid write the padding, if there is any
+    if (blockIdx.x < pad_blocks) {
+      zero_scale_padding(scales, rows, kblocks, int64_t(blockIdx.x) * kThreads + threadIdx.x, int64_t(pad_blocks) * kThreads);
+      return;
+    }
+  }
+  for (int64_t tile = blockIdx.x - (BLOCKED ? pad_blocks : 0); tile * kTile < nchunks; tile += gridDim.x) {
     const int64_t warp_first = tile * kTile + int64_t(warp) * (32 * kUnroll);
     uint4 v[kUnroll];
 #pragma unroll
@@ -66,7 +72,9 @@ mx_stream_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, ui
 template <bool BLOCKED>
 __global__ void __launch_bounds__(kThreads)
 mx_scalar_kernel(const uint16_t *__restrict__ in, uint8_t *__restrict__ payload, uint8_t *__restrict__ scales,
-                 int64_t nblocks, int64_t kblocks, int64_t katoms) {
+                 int64_t nblocks, int64_t kblocks, int64_t katoms, int64_t rows) {
+  if constexpr (BLOCKED)
+    zero_scale_padding(scales, rows, kblocks, int64_t(blockIdx.x) * kThreads + threadIdx.x, int64_t(gridDim.x) * kThreads);
   for (int64_t b = int64_t(blockIdx.x) * kThreads + threadIdx.x; b < nblocks; b += int64_t(gridDim.x) * kThreads) {
     const uint16_t *x = in + b * 32;
     uint32_t mag = 0;
@@ -99,16 +107,18 @@ int launch_mx(const void *in_bf16, void *payload, void *scales_e8m0, int64_t row
   if (aligned_to(in_bf16, 16) && aligned_to(payload, 8)) {
     const int64_t nchunks = numel / 8;
     const int64_t tiles = ceil_div64(nchunks, int64_t(kThreads) * kUnroll);
-    const int grid = balanced_grid(tiles, max_grid);
+    const int64_t pad_blocks = BLOCKED ? scale_padding_blocks(rows, kblocks, kThreads) : 0;
+    const int grid = balanced_grid(tiles, max_grid) + static_cast<int>(pad_blocks);
     return cuda_status(launch_after_dependency(mx_stream_kernel<BLOCKED>, dim3(grid), dim3(kThreads), 0, st,
                                                static_cast<const uint4 *>(in_bf16), static_cast<uint8_t *>(payload),
-                                               static_cast<uint8_t *>(scales_e8m0), nchunks, kblocks, katoms));
+                                               static_cast<uint8_t *>(scales_e8m0), nchunks, kblocks, katoms, rows,
+                                               static_cast<unsigned>(pad_blocks)));
   } else {
     const int64_t blocks = ceil_div64(numel / 32, kThreads);
     const int grid = static_cast<int>(blocks < max_grid ? blocks : max_grid);
     mx_scalar_kernel<BLOCKED><<<grid, kThreads, 0, st>>>(static_cast<const uint16_t *>(in_bf16),
                                                          static_cast<uint8_t *>(payload),
-                                                         static_cast<uint8_t *>(scales_e8m0), numel / 32, kblocks, katoms);
+                                                         static_cast<uint8_t *>(scales_e8m0), numel / 32, kblocks, katoms, rows);
   }
   return cuda_status(cudaGetLastError());
 }

@@ -17,6 +17,8 @@
 // conflicts).  Column direction: a lane owns two neighbouring columns x 16 rows (sixteen 32-bit
 // shared loads), lanes l and l^1 together hold one MX block of each column; the eight lanes of a
 // column pair write 128 contiguous bytes of a row of the transposed payload.
+// Blocked scales: a tile's 128 rows x 4 blocks are exactly one 512-byte atom of either scale array, so both atoms are put
+// together in shared memory and leave as 16-byte stores, the zeros of the padding included.
 // CTAs are numbered so that eight row tiles of one column tile run back to back, then the next
 // column tile: the 4-byte scale fragments that neighbouring tiles add to one 32-byte sector of
 // either scale array arrive close together in time.
@@ -39,13 +41,13 @@ constexpr int kGroupRowTiles = 8;
 // One tile.  FULL: the tile lies inside the matrix, no access is predicated.  ROW_OUT: the row-major payload
 // and scales are wanted too (otherwise the row direction only loads the tile and parks it).
 template <bool FULL, bool BLOCKED, bool ROW_OUT>
-__device__ __forceinline__ void dual_tile(uint32_t (&tile)[kTile][kTileWords], const uint16_t *__restrict__ in,
+__device__ __forceinline__ void dual_tile(uint32_t (&tile)[kTile][kTileWords], uint8_t (&atoms)[2][512], const uint16_t *__restrict__ in,
                                           uint8_t *__restrict__ payload, uint8_t *__restrict__ scales,
                                           uint8_t *__restrict__ payload_t, uint8_t *__restrict__ scales_t, int64_t rows,
-                                          int64_t cols, int64_t row0, int64_t col0) {
+                                          int64_t cols, int64_t row0, int64_t col0, bool atoms_aligned) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t kblocks = cols / 32, katoms = (kblocks + 3) / 4;          // scale grid of x: [rows, kblocks]
-  const int64_t row_blocks = rows / 32, row_atoms = (row_blocks + 3) / 4;  // scale grid of x^T: [cols, row_blocks]
+  const int64_t kblocks = cols / 32;      // scale grid of x: [rows, kblocks]
+  const int64_t row_blocks = rows / 32;   // scale grid of x^T: [cols, row_blocks]
 
   // ---- row direction: in pass p warp w owns tile rows 16p + 2w and + 1; lane l the columns 8(l&15) .. +7
   const int chunk = lane & 15;
@@ -73,8 +75,13 @@ __device__ __forceinline__ void dual_tile(uint32_t (&tile)[kTile][kTileWords], c
     // every lane has one byte to store after four passes instead of a quarter of the lanes after each.
     if ((lane & 3) == (p & 3)) my_scale = biased;
     if ((p & 3) == 3) {
-      const int64_t sr = row0 + (p - 3 + (lane & 3)) * kPassRows + warp * 2 + (lane >> 4);
-      if (FULL || (col_live && sr < rows)) scales[scale_offset<BLOCKED>(sr * kblocks + (c >> 5), kblocks, katoms)] = mx_scale_byte(my_scale);
+      if constexpr (BLOCKED) {  // outside the matrix the tile is zero, and so is the scale byte
+        const int srt = (p - 3 + (lane & 3)) * kPassRows + warp * 2 + (lane >> 4);
+        atoms[0][(srt & 31) * 16 + (srt >> 5) * 4 + (chunk >> 2)] = mx_scale_byte(my_scale);
+      } else {
+        const int64_t sr = row0 + (p - 3 + (lane & 3)) * kPassRows + warp * 2 + (lane >> 4);
+        if (FULL || (col_live && sr < rows)) scales[scale_offset<false>(sr * kblocks + (c >> 5), kblocks, 0)] = mx_scale_byte(my_scale);
+      }
     }
   }
   __syncthreads();
@@ -108,10 +115,30 @@ __device__ __forceinline__ void dual_tile(uint32_t (&tile)[kTile][kTileWords], c
       uint8_t *dst = payload_t + col_a * rows + r_first;  // 16 consecutive bytes of row col_a of the transpose
       stg_stream(dst, make_uint4(a[0] | (a[1] << 16), a[2] | (a[3] << 16), a[4] | (a[5] << 16), a[6] | (a[7] << 16)));
       stg_stream(dst + rows, make_uint4(b[0] | (b[1] << 16), b[2] | (b[3] << 16), b[4] | (b[5] << 16), b[6] | (b[7] << 16)));
-      if ((g & 1) == 0) {
+      if (!BLOCKED && (g & 1) == 0) {
         const int64_t blk = col_a * row_blocks + (r_first >> 5);
-        scales_t[scale_offset<BLOCKED>(blk, row_blocks, row_atoms)] = mx_scale_byte(biased_a);
-        scales_t[scale_offset<BLOCKED>(blk + row_blocks, row_blocks, row_atoms)] = mx_scale_byte(biased_b);
+        scales_t[blk] = mx_scale_byte(biased_a);
+        scales_t[blk + row_blocks] = mx_scale_byte(biased_b);
+      }
+    }
+    if (BLOCKED && (g & 1) == 0) {
+      const int ct = word * 2;  // even, so ct and ct + 1 are in the same quarter of the atom
+      uint8_t *p = &atoms[1][(ct & 31) * 16 + (ct >> 5) * 4 + (g >> 1)];
+      p[0] = mx_scale_byte(biased_a);
+      p[16] = mx_scale_byte(biased_b);
+    }
+  }
+  if constexpr (BLOCKED) {
+    __syncthreads();
+    const int64_t katoms = (cols + 127) / 128, row_atoms = (rows + 127) / 128;
+    if (threadIdx.x < 64 && (ROW_OUT || threadIdx.x >= 32)) {
+      const bool t = threadIdx.x >= 32;
+      uint8_t *dst = (t ? scales_t + ((col0 >> 7) * row_atoms + (row0 >> 7)) * 512 : scales + ((row0 >> 7) * katoms + (col0 >> 7)) * 512) + lane * 16;
+      const uint4 v16 = *reinterpret_cast<const uint4 *>(&atoms[t][lane * 16]);
+      if (atoms_aligned) {
+        *reinterpret_cast<uint4 *>(dst) = v16;
+      } else {
+        for (int i = 0; i < 16; ++i) dst[i] = atoms[t][lane * 16 + i];
       }
     }
   }
@@ -120,11 +147,12 @@ __device__ __forceinline__ void dual_tile(uint32_t (&tile)[kTile][kTileWords], c
 // 5 CTAs of 256 threads per SM (48 registers) measured 4 % faster than 4 (64 registers); 6 (40 registers) 12 % slower
 constexpr int kDualMinBlocks = kThreadsDual == 256 ? 5 : 2;
 template <bool BLOCKED, bool ROW_OUT>
-__global__ void __launch_bounds__(kThreadsDual, BLOCKED ? kDualMinBlocks - 1 : kDualMinBlocks)  // the blocked offsets need the registers
+__global__ void __launch_bounds__(kThreadsDual, kDualMinBlocks)
 mx_dual_kernel(const uint16_t *__restrict__ in, uint8_t *__restrict__ payload, uint8_t *__restrict__ scales,
                uint8_t *__restrict__ payload_t, uint8_t *__restrict__ scales_t, int64_t rows, int64_t cols,
-               int64_t row_tiles, int64_t col_tiles) {
+               int64_t row_tiles, int64_t col_tiles, bool atoms_aligned) {
   __shared__ __align__(16) uint32_t tile[kTile][kTileWords];
+  __shared__ __align__(16) uint8_t atoms[2][512];  // blocked scales of the tile, of x and of x^T
   // programmatic dependent launch, both ways (see dtq_device.cuh): blocks may become resident under the tail of the
   // kernel before this one, and what is queued behind this one under its own tail
   pdl_launch_dependents();
@@ -138,9 +166,9 @@ mx_dual_kernel(const uint16_t *__restrict__ in, uint8_t *__restrict__ payload, u
   const int64_t row0 = (first_row_tile + in_group % group_rows) * kTile;
   const int64_t col0 = (in_group / group_rows) * kTile;
   if (row0 + kTile <= rows && col0 + kTile <= cols)
-    dual_tile<true, BLOCKED, ROW_OUT>(tile, in, payload, scales, payload_t, scales_t, rows, cols, row0, col0);
+    dual_tile<true, BLOCKED, ROW_OUT>(tile, atoms, in, payload, scales, payload_t, scales_t, rows, cols, row0, col0, atoms_aligned);
   else
-    dual_tile<false, BLOCKED, ROW_OUT>(tile, in, payload, scales, payload_t, scales_t, rows, cols, row0, col0);
+    dual_tile<false, BLOCKED, ROW_OUT>(tile, atoms, in, payload, scales, payload_t, scales_t, rows, cols, row0, col0, atoms_aligned);
 }
 
 }  // namespace
@@ -166,7 +194,8 @@ int launch_dual(const void *in_bf16, void *payload, void *scales_e8m0, void *pay
                                              static_cast<cudaStream_t>(stream), static_cast<const uint16_t *>(in_bf16),
                                              static_cast<uint8_t *>(payload), static_cast<uint8_t *>(scales_e8m0),
                                              static_cast<uint8_t *>(payload_t), static_cast<uint8_t *>(scales_t_e8m0), rows, cols,
-                                             row_tiles, col_tiles));
+                                             row_tiles, col_tiles,
+                                             (!row_out || aligned_to(scales_e8m0, 16)) && aligned_to(scales_t_e8m0, 16)));
 }
 }  // namespace
 }  // namespace dtq

@@ -146,7 +146,8 @@ __device__ __forceinline__ void convert_store(const float (&f)[N], float inv, ui
 template <int IN, int FMT>
 __global__ void __launch_bounds__(kThreadsF, 2048 / kThreadsF)
 mx_formats_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, uint8_t *__restrict__ scales,
-                  int64_t nchunks, int64_t kblocks) {  // kblocks > 0: scales in the MX GEMM's blocked layout, that many per row
+                  int64_t nchunks, int64_t kblocks,  // kblocks > 0: scales in the MX GEMM's blocked layout, that many per row
+                  int64_t rows, unsigned pad_blocks) {
   // programmatic dependent launch, both ways (see dtq_device.cuh): blocks may become resident under the tail of the
   // kernel before this one, and what is queued behind this one under its own tail
   pdl_launch_dependents();
@@ -155,19 +156,28 @@ mx_formats_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, u
   using O = MxOut<FMT>;
   constexpr int kLanes = 32 / I::kElems;                        // lanes per MX block
   constexpr int kChunkBytesOut = I::kElems * O::kBitsPerElem / 8;
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int64_t kTile = int64_t(kThreadsF) * kUnrollF;
-  for (int64_t tile = blockIdx.x; tile * kTile < nchunks; tile += gridDim.x) {
-    const int64_t first = tile * kTile + threadIdx.x;
+  if (blockIdx.x < pad_blocks) {  // the first blocks of the grid write the padding of blocked scales, if there is any
+    zero_scale_padding(scales, rows, kblocks, int64_t(blockIdx.x) * kThreadsF + threadIdx.x, int64_t(pad_blocks) * kThreadsF);
+    return;
+  }
+  // A warp owns kUnrollF consecutive rows of 32 chunks, so that after the last of them every lane (every second one for
+  // fp32) has one scale byte to place: with a scale per block placed by one lane of it in each step, finding the place
+  // in the blocked layout (a division) ran four times as often, and 64 bits wide it was most of the kernel.
+  // Measured, MXFP4 with blocked scales: see mx_quantize_any.
+  for (int64_t tile = blockIdx.x - pad_blocks; tile * kTile < nchunks; tile += gridDim.x) {
+    const int64_t first = tile * kTile + int64_t(warp) * (32 * kUnrollF) + lane;
     uint4 v[kUnrollF];
+    int my_scale = 0;
 #pragma unroll
     for (int u = 0; u < kUnrollF; ++u) {
-      const int64_t c = first + u * kThreadsF;  // nchunks % kLanes == 0: a block is inside or outside as a whole
+      const int64_t c = first + u * 32;  // nchunks % kLanes == 0: a block is inside or outside as a whole
       v[u] = c < nchunks ? ldg_stream(in + c) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int u = 0; u < kUnrollF; ++u) {
-      const int64_t c = first + u * kThreadsF;
+      const int64_t c = first + u * 32;
       uint32_t key = I::key(v[u]);
 #pragma unroll
       for (int d = 1; d < kLanes; d <<= 1) key = max(key, __shfl_xor_sync(0xFFFFFFFFu, key, d));
@@ -176,36 +186,41 @@ mx_formats_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, u
         float f[I::kElems];
         I::unpack(v[u], f);
         convert_store<I::kElems, FMT>(f, inverse_scale_wide(biased), payload + c * kChunkBytesOut);
-        if ((lane & (kLanes - 1)) == 0) {
-          const int64_t blk = c / kLanes;
-          scales[kblocks > 0 ? scale_offset<true>(blk, kblocks, (kblocks + 3) / 4) : blk] = static_cast<uint8_t>(biased);
-        }
       }
+      if ((lane & (kLanes - 1)) == u) my_scale = biased;
     }
+    // lane = kLanes * k + j holds the scale of step j's k-th block
+    const int j = lane & (kLanes - 1);
+    const int64_t blk = (first - lane + j * 32) / kLanes + lane / kLanes;
+    if (j < kUnrollF && blk * kLanes < nchunks)
+      scales[kblocks > 0 ? scale_offset<true>(blk, kblocks, (kblocks + 3) / 4) : blk] = static_cast<uint8_t>(my_scale);
   }
 }
 
 template <int IN, int FMT>
-int launch_formats(const void *in, void *payload, void *scales, int64_t numel, int64_t kblocks, const DeviceInfo &dev,
+int launch_formats(const void *in, void *payload, void *scales, int64_t numel, int64_t kblocks, int64_t rows, const DeviceInfo &dev,
                    cudaStream_t st) {
   using I = MxIn<IN>;
   constexpr int kChunkBytesOut = I::kElems * MxOut<FMT>::kBitsPerElem / 8;
+  static_assert(kUnrollF == 4, "a lane keeps the scale of one of its group's four steps");
   if (!aligned_to(in, 16) || !aligned_to(payload, kChunkBytesOut)) return DTQ_ERR_INVALID_ARGUMENT;
   const int64_t nchunks = numel / I::kElems;
   const int64_t tiles = ceil_div64(nchunks, int64_t(kThreadsF) * kUnrollF);
-  const int grid = balanced_grid(tiles, int64_t(dev.sm_count) * (1 << 20));
+  const int64_t pad_blocks = kblocks > 0 ? scale_padding_blocks(rows, kblocks, kThreadsF) : 0;
+  const int grid = balanced_grid(tiles, int64_t(dev.sm_count) * (1 << 20)) + static_cast<int>(pad_blocks);
   return cuda_status(launch_after_dependency(mx_formats_kernel<IN, FMT>, dim3(grid), dim3(kThreadsF), 0, st,
                                              static_cast<const uint4 *>(in), static_cast<uint8_t *>(payload),
-                                             static_cast<uint8_t *>(scales), nchunks, kblocks));
+                                             static_cast<uint8_t *>(scales), nchunks, kblocks, rows,
+                                             static_cast<unsigned>(pad_blocks)));
 }
 
 template <int IN>
 int launch_by_format(int fmt, const void *in, void *payload, void *scales, int64_t numel, int64_t kblocks,
-                     const DeviceInfo &dev, cudaStream_t st) {
+                     int64_t rows, const DeviceInfo &dev, cudaStream_t st) {
   switch (fmt) {
-    case DTQ_E4M3: return launch_formats<IN, DTQ_E4M3>(in, payload, scales, numel, kblocks, dev, st);
-    case DTQ_E5M2: return launch_formats<IN, DTQ_E5M2>(in, payload, scales, numel, kblocks, dev, st);
-    default: return launch_formats<IN, DTQ_E2M1>(in, payload, scales, numel, kblocks, dev, st);
+    case DTQ_E4M3: return launch_formats<IN, DTQ_E4M3>(in, payload, scales, numel, kblocks, rows, dev, st);
+    case DTQ_E5M2: return launch_formats<IN, DTQ_E5M2>(in, payload, scales, numel, kblocks, rows, dev, st);
+    default: return launch_formats<IN, DTQ_E2M1>(in, payload, scales, numel, kblocks, rows, dev, st);
   }
 }
 
@@ -223,9 +238,9 @@ int mx_quantize_any(const void *in, void *payload, void *scales_e8m0, int64_t ro
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t kblocks = blocked ? cols / 32 : 0;
   switch (in_dtype) {
-    case DTQ_BF16: return launch_by_format<DTQ_BF16>(elem_format, in, payload, scales_e8m0, numel, kblocks, dev, st);
-    case DTQ_F16: return launch_by_format<DTQ_F16>(elem_format, in, payload, scales_e8m0, numel, kblocks, dev, st);
-    default: return launch_by_format<DTQ_F32>(elem_format, in, payload, scales_e8m0, numel, kblocks, dev, st);
+    case DTQ_BF16: return launch_by_format<DTQ_BF16>(elem_format, in, payload, scales_e8m0, numel, kblocks, rows, dev, st);
+    case DTQ_F16: return launch_by_format<DTQ_F16>(elem_format, in, payload, scales_e8m0, numel, kblocks, rows, dev, st);
+    default: return launch_by_format<DTQ_F32>(elem_format, in, payload, scales_e8m0, numel, kblocks, rows, dev, st);
   }
 }
 

@@ -324,8 +324,7 @@ std::tuple<at::Tensor, at::Tensor> mx_fp4_quantize(at::Tensor input, bool blocke
   c10::cuda::CUDAGuard guard(input.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   if (blocked) {  // scales in the layout mx_fp4_bf16 takes, zero in the padding
-    at::Tensor scale = at::zeros({static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, input.options().dtype(at::kByte))
-                           .view(at::kFloat8_e8m0fnu);
+    at::Tensor scale = at::empty({static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, input.options().dtype(at::kFloat8_e8m0fnu));
     check_status(dtq_mx_quantize_blocked(input.data_ptr(), out.data_ptr(), scale.data_ptr(), m, n, mx_in_code(in_type),
                                          DTQ_E2M1, stream.stream()),
                  "mx_fp4_quantize");
@@ -352,9 +351,8 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> mx_fp8_quantize_dual(
   at::Tensor out = at::empty({m, n}, fp8), out_t = at::empty({n, m}, fp8);
   at::Tensor scale, scale_t;
   if (blocked) {
-    auto bytes = input.options().dtype(at::kByte);
-    scale = at::zeros({static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, bytes).view(at::kFloat8_e8m0fnu);
-    scale_t = at::zeros({static_cast<int64_t>(dtq_mx_blocked_scale_bytes(n, m))}, bytes).view(at::kFloat8_e8m0fnu);
+    scale = at::empty({static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, e8m0);
+    scale_t = at::empty({static_cast<int64_t>(dtq_mx_blocked_scale_bytes(n, m))}, e8m0);
   } else {
     scale = at::empty({m * (n / 32)}, e8m0);
     scale_t = at::empty({n * (m / 32)}, e8m0);
@@ -378,10 +376,7 @@ std::tuple<at::Tensor, at::Tensor> mx_fp8_quantize_blocked(at::Tensor input) {
   const int64_t m = input.size(0), n = input.size(1);
   TORCH_CHECK(n % 32 == 0, "The last dimension must be a multiple of the block size 32, but got ", n);
   at::Tensor out = at::empty_like(input, input.options().dtype(at::kFloat8_e4m3fn));
-  const int64_t nbytes = static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n));
-  const bool padded = m % 128 != 0 || (n / 32) % 4 != 0;
-  at::Tensor scale = padded ? at::zeros({nbytes}, input.options().dtype(at::kByte)).view(at::kFloat8_e8m0fnu)
-                            : at::empty({nbytes}, input.options().dtype(at::kFloat8_e8m0fnu));
+  at::Tensor scale = at::empty({static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, input.options().dtype(at::kFloat8_e8m0fnu));
   c10::cuda::CUDAGuard guard(input.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   check_status(dtq_mx_fp8_quantize_blocked(input.data_ptr(), out.data_ptr(), scale.data_ptr(), m, n, stream.stream()),

@@ -263,8 +263,7 @@ int dtq_mx_quantize(const void *in, void *payload, void *scales_e8m0, int64_t ro
                     int elem_format, void *stream);
 /*
  * The same with the scales in the blocked layout of dtq_mx_fp8_quantize_blocked (dtq_mx_blocked_scale_bytes(rows,
- * cols) bytes; bytes of padding rows / blocks are not written: zero the buffer first if the shape is not a
- * multiple of (128, 128)): the operands of dtq_mx_fp4_bf16 straight from the cast.
+ * cols) bytes; bytes of padding rows / blocks are written as zeros): the operands of dtq_mx_fp4_bf16 straight from the cast.
  */
 int dtq_mx_quantize_blocked(const void *in, void *payload, void *scales_blocked, int64_t rows, int64_t cols, int in_dtype,
                             int elem_format, void *stream);
@@ -286,8 +285,8 @@ int dtq_mx_fp8_quantize_dual(const void *in_bf16, void *payload, void *scales_e8
 /*
  * The same with both scale arrays in the blocked layout of dtq_mx_fp8_quantize_blocked: `scales`
  * for the [rows, cols/32] grid (dtq_mx_blocked_scale_bytes(rows, cols) bytes), `scales_t` for the
- * [cols, rows/32] grid (dtq_mx_blocked_scale_bytes(cols, rows) bytes); padding bytes are not
- * written (zero-fill the arrays when rows or cols is not a multiple of 128).  Both operands of the
+ * [cols, rows/32] grid (dtq_mx_blocked_scale_bytes(cols, rows) bytes); padding bytes are
+ * written as zeros.  Both operands of the
  * reference's mx_fp8_bf16 (src/mx_fp8_bf16.cu:197-205) for x and for x^T from one read, with no
  * transpose, second cast or to_blocked pass.
  */
@@ -315,8 +314,7 @@ int dtq_mx_fp8_quantize_tma(const void *in_bf16, void *payload, void *scales_e8m
  * reference reaches that layout with a separate re-layout pass over the row-major scales
  * (`to_blocked`, test/test_mx.py:28-32); emitting it here saves that pass.
  * `scales_blocked` holds dtq_mx_blocked_scale_bytes(rows, cols) bytes; bytes that belong to
- * padding rows / blocks (rows % 128, (cols/32) % 4) are not written: zero the buffer first if
- * the shape is not a multiple of (128, 128).
+ * padding rows / blocks (rows % 128, (cols/32) % 4) are written as zeros.
  */
 size_t dtq_mx_blocked_scale_bytes(int64_t rows, int64_t cols);
 int dtq_mx_fp8_quantize_blocked(const void *in_bf16, void *payload, void *scales_blocked, int64_t rows,

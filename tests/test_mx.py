@@ -469,3 +469,37 @@ def test_dual_with_blocked_scales(rows, cols):
     q, qs = dt.mx_fp8_quantize_blocked(a.cuda())
     qt, qts = dt.mx_fp8_quantize_blocked(a.t().contiguous().cuda())
     assert torch.equal(as_bytes(s), as_bytes(qs)) and torch.equal(as_bytes(s_t), as_bytes(qts))
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 32), (32, 96), (127, 128), (128, 160), (160, 32), (288, 4128)])
+@pytest.mark.parametrize("offset", [0, 1])  # byte offset of the scale array
+def test_padding_of_blocked_scales_is_written(rows, cols, offset):
+    from driss_torch_b200 import _cabi
+
+    a = workloads.make_cfg3(rows=rows, cols=cols)
+
+    def scale_room(r, c):
+        n = _cabi.load().dtq_mx_blocked_scale_bytes(r, c)
+        room = torch.full((n + 96,), 0xAA, dtype=torch.uint8, device="cuda")
+        return room, room[48 + offset:48 + offset + n]
+
+    def check(room, got, want_rm, r, c):
+        assert torch.equal(got.cpu(), as_bytes(qo.to_blocked(want_rm.cpu().view(torch.uint8), r, c // 32)))
+        assert (room[:48 + offset] == 0xAA).all() and (room[48 + offset + got.numel():] == 0xAA).all()
+
+    x = a.cuda()
+    _, want = _cabi.mx_fp8_quantize(x)
+    shifted = torch.empty(rows * cols + 1, dtype=torch.bfloat16, device="cuda")[1:].view(rows, cols).copy_(x)
+    for inp in (x, shifted):  # the stream kernel and the scalar one
+        room, s = scale_room(rows, cols)
+        _cabi.mx_fp8_quantize_blocked(inp, scales=s)
+        check(room, s, want, rows, cols)
+    for dtype in (torch.bfloat16, torch.float16, torch.float32):
+        room, s = scale_room(rows, cols)
+        _cabi.mx_quantize(x.to(dtype), "e2m1", scales=s, blocked=True)
+        check(room, s, _cabi.mx_quantize(x.to(dtype), "e2m1")[1], rows, cols)
+    if rows % 32 == 0:
+        (room, s), (room_t, s_t) = scale_room(rows, cols), scale_room(cols, rows)
+        _cabi.mx_fp8_quantize_dual(x, scales=s, scales_t=s_t, blocked=True)
+        check(room, s, want, rows, cols)
+        check(room_t, s_t, _cabi.mx_fp8_quantize(x.t().contiguous())[1], cols, rows)
