@@ -10,6 +10,7 @@
 // Each op: check -> allocate outputs with the caching allocator -> one C-ABI call.  Nothing
 // here computes.
 #include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/DispatchKey.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -31,6 +32,15 @@ void check_status(int status, const char *what) {
 
 int in_code(at::ScalarType t) { return t == at::kBFloat16 ? DTQ_BF16 : DTQ_F32; }
 int out_code(at::ScalarType t) { return t == at::kFloat8_e4m3fn ? DTQ_E4M3 : DTQ_E5M2; }
+
+// Outputs straight from the CUDA allocator: what at::empty / at::empty_like end in, without a second and third trip
+// through the dispatcher.  The smallest calls are bound by the host, and each at::empty was 0.4 us of their 5 to 9.
+at::Tensor new_on_device_of(const at::Tensor &like, at::IntArrayRef sizes, at::ScalarType dtype) {
+  return at::Tensor(at::detail::empty_cuda(sizes, dtype, like.device(), std::nullopt));
+}
+at::Tensor new_same_layout(const at::Tensor &like, at::ScalarType dtype) {  // `like` is dense: its strides are kept as they are
+  return at::Tensor(at::detail::empty_strided_cuda(like.sizes(), like.strides(), dtype, like.device()));
+}
 
 void check_fp8(at::ScalarType dtype) {
   TORCH_CHECK(dtype == at::kFloat8_e4m3fn || dtype == at::kFloat8_e5m2,
@@ -97,7 +107,7 @@ at::Tensor saturated_cast(const at::Tensor &input, const at::Tensor &scale, at::
   const bool transposed = strides[0] == 1 && strides[1] == input.size(0);
   const bool as_is = (input.is_contiguous() || transposed) && input.storage_offset() == 0;
   const at::Tensor x = as_is ? input : input.contiguous();
-  at::Tensor out = at::empty_like(x, x.options().dtype(dtype));
+  at::Tensor out = new_same_layout(x, dtype);
   c10::cuda::CUDAGuard guard(x.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   check_status(dtq_saturated_cast(x.data_ptr(), out.data_ptr(), scale.data_ptr<float>(), x.numel(),
@@ -116,8 +126,8 @@ std::tuple<at::Tensor, at::Tensor> cast_transposed(const at::Tensor &input, cons
   TORCH_CHECK(scale.is_cuda() && scale.device() == input.device(), "Scale tensor must live on the input's device");
   const at::Tensor x = input.contiguous();
   const int64_t rows = x.size(0), cols = x.size(1);
-  at::Tensor out_t = at::empty({cols, rows}, x.options().dtype(dtype));
-  at::Tensor out = both ? at::empty({rows, cols}, x.options().dtype(dtype)) : at::Tensor();
+  at::Tensor out_t = new_on_device_of(x, {cols, rows}, dtype);
+  at::Tensor out = both ? new_on_device_of(x, {rows, cols}, dtype) : at::Tensor();
   c10::cuda::CUDAGuard guard(x.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   check_status(dtq_saturated_cast_transposed(x.data_ptr(), both ? out.data_ptr() : nullptr, out_t.data_ptr(),
@@ -146,9 +156,9 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> cast_with_amax_dual(const at::Ten
                   amax_value.device() == input.device(),
               "amax must be a one-element fp32 tensor on the input's device");
   const int64_t rows = input.size(0), cols = input.size(1);
-  at::Tensor out = at::empty({rows, cols}, input.options().dtype(dtype));
-  at::Tensor out_t = at::empty({cols, rows}, input.options().dtype(dtype));
-  at::Tensor scale = at::empty({1}, input.options().dtype(at::kFloat));
+  at::Tensor out = new_on_device_of(input, {rows, cols}, dtype);
+  at::Tensor out_t = new_on_device_of(input, {cols, rows}, dtype);
+  at::Tensor scale = new_on_device_of(input, {1}, at::kFloat);
   c10::cuda::CUDAGuard guard(input.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   if (input.numel() == 0) {  // nothing is launched: derive the scale like the cast kernels do
@@ -170,15 +180,15 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> dynamic_scaled_quant_
   check_input(input);
   TORCH_CHECK(input.is_contiguous(), "Input tensor must be contiguous");
   const int64_t rows = input.size(0), cols = input.size(1);
-  at::Tensor out = at::empty({rows, cols}, input.options().dtype(dtype));
-  at::Tensor out_t = at::empty({cols, rows}, input.options().dtype(dtype));
+  at::Tensor out = new_on_device_of(input, {rows, cols}, dtype);
+  at::Tensor out_t = new_on_device_of(input, {cols, rows}, dtype);
   if (input.numel() == 0) {  // nothing is launched: the fused op's maximum starts at 0
     at::Tensor amax_value = at::zeros({1}, input.options().dtype(at::kFloat));
     at::Tensor scale = at::full({1}, (dtype == at::kFloat8_e4m3fn ? 448.0 : 57344.0) / 1e-12, input.options().dtype(at::kFloat));
     return {out, out_t, amax_value, scale};
   }
-  at::Tensor amax_value = at::empty({1}, input.options().dtype(at::kFloat));
-  at::Tensor scale = at::empty({1}, input.options().dtype(at::kFloat));
+  at::Tensor amax_value = new_on_device_of(input, {1}, at::kFloat);
+  at::Tensor scale = new_on_device_of(input, {1}, at::kFloat);
   c10::cuda::CUDAGuard guard(input.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   check_status(dtq_dynamic_scaled_quant_dual(input.data_ptr(), out.data_ptr(), out_t.data_ptr(), amax_value.data_ptr<float>(),
@@ -193,7 +203,7 @@ at::Tensor amax(const at::Tensor &input) {
   check_input(input);
   // max is order independent, so any dense layout can be reduced over its storage.
   const at::Tensor x = input.is_non_overlapping_and_dense() ? input : input.contiguous();
-  at::Tensor out = at::empty({1}, x.options().dtype(at::kFloat));
+  at::Tensor out = new_on_device_of(x, {1}, at::kFloat);
   c10::cuda::CUDAGuard guard(x.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   check_status(dtq_amax(x.data_ptr(), out.data_ptr<float>(), x.numel(), in_code(x.scalar_type()),
@@ -207,9 +217,9 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> dynamic_scaled_quant_with_scale(c
   check_fp8(dtype);
   check_input(input);
   TORCH_CHECK(input.is_contiguous(), "Input tensor must be contiguous");
-  at::Tensor out = at::empty_like(input, input.options().dtype(dtype));
-  at::Tensor amax_value = at::empty({1}, input.options().dtype(at::kFloat));
-  at::Tensor scale = at::empty({1}, input.options().dtype(at::kFloat));
+  at::Tensor out = new_same_layout(input, dtype);
+  at::Tensor amax_value = new_on_device_of(input, {1}, at::kFloat);
+  at::Tensor scale = new_on_device_of(input, {1}, at::kFloat);
   c10::cuda::CUDAGuard guard(input.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   check_status(dtq_dynamic_scaled_quant(input.data_ptr(), out.data_ptr(), amax_value.data_ptr<float>(),
@@ -224,7 +234,7 @@ at::Tensor dynamic_scaled_quant(const at::Tensor &input, at::ScalarType dtype) {
   check_fp8(dtype);
   check_input(input);
   TORCH_CHECK(input.is_contiguous(), "Input tensor must be contiguous");
-  at::Tensor out = at::empty_like(input, input.options().dtype(dtype));
+  at::Tensor out = new_same_layout(input, dtype);
   c10::cuda::CUDAGuard guard(input.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   check_status(dtq_dynamic_scaled_quant(input.data_ptr(), out.data_ptr(), nullptr, nullptr, input.numel(),
@@ -262,8 +272,8 @@ std::tuple<at::Tensor, at::Tensor> mx_fp8_quantize(at::Tensor input, int64_t blo
     TORCH_CHECK(in_type == at::kBFloat16 && fp8_type == at::kFloat8_e4m3fn,
                 "axis=0 / transpose=True need a bfloat16 input and an e4m3 payload");
     TORCH_CHECK(m % 32 == 0 && n % 32 == 0, "Both dimensions must be multiples of the block size 32, but got ", m, " x ", n);
-    at::Tensor out_t = at::empty({n, m}, input.options().dtype(fp8_type));
-    at::Tensor scale_t = at::empty({n * (m / 32)}, input.options().dtype(at::kFloat8_e8m0fnu));
+    at::Tensor out_t = new_on_device_of(input, {n, m}, fp8_type);
+    at::Tensor scale_t = new_on_device_of(input, {n * (m / 32)}, at::kFloat8_e8m0fnu);
     c10::cuda::CUDAGuard guard(input.device());
     auto stream = c10::cuda::getCurrentCUDAStream();
     check_status(dtq_mx_fp8_quantize_dual(input.data_ptr(), nullptr, nullptr, out_t.data_ptr(), scale_t.data_ptr(), m, n,
@@ -272,8 +282,8 @@ std::tuple<at::Tensor, at::Tensor> mx_fp8_quantize(at::Tensor input, int64_t blo
     return {transpose ? out_t : out_t.t(), scale_t};
   }
   TORCH_CHECK(n % 32 == 0, "The last dimension must be a multiple of the block size 32, but got ", n);
-  at::Tensor out = at::empty_like(input, input.options().dtype(fp8_type));
-  at::Tensor scale = at::empty({m * (n / 32)}, input.options().dtype(at::kFloat8_e8m0fnu));
+  at::Tensor out = new_same_layout(input, fp8_type);
+  at::Tensor scale = new_on_device_of(input, {m * (n / 32)}, at::kFloat8_e8m0fnu);
   c10::cuda::CUDAGuard guard(input.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   if (in_type == at::kBFloat16 && fp8_type == at::kFloat8_e4m3fn) {
@@ -298,9 +308,9 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> mx_fp8_quantize_with_amax(at::Ten
   TORCH_CHECK(input.scalar_type() == at::kBFloat16, "Input tensor must be bfloat16, but got ", input.dtype());
   const int64_t m = input.size(0), n = input.size(1);
   TORCH_CHECK(n % 32 == 0, "The last dimension must be a multiple of the block size 32, but got ", n);
-  at::Tensor out = at::empty_like(input, input.options().dtype(at::kFloat8_e4m3fn));
-  at::Tensor scale = at::empty({m * (n / 32)}, input.options().dtype(at::kFloat8_e8m0fnu));
-  at::Tensor amax = at::empty({1}, input.options().dtype(at::kFloat));
+  at::Tensor out = new_same_layout(input, at::kFloat8_e4m3fn);
+  at::Tensor scale = new_on_device_of(input, {m * (n / 32)}, at::kFloat8_e8m0fnu);
+  at::Tensor amax = new_on_device_of(input, {1}, at::kFloat);
   c10::cuda::CUDAGuard guard(input.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   check_status(dtq_mx_fp8_quantize_amax(input.data_ptr(), out.data_ptr(), scale.data_ptr(), amax.data_ptr<float>(), m, n,
@@ -320,17 +330,17 @@ std::tuple<at::Tensor, at::Tensor> mx_fp4_quantize(at::Tensor input, bool blocke
               "Input tensor must be bfloat16, float16 or float32, but got ", input.dtype());
   const int64_t m = input.size(0), n = input.size(1);
   TORCH_CHECK(n % 32 == 0, "The last dimension must be a multiple of the block size 32, but got ", n);
-  at::Tensor out = at::empty({m, n / 2}, input.options().dtype(at::kByte));
+  at::Tensor out = new_on_device_of(input, {m, n / 2}, at::kByte);
   c10::cuda::CUDAGuard guard(input.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   if (blocked) {  // scales in the layout mx_fp4_bf16 takes, zero in the padding
-    at::Tensor scale = at::empty({static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, input.options().dtype(at::kFloat8_e8m0fnu));
+    at::Tensor scale = new_on_device_of(input, {static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, at::kFloat8_e8m0fnu);
     check_status(dtq_mx_quantize_blocked(input.data_ptr(), out.data_ptr(), scale.data_ptr(), m, n, mx_in_code(in_type),
                                          DTQ_E2M1, stream.stream()),
                  "mx_fp4_quantize");
     return {out, scale};
   }
-  at::Tensor scale = at::empty({m * (n / 32)}, input.options().dtype(at::kFloat8_e8m0fnu));
+  at::Tensor scale = new_on_device_of(input, {m * (n / 32)}, at::kFloat8_e8m0fnu);
   check_status(dtq_mx_quantize(input.data_ptr(), out.data_ptr(), scale.data_ptr(), m, n, mx_in_code(in_type), DTQ_E2M1,
                                stream.stream()),
                "mx_fp4_quantize");
@@ -346,16 +356,14 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> mx_fp8_quantize_dual(
   TORCH_CHECK(input.scalar_type() == at::kBFloat16, "Input tensor must be bfloat16, but got ", input.dtype());
   const int64_t m = input.size(0), n = input.size(1);
   TORCH_CHECK(m % 32 == 0 && n % 32 == 0, "Both dimensions must be multiples of the block size 32, but got ", m, " x ", n);
-  auto fp8 = input.options().dtype(at::kFloat8_e4m3fn);
-  auto e8m0 = input.options().dtype(at::kFloat8_e8m0fnu);
-  at::Tensor out = at::empty({m, n}, fp8), out_t = at::empty({n, m}, fp8);
+  at::Tensor out = new_on_device_of(input, {m, n}, at::kFloat8_e4m3fn), out_t = new_on_device_of(input, {n, m}, at::kFloat8_e4m3fn);
   at::Tensor scale, scale_t;
   if (blocked) {
-    scale = at::empty({static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, e8m0);
-    scale_t = at::empty({static_cast<int64_t>(dtq_mx_blocked_scale_bytes(n, m))}, e8m0);
+    scale = new_on_device_of(input, {static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, at::kFloat8_e8m0fnu);
+    scale_t = new_on_device_of(input, {static_cast<int64_t>(dtq_mx_blocked_scale_bytes(n, m))}, at::kFloat8_e8m0fnu);
   } else {
-    scale = at::empty({m * (n / 32)}, e8m0);
-    scale_t = at::empty({n * (m / 32)}, e8m0);
+    scale = new_on_device_of(input, {m * (n / 32)}, at::kFloat8_e8m0fnu);
+    scale_t = new_on_device_of(input, {n * (m / 32)}, at::kFloat8_e8m0fnu);
   }
   c10::cuda::CUDAGuard guard(input.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
@@ -375,8 +383,8 @@ std::tuple<at::Tensor, at::Tensor> mx_fp8_quantize_blocked(at::Tensor input) {
   TORCH_CHECK(input.scalar_type() == at::kBFloat16, "Input tensor must be bfloat16, but got ", input.dtype());
   const int64_t m = input.size(0), n = input.size(1);
   TORCH_CHECK(n % 32 == 0, "The last dimension must be a multiple of the block size 32, but got ", n);
-  at::Tensor out = at::empty_like(input, input.options().dtype(at::kFloat8_e4m3fn));
-  at::Tensor scale = at::empty({static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, input.options().dtype(at::kFloat8_e8m0fnu));
+  at::Tensor out = new_same_layout(input, at::kFloat8_e4m3fn);
+  at::Tensor scale = new_on_device_of(input, {static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, at::kFloat8_e8m0fnu);
   c10::cuda::CUDAGuard guard(input.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   check_status(dtq_mx_fp8_quantize_blocked(input.data_ptr(), out.data_ptr(), scale.data_ptr(), m, n, stream.stream()),
@@ -391,9 +399,9 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> dynamic_scaled_quant_rowwise(cons
   TORCH_CHECK(input.is_contiguous(), "Input tensor must be contiguous");
   const int64_t m = input.size(0), n = input.size(1);
   TORCH_CHECK(m == 0 || n > 0, "Rows must not be empty");
-  at::Tensor out = at::empty_like(input, input.options().dtype(dtype));
-  at::Tensor amax_rows = at::empty({m, 1}, input.options().dtype(at::kFloat));
-  at::Tensor scale_rows = at::empty({m, 1}, input.options().dtype(at::kFloat));
+  at::Tensor out = new_same_layout(input, dtype);
+  at::Tensor amax_rows = new_on_device_of(input, {m, 1}, at::kFloat);
+  at::Tensor scale_rows = new_on_device_of(input, {m, 1}, at::kFloat);
   c10::cuda::CUDAGuard guard(input.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   check_status(dtq_dynamic_scaled_quant_rowwise(input.data_ptr(), out.data_ptr(), amax_rows.data_ptr<float>(),
@@ -411,8 +419,8 @@ std::tuple<at::Tensor, at::Tensor> cast_with_amax(const at::Tensor &input, const
   TORCH_CHECK(amax_value.scalar_type() == at::kFloat && amax_value.numel() == 1 && amax_value.is_cuda() &&
                   amax_value.device() == input.device(),
               "amax must be one fp32 value on the input's device");
-  at::Tensor out = at::empty_like(input, input.options().dtype(dtype));
-  at::Tensor scale = at::empty({1}, input.options().dtype(at::kFloat));
+  at::Tensor out = new_same_layout(input, dtype);
+  at::Tensor scale = new_on_device_of(input, {1}, at::kFloat);
   c10::cuda::CUDAGuard guard(input.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   check_status(dtq_cast_with_amax(input.data_ptr(), out.data_ptr(), amax_value.data_ptr<float>(),
@@ -450,7 +458,7 @@ at::Tensor mx_fp8_bf16(at::Tensor a, at::Tensor b, at::Tensor a_scale, at::Tenso
   TORCH_CHECK(a_scale.is_contiguous() && b_scale.is_contiguous(), "scale tensors must be contiguous");
   TORCH_CHECK(a.stride(1) == 1 && a.stride(0) == K, "Input tensor 'a' must be contiguous in the K dimension (row-major)");
   TORCH_CHECK(b.stride(0) == 1 && b.stride(1) == K, "Input tensor 'b' must be contiguous in the K dimension (column-major)");
-  at::Tensor out = at::empty({M, N}, a.options().dtype(at::kBFloat16));
+  at::Tensor out = new_on_device_of(a, {M, N}, at::kBFloat16);
   c10::cuda::CUDAGuard guard(a.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   check_status(dtq_mx_fp8_bf16(a.data_ptr(), b.data_ptr(), a_scale.data_ptr(), b_scale.data_ptr(), out.data_ptr(), M, N, K,
@@ -482,7 +490,7 @@ at::Tensor mx_fp4_bf16(at::Tensor a, at::Tensor b, at::Tensor a_scale, at::Tenso
   TORCH_CHECK(a_scale.is_contiguous() && b_scale.is_contiguous(), "scale tensors must be contiguous");
   TORCH_CHECK(a.stride(1) == 1 && a.stride(0) == Kb, "Input tensor 'a' must be contiguous in the K dimension (row-major)");
   TORCH_CHECK(b.stride(0) == 1 && b.stride(1) == Kb, "Input tensor 'b' must be contiguous in the K dimension (column-major)");
-  at::Tensor out = at::empty({M, N}, a.options().dtype(at::kBFloat16));
+  at::Tensor out = new_on_device_of(a, {M, N}, at::kBFloat16);
   c10::cuda::CUDAGuard guard(a.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   check_status(dtq_mx_fp4_bf16(a.data_ptr(), b.data_ptr(), a_scale.data_ptr(), b_scale.data_ptr(), out.data_ptr(), M, N, K,
@@ -521,7 +529,7 @@ at::Tensor sweep_mm(at::Tensor XQ, at::Tensor WQ, at::Tensor x_scale, at::Tensor
     bias_ptr = bias->data_ptr();
     bias_code = bias->scalar_type() == at::kBFloat16 ? DTQ_BF16 : DTQ_F32;
   }
-  at::Tensor out = at::empty({M, N}, XQ.options().dtype(out_dtype));
+  at::Tensor out = new_on_device_of(XQ, {M, N}, out_dtype);
   c10::cuda::CUDAGuard guard(XQ.device());
   auto stream = c10::cuda::getCurrentCUDAStream();
   check_status(dtq_rowwise_fp8_bf16(XQ.data_ptr(), WQ.data_ptr(), x_scale.data_ptr<float>(), w_scale.data_ptr<float>(), bias_ptr,
