@@ -298,6 +298,22 @@ __device__ __forceinline__ void apply_rowwise(uint32_t (&v)[32], float xs, float
   }
 }
 
+// The same with the 32 columns' scales and biases (null: none) in shared memory, 16-byte aligned.
+__device__ __forceinline__ void apply_rowwise_shared(uint32_t (&v)[32], float xs, const float *cs, const float *bs) {
+#pragma unroll
+  for (int i = 0; i < 32; i += 4) {
+    const float4 s = *reinterpret_cast<const float4 *>(cs + i);
+    float f[4] = {__fmul_rn(__fmul_rn(__uint_as_float(v[i]), xs), s.x), __fmul_rn(__fmul_rn(__uint_as_float(v[i + 1]), xs), s.y),
+                  __fmul_rn(__fmul_rn(__uint_as_float(v[i + 2]), xs), s.z), __fmul_rn(__fmul_rn(__uint_as_float(v[i + 3]), xs), s.w)};
+    if (bs) {
+      const float4 b = *reinterpret_cast<const float4 *>(bs + i);
+      f[0] = __fadd_rn(f[0], b.x), f[1] = __fadd_rn(f[1], b.y), f[2] = __fadd_rn(f[2], b.z), f[3] = __fadd_rn(f[3], b.w);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[i + j] = __float_as_uint(f[j]);
+  }
+}
+
 // 32 accumulator columns of this thread's lane of tensor memory into registers (asynchronous: tmem_load_wait).
 __device__ __forceinline__ void tmem_load_32(uint32_t (&v)[32], uint32_t taddr) {
   asm volatile(
@@ -320,26 +336,6 @@ __device__ __forceinline__ void tmem_load_wait(uint32_t (&v)[32]) {
                  "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])
                :
                : "memory");
-}
-
-// 32 bf16 of one output row (64 bytes at `dst`), of which the first `live` columns exist (a multiple of 8).  A lane owns
-// a row, so a warp-wide store of 16 bytes per lane touches 32 half sectors and L2 sees every sector twice; where the
-// row pitch allows it (`wide`: output and pitch 32-byte aligned) a lane stores whole 32-byte sectors.  Streaming: the
-// output must not push the operands out of L2.
-__device__ __forceinline__ void store_row_32(uint16_t *dst, const uint32_t (&p)[16], int64_t live, bool wide) {
-  if (wide) {
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-      if (q * 16 < live)  // N % 16 == 0 here
-        asm volatile("st.global.cs.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + q * 16), "r"(p[8 * q]),
-                     "r"(p[8 * q + 1]), "r"(p[8 * q + 2]), "r"(p[8 * q + 3]), "r"(p[8 * q + 4]), "r"(p[8 * q + 5]),
-                     "r"(p[8 * q + 6]), "r"(p[8 * q + 7])
-                     : "memory");
-  } else {
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (q * 8 < live) stg_stream(dst + q * 8, make_uint4(p[4 * q], p[4 * q + 1], p[4 * q + 2], p[4 * q + 3]));
-  }
 }
 
 struct GemmParams {
@@ -585,7 +581,8 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 //     address space.
 // Every wait is bounded as above; an abort is forwarded to the other CTA, and both always meet at the cluster
 // barrier before tensor memory is freed.
-constexpr int kPairStages = 6;
+template <int MODE>
+constexpr int PairStages = MODE == kMxFp4 ? 5 : 6;  // what fits beside the output staging (MXFP4 has twice the scale atoms)
 constexpr int kPairBN = 256;  // tile columns; each CTA holds kPairBN / 2 rows of B
 
 // Tensor memory of the pair kernel: two accumulators of 256 columns.  Without block scales they fill the 512 columns
@@ -605,12 +602,14 @@ struct PairTmem {
 
 template <int MODE>
 struct __align__(1024) PairSmem {
-  uint8_t a[kPairStages][kBM * kBK];             // this CTA's 128 rows of A
-  uint8_t b[kPairStages][kPairBN / 2 * kBK];     // this CTA's 128 of the tile's 256 rows of B
-  uint8_t sfa[kPairStages][Format<MODE>::kKAtoms * 512];      // scales of this CTA's 128 rows of A
-  uint8_t sfb[kPairStages][2 * Format<MODE>::kKAtoms * 512];  // scales of all 256 rows of B: [128 columns][atom along K]
-  uint64_t full[kPairStages];                    // used in the leader CTA only
-  uint64_t empty[kPairStages];
+  uint8_t a[PairStages<MODE>][kBM * kBK];             // this CTA's 128 rows of A
+  uint8_t b[PairStages<MODE>][kPairBN / 2 * kBK];     // this CTA's 128 of the tile's 256 rows of B
+  uint8_t sfa[PairStages<MODE>][Format<MODE>::kKAtoms * 512];      // scales of this CTA's 128 rows of A
+  uint8_t sfb[PairStages<MODE>][2 * Format<MODE>::kKAtoms * 512];  // scales of all 256 rows of B: [128 columns][atom along K]
+  uint8_t out[kEpilogueWarps][32 * 64];          // per epilogue warp 32 rows x 32 bf16 on their way out (64-byte swizzle)
+  float scales[MODE == kRowwise ? kEpilogueWarps : 1][2][128];  // per epilogue warp its columns' scales and biases
+  uint64_t full[PairStages<MODE>];               // used in the leader CTA only
+  uint64_t empty[PairStages<MODE>];
   uint64_t tmem_full[2];                         // one per accumulator
   uint64_t tmem_empty[2];                        // used in the leader CTA only
   uint32_t tmem_base;
@@ -661,20 +660,35 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t *bar) {
                : "memory");
 }
 
+// TMA store of a box of the output from shared memory (bulk group of the issuing thread), and the waits for it.
+__device__ __forceinline__ uint64_t l2_policy_evict_first() {
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, const void *src, int x, int y, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group.L2::cache_hint [%0, {%2, %3}], [%1], %4;\n\t"
+      "cp.async.bulk.commit_group;" ::"l"(reinterpret_cast<uint64_t>(map)),
+      "r"(smem_addr(src)), "r"(x), "r"(y), "l"(policy)
+      : "memory");
+}
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 struct PairParams {
   RowwiseEpilogue rowwise;
-  uint16_t *out;  // bf16 [M, N]
   int M, N;
   int m_pairs, n_tiles, k_stages;  // 256-row tile rows, 256-column tile columns, 128-byte K stages
-  bool wide_stores;                // rows of the output start on 32-byte boundaries
   int *status;
 };
 
 template <int MODE>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                    const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb, PairParams p) {
-  constexpr int kKAtoms = Format<MODE>::kKAtoms;
+                    const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb,
+                    const __grid_constant__ CUtensorMap map_out, PairParams p) {
+  constexpr int kKAtoms = Format<MODE>::kKAtoms, kPairStages = PairStages<MODE>;
   extern __shared__ unsigned char smem_raw[];
   PairSmem<MODE> &sm = *reinterpret_cast<PairSmem<MODE> *>(smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u));
   const int warp = int(warp_uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
@@ -813,10 +827,14 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   } else {
     // ---- epilogue: this CTA's 128 rows of the tile, 8 warps as in the single-CTA kernel --------------------
     // A warp's 128 columns go 32 at a time, the next 32 on their way from tensor memory while these are converted and
-    // stored.  The half that holds the shared columns starts with them: half 1 at its end (columns 255..224 of the first
+    // staged in shared memory, from where a TMA store takes them (which also cuts off what lies past the edges).  With
+    // stores from registers a lane owned a row, a warp's store touched 32 lines, and the epilogue took longer than the
+    // MMAs of 1024 bytes of K; see launch_pair for the figures.  The half that holds the shared columns starts with them: half 1 at its end (columns 255..224 of the first
     // accumulator), half 0 at its beginning (columns 0..31 of the second, the same columns of tensor memory).
     const int quad = warp & 3, half = (warp - 2) >> 2;
     const uint32_t leader_empty[2] = {map_to_cta(smem_addr(&sm.tmem_empty[0]), 0), map_to_cta(smem_addr(&sm.tmem_empty[1]), 0)};
+    uint8_t *staging = sm.out[warp - 2];
+    const uint64_t stream_policy = l2_policy_evict_first();  // the output must not push the operands out of L2
     int local_tile = 0;
     for (int tile = cluster_id; tile < total_tiles; tile += n_clusters, ++local_tile) {
       int mp, nt;
@@ -824,8 +842,20 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const int64_t row = int64_t(mp) * 256 + int64_t(rank) * kBM + quad * 32 + lane;
       const int64_t col0 = int64_t(nt) * kPairBN + half * 128;
       const int acc = local_tile & 1;
-      RowwiseRegs<4> rw;
-      if constexpr (MODE == kRowwise) load_rowwise<4>(rw, p.rowwise, row, col0, lane, p.M, p.N);
+      float xs = 0.0f;
+      if constexpr (MODE == kRowwise) {
+        // before the wait: the row's scale, and the columns' scales and biases to shared memory, read there by all lanes
+        RowwiseRegs<4> rw;
+        load_rowwise<4>(rw, p.rowwise, row, col0, lane, p.M, p.N);
+        xs = rw.xs;
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          sm.scales[warp - 2][0][c * 32 + lane] = rw.cs[c];
+          sm.scales[warp - 2][1][c * 32 + lane] = rw.bs[c];
+        }
+        __syncwarp();
+      }
       if (!mbar_wait(&sm.tmem_full[acc], (local_tile >> 1) & 1u, abort)) {
         if (lane == 0) {
           atomicExch(p.status, DTQ_ERR_TIMEOUT);
@@ -836,7 +866,6 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       }
       tmem_fence_after();
       const uint32_t taddr = tmem + (uint32_t(quad * 32) << 16) + uint32_t((acc ? PairTmem<MODE>::kAcc1 : 0) + half * 128);
-      uint16_t *dst = p.out + row * p.N + col0;
       // the i-th 32 columns of this warp in the order it takes them
       auto chunk_at = [&](int i) { return PairTmem<MODE>::kShared && half ? 3 - i : i; };
       // handed back after the shared columns (the other half has none to wait for) or after everything
@@ -855,13 +884,24 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if (i == release_after) hand_back();
         if (i < 3) tmem_load_32(v[(i + 1) & 1], taddr + chunk_at(i + 1) * 32);
         const int c = chunk_at(i);
-        if constexpr (MODE == kRowwise) apply_rowwise(v[i & 1], rw.xs, rw.cs[i], rw.bs[i], rw.has_bias);  // c == i
+        if constexpr (MODE == kRowwise)
+          apply_rowwise_shared(v[i & 1], xs, &sm.scales[warp - 2][0][c * 32], p.rowwise.bias ? &sm.scales[warp - 2][1][c * 32] : nullptr);
         uint32_t packed[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) packed[j] = pack_bf16(v[i & 1][2 * j], v[i & 1][2 * j + 1]);
-        if (row < p.M) store_row_32(dst + c * 32, packed, p.N - (col0 + c * 32), p.wide_stores);
+        if (lane == 0) tma_store_wait_read();  // the staging buffer has been read
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          *reinterpret_cast<uint4 *>(staging + lane * 64 + ((q ^ ((lane >> 1) & 3)) * 16)) =
+              make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0 && row < p.M && col0 + c * 32 < p.N)
+          tma_store_2d(&map_out, staging, static_cast<int>(col0) + c * 32, static_cast<int>(row), stream_policy);
       }
     }
+    if (lane == 0) tma_store_wait_all();
   }
 
   // ---- teardown ---------------------------------------------------------------------------------------------
@@ -1173,6 +1213,20 @@ int make_operand_map(CUtensorMap *map, const void *base, int64_t rows, int64_t k
   return r == CUDA_SUCCESS ? DTQ_OK : DTQ_ERR_INVALID_ARGUMENT;
 }
 
+// Map of the bf16 output [rows, cols] for stores of boxes of 32 x 32 (64-byte swizzle).
+int make_output_map(CUtensorMap *map, void *base, int64_t rows, int64_t cols) {
+  EncodeTiledFn encode = nullptr;
+  if (int e = encode_tiled_fn(&encode)) return e;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 2};
+  const cuuint32_t box[2] = {32, 32};
+  const cuuint32_t elem_strides[2] = {1, 1};
+  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, elem_strides,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? DTQ_OK : DTQ_ERR_INVALID_ARGUMENT;
+}
+
 // Map of a blocked scale array as [atom rows][atoms along K][512 bytes]: boxes of `box_rows` x `box_katoms` atoms.
 // Atoms past the end are delivered as zeros.
 int make_scale_map(CUtensorMap *map, const void *base, int64_t atom_rows, int64_t katoms, int box_rows, int box_katoms) {
@@ -1247,9 +1301,13 @@ struct GemmCall {
   cudaStream_t st;
 };
 
+// Stores from registers against TMA stores from staged boxes (and, row-wise, scales by shuffle against shared memory),
+// us, B200: K of 512 bytes, 32768 x 4096 outputs, where the epilogue is as long as the MMAs: row-wise 118.6 -> 83.1, MXFP8
+// 89.0 -> 80.2, MXFP4 (K 512) 82.7 -> 67.2; K of 1024, 2048 x 9472: row-wise 23.0 -> 18.7; K of 4096 and more within 1 %
+// (MXFP4 8192^3 170 -> 173, for the stage that its staging costs).
 template <int MODE>
 int launch_pair(const GemmCall &c, int max_clusters) {
-  CUtensorMap map_a, map_b, map_sfa, map_sfb;
+  CUtensorMap map_a, map_b, map_sfa, map_sfb, map_out;
   constexpr int kKAtoms = Format<MODE>::kKAtoms;
   if (int e = make_operand_map(&map_a, c.a, c.m, c.k_bytes, kBM)) return e;
   if (int e = make_operand_map(&map_b, c.b, c.n, c.k_bytes, kPairBN / 2)) return e;
@@ -1260,12 +1318,11 @@ int launch_pair(const GemmCall &c, int max_clusters) {
     map_sfa = map_a;
     map_sfb = map_a;
   }
+  if (int e = make_output_map(&map_out, c.out, c.m, c.n)) return e;
   PairParams p;
   p.rowwise = c.rowwise;
-  p.out = static_cast<uint16_t *>(c.out);
   p.M = static_cast<int>(c.m);
   p.N = static_cast<int>(c.n);
-  p.wide_stores = c.n % 16 == 0 && aligned_to(c.out, 32);
   p.m_pairs = static_cast<int>(ceil_div64(c.m, 256));
   p.n_tiles = static_cast<int>(ceil_div64(c.n, kPairBN));
   p.k_stages = static_cast<int>(ceil_div64(c.k_bytes, kBK));
@@ -1275,7 +1332,7 @@ int launch_pair(const GemmCall &c, int max_clusters) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
   cluster_launch_config(&cfg, attr, 2 * clusters, kGemmThreads, 2, sizeof(PairSmem<MODE>) + 1024, c.st);
-  return cuda_status(cudaLaunchKernelEx(&cfg, mx_gemm_pair_kernel<MODE>, map_a, map_b, map_sfa, map_sfb, p));
+  return cuda_status(cudaLaunchKernelEx(&cfg, mx_gemm_pair_kernel<MODE>, map_a, map_b, map_sfa, map_sfb, map_out, p));
 }
 
 // One CTA per tile, tile shape SH.
