@@ -59,33 +59,39 @@ constexpr int kThreads = 256;
 constexpr int64_t kCastBlocksPerSmCap = 1 << 20;
 
 // ---- per-chunk arithmetic ----------------------------------------------------------------------
-// BOUNDED: |x| <= amax is guaranteed (amax was computed from the same data in this launch).
-template <int IN, int OUT, bool BOUNDED = false>
+template <int IN, int OUT>
 struct DsqChunk;
 
-template <int OUT, bool BOUNDED>
-struct DsqChunk<DTQ_BF16, OUT, BOUNDED> {
+template <int OUT>
+struct DsqChunk<DTQ_BF16, OUT> {
   static constexpr int kElems = 8;
   static constexpr int kElemBytes = 2;
   static constexpr int kOutAlign = 8;
   __device__ static void convert_store(uint4 v, const DsqScale &s, uint8_t *out, int64_t chunk) {
-    stg_stream(out + chunk * kElems, dsq_convert_bf16x8<OUT, BOUNDED>(v, s));
+    stg_stream(out + chunk * kElems, dsq_convert_bf16x8<OUT>(v, s));
   }
   __device__ static float load_one(const void *in, int64_t i) {
     return __uint_as_float(uint32_t(static_cast<const uint16_t *>(in)[i]) << 16);
   }
-  __device__ static void absmax(float &a, float &b, uint4 v) {
-    // packed |x| and max on bf16 pairs, NaNs dropped
-    __nv_bfloat162 m = __hmax2(as_bf162(v.x & 0x7FFF7FFFu), as_bf162(v.y & 0x7FFF7FFFu));
-    __nv_bfloat162 n = __hmax2(as_bf162(v.z & 0x7FFF7FFFu), as_bf162(v.w & 0x7FFF7FFFu));
-    m = __hmax2(m, n);
-    a = fmaxf(a, __bfloat162float(m.x));
-    b = fmaxf(b, __bfloat162float(m.y));
+  // Running per-half max(|acc|, |w|) of packed bf16: one instruction per word.  The sign bits are garbage until
+  // `finish` masks them; a NaN is dropped, and the accumulators start at 0, so they are never NaN.
+  using Acc = uint32_t;
+  __device__ static Acc fold1(Acc acc, uint32_t w) {
+    asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(acc) : "r"(acc), "r"(w));
+    return acc;
+  }
+  __device__ static void absmax(Acc &a, Acc &b, uint4 v) {
+    a = fold1(fold1(a, v.x), v.z);
+    b = fold1(fold1(b, v.y), v.w);
+  }
+  __device__ static float finish(Acc a, Acc b) {
+    const uint32_t m = fold1(a, b) & 0x7FFF7FFFu;
+    return fmaxf(bf16_lo(m), bf16_hi(m));
   }
 };
 
-template <int OUT, bool BOUNDED>
-struct DsqChunk<DTQ_F32, OUT, BOUNDED> {
+template <int OUT>
+struct DsqChunk<DTQ_F32, OUT> {
   static constexpr int kElems = 4;
   static constexpr int kElemBytes = 4;
   static constexpr int kOutAlign = 4;
@@ -93,10 +99,12 @@ struct DsqChunk<DTQ_F32, OUT, BOUNDED> {
     stg_stream(out + chunk * kElems, dsq_convert_f32x4<OUT>(v, s));
   }
   __device__ static float load_one(const void *in, int64_t i) { return static_cast<const float *>(in)[i]; }
-  __device__ static void absmax(float &a, float &b, uint4 v) {
+  using Acc = float;
+  __device__ static void absmax(Acc &a, Acc &b, uint4 v) {
     a = fmaxf(a, fmaxf(fabsf(__uint_as_float(v.x)), fabsf(__uint_as_float(v.y))));
     b = fmaxf(b, fmaxf(fabsf(__uint_as_float(v.z)), fabsf(__uint_as_float(v.w))));
   }
+  __device__ static float finish(Acc a, Acc b) { return fmaxf(a, b); }
 };
 
 // ---- fused single launch -------------------------------------------------------------------------
@@ -158,7 +166,7 @@ template <int IN, int OUT, int UNROLL, bool P2P>
 __global__ void __launch_bounds__(kFusedThreads, kFusedBlocksPerSm)
 dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float *__restrict__ amax_out,
                  float *__restrict__ scale_out, int64_t numel, Workspace *ws, int smem_tiles, PeerExchange px) {
-  using C = DsqChunk<IN, OUT, true>;
+  using C = DsqChunk<IN, OUT>;
   extern __shared__ uint4 kept_smem[];  // [smem_tiles][UNROLL][kFusedThreads]
   __shared__ float smem32[32];
   __shared__ int flag;
@@ -181,14 +189,14 @@ dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float 
   // the newest kFusedL2KeepMB of the streamed tiles (phase 2 starts with them); never a kept tile
   const int64_t hint_tiles = (kFusedL2KeepMB << 20) / (G * kTile * 16);
   const int64_t hint_from = count - hint_tiles > kept ? count - hint_tiles : kept;
-  float a = 0.0f, b = 0.0f;
+  typename C::Acc acc0 = 0, acc1 = 0;
   uint4 first_tile[UNROLL];
 #pragma unroll
   for (int u = 0; u < UNROLL; ++u) first_tile[u] = make_uint4(0, 0, 0, 0);
   if (kRegTiles && count > 0) {
     load_tile<UNROLL>(first_tile, in, blockIdx.x, nchunks);
 #pragma unroll
-    for (int u = 0; u < UNROLL; ++u) C::absmax(a, b, first_tile[u]);
+    for (int u = 0; u < UNROLL; ++u) C::absmax(acc0, acc1, first_tile[u]);
   }
   for (int64_t k = kRegTiles; k < count; k += 2) {  // two tiles (2 * UNROLL loads) in flight
     uint4 v[UNROLL], w[UNROLL];
@@ -201,7 +209,7 @@ dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float 
       else load_tile<UNROLL>(w, in, blockIdx.x + (k + 1) * G, nchunks);
     }
 #pragma unroll
-    for (int u = 0; u < UNROLL; ++u) C::absmax(a, b, v[u]);
+    for (int u = 0; u < UNROLL; ++u) C::absmax(acc0, acc1, v[u]);
     if (k < kept) {
       uint4 *slot = kept_smem + (k - kRegTiles) * kTile + threadIdx.x;
 #pragma unroll
@@ -209,7 +217,7 @@ dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float 
     }
     if (second) {
 #pragma unroll
-      for (int u = 0; u < UNROLL; ++u) C::absmax(a, b, w[u]);
+      for (int u = 0; u < UNROLL; ++u) C::absmax(acc0, acc1, w[u]);
       if (k + 1 < kept) {
         uint4 *slot = kept_smem + (k + 1 - kRegTiles) * kTile + threadIdx.x;
 #pragma unroll
@@ -217,10 +225,11 @@ dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float 
       }
     }
   }
+  float a = C::finish(acc0, acc1);
   if (blockIdx.x == 0 && tail0 + threadIdx.x < numel) a = fmaxf(a, fabsf(C::load_one(in, tail0 + threadIdx.x)));
 
   // finish
-  const float block_value = block_max_nonneg(fmaxf(a, b), smem32, 0.0f);
+  const float block_value = block_max_nonneg(a, smem32, 0.0f);
   __shared__ float amax_shared;
   float amax;
   bool met;
@@ -260,12 +269,11 @@ dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float 
 
 // ---- cast phase alone ---------------------------------------------------------------------------------
 constexpr int kCastPrefetchTiles = 6;  // tiles per block asked of L2 while the block waits for the amax
-// BOUNDED: *amax_p is the maximum of this very input (no product can overflow).
-template <int IN, int OUT, int UNROLL, bool BOUNDED>
+template <int IN, int OUT, int UNROLL>
 __global__ void __launch_bounds__(kThreads, 2048 / kThreads)
 cast_with_amax_stream(const uint4 *__restrict__ in, uint8_t *__restrict__ out, const float *__restrict__ amax_p,
                       float *__restrict__ scale_out, float *__restrict__ amax_out, int64_t numel) {
-  using C = DsqChunk<IN, OUT, BOUNDED>;
+  using C = DsqChunk<IN, OUT>;
   pdl_launch_dependents();
   const int64_t nchunks = numel / C::kElems;
   constexpr int64_t kTile = int64_t(kThreads) * UNROLL;
@@ -419,7 +427,7 @@ int launch_fused(const void *in, void *out, float *amax_out, float *scale_out, i
     if (int e = launch_amax(in, &ws->amax, numel, IN, ws, dev, st)) return e;
     const int64_t tiles = ceil_div64(numel / C::kElems, int64_t(kThreads) * kUnroll);
     const int grid = balanced_grid(tiles, int64_t(dev.sm_count) * kCastBlocksPerSmCap);
-    return cuda_status(launch_after_dependency(cast_with_amax_stream<IN, OUT, kUnroll, true>, dim3(grid), dim3(kThreads),
+    return cuda_status(launch_after_dependency(cast_with_amax_stream<IN, OUT, kUnroll>, dim3(grid), dim3(kThreads),
                                                0, st, static_cast<const uint4 *>(in), o, &ws->amax, scale_out, amax_out,
                                                numel));
   }
@@ -442,7 +450,7 @@ int launch_cast(const void *in, void *out, const float *amax, float *scale_out, 
   if (aligned_to(in, 16) && aligned_to(out, C::kOutAlign)) {
     const int64_t tiles = ceil_div64(numel / C::kElems, int64_t(kThreads) * kUnroll);
     const int grid = balanced_grid(tiles, max_grid);
-    return cuda_status(launch_after_dependency(cast_with_amax_stream<IN, OUT, kUnroll, false>, dim3(grid),
+    return cuda_status(launch_after_dependency(cast_with_amax_stream<IN, OUT, kUnroll>, dim3(grid),
                                                dim3(kThreads), 0, st, static_cast<const uint4 *>(in), o, amax, scale_out,
                                                static_cast<float *>(nullptr), numel));
   } else {

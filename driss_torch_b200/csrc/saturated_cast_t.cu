@@ -95,7 +95,7 @@ struct DynCast<DTQ_BF16, OUT> {
   using Scale = DsqScale;
   __device__ static Scale load_scale(const float *amax) { return make_dsq_scale<OUT>(fmaxf(*amax, 0.0f)); }
   __device__ static float scale_value(const Scale &s) { return static_cast<float>(s.sd); }
-  __device__ static Bytes convert(uint4 v, const Scale &s) { return dsq_convert_bf16x8<OUT, false>(v, s); }
+  __device__ static Bytes convert(uint4 v, const Scale &s) { return dsq_convert_bf16x8<OUT>(v, s); }
   __device__ static uint8_t one(const void *in, int64_t i, const Scale &s) {
     return cvt_fp8<OUT>(dsq_mul(s.sd, __uint_as_float(uint32_t(static_cast<const uint16_t *>(in)[i]) << 16)));
   }
