@@ -29,6 +29,7 @@
 // abort flag, the roles drain what they have in flight, tensor memory is freed and the kernel returns.
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 
@@ -1426,35 +1427,43 @@ constexpr int kGemmSplit = DTQ_GEMM_NARROW + 1;  // only launch_gemm itself choo
 
 template <int MODE>
 int launch_gemm(const GemmCall &c, int kernel, const DeviceInfo &dev) {
-  // Which kernel: estimated time = a fixed part (launch, set-up, filling the pipeline, the last epilogue) plus
-  // rounds of tiles on the busiest SM x stages of 128 operand bytes along K x the time of such a stage, all in
-  // microseconds as measured on a B200 (steady state, 1.3 to 1.5 GHz under the power cap): the SM pair's
-  // 256 x 256 tile costs 0.36 per stage but 10 to start, a 128 x 256 tile 0.42 and 8, a 128 x 128 tile 0.30 and 6.
-  // So large problems run on SM pairs, and problems of a tile or two per SM on the narrow kernel, whose
-  // smaller tiles also spread a small output over more SMs.
+  // Which kernel: estimated time, in microseconds as measured on a B200 = a fixed part (launch, set-up, filling the
+  // pipeline, the last epilogue) plus, for every round of tiles on the busiest SM, the stages of 128 operand bytes along K
+  // at the time of one, and what a tile costs besides; a tile never takes less than its epilogue.
+  //   pair   256 x 256 tiles on SM pairs: 5.6 + rounds x max(0.333 stages + 0.6, 1.8; row-wise 2.2)
+  //   wide   128 x 256 on one SM: 4.2 + rounds x max(0.36 stages + 1.9, 2.6; row-wise 4.6), its epilogue not overlapped
+  //   narrow 128 x 128 on one SM: 3.2 + rounds x max(0.25 stages + 1.1, 1.5; row-wise 0.25 stages + 1.3, 2.4)
+  // So large problems run on SM pairs, and problems of about a tile per SM on the narrow kernel, whose smaller tiles also
+  // spread a small output over more SMs.  Measured, us, narrow / wide / pair: row-wise 512 x 4096 x 2048 8.9 / 12.0 / 10.7,
+  // 500 x 8192 x 1024 10.2 / 10.0 / 8.6, 1024 x 8192 x 2048 23.8 / 21.1 / 16.5, 16384 x 1024 x 1024 28.6 / 29.7 / 19.3;
+  // MXFP8 3000 x 1000 x 5120 25.5 / 18.9 / 19.6; MXFP4 1000 x 4096 x 512 6.1 / 6.5 / 6.5, 4096 x 4096 x 256 13.6 / 14.7 / 12.3.
+  // Over 26 shapes in each of the three modes the kernel chosen took at most 6 % longer than the quickest (before: 53 %).
   const int64_t m_tiles = ceil_div64(c.m, kBM);
   const double stages = static_cast<double>(ceil_div64(c.k_bytes, kBK));
-  const double wide = 8.0 + static_cast<double>(ceil_div64(m_tiles * ceil_div64(c.n, 256), dev.sm_count)) * stages * 0.42;
-  const double narrow = 6.0 + static_cast<double>(ceil_div64(m_tiles * ceil_div64(c.n, 128), dev.sm_count)) * stages * 0.30;
+  constexpr bool kRow = MODE == kRowwise;
+  auto rounds = [](int64_t tiles, int64_t slots) { return static_cast<double>(ceil_div64(tiles, slots)); };
+  const double wide = 4.2 + rounds(m_tiles * ceil_div64(c.n, 256), dev.sm_count) * std::max(0.36 * stages + 1.9, kRow ? 4.6 : 2.6);
+  const double narrow =
+      3.2 + rounds(m_tiles * ceil_div64(c.n, 128), dev.sm_count) * std::max(0.25 * stages + (kRow ? 1.3 : 1.1), kRow ? 2.4 : 1.5);
   int dev_id = 0, max_clusters = 0;
   DTQ_CUDA_TRY(cudaGetDevice(&dev_id));
   if (int e = pair_cluster_capacity<MODE>(dev_id, &max_clusters)) return e;
-  const double pair =
-      max_clusters > 0
-          ? 10.0 + static_cast<double>(ceil_div64(ceil_div64(c.m, 256) * ceil_div64(c.n, 256), max_clusters)) * stages * 0.36
-          : 1e30;
+  const double pair = max_clusters > 0 ? 5.6 + rounds(ceil_div64(c.m, 256) * ceil_div64(c.n, 256), max_clusters) *
+                                                   std::max(0.333 * stages + 0.6, kRow ? 2.2 : 1.8)
+                                       : 1e30;
   if (kernel == DTQ_GEMM_PAIR && max_clusters <= 0) return DTQ_ERR_CUDA_BASE + static_cast<int>(cudaErrorNotSupported);
-  // Few tiles and a long K: the split kernel, once it gets four CTAs per tile, or two where a tile is only 32 tokens wide.
-  // Measured split against the best of the others, us: four CTAs, row-wise 64 x 8192 x 4096 9.9 / 12.1, 128 x 4096 x 4096
-  // 10.3 / 12.4, 300 x 2048 x 8192 14.3 / 19.4, MXFP4 512 x 1024 x 8192 10.3 / 12.0; two CTAs, 16 x 16384 x 8192 24.0 / 27.0,
-  // MXFP4 16 x 8192 x 4096 6.7 / 9.2, but 512 x 4096 x 4096 14.3 / 13.4 and MXFP4 64 x 8192 x 4096 8.1 / 8.0; one CTA,
-  // 32 x 1024 x 1024 6.1 / 4.9.
+  // Few tiles and a long K: the split kernel, once it gets four CTAs per tile, or two where a tile is only 32 tokens wide or,
+  // with 32 stages of K or more, 64.  Measured split against the best of the others, us: four CTAs, row-wise 64 x 8192 x 4096
+  // 9.9 / 12.1, 128 x 4096 x 4096 10.3 / 12.4, 300 x 2048 x 8192 14.3 / 19.4, MXFP4 512 x 1024 x 8192 10.3 / 12.0; two CTAs,
+  // 16 x 16384 x 8192 24.0 / 27.0, 64 x 16384 x 8192 25.8 / 28.7, MXFP4 16 x 8192 x 4096 6.7 / 9.2, but 512 x 4096 x 4096
+  // 14.3 / 13.4 and MXFP4 64 x 8192 x 4096 8.1 / 8.0; one CTA, 32 x 1024 x 1024 6.1 / 4.9.
   if (kernel == DTQ_GEMM_AUTO) {
     const int64_t tiles = ceil_div64(c.n, 128) * ceil_div64(c.m, split_tokens(c.m));
-    if (split_count(tiles, ceil_div64(c.k_bytes, kBK), dev) >= (c.m <= 32 ? 2 : 4)) kernel = kGemmSplit;
+    const bool two_pay = c.m <= 32 || (c.m <= 64 && stages >= 32);
+    if (split_count(tiles, ceil_div64(c.k_bytes, kBK), dev) >= (two_pay ? 2 : 4)) kernel = kGemmSplit;
   }
   if (kernel == DTQ_GEMM_AUTO)
-    kernel = (pair <= wide && pair <= narrow) ? DTQ_GEMM_PAIR : (narrow < wide ? DTQ_GEMM_NARROW : DTQ_GEMM_WIDE);
+    kernel = (pair < wide && pair < narrow) ? DTQ_GEMM_PAIR : (narrow <= wide ? DTQ_GEMM_NARROW : DTQ_GEMM_WIDE);
   if (kernel == kGemmSplit) {
     switch (split_tokens(c.m)) {
       case 32: return launch_split<32, 5, MODE>(c, dev);
