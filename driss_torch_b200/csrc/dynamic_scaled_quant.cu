@@ -52,7 +52,8 @@ constexpr int kFusedRegTiles = 1;
 // Inputs above this many bytes are quantised as amax kernel + cast kernel instead of the single
 // fused launch: what the chip can keep between the two looks (about 140 MB) no longer matters at
 // that size, and the two stream kernels run at higher occupancy than the persistent fused one
-// (measured at 512 MiB: 199 us against 209 us; at 128 MiB the fused launch wins 48 us to 60 us).
+// (measured, bf16, fused / two launches: 128 MiB 44.8 / 49.5 us, 256 MiB 94.3 / 100.8, 320 MiB 118.3 / 120.2; fp32 320 MiB
+// 105.7 / 104.9).
 constexpr int64_t kFusedMaxBytes = int64_t(320) << 20;
 // The stand-alone cast kernel: one tile per block (no grid cap), see saturated_cast.cu.
 constexpr int kThreads = 256;
@@ -115,7 +116,7 @@ struct DsqChunk<DTQ_F32, OUT> {
 // policy, so that they survive the rest of the streaming traffic until phase 2 comes back for them (newest
 // first).  Measured on B200, 128 MiB input: 53.2 us without the hint, 52.6 / 50.9 / 50.0 / 49.3 us with
 // 32 / 48 / 64 / 80 MB, 49.8 us with every streamed tile marked (more than L2 holds: the marked lines evict
-// each other).
+// each other).  With the two-instruction product (dtq_device.cuh): 44.8 / 44.7 / 44.6 us with 64 / 80 / 100 MB.
 constexpr int64_t kFusedL2KeepMB = 80;
 
 template <int UNROLL>

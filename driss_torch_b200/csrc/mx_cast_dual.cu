@@ -18,7 +18,8 @@
 // shared loads), lanes l and l^1 together hold one MX block of each column; the eight lanes of a
 // column pair write 128 contiguous bytes of a row of the transposed payload.
 // Blocked scales: a tile's 128 rows x 4 blocks are exactly one 512-byte atom of either scale array, so both atoms are put
-// together in shared memory and leave as 16-byte stores, the zeros of the padding included.
+// together in shared memory and leave as 16-byte stores, the zeros of the padding included (8192 x 8192: 51.8 us with a
+// byte store and a division per scale, 46.7 now, 48.0 with row-major scales).
 // CTAs are numbered so that eight row tiles of one column tile run back to back, then the next
 // column tile: the 4-byte scale fragments that neighbouring tiles add to one 32-byte sector of
 // either scale array arrive close together in time.

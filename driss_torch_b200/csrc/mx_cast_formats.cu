@@ -165,7 +165,8 @@ mx_formats_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, u
   // A warp owns kUnrollF consecutive rows of 32 chunks, so that after the last of them every lane (every second one for
   // fp32) has one scale byte to place: with a scale per block placed by one lane of it in each step, finding the place
   // in the blocked layout (a division) ran four times as often, and 64 bits wide it was most of the kernel.
-  // Measured, MXFP4 with blocked scales: see mx_quantize_any.
+  // Measured, bf16 -> MXFP4 with blocked scales: 8192 x 8192 38.0 -> 26.9 us (row-major scales 24.7), 16384 x 8192
+  // 73.1 -> 53.2 (50.2); from fp32 129 -> 91.
   for (int64_t tile = blockIdx.x - pad_blocks; tile * kTile < nchunks; tile += gridDim.x) {
     const int64_t first = tile * kTile + int64_t(warp) * (32 * kUnrollF) + lane;
     uint4 v[kUnrollF];
