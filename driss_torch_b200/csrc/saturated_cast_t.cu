@@ -20,10 +20,9 @@
 // 16 rows, transposes its 4 x 4 byte blocks with byte permutes, and stores 16 contiguous bytes to
 // each of four rows of out_t; the eight lanes of a word column cover full 128-byte lines.
 // Any other number of rows (or alignment of out_t): the rows of out_t start at every byte offset, so no 16-byte store
-// fits.  The transposed tile goes through shared memory once more, and a warp writes one row segment of out_t (up to 128
-// bytes) at a time: each lane one aligned 4-byte word, cut out of two words of shared memory by a funnel shift, and up to
-// six single bytes for the ends.  That costs a quarter more than aligned rows, by the issue of those
-// stores (16 row segments per warp); launch_transposed has the figures.
+// fits as it is.  The transposed tile goes through shared memory once more, and a warp writes four row segments of out_t
+// (up to 128 bytes) at a time: eight lanes each, one aligned 16 bytes per lane, cut out of five words of shared memory by
+// funnel shifts, and single bytes for the ends.  launch_transposed has the figures.
 // Rows of input that are not 16-byte aligned, or few tiles of ragged rows: a 32 x 32 byte-tile kernel, one element per thread.
 #include "dtq_device.cuh"
 #include "dtq_host.h"
@@ -38,6 +37,7 @@ namespace {
 
 constexpr int kTileRows = 128;
 constexpr int kTileWords = 32;  // 32-bit words of fp8 bytes per shared-memory row (fp32 input uses 16 of them)
+constexpr int kRaggedPitch = 36;  // words between byte columns of the transposed tile when its rows start at any byte
 constexpr int kThreadsT = 256;
 constexpr int kRowPasses = kTileRows / 16;  // a pass of 8 warps covers 16 rows (2 per warp)
 
@@ -170,27 +170,34 @@ __device__ __forceinline__ void transposed_tile(uint32_t (&tile)[kTileRows][kTil
     t[3][k] = __byte_perm(a1, b1, 0x7632);
   }
   if constexpr (RAGGED) {
-    // the tile again, now as [byte column][row]: 32 words of rows per column
+    // the tile again, now as [byte column][row]: 32 words of rows per column, 36 words apart
     uint32_t *tile_t = &tile[0][0];
     __syncthreads();
     if (word < kRowWords) {
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        *reinterpret_cast<uint4 *>(tile_t + (word * 4 + j) * kTileWords + g * 4) = make_uint4(t[j][0], t[j][1], t[j][2], t[j][3]);
+        *reinterpret_cast<uint4 *>(tile_t + (word * 4 + j) * kRaggedPitch + g * 4) = make_uint4(t[j][0], t[j][1], t[j][2], t[j][3]);
     }
     __syncthreads();
     const int len = FULL ? kTileRows : static_cast<int>(min(rows - row0, int64_t(kTileRows)));
     const int ncols = FULL ? 4 * kRowWords : static_cast<int>(min(cols - col0, int64_t(4 * kRowWords)));
-    for (int cc = warp; cc < ncols; cc += kThreadsT / 32) {
+    // a warp takes four columns at a time, eight lanes each: lane l an aligned 16 bytes of the segment
+    const int l = lane & 7;
+    for (int cc = warp * 4 + (lane >> 3); cc < ncols; cc += kThreadsT / 8) {
       uint8_t *dst = out_t + (col0 + cc) * rows + row0;
-      const uint32_t *src = tile_t + cc * kTileWords;
-      const int head = min(static_cast<int>(-reinterpret_cast<uintptr_t>(dst) & 3), len);  // bytes before the first aligned word
-      const int words = (len - head) >> 2, tail = (len - head) & 3;
-      if (lane < words)
-        *reinterpret_cast<uint32_t *>(dst + head + 4 * lane) = __funnelshift_r(src[lane], src[(lane + 1) & 31], 8 * head);
-      if (lane < head + tail) {
-        const int i = lane < head ? lane : len - tail + lane - head;
-        dst[i] = reinterpret_cast<const uint8_t *>(src)[i];
+      const uint32_t *src = tile_t + cc * kRaggedPitch;
+      const int head = min(static_cast<int>(-reinterpret_cast<uintptr_t>(dst) & 15), len);  // bytes before the first aligned 16
+      const int vectors = (len - head) >> 4;
+      if (l < vectors) {
+        const int first = head + 16 * l, shift = 8 * (first & 3);
+        const uint32_t *p = src + (first >> 2);  // five words, the fifth only looked at when shift > 0
+        const uint32_t w0 = p[0], w1 = p[1], w2 = p[2], w3 = p[3], w4 = p[4];
+        *reinterpret_cast<uint4 *>(dst + first) = make_uint4(__funnelshift_r(w0, w1, shift), __funnelshift_r(w1, w2, shift),
+                                                             __funnelshift_r(w2, w3, shift), __funnelshift_r(w3, w4, shift));
+      }
+      for (int i = l; i < len - 16 * vectors; i += 8) {  // the ends
+        const int b = i < head ? i : i + 16 * vectors;
+        dst[b] = reinterpret_cast<const uint8_t *>(src)[b];
       }
     }
     return;
@@ -211,7 +218,8 @@ __global__ void __launch_bounds__(kThreadsT, kTransposedMinBlocks)
 cast_transposed_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, uint8_t *__restrict__ out_t,
                        const float *__restrict__ scale, float *__restrict__ scale_out, float *__restrict__ amax_out,
                        int64_t rows, int64_t cols, int64_t col_tiles) {
-  __shared__ __align__(16) uint32_t tile[kTileRows][kTileWords];
+  __shared__ __align__(16) uint32_t buffer[kTileRows * (RAGGED ? kRaggedPitch : kTileWords)];
+  uint32_t (&tile)[kTileRows][kTileWords] = *reinterpret_cast<uint32_t (*)[kTileRows][kTileWords]>(buffer);
   constexpr int kTileCols = 16 * C::kChunkElems;
   pdl_launch_dependents();
   pdl_wait();  // may have become resident under the tail of the kernel that delivers *scale
@@ -270,8 +278,10 @@ int launch_transposed(const void *in, void *out, void *out_t, const float *scale
   // Tiles where the input's rows can be read 16 bytes at a time; 16-byte stores of the transposed output where all its
   // rows start on 16 bytes, else the byte-shifted ones, unless there are fewer tiles than SMs: then the smaller tiles of
   // the byte kernel are quicker.  Measured, both orientations from bf16, byte tiles / shifted rows: 33 x 256 (2 tiles)
-  // 1.7 / 3.2 us, 333 x 1000 (24) 2.9 / 4.1, 40 x 8192 (64) 3.0 / 3.4, 1001 x 4096 (256) 8.8 / 7.3, 5003 x 4096
-  // (1280) 37.0 / 15.7, 16383 x 8192 232 / 112; 16384 x 8192 with aligned rows 88.
+  // 1.7 / 3.2 us, 333 x 1000 (24) 2.9 / 4.1, 40 x 8192 (64) 3.0 / 3.4, 1001 x 4096 (256) 8.8 / 6.9, 5003 x 4096
+  // (1280) 37.0 / 13.8, 16383 x 8192 232 / 115; with aligned rows 5008 x 4096 11.9, 16384 x 8192 88.  (One aligned word per
+  // lane and row segment instead of 16 bytes: 7.3, 15.5 and 112 us.  Row tiles fastest, so that neighbours share the sectors
+  // at their segments' ends while those are in L2: 7.2, 15.4 and 115.)
   const bool readable = cols % C::kChunkElems == 0 && aligned_to(in, 16) && (!BOTH || aligned_to(out, 8));
   const bool aligned_rows = rows % 16 == 0 && aligned_to(out_t, 16);
   DeviceInfo dev;
