@@ -26,7 +26,9 @@ struct alignas(256) Workspace {
   // into word b % 32) instead of publishing partials; a one-warp finishing launch takes them and
   // leaves zeros behind.
   unsigned int slot_max[32];
-  unsigned int pad[24];
+  // Limit of a wait in the GEMMs, in microseconds; 0, as initialised, is two seconds.  Tests shorten it to see one run out.
+  unsigned int wait_limit_us;
+  unsigned int pad[23];
   float partials[kMaxGridBlocks];
 };
 

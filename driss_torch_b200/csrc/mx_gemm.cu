@@ -82,7 +82,7 @@ struct GemmShape {
 };
 using WideShape = GemmShape<256, 4, 1>;
 using NarrowShape = GemmShape<128, 6, 2>;
-constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // a wait gives up after two seconds of wall time
+constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // a wait gives up after two seconds of wall time (Workspace::wait_limit_us)
 
 template <typename SH, int MODE>
 struct __align__(1024) GemmSmem {
@@ -94,6 +94,7 @@ struct __align__(1024) GemmSmem {
   uint64_t empty[SH::STAGES];
   uint64_t tmem_full[SH::ACC];
   uint64_t tmem_empty[SH::ACC];
+  uint64_t drained;  // only the way out of an abort commits to it: the others may still have commits on their way
   uint32_t tmem_base;
   int abort;
 };
@@ -126,9 +127,19 @@ __device__ __forceinline__ bool mbar_poll(uint32_t addr, unsigned parity) {
       : "memory");
   return done != 0;
 }
-// Bounded wait for the phase of the given parity: false if it has not completed after kWaitLimitNs of
-// wall time, or if the CTA is aborting (`abort` may be null for a wait that must not be cut short).
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, volatile int *abort) {
+// What every wait of a role looks at besides its barrier: the CTA's abort flag, and the caller's workspace, which holds
+// the limit and takes the status when a wait gives up.
+struct Bounds {
+  volatile int *abort;
+  Workspace *ws;
+  __device__ __forceinline__ void give_up() const {
+    atomicExch(&ws->status, DTQ_ERR_TIMEOUT);
+    *abort = 1;
+  }
+};
+// Bounded wait of one thread for the phase of the given parity: false if it has not completed within the limit of wall
+// time, or (`abort` not null) if the CTA is aborting.  Behind the two functions below, which the roles use.
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, volatile int *abort, const Workspace *ws) {
   const uint32_t addr = smem_addr(bar);
   if (mbar_poll(addr, parity)) return true;
   const unsigned long long start = global_ns();
@@ -136,14 +147,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, volati
     if (mbar_poll(addr, parity)) return true;
     if ((spins & 63u) == 0) {
       if (abort && *abort) return false;
-      if (global_ns() - start > kWaitLimitNs) return false;
+      const unsigned int us = ws ? *const_cast<const volatile unsigned int *>(&ws->wait_limit_us) : 0u;
+      if (global_ns() - start > (us ? us * 1000ull : kWaitLimitNs)) return false;
     }
   }
 }
-// The same wait by all lanes of a converged warp, with one answer for the warp.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, unsigned parity, volatile int *abort) {
-  return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort));
+// The wait of a role, by all lanes of a converged warp, with one answer for the warp: what follows it is warp-wide
+// (tcgen05.ld, shuffles, elect.sync), so no lane may leave on a flag that another lane has not seen.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, unsigned parity, const Bounds &b) {
+  return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, b.abort, b.ws));
 }
+// The wait of a single lane for its own copies or MMAs in flight on the way out; an abort does not cut it short.
+__device__ __forceinline__ void mbar_drain(uint64_t *bar, unsigned parity) { mbar_wait(bar, parity, nullptr, nullptr); }
 // True in one lane of a converged warp, the same lane every time.  The producer and the MMA issuer walk their
 // loops as whole warps and let the elected lane issue the asynchronous instructions: everything those
 // instructions take as operands (descriptors, coordinates, barrier addresses) is then the same in all lanes,
@@ -344,7 +359,7 @@ struct GemmParams {
   uint16_t *out;  // bf16 [M, N]
   int M, N, K;
   int m_tiles, n_tiles, k_stages;
-  int *status;
+  Workspace *ws;
 };
 
 template <typename SH, int MODE>
@@ -357,7 +372,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   GemmSmem<SH, MODE> &sm =
       *reinterpret_cast<GemmSmem<SH, MODE> *>(smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u));
   const int warp = int(warp_uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
-  volatile int *abort = &sm.abort;
+  const Bounds bounds{&sm.abort, p.ws};
   // Programmatic dependent launch, both ways: what is queued behind this kernel with that attribute may become
   // resident as this grid's CTAs leave, and this kernel's own set-up below (barriers, tensor memory, the tensor
   // maps in its parameters) may run under the tail of the kernel before it; nothing in global memory is touched
@@ -373,6 +388,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       mbar_init(&sm.tmem_full[i], 1);
       mbar_init(&sm.tmem_empty[i], kEpilogueWarps);
     }
+    mbar_init(&sm.drained, 1);
     sm.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -398,7 +414,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       tile_coords(tile, p.m_tiles, p.n_tiles, &mt, &nt);
       for (int ks = 0; ks < p.k_stages; ++ks) {
         // the MMAs that read this stage's previous contents (one pass ago) must have finished
-        if (!first_pass && !mbar_wait_warp(&sm.empty[stage], phase ^ 1u, abort)) {
+        if (!first_pass && !mbar_wait_warp(&sm.empty[stage], phase ^ 1u, bounds)) {
           ok = false;
           break;
         }
@@ -425,11 +441,10 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       // Give up, but not with copies on their way into this CTA's shared memory: wait (bounded) for the newest
       // copy of every stage (this pass's below `stage`, the previous pass's from there on); they complete
       // without anybody's help.
-      atomicExch(p.status, DTQ_ERR_TIMEOUT);
-      *abort = 1;
+      bounds.give_up();
       for (uint32_t j = 0; j < uint32_t(kStagesG); ++j) {
-        if (j < stage) mbar_wait(&sm.full[j], phase, nullptr);
-        else if (!first_pass) mbar_wait(&sm.full[j], phase ^ 1u, nullptr);
+        if (j < stage) mbar_drain(&sm.full[j], phase);
+        else if (!first_pass) mbar_drain(&sm.full[j], phase ^ 1u);
       }
     }
   } else if (warp == 1) {
@@ -440,14 +455,14 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++local_tile) {
       // the epilogue must have taken this accumulator's previous tile out of tensor memory
       const int acc = local_tile % kAcc, use = local_tile / kAcc;
-      if (use > 0 && !mbar_wait_warp(&sm.tmem_empty[acc], (use - 1) & 1u, abort)) {
+      if (use > 0 && !mbar_wait_warp(&sm.tmem_empty[acc], (use - 1) & 1u, bounds)) {
         ok = false;
         break;
       }
       tmem_fence_after();
       const uint32_t d_tmem = tmem + uint32_t(acc * kBN);
       for (int ks = 0; ks < p.k_stages; ++ks) {
-        if (!mbar_wait_warp(&sm.full[stage], phase, abort)) {
+        if (!mbar_wait_warp(&sm.full[stage], phase, bounds)) {
           ok = false;
           break;
         }
@@ -487,8 +502,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       __syncwarp();
     }
     if (!ok && lane == 0) {
-      atomicExch(p.status, DTQ_ERR_TIMEOUT);
-      *abort = 1;
+      bounds.give_up();
     }
   } else {
     // ---- epilogue: 8 warps; warp w reads lanes 32 (w % 4) .. + 31, column half (w - 2) / 4 -------------------
@@ -503,10 +517,9 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       RowwiseRegs<kChunks> rw;
       if constexpr (MODE == kRowwise)
         load_rowwise<kChunks>(rw, p.rowwise, row, int64_t(nt) * kBN + half * kHalfCols, lane, p.M, p.N);
-      if (!mbar_wait(&sm.tmem_full[acc], use & 1u, abort)) {
+      if (!mbar_wait_warp(&sm.tmem_full[acc], use & 1u, bounds)) {
         if (lane == 0) {
-          atomicExch(p.status, DTQ_ERR_TIMEOUT);
-          *abort = 1;
+          bounds.give_up();
         }
         break;
       }
@@ -551,12 +564,10 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   tmem_fence_before();
   __syncthreads();
   if (warp == 1) {
-    if (*abort && elect_one()) {  // the lane that issued the MMAs: a commit follows the issuing thread's own
+    if (*bounds.abort && elect_one()) {  // the lane that issued the MMAs: a commit follows the issuing thread's own
       // MMAs may still be in flight: a commit that arrives on a barrier nobody else uses, and a bounded wait for it
-      mbar_init(&sm.tmem_full[0], 1);
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-      umma_commit(&sm.tmem_full[0]);
-      mbar_wait(&sm.tmem_full[0], 0u, nullptr);
+      umma_commit(&sm.drained);
+      mbar_drain(&sm.drained, 0u);
     }
     __syncwarp();
     tmem_fence_after();
@@ -681,7 +692,7 @@ struct PairParams {
   RowwiseEpilogue rowwise;
   int M, N;
   int m_pairs, n_tiles, k_stages;  // 256-row tile rows, 256-column tile columns, 128-byte K stages
-  int *status;
+  Workspace *ws;
 };
 
 template <int MODE>
@@ -696,7 +707,7 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const uint32_t rank = warp_uniform(cluster_ctarank());  // 0 = leader
   const bool leader = rank == 0;
   const uint32_t peer = rank ^ 1u;
-  volatile int *abort = &sm.abort;
+  const Bounds bounds{&sm.abort, p.ws};
   const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
   const int total_tiles = p.m_pairs * p.n_tiles;
   pdl_launch_dependents();  // as in the single-CTA kernel
@@ -734,7 +745,7 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       int mp, nt;
       tile_coords(tile, p.m_pairs, p.n_tiles, &mp, &nt);
       for (int ks = 0; ks < p.k_stages; ++ks) {
-        if (!first_pass && !mbar_wait_warp(&sm.empty[stage], phase ^ 1u, abort)) {
+        if (!first_pass && !mbar_wait_warp(&sm.empty[stage], phase ^ 1u, bounds)) {
           ok = false;
           break;
         }
@@ -759,8 +770,7 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       }
     }
     if (!ok && lane == 0) {
-      atomicExch(p.status, DTQ_ERR_TIMEOUT);
-      *abort = 1;
+      bounds.give_up();
       st_cluster_u32(map_to_cta(smem_addr(&sm.abort), peer), 1u);
     }
   } else if (warp == 1) {
@@ -774,14 +784,14 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         // tiles ago); separate accumulators: for the tile two before this one
         constexpr int kBack = PairTmem<MODE>::kShared ? 1 : 2;
         const int before = local_tile - kBack;
-        if (before >= 0 && !mbar_wait_warp(&sm.tmem_empty[before & 1], (before >> 1) & 1u, abort)) {
+        if (before >= 0 && !mbar_wait_warp(&sm.tmem_empty[before & 1], (before >> 1) & 1u, bounds)) {
           ok = false;
           break;
         }
         tmem_fence_after();
         const uint32_t d_tmem = tmem + ((local_tile & 1) ? PairTmem<MODE>::kAcc1 : 0);
         for (int ks = 0; ks < p.k_stages; ++ks) {
-          if (!mbar_wait_warp(&sm.full[stage], phase, abort)) {
+          if (!mbar_wait_warp(&sm.full[stage], phase, bounds)) {
             ok = false;
             break;
           }
@@ -820,8 +830,7 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         __syncwarp();
       }
       if (!ok && lane == 0) {
-        atomicExch(p.status, DTQ_ERR_TIMEOUT);
-        *abort = 1;
+        bounds.give_up();
         st_cluster_u32(map_to_cta(smem_addr(&sm.abort), peer), 1u);
       }
     }
@@ -857,10 +866,9 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
         __syncwarp();
       }
-      if (!mbar_wait(&sm.tmem_full[acc], (local_tile >> 1) & 1u, abort)) {
+      if (!mbar_wait_warp(&sm.tmem_full[acc], (local_tile >> 1) & 1u, bounds)) {
         if (lane == 0) {
-          atomicExch(p.status, DTQ_ERR_TIMEOUT);
-          *abort = 1;
+          bounds.give_up();
           st_cluster_u32(map_to_cta(smem_addr(&sm.abort), peer), 1u);
         }
         break;
@@ -909,7 +917,7 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   // whoever gave up has already raised both CTAs' abort flags
   tmem_fence_before();
   __syncthreads();
-  if (*abort) {
+  if (*bounds.abort) {
     // Copies and MMAs may still be in flight into or out of this CTA's memories.  Loads complete by themselves
     // within microseconds and the leader's MMAs within a tile's time; neither CTA leaves before the other
     // (cluster barrier below), and a short sleep here covers what was issued last.
@@ -951,6 +959,7 @@ struct __align__(1024) SplitSmem {
   uint64_t full[STAGES];
   uint64_t empty[STAGES];
   uint64_t tmem_full;
+  uint64_t drained;  // as in GemmSmem
   uint32_t tmem_base;
   int abort;
 };
@@ -960,7 +969,7 @@ struct SplitParams {
   uint16_t *out;  // bf16 [M, N]
   int M, N;
   int n_tiles, k_stages, splits;  // 128-column tiles of the output, 128-byte K stages, CTAs per cluster
-  int *status;
+  Workspace *ws;
 };
 
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
@@ -986,7 +995,7 @@ mx_gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   Smem &sm = *reinterpret_cast<Smem *>(smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u));
   const int warp = int(warp_uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int rank = int(warp_uniform(cluster_ctarank()));
-  volatile int *abort = &sm.abort;
+  const Bounds bounds{&sm.abort, p.ws};
   const int tile = blockIdx.x / p.splits;
   const int nt = tile % p.n_tiles, tt = tile / p.n_tiles;
   const int k0 = int(int64_t(p.k_stages) * rank / p.splits), k1 = int(int64_t(p.k_stages) * (rank + 1) / p.splits);
@@ -997,6 +1006,7 @@ mx_gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       mbar_init(&sm.empty[s], 1);
     }
     mbar_init(&sm.tmem_full, 1);
+    mbar_init(&sm.drained, 1);
     sm.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     for (int ks = k0; ks < k1 && ks < k0 + kSplitPrefetch; ++ks) tma_prefetch_2d(&map_w, ks * kBK, nt * kBM);
@@ -1019,7 +1029,7 @@ mx_gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     uint32_t stage = 0, phase = 0;
     bool first_pass = true, ok = true;
     for (int ks = k0; ks < k1; ++ks) {
-      if (!first_pass && !mbar_wait_warp(&sm.empty[stage], phase ^ 1u, abort)) {
+      if (!first_pass && !mbar_wait_warp(&sm.empty[stage], phase ^ 1u, bounds)) {
         ok = false;
         break;
       }
@@ -1040,11 +1050,10 @@ mx_gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       }
     }
     if (!ok && lane == 0) {  // as in the single-CTA kernel: no copies left on their way when the CTA leaves
-      atomicExch(p.status, DTQ_ERR_TIMEOUT);
-      *abort = 1;
+      bounds.give_up();
       for (uint32_t j = 0; j < uint32_t(STAGES); ++j) {
-        if (j < stage) mbar_wait(&sm.full[j], phase, nullptr);
-        else if (!first_pass) mbar_wait(&sm.full[j], phase ^ 1u, nullptr);
+        if (j < stage) mbar_drain(&sm.full[j], phase);
+        else if (!first_pass) mbar_drain(&sm.full[j], phase ^ 1u);
       }
     }
   } else if (warp == 1) {
@@ -1052,7 +1061,7 @@ mx_gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     uint32_t stage = 0, phase = 0;
     bool ok = true;
     for (int ks = k0; ks < k1; ++ks) {
-      if (!mbar_wait_warp(&sm.full[stage], phase, abort)) {
+      if (!mbar_wait_warp(&sm.full[stage], phase, bounds)) {
         ok = false;
         break;
       }
@@ -1085,8 +1094,7 @@ mx_gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     if (ok && elect_one()) umma_commit(&sm.tmem_full);
     __syncwarp();
     if (!ok && lane == 0) {
-      atomicExch(p.status, DTQ_ERR_TIMEOUT);
-      *abort = 1;
+      bounds.give_up();
     }
   }
 
@@ -1114,10 +1122,9 @@ mx_gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   if (warp >= 2) {
     const int quad = warp & 3;  // the quarter of tensor memory that this warp can read
     // the barrier completes when all MMAs have, so nothing reads the stage buffers any more
-    if (!mbar_wait(&sm.tmem_full, 0u, abort)) {
+    if (!mbar_wait_warp(&sm.tmem_full, 0u, bounds)) {
       if (lane == 0) {
-        atomicExch(p.status, DTQ_ERR_TIMEOUT);
-        *abort = 1;
+        bounds.give_up();
       }
     } else {
       tmem_fence_after();
@@ -1139,7 +1146,7 @@ mx_gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   cluster_sync_all();
 
   // ---- sum over the cluster: token t by CTA t % splits, a warp per token, four outputs per lane --------------
-  if (!*abort) {
+  if (!*bounds.abort) {
     for (int t = rank + p.splits * warp; t < live; t += p.splits * kSplitWarps) {
       const uint32_t mine = smem_addr(partial + t * kBM + lane * 4);
       float4 part[kMaxSplits];
@@ -1164,11 +1171,9 @@ mx_gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     }
   }
   __syncwarp();
-  if (warp == 1 && *abort && elect_one()) {  // MMAs may still be in flight: wait (bounded) for them, as in the single-CTA kernel
-    mbar_init(&sm.tmem_full, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    umma_commit(&sm.tmem_full);
-    mbar_wait(&sm.tmem_full, 0u, nullptr);
+  if (warp == 1 && *bounds.abort && elect_one()) {  // MMAs may still be in flight: wait (bounded) for them, as in the single-CTA kernel
+    umma_commit(&sm.drained);
+    mbar_drain(&sm.drained, 0u);
   }
   __syncwarp();
   cluster_sync_all();  // nobody leaves while another CTA may still read its partial sums
@@ -1292,13 +1297,13 @@ int pair_cluster_capacity(int dev_id, int *max_clusters) {
   return DTQ_OK;
 }
 
-// What every launcher needs: operand pointers, sizes (k_bytes = bytes per operand row), where the status word is.
+// What every launcher needs: operand pointers, sizes (k_bytes = bytes per operand row), the caller's workspace.
 struct GemmCall {
   RowwiseEpilogue rowwise;  // all zero for the block-scaled modes
   const void *a, *b, *sfa, *sfb;
   void *out;
   int64_t m, n, k_bytes, katoms;
-  int *status;
+  Workspace *ws;
   cudaStream_t st;
 };
 
@@ -1327,7 +1332,7 @@ int launch_pair(const GemmCall &c, int max_clusters) {
   p.m_pairs = static_cast<int>(ceil_div64(c.m, 256));
   p.n_tiles = static_cast<int>(ceil_div64(c.n, kPairBN));
   p.k_stages = static_cast<int>(ceil_div64(c.k_bytes, kBK));
-  p.status = c.status;
+  p.ws = c.ws;
   const int64_t tiles = int64_t(p.m_pairs) * p.n_tiles;
   const int clusters = static_cast<int>(tiles < max_clusters ? tiles : max_clusters);
   cudaLaunchConfig_t cfg;
@@ -1367,7 +1372,7 @@ int launch_shape(const GemmCall &c, const DeviceInfo &dev) {
   p.m_tiles = static_cast<int>(ceil_div64(c.m, kBM));
   p.n_tiles = static_cast<int>(ceil_div64(c.n, SH::BN));
   p.k_stages = static_cast<int>(ceil_div64(c.k_bytes, kBK));
-  p.status = c.status;
+  p.ws = c.ws;
   const int64_t tiles = int64_t(p.m_tiles) * p.n_tiles;
   const int grid = static_cast<int>(tiles < dev.sm_count ? tiles : dev.sm_count);
   return cuda_status(launch_after_dependency(mx_gemm_kernel<SH, MODE>, dim3(grid), dim3(kGemmThreads), size_t(smem), c.st, map_a,
@@ -1414,7 +1419,7 @@ int launch_split(const GemmCall &c, const DeviceInfo &dev) {
   p.N = static_cast<int>(c.n);
   p.n_tiles = static_cast<int>(ceil_div64(c.n, kBM));
   p.k_stages = static_cast<int>(ceil_div64(c.k_bytes, kBK));
-  p.status = c.status;
+  p.ws = c.ws;
   const int64_t tiles = int64_t(p.n_tiles) * ceil_div64(c.m, BN);
   p.splits = split_count(tiles, p.k_stages, dev);
   cudaLaunchConfig_t cfg;
@@ -1514,7 +1519,7 @@ extern "C" int dtq_mx_gemm_bf16(const void *a, const void *b, const void *a_scal
   c.n = n;
   c.k_bytes = elem_format == DTQ_E2M1 ? k / 2 : k;
   c.katoms = ceil_div64(k / 32, 4);
-  c.status = &static_cast<Workspace *>(workspace)->status;
+  c.ws = static_cast<Workspace *>(workspace);
   c.st = st;
   return elem_format == DTQ_E2M1 ? launch_gemm<kMxFp4>(c, kernel, dev) : launch_gemm<kMxFp8>(c, kernel, dev);
 }
@@ -1550,7 +1555,7 @@ extern "C" int dtq_rowwise_fp8_bf16(const void *a, const void *b, const float *a
   c.n = n;
   c.k_bytes = k;
   c.katoms = 0;
-  c.status = &static_cast<Workspace *>(workspace)->status;
+  c.ws = static_cast<Workspace *>(workspace);
   c.st = static_cast<cudaStream_t>(stream);
   return launch_gemm<kRowwise>(c, kernel, dev);
 }

@@ -312,3 +312,49 @@ def test_few_tiles_split_along_k(tokens, n, kb, mode):
         kb = kb // 32 * 32
     _check_exact_on_device(mode, tokens, n, kb * 2 if mode == "mx4" else kb, "auto",
                            a_dtype=torch.float8_e5m2 if tokens % 2 else E4M3, bias=[None, torch.float32, torch.bfloat16][tokens % 3])
+
+
+# ---- the way out of a wait that runs out ---------------------------------------------------------------------------
+
+def test_waits_of_the_gemm_roles_are_warp_wide():
+    # What follows a role's wait is warp-wide (tcgen05.ld, elect.sync), and an abort flag raised between two lanes' polls
+    # would split a warp that polls lane by lane.  So nothing but the two wrappers calls the per-thread wait.
+    import re
+    from pathlib import Path
+
+    source = (Path(__file__).resolve().parents[1] / "driss_torch_b200" / "csrc" / "mx_gemm.cu").read_text()
+    calls = re.findall(r"^.*\bmbar_wait\(.*$", source, flags=re.M)
+    assert len(calls) == 3, calls  # its definition and the two wrappers
+    # and the barrier that the way out waits for is committed to by nobody else
+    assert len(re.findall(r"umma_commit\(&sm\.drained\)", source)) == len(re.findall(r"mbar_drain\(&sm\.drained", source)) == 2
+
+
+_WAIT_LIMIT_WORD = 40  # Workspace::wait_limit_us, csrc/dtq_host.h
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["mx8", "rowwise"])
+@pytest.mark.parametrize("kernel,m,n,k", [("pair", 256, 256, 1 << 18), ("wide", 256, 256, 1 << 18), ("narrow", 256, 256, 1 << 18),
+                                          ("auto", 32, 128, 1 << 21)])  # split along K
+def test_a_wait_that_runs_out_is_reported_and_stores_nothing(mode, kernel, m, n, k):
+    # a sound launch whose epilogue waits hundreds of microseconds for its accumulator, under a limit of one
+    from driss_torch_b200 import _cabi
+
+    a, b = (torch.zeros(rows, k, dtype=torch.uint8, device="cuda").view(E4M3) for rows in (m, n))
+
+    def run(ws):
+        out = torch.full((m, n), 7.0, dtype=torch.bfloat16, device="cuda")
+        if mode == "rowwise":
+            _cabi.rowwise_fp8_bf16(a, b, torch.ones(m, device="cuda"), torch.ones(n, device="cuda"), out=out, ws=ws, kernel=kernel)
+        else:
+            sa, sb = (torch.full((_cabi.load().dtq_mx_gemm_scale_bytes(rows, k),), 127, dtype=torch.uint8, device="cuda") for rows in (m, n))
+            _cabi.mx_fp8_bf16(a, b, sa, sb, out=out, ws=ws, kernel=kernel)
+        return out
+
+    ws = torch.zeros(_cabi.load().dtq_workspace_bytes(), dtype=torch.uint8, device="cuda")
+    ws.view(torch.int32)[_WAIT_LIMIT_WORD] = 1
+    out = run(ws)
+    assert _cabi.workspace_status(ws) == 5  # DTQ_ERR_TIMEOUT
+    assert (out == 7.0).all()
+    ws = torch.zeros_like(ws)  # the context is as good as before
+    assert (run(ws) == 0.0).all() and _cabi.workspace_status(ws) == 0
