@@ -977,6 +977,11 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
   return v;
 }
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t cluster_addr) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap *map, int x, int y) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y)
                : "memory");
@@ -1146,29 +1151,31 @@ mx_gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   cluster_sync_all();
 
   // ---- sum over the cluster: token t by CTA t % splits, a warp per token, four outputs per lane --------------
-  if (!*bounds.abort) {
-    for (int t = rank + p.splits * warp; t < live; t += p.splits * kSplitWarps) {
-      const uint32_t mine = smem_addr(partial + t * kBM + lane * 4);
-      float4 part[kMaxSplits];
+  // A CTA that gave up has operand bytes where its partial sums should be: if there is one, nobody in the cluster stores.
+  // Lane j asks CTA j, and the answer is looked at behind the first loads of partial sums.
+  const uint32_t gave_up = lane < p.splits ? ld_cluster_u32(map_to_cta(smem_addr(&sm.abort), lane)) : 0u;
+  for (int t = rank + p.splits * warp; t < live; t += p.splits * kSplitWarps) {
+    const uint32_t mine = smem_addr(partial + t * kBM + lane * 4);
+    float4 part[kMaxSplits];
 #pragma unroll
-      for (int j = 0; j < kMaxSplits; ++j)
-        if (j < p.splits) part[j] = ld_cluster_f4(map_to_cta(mine, j));
-      float4 f = part[0];
+    for (int j = 0; j < kMaxSplits; ++j)
+      if (j < p.splits) part[j] = ld_cluster_f4(map_to_cta(mine, j));
+    if (__any_sync(0xFFFFFFFFu, gave_up != 0)) break;
+    float4 f = part[0];
 #pragma unroll
-      for (int j = 1; j < kMaxSplits; ++j)
-        if (j < p.splits) f = make_float4(f.x + part[j].x, f.y + part[j].y, f.z + part[j].z, f.w + part[j].w);
-      const int64_t row = int64_t(tt) * BN + t;
-      if constexpr (MODE == kRowwise) {  // the same steps as apply_rowwise
-        const float xs = __ldg(p.rowwise.row_scale + row);
-        f = make_float4(__fmul_rn(__fmul_rn(f.x, xs), cs.x), __fmul_rn(__fmul_rn(f.y, xs), cs.y), __fmul_rn(__fmul_rn(f.z, xs), cs.z),
-                        __fmul_rn(__fmul_rn(f.w, xs), cs.w));
-        if (p.rowwise.bias)
-          f = make_float4(__fadd_rn(f.x, bs.x), __fadd_rn(f.y, bs.y), __fadd_rn(f.z, bs.z), __fadd_rn(f.w, bs.w));
-      }
-      if (n_live)
-        stg_stream(p.out + row * p.N + n0,
-                   make_uint2(pack_bf16(__float_as_uint(f.x), __float_as_uint(f.y)), pack_bf16(__float_as_uint(f.z), __float_as_uint(f.w))));
+    for (int j = 1; j < kMaxSplits; ++j)
+      if (j < p.splits) f = make_float4(f.x + part[j].x, f.y + part[j].y, f.z + part[j].z, f.w + part[j].w);
+    const int64_t row = int64_t(tt) * BN + t;
+    if constexpr (MODE == kRowwise) {  // the same steps as apply_rowwise
+      const float xs = __ldg(p.rowwise.row_scale + row);
+      f = make_float4(__fmul_rn(__fmul_rn(f.x, xs), cs.x), __fmul_rn(__fmul_rn(f.y, xs), cs.y), __fmul_rn(__fmul_rn(f.z, xs), cs.z),
+                      __fmul_rn(__fmul_rn(f.w, xs), cs.w));
+      if (p.rowwise.bias)
+        f = make_float4(__fadd_rn(f.x, bs.x), __fadd_rn(f.y, bs.y), __fadd_rn(f.z, bs.z), __fadd_rn(f.w, bs.w));
     }
+    if (n_live)
+      stg_stream(p.out + row * p.N + n0,
+                 make_uint2(pack_bf16(__float_as_uint(f.x), __float_as_uint(f.y)), pack_bf16(__float_as_uint(f.z), __float_as_uint(f.w))));
   }
   __syncwarp();
   if (warp == 1 && *bounds.abort && elect_one()) {  // MMAs may still be in flight: wait (bounded) for them, as in the single-CTA kernel

@@ -329,6 +329,18 @@ def test_waits_of_the_gemm_roles_are_warp_wide():
     assert len(re.findall(r"umma_commit\(&sm\.drained\)", source)) == len(re.findall(r"mbar_drain\(&sm\.drained", source)) == 2
 
 
+def test_split_kernel_stores_only_if_no_cta_of_the_cluster_gave_up():
+    # The abort flag is a CTA's own.  Every CTA adds up and stores all CTAs' partial sums of its tokens, so the flags of
+    # all of them have to be asked for between the cluster barrier behind the partial sums and the stores.
+    from pathlib import Path
+
+    source = (Path(__file__).resolve().parents[1] / "driss_torch_b200" / "csrc" / "mx_gemm.cu").read_text()
+    body = source[source.index("\nmx_gemm_split_kernel("):source.index("// ---- host side")]
+    barrier, store = body.index("cluster_sync_all();"), body.index("stg_stream(p.out")
+    assert "ld_cluster_u32(map_to_cta(smem_addr(&sm.abort), lane))" in body[barrier:store]
+    assert "if (__any_sync(0xFFFFFFFFu, gave_up != 0)) break;" in body[barrier:store]
+
+
 _WAIT_LIMIT_WORD = 40  # Workspace::wait_limit_us, csrc/dtq_host.h
 
 
