@@ -100,7 +100,11 @@ def mx_fp8_bf16(a: Tensor, b: Tensor, a_scale: Tensor, b_scale: Tensor) -> Tenso
     """Matrix multiplication of two MX-quantised e4m3 operands with E8M0 scales of 32 elements along K
     (driss_torch/__init__.py:80-95): ``a`` [M, K] row-major, ``b`` [K, N] column-major (``w.t()`` of a
     row-major [N, K] payload), ``a_scale`` / ``b_scale`` in the blocked layout ``mx_fp8_quantize_blocked``
-    writes; returns bf16 [M, N]."""
+    writes; returns bf16 [M, N].
+
+    The bits are those of the straight sum over K, except for few rows and a long K, where K is split and the parts'
+    fp32 sums are added in order: there a row's result may differ in the last bit from the same row's in a larger batch
+    (``DTQ_GEMM_AUTO`` in ``include/dtq_b200.h`` has the rule, and the kernels that a C caller can name instead)."""
     return ops.mx_fp8_bf16(a, b, a_scale, b_scale)
 
 
@@ -122,7 +126,8 @@ def sweep_mm(
     row-major, ``w`` [K, N] e4m3 column-major, ``x_scale`` [M, 1] and ``w_scale`` [1, N] fp32 dequantisation scales
     (the reciprocals of ``dynamic_scaled_quant_rowwise``'s), optional ``bias`` [N]; returns
     ``bf16((acc * x_scale) * w_scale + bias)``.  The arguments after ``out_dtype`` tune the reference's Hopper
-    kernels and have no effect here."""
+    kernels and have no effect here.  For few rows and a long K the last bit may depend on the number of rows, see
+    ``mx_fp8_bf16``."""
     return ops.sweep_mm(x, w, x_scale, w_scale, bias, out_dtype, use_fast_accum, cluster_shape_x, cluster_shape_y,
                         cluster_shape_z, transposed, swizzle)
 
@@ -131,7 +136,8 @@ def mx_fp4_bf16(a: Tensor, b: Tensor, a_scale: Tensor, b_scale: Tensor) -> Tenso
     """Matrix multiplication of two MXFP4 operands (e2m1 values packed two per byte, the lower index in the low
     nibble; E8M0 scales of 32 elements along K, blocked layout) (driss_torch/__init__.py:98-111): ``a`` [M, K/2]
     bytes row-major, ``b`` [K/2, N] column-major (``w.t()`` of a row-major [N, K/2] payload); returns bf16 [M, N].
-    ``mx_fp4_quantize(x, blocked=True)`` produces the payloads and the scales in that layout."""
+    ``mx_fp4_quantize(x, blocked=True)`` produces the payloads and the scales in that layout.  For few rows and a long K
+    the last bit may depend on the number of rows, see ``mx_fp8_bf16``."""
     return ops.mx_fp4_bf16(a, b, a_scale, b_scale)
 
 

@@ -368,14 +368,14 @@ def dynamic_scaled_quant_dual(x, out_dtype, out=None, out_t=None, amax_out=None,
     return out, out_t
 
 
-GEMM_KERNELS = {"auto": 0, "pair": 1, "wide": 2, "narrow": 3}
+GEMM_KERNELS = {"auto": 0, "pair": 1, "wide": 2, "narrow": 3, "split": 4}
 
 
 @_on_device_of_first_tensor
 def mx_fp8_bf16(a, b_nk, a_scale_blocked, b_scale_blocked, out=None, ws=None, kernel="auto", fp4=False):
     """MX block-scaled GEMM: ``a`` [M, K] e4m3, ``b_nk`` [N, K] e4m3 (the memory of the reference's column-major
     [K, N] operand), blocked E8M0 scales -> bf16 [M, N].  ``fp4``: the operands are packed e2m1 bytes, [M, K/2] and
-    [N, K/2].  ``kernel``: "auto", or one of "pair", "wide", "narrow"."""
+    [N, K/2].  ``kernel``: "auto", or one of "pair", "wide", "narrow" (the same bits each) and "split" (parts of K)."""
     m = a.shape[0]
     k = a.shape[1] * (2 if fp4 else 1)
     n = b_nk.shape[0]

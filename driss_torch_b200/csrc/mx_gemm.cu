@@ -1435,8 +1435,6 @@ int launch_split(const GemmCall &c, const DeviceInfo &dev) {
   return cuda_status(cudaLaunchKernelEx(&cfg, mx_gemm_split_kernel<BN, STAGES, MODE>, map_w, map_x, map_sfw, map_sfx, p));
 }
 
-constexpr int kGemmSplit = DTQ_GEMM_NARROW + 1;  // only launch_gemm itself chooses it
-
 template <int MODE>
 int launch_gemm(const GemmCall &c, int kernel, const DeviceInfo &dev) {
   // Which kernel: estimated time, in microseconds as measured on a B200 = a fixed part (launch, set-up, filling the
@@ -1469,14 +1467,15 @@ int launch_gemm(const GemmCall &c, int kernel, const DeviceInfo &dev) {
   // 9.9 / 12.1, 128 x 4096 x 4096 10.3 / 12.4, 300 x 2048 x 8192 14.3 / 19.4, MXFP4 512 x 1024 x 8192 10.3 / 12.0; two CTAs,
   // 16 x 16384 x 8192 24.0 / 27.0, 64 x 16384 x 8192 25.8 / 28.7, MXFP4 16 x 8192 x 4096 6.7 / 9.2, but 512 x 4096 x 4096
   // 14.3 / 13.4 and MXFP4 64 x 8192 x 4096 8.1 / 8.0; one CTA, 32 x 1024 x 1024 6.1 / 4.9.
+  const int splits = split_count(ceil_div64(c.n, 128) * ceil_div64(c.m, split_tokens(c.m)), ceil_div64(c.k_bytes, kBK), dev);
   if (kernel == DTQ_GEMM_AUTO) {
-    const int64_t tiles = ceil_div64(c.n, 128) * ceil_div64(c.m, split_tokens(c.m));
     const bool two_pay = c.m <= 32 || (c.m <= 64 && stages >= 32);
-    if (split_count(tiles, ceil_div64(c.k_bytes, kBK), dev) >= (two_pay ? 2 : 4)) kernel = kGemmSplit;
+    if (splits >= (two_pay ? 2 : 4)) kernel = DTQ_GEMM_SPLIT;
   }
   if (kernel == DTQ_GEMM_AUTO)
     kernel = (pair < wide && pair < narrow) ? DTQ_GEMM_PAIR : (narrow <= wide ? DTQ_GEMM_NARROW : DTQ_GEMM_WIDE);
-  if (kernel == kGemmSplit) {
+  if (kernel == DTQ_GEMM_SPLIT) {
+    if (splits < 2) return DTQ_ERR_SHAPE;  // named, but too many tiles or too little of K to split anything
     switch (split_tokens(c.m)) {
       case 32: return launch_split<32, 5, MODE>(c, dev);
       case 64: return launch_split<64, 4, MODE>(c, dev);
@@ -1502,7 +1501,7 @@ extern "C" int dtq_mx_gemm_bf16(const void *a, const void *b, const void *a_scal
   using namespace dtq;
   if (m < 0 || n < 0 || k < 0) return DTQ_ERR_INVALID_ARGUMENT;
   if (elem_format != DTQ_E4M3 && elem_format != DTQ_E2M1) return DTQ_ERR_UNSUPPORTED_DTYPE;
-  if (kernel < DTQ_GEMM_AUTO || kernel > DTQ_GEMM_NARROW) return DTQ_ERR_INVALID_ARGUMENT;
+  if (kernel < DTQ_GEMM_AUTO || kernel > DTQ_GEMM_SPLIT) return DTQ_ERR_INVALID_ARGUMENT;
   if (n % 8 != 0 || k % 32 != 0) return DTQ_ERR_SHAPE;  // 16-byte output vectors; whole MX blocks (also the TMA row pitch)
   if (m > 0x7FFFFFFF - 256 || n > 0x7FFFFFFF - 256 || k > 0x7FFFFFFF - 256) return DTQ_ERR_TOO_LARGE;
   if (!workspace || workspace_bytes < sizeof(Workspace) || !aligned_to(workspace, 256)) return DTQ_ERR_WORKSPACE;
@@ -1538,7 +1537,7 @@ extern "C" int dtq_rowwise_fp8_bf16(const void *a, const void *b, const float *a
   if (m < 0 || n < 0 || k < 0) return DTQ_ERR_INVALID_ARGUMENT;
   if (a_format != DTQ_E4M3 && a_format != DTQ_E5M2) return DTQ_ERR_UNSUPPORTED_DTYPE;
   if (bias && bias_dtype != DTQ_F32 && bias_dtype != DTQ_BF16) return DTQ_ERR_UNSUPPORTED_DTYPE;
-  if (kernel < DTQ_GEMM_AUTO || kernel > DTQ_GEMM_NARROW) return DTQ_ERR_INVALID_ARGUMENT;
+  if (kernel < DTQ_GEMM_AUTO || kernel > DTQ_GEMM_SPLIT) return DTQ_ERR_INVALID_ARGUMENT;
   if (n % 8 != 0 || k % 16 != 0) return DTQ_ERR_SHAPE;  // 16-byte output vectors; 16-byte operand row pitch (TMA)
   if (m > 0x7FFFFFFF - 256 || n > 0x7FFFFFFF - 256 || k > 0x7FFFFFFF - 256) return DTQ_ERR_TOO_LARGE;
   if (!workspace || workspace_bytes < sizeof(Workspace) || !aligned_to(workspace, 256)) return DTQ_ERR_WORKSPACE;

@@ -352,20 +352,28 @@ int dtq_mx_fp4_bf16(const void *a, const void *b, const void *a_scales_blocked, 
 
 /*
  * Both GEMMs with the element format (DTQ_E4M3 or DTQ_E2M1) and the kernel named instead of chosen from the
- * problem size (for benchmarks, and for tests that run every kernel on every size; the results of the named kernels
- * are bit-identical):
+ * problem size:
  *   DTQ_GEMM_PAIR    two CTAs of a cluster (an SM pair) per 256 x 256 tile, tcgen05.mma.cta_group::2: least
  *                    operand traffic per SM, what large problems use;
  *   DTQ_GEMM_WIDE    one CTA per 128 x 256 tile;
  *   DTQ_GEMM_NARROW  one CTA per 128 x 128 tile, two accumulators (epilogue under the next tile's MMAs);
- *   DTQ_GEMM_AUTO    one of these, or for few output tiles and operand rows of at least 2 KB a cluster per tile whose CTAs
- *                    take a part of K each (fp32 partial sums added in the order of K, so the last bit may differ).
+ *   DTQ_GEMM_SPLIT   a cluster of 2, 4 or 8 CTAs per tile of 128 columns x 32, 64 or 128 rows, each with a part of K:
+ *                    few rows against large weights.  DTQ_ERR_SHAPE where there is nothing to split (so many tiles that
+ *                    two CTAs each exceed two per SM, or less than 16 stages of 128 operand bytes along K);
+ *   DTQ_GEMM_AUTO    the one expected to be quickest.  SPLIT only for operand rows of more than 15 * 128 bytes (up to
+ *                    32 rows of a) or 31 * 128 bytes (more rows), and only with four CTAs per tile, or two with at
+ *                    most 64 rows.
+ * PAIR, WIDE and NARROW give the same bits for every size: the straight sum over K.  SPLIT adds the fp32 sums of its
+ * parts in the order of K, so the last bit of a result may differ from theirs; with AUTO a row's result may therefore
+ * differ in the last bit with the number of rows it is multiplied with (name NARROW where that matters).  Sums beyond the range of
+ * fp32, which only extreme MX scales reach, may overflow in one order and not in the other, or give NaN for an infinity.
  * No reference counterpart (the reference fixes one CUTLASS tile shape, src/mx_fp8_bf16.cu:231-233).
  */
 #define DTQ_GEMM_AUTO 0
 #define DTQ_GEMM_PAIR 1
 #define DTQ_GEMM_WIDE 2
 #define DTQ_GEMM_NARROW 3
+#define DTQ_GEMM_SPLIT 4
 int dtq_mx_gemm_bf16(const void *a, const void *b, const void *a_scales_blocked, const void *b_scales_blocked,
                      void *out_bf16, int64_t m, int64_t n, int64_t k, int elem_format, int kernel, void *workspace,
                      size_t workspace_bytes, void *stream);

@@ -263,10 +263,53 @@ def test_fp4_reference_size_grid_sqnr(size):
     dt.check_device_status()
 
 
-def _check_exact_on_device(mode, m, n, k, kernel, a_dtype=E4M3, bias=None):
-    # exactly summable inputs, so that fp64 on the device gives the same bits whatever the order of the sums
+_E2M1 = (0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0, -0.0, -0.5, -1.0, -1.5, -2.0, -3.0, -4.0, -6.0)
+
+
+def _product(mode, operands, kernel):
+    """One product through the C ABI, into an output with a poisoned margin on both sides."""
     from driss_torch_b200 import _cabi
 
+    a, b, sa, sb, bias = operands
+    m, n = a.shape[0], b.shape[0]
+    room = torch.full((m * n + 128,), 0x5555, dtype=torch.int16, device="cuda")
+    out = room[64:64 + m * n].view(torch.bfloat16).view(m, n)
+    if mode == "rowwise":
+        _cabi.rowwise_fp8_bf16(a, b, sa, sb, bias=bias, out=out, kernel=kernel)
+    else:
+        sab, sbb = (qo.to_blocked(s.cpu(), s.shape[0], s.shape[1]).cuda() for s in (sa, sb))
+        (_cabi.mx_fp8_bf16 if mode == "mx8" else _cabi.mx_fp4_bf16)(a, b, sab, sbb, out=out, kernel=kernel)
+    assert (room[:64] == 0x5555).all() and (room[64 + m * n:] == 0x5555).all(), "bytes outside the output were written"
+    assert _cabi.workspace_status(_cabi.workspace(torch.device("cuda", torch.cuda.current_device()))) == 0
+    return out
+
+
+def _operands64(mode, operands):
+    """The operands as fp64 matrices, block scales multiplied in."""
+    a, b, sa, sb, _ = operands
+    if mode == "rowwise":
+        return a.double(), b.double()
+
+    def full(v, s):
+        if mode == "mx4":
+            table = torch.tensor(_E2M1, dtype=torch.float64, device=v.device)
+            v = torch.stack([table[(v & 0xF).long()], table[(v >> 4).long()]], dim=-1).view(v.shape[0], -1)
+        scale = torch.where(s == 255, torch.full((), float("nan"), dtype=torch.float64, device=v.device), torch.exp2(s.double() - 127))
+        return (v.double().view(v.shape[0], -1, 32) * scale.unsqueeze(2)).view(v.shape[0], -1)
+
+    return full(a, sa), full(b, sb)
+
+
+def _finish64(mode, operands, acc):
+    if mode == "rowwise":
+        acc = acc * operands[2].double()[:, None] * operands[3].double()[None, :]
+        if operands[4] is not None:
+            acc = acc + operands[4].double()
+    return acc
+
+
+def _check_exact_on_device(mode, m, n, k, kernel, a_dtype=E4M3, bias=None):
+    # exactly summable inputs, so that fp64 on the device gives the same bits whatever the order of the sums
     g = torch.Generator(device="cuda").manual_seed(m + n + k)
     a = torch.randint(-3, 4, (m, k), generator=g, device="cuda").float()
     b = torch.randint(-3, 4, (n, k), generator=g, device="cuda").float()
@@ -274,22 +317,21 @@ def _check_exact_on_device(mode, m, n, k, kernel, a_dtype=E4M3, bias=None):
         xs = torch.exp2(torch.randint(-3, 3, (m,), generator=g, device="cuda").float())
         ws = torch.exp2(torch.randint(-3, 3, (n,), generator=g, device="cuda").float())
         bias_d = None if bias is None else (torch.randint(-8, 9, (n,), generator=g, device="cuda") * 0.5).to(bias)
-        got = _cabi.rowwise_fp8_bf16(a.to(a_dtype), b.to(E4M3), xs, ws, bias=bias_d, kernel=kernel)
-        want = (a.double() @ b.double().t()) * xs[:, None] * ws[None, :] + (0.0 if bias is None else bias_d.double())
+        operands = (a.to(a_dtype), b.to(E4M3), xs, ws, bias_d)
     else:
-        sa = torch.randint(125, 130, (m, k // 32), generator=g, device="cuda")
-        sb = torch.randint(125, 130, (n, k // 32), generator=g, device="cuda")
-        sab, sbb = (qo.to_blocked(s.cpu().to(torch.uint8), s.shape[0], k // 32).cuda() for s in (sa, sb))
-        full = [(v.double().view(-1, k // 32, 32) * torch.exp2(s.double() - 127).unsqueeze(2)).view(-1, k) for v, s in ((a, sa), (b, sb))]
-        want = full[0] @ full[1].t()
+        sa = torch.randint(125, 130, (m, k // 32), generator=g, device="cuda").to(torch.uint8)
+        sb = torch.randint(125, 130, (n, k // 32), generator=g, device="cuda").to(torch.uint8)
         if mode == "mx8":
-            got = _cabi.mx_fp8_bf16(a.to(E4M3), b.to(E4M3), sab, sbb, kernel=kernel)
+            pa, pb = a.to(E4M3), b.to(E4M3)
         else:
             code = torch.tensor([13, 12, 10, 0, 2, 4, 5], dtype=torch.uint8, device="cuda")  # e2m1 of -3 .. 3
             pa, pb = (code[(v + 3).long()] for v in (a, b))
-            got = _cabi.mx_fp4_bf16(pa[:, ::2] | (pa[:, 1::2] << 4), pb[:, ::2] | (pb[:, 1::2] << 4), sab, sbb, kernel=kernel)
+            pa, pb = pa[:, ::2] | (pa[:, 1::2] << 4), pb[:, ::2] | (pb[:, 1::2] << 4)
+        operands = (pa, pb, sa, sb, None)
+    got = _product(mode, operands, kernel)
+    a64, b64 = _operands64(mode, operands)
+    want = _finish64(mode, operands, a64 @ b64.t())
     assert torch.equal(got.view(torch.int16), want.to(torch.bfloat16).view(torch.int16))
-    assert _cabi.workspace_status(_cabi.workspace(torch.device("cuda", torch.cuda.current_device()))) == 0
 
 
 @pytest.mark.gpu
@@ -370,3 +412,100 @@ def test_a_wait_that_runs_out_is_reported_and_stores_nothing(mode, kernel, m, n,
     assert (out == 7.0).all()
     ws = torch.zeros_like(ws)  # the context is as good as before
     assert (run(ws) == 0.0).all() and _cabi.workspace_status(ws) == 0
+
+
+# ---- the kernel that splits K, by name ----------------------------------------------------------------------------
+
+_SPLIT_SHAPES = [(1, 8, 2048), (32, 136, 2064), (31, 9600, 4080), (33, 264, 4096), (64, 1000, 8192), (65, 520, 4208),
+                 (128, 4096, 8176), (129, 136, 8192), (300, 2056, 4096), (16, 8192, 16384)]  # tokens, outputs, bytes of K
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["mx8", "mx4", "rowwise"])
+@pytest.mark.parametrize("tokens,n,kb", _SPLIT_SHAPES + [(33, 264, 2048)])
+def test_split_kernel_by_name_on_exactly_summable_inputs(tokens, n, kb, mode):
+    if mode != "rowwise":
+        kb = kb // 32 * 32
+    _check_exact_on_device(mode, tokens, n, kb * 2 if mode == "mx4" else kb, "split",
+                           a_dtype=torch.float8_e5m2 if tokens % 2 else E4M3, bias=[None, torch.float32, torch.bfloat16][tokens % 3])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["mx8", "rowwise"])
+def test_split_kernel_is_refused_where_there_is_nothing_to_split(mode):
+    for tokens, n, kb in [(8, 19200, 4096), (8, 256, 1920)]:  # two CTAs for each of 150 tiles; 15 stages of K
+        with pytest.raises(RuntimeError, match="unsupported shape"):
+            _check_exact_on_device(mode, tokens, n, kb, "split")
+
+
+def _random_operands(mode, m, n, kb, special=False):
+    """Operands as the casts write them; ``special``: any byte as an element, and a few scales at either end."""
+    g = torch.Generator(device="cuda").manual_seed(m * 7 + n * 3 + kb)
+
+    def rand_bytes(rows, cols, poison):
+        v = torch.randint(0, 256, (rows, cols), generator=g, device="cuda", dtype=torch.int32).to(torch.uint8)
+        # most rows free of NaN and infinity (e4m3 x1111111; e5m2 x11111yy), so that finite results are compared too
+        return torch.where((v & 0x7C) == 0x7C, v & 0xBF, v) if not poison else torch.cat([v[:2], torch.where((v[2:] & 0x7C) == 0x7C, v[2:] & 0xBF, v[2:])])
+
+    a_dtype = torch.float8_e5m2 if mode == "rowwise" else E4M3
+    if mode == "mx4":
+        a, b = (torch.randint(0, 256, (r, kb), generator=g, device="cuda", dtype=torch.int32).to(torch.uint8) for r in (m, n))
+    elif special:
+        a, b = rand_bytes(m, kb, True).view(a_dtype), rand_bytes(n, kb, True).view(E4M3)
+    else:
+        a = torch.randn(m, kb, generator=g, device="cuda").to(a_dtype)
+        b = torch.randn(n, kb, generator=g, device="cuda").to(E4M3)
+    if mode == "rowwise":
+        return a, b, torch.rand(m, generator=g, device="cuda") + 0.5, torch.rand(n, generator=g, device="cuda") + 0.5, \
+            torch.randn(n, generator=g, device="cuda")
+    blocks = kb * (2 if mode == "mx4" else 1) // 32
+    sa, sb = (torch.randint(118, 136, (r, blocks), generator=g, device="cuda", dtype=torch.int32).to(torch.uint8) for r in (m, n))
+    if special:
+        sa[m - 1, blocks - 1], sb[n - 1, 0], sb[n - 2, blocks // 2] = 255, 255, 0
+        sa[0, 1] = 0
+    return a, b, sa, sb, None
+
+
+def _accumulation_bound(mode, operands, parts):
+    """Largest distance of a correct result from the fp64 product: every step of 32 bytes of K and every part adds once
+    in fp32 (an error below 2^-23 of the sum of magnitudes, truncation allowed), then one rounding to bf16, whose eight
+    significant bits leave at most 2^-8 of the value."""
+    a64, b64 = _operands64(mode, operands)
+    steps = operands[0].shape[1] // 32 + parts + 4  # and the epilogue's three roundings
+    want = _finish64(mode, operands, a64 @ b64.t())
+    magnitude = _finish64(mode, operands[:4] + (None if operands[4] is None else operands[4].abs(),), a64.abs() @ b64.abs().t())
+    slack = steps * 2.0**-23 * magnitude
+    return want, slack + 2.0**-8 * (want.abs() + slack)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["mx8", "mx4", "rowwise"])
+@pytest.mark.parametrize("tokens,n,kb", _SPLIT_SHAPES)
+def test_split_kernel_on_inexact_sums(tokens, n, kb, mode):
+    if mode != "rowwise":
+        kb = kb // 32 * 32
+    operands = _random_operands(mode, tokens, n, kb)
+    want, bound = _accumulation_bound(mode, operands, 8)
+    split, straight, auto = (_product(mode, operands, kernel) for kernel in ("split", "narrow", "auto"))
+    for got in (split, straight):
+        assert ((got.double() - want).abs() <= bound).all()
+    # further from fp64 than the straight sum by no more than chance (a handful of roundings in the smallest outputs)
+    off = [float((got.double() - want).norm() / want.norm()) for got in (split, straight)]
+    assert off[0] <= off[1] * (1.0 + 4.0 / want.numel() ** 0.5), off
+    # and these shapes are what the default choice sends to this kernel
+    assert torch.equal(auto.view(torch.int16), split.view(torch.int16))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["mx8", "mx4", "rowwise"])
+@pytest.mark.parametrize("tokens,n,kb", [(5, 256, 4096), (40, 136, 4096), (130, 264, 8192)])
+def test_split_kernel_on_special_values(tokens, n, kb, mode):
+    # NaN and (e5m2) infinite elements, scale bytes 0 and 255: what the straight sum makes of them, everywhere
+    operands = _random_operands(mode, tokens, n, kb, special=True)
+    split, straight = (_product(mode, operands, kernel) for kernel in ("split", "narrow"))
+    assert torch.equal(split.isnan(), straight.isnan()) and torch.equal(split.isinf(), straight.isinf())
+    assert torch.equal(split[split.isinf()], straight[split.isinf()])
+    want, bound = _accumulation_bound(mode, operands, 8)
+    finite = split.isfinite()
+    assert finite.any() and not finite.all()
+    assert ((split.double() - want).abs() <= bound)[finite].all()
