@@ -54,6 +54,7 @@ SIGNATURES = {
     "dtq_mx_fp4_bf16": ([_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _sz, _vp], _i32),
     "dtq_rowwise_fp8_bf16": ([_vp, _vp, _vp, _vp, _vp, _i32, _vp, _i64, _i64, _i64, _i32, _i32, _vp, _sz, _vp], _i32),
     "dtq_mx_gemm_bf16": ([_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i32, _i32, _vp, _sz, _vp], _i32),
+    "dtq_gemm_kernel_for": ([_i32, _i64, _i64, _i64, _i32, _i32, _i32], _i32),
     "dtq_mx_fp8_quantize_blocked": ([_vp, _vp, _vp, _i64, _i64, _vp], _i32),
 }
 

@@ -1386,28 +1386,58 @@ int launch_shape(const GemmCall &c, const DeviceInfo &dev) {
                                              map_b, map_sfa, map_sfb, p));
 }
 
-// Token rows per tile of the split kernel.
+// Token rows per tile of the split kernel, and its stages.
 int split_tokens(int64_t m) { return m <= 32 ? 32 : (m <= 64 ? 64 : 128); }
+template <int BN>
+constexpr int SplitStages = BN == 32 ? 5 : (BN == 64 ? 4 : 3);
 
 // CTAs per tile of the split kernel: as many (1, 2, 4, 8) as fill the device's two CTAs per SM, with at least eight K
 // stages each.
-int split_count(int64_t tiles, int64_t stages, const DeviceInfo &dev) {
+int split_count(int64_t m, int64_t n, int64_t stages, int sm_count) {
+  const int64_t tiles = ceil_div64(n, 128) * ceil_div64(m, split_tokens(m));
   int splits = 1;
-  while (splits < kMaxSplits && tiles * splits * 2 <= 2 * dev.sm_count && stages >= 16 * splits) splits *= 2;
+  while (splits < kMaxSplits && tiles * splits * 2 <= 2 * sm_count && stages >= 16 * splits) splits *= 2;
   return splits;
 }
 
-template <int BN, int STAGES, int MODE>
-int launch_split(const GemmCall &c, const DeviceInfo &dev) {
-  static std::atomic<int> configured[kMaxGemmDevices];
-  int dev_id = 0;
-  DTQ_CUDA_TRY(cudaGetDevice(&dev_id));
+// How many clusters of `splits` CTAs of the split kernel the device can hold at once, asked once per device and size; 0
+// where it cannot launch them.
+template <int BN, int MODE>
+int split_cluster_capacity(int dev_id, int splits, int *max_clusters) {
+  static std::atomic<int> known[kMaxGemmDevices][kMaxSplits + 1];  // 0: not asked yet, else the answer + 1
+  auto kernel = mx_gemm_split_kernel<BN, SplitStages<BN>, MODE>;
   if (dev_id < 0 || dev_id >= kMaxGemmDevices) return DTQ_ERR_INVALID_ARGUMENT;
-  const int smem = static_cast<int>(sizeof(SplitSmem<BN, STAGES, MODE>)) + 1024;
-  if (!configured[dev_id].load(std::memory_order_acquire)) {  // setting the attribute twice is harmless
-    DTQ_CUDA_TRY(cudaFuncSetAttribute(mx_gemm_split_kernel<BN, STAGES, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    configured[dev_id].store(1, std::memory_order_release);
+  int value = known[dev_id][splits].load(std::memory_order_acquire);
+  if (value == 0) {  // asking twice is harmless
+    const int smem = static_cast<int>(sizeof(SplitSmem<BN, SplitStages<BN>, MODE>)) + 1024;
+    int n = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess) {
+      cudaLaunchConfig_t cfg;
+      cudaLaunchAttribute attr[2];
+      cluster_launch_config(&cfg, attr, splits, kSplitThreads, splits, smem, nullptr);
+      cfg.numAttrs = 1;  // the occupancy query wants the cluster shape only
+      if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) n = 0;
+    }
+    (void)cudaGetLastError();  // a device without such clusters is not an error of this call
+    value = n + 1;
+    known[dev_id][splits].store(value, std::memory_order_release);
   }
+  *max_clusters = value - 1;
+  return DTQ_OK;
+}
+template <int MODE>
+int split_cluster_capacity(int dev_id, int64_t m, int splits, int *max_clusters) {
+  switch (split_tokens(m)) {
+    case 32: return split_cluster_capacity<32, MODE>(dev_id, splits, max_clusters);
+    case 64: return split_cluster_capacity<64, MODE>(dev_id, splits, max_clusters);
+    default: return split_cluster_capacity<128, MODE>(dev_id, splits, max_clusters);
+  }
+}
+
+// split_cluster_capacity has been asked for these sizes: it also sets the kernel's shared-memory attribute.
+template <int BN, int MODE>
+int launch_split(const GemmCall &c, int splits) {
+  const size_t smem = sizeof(SplitSmem<BN, SplitStages<BN>, MODE>) + 1024;
   CUtensorMap map_w, map_x, map_sfw, map_sfx;
   if (int e = make_operand_map(&map_w, c.b, c.n, c.k_bytes, kBM)) return e;
   if (int e = make_operand_map(&map_x, c.a, c.m, c.k_bytes, BN)) return e;
@@ -1428,67 +1458,87 @@ int launch_split(const GemmCall &c, const DeviceInfo &dev) {
   p.k_stages = static_cast<int>(ceil_div64(c.k_bytes, kBK));
   p.ws = c.ws;
   const int64_t tiles = int64_t(p.n_tiles) * ceil_div64(c.m, BN);
-  p.splits = split_count(tiles, p.k_stages, dev);
+  p.splits = splits;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
   cluster_launch_config(&cfg, attr, static_cast<int>(tiles * p.splits), kSplitThreads, p.splits, smem, c.st);
-  return cuda_status(cudaLaunchKernelEx(&cfg, mx_gemm_split_kernel<BN, STAGES, MODE>, map_w, map_x, map_sfw, map_sfx, p));
+  return cuda_status(cudaLaunchKernelEx(&cfg, mx_gemm_split_kernel<BN, SplitStages<BN>, MODE>, map_w, map_x, map_sfw, map_sfx, p));
+}
+
+// The CTAs per tile that the split kernel gets in the choice below; 1: the call is not one for it.
+// Few tiles and a long K: once it gets four CTAs per tile, or two where a tile is only 32 tokens wide or, with 32 stages of K
+// or more, 64.  Measured split against the best of the others, us: four CTAs, row-wise 64 x 8192 x 4096 9.9 / 12.1,
+// 128 x 4096 x 4096 10.3 / 12.4, 300 x 2048 x 8192 14.3 / 19.4, MXFP4 512 x 1024 x 8192 10.3 / 12.0; two CTAs,
+// 16 x 16384 x 8192 24.0 / 27.0, 64 x 16384 x 8192 25.8 / 28.7, MXFP4 16 x 8192 x 4096 6.7 / 9.2, but 512 x 4096 x 4096
+// 14.3 / 13.4 and MXFP4 64 x 8192 x 4096 8.1 / 8.0; one CTA, 32 x 1024 x 1024 6.1 / 4.9.
+int split_worthwhile(int64_t m, int64_t n, int64_t stages, int sm_count) {
+  const int splits = split_count(m, n, stages, sm_count);
+  const bool two_pay = m <= 32 || (m <= 64 && stages >= 32);
+  return splits >= (two_pay ? 2 : 4) ? splits : 1;
+}
+
+// Which kernel, for a device with `sm_count` SMs that holds `pair_clusters` SM pairs and `split_clusters` clusters of the split
+// kernel (0: cannot launch them).  Estimated time, in microseconds as measured on a B200 = a fixed part (launch, set-up,
+// filling the pipeline, the last epilogue) plus, for every round of tiles on the busiest SM, the stages of 128 operand bytes
+// along K at the time of one, and what a tile costs besides; a tile never takes less than its epilogue.
+//   pair   256 x 256 tiles on SM pairs: 5.6 + rounds x max(0.333 stages + 0.6, 1.8; row-wise 2.2)
+//   wide   128 x 256 on one SM: 4.2 + rounds x max(0.36 stages + 1.9, 2.6; row-wise 4.6), its epilogue not overlapped
+//   narrow 128 x 128 on one SM: 3.2 + rounds x max(0.25 stages + 1.1, 1.5; row-wise 0.25 stages + 1.3, 2.4)
+// So large problems run on SM pairs, and problems of about a tile per SM on the narrow kernel, whose smaller tiles also
+// spread a small output over more SMs.  Measured, us, narrow / wide / pair: row-wise 512 x 4096 x 2048 8.9 / 12.0 / 10.7,
+// 500 x 8192 x 1024 10.2 / 10.0 / 8.6, 1024 x 8192 x 2048 23.8 / 21.1 / 16.5, 16384 x 1024 x 1024 28.6 / 29.7 / 19.3;
+// MXFP8 3000 x 1000 x 5120 25.5 / 18.9 / 19.6; MXFP4 1000 x 4096 x 512 6.1 / 6.5 / 6.5, 4096 x 4096 x 256 13.6 / 14.7 / 12.3.
+// Over 26 shapes in each of the three modes the kernel chosen took at most 6 % longer than the quickest (before: 53 %).
+int choose_kernel(bool row_wise, int64_t m, int64_t n, int64_t k_bytes, int sm_count, int pair_clusters, int split_clusters) {
+  const int64_t k_stages = ceil_div64(k_bytes, kBK), m_tiles = ceil_div64(m, kBM);
+  if (split_clusters > 0 && split_worthwhile(m, n, k_stages, sm_count) > 1) return DTQ_GEMM_SPLIT;
+  const double stages = static_cast<double>(k_stages);
+  auto rounds = [](int64_t tiles, int64_t slots) { return static_cast<double>(ceil_div64(tiles, slots)); };
+  const double wide = 4.2 + rounds(m_tiles * ceil_div64(n, 256), sm_count) * std::max(0.36 * stages + 1.9, row_wise ? 4.6 : 2.6);
+  const double narrow =
+      3.2 + rounds(m_tiles * ceil_div64(n, 128), sm_count) * std::max(0.25 * stages + (row_wise ? 1.3 : 1.1), row_wise ? 2.4 : 1.5);
+  const double pair = pair_clusters > 0 ? 5.6 + rounds(ceil_div64(m, 256) * ceil_div64(n, 256), pair_clusters) *
+                                                    std::max(0.333 * stages + 0.6, row_wise ? 2.2 : 1.8)
+                                        : 1e30;
+  return (pair < wide && pair < narrow) ? DTQ_GEMM_PAIR : (narrow <= wide ? DTQ_GEMM_NARROW : DTQ_GEMM_WIDE);
 }
 
 template <int MODE>
 int launch_gemm(const GemmCall &c, int kernel, const DeviceInfo &dev) {
-  // Which kernel: estimated time, in microseconds as measured on a B200 = a fixed part (launch, set-up, filling the
-  // pipeline, the last epilogue) plus, for every round of tiles on the busiest SM, the stages of 128 operand bytes along K
-  // at the time of one, and what a tile costs besides; a tile never takes less than its epilogue.
-  //   pair   256 x 256 tiles on SM pairs: 5.6 + rounds x max(0.333 stages + 0.6, 1.8; row-wise 2.2)
-  //   wide   128 x 256 on one SM: 4.2 + rounds x max(0.36 stages + 1.9, 2.6; row-wise 4.6), its epilogue not overlapped
-  //   narrow 128 x 128 on one SM: 3.2 + rounds x max(0.25 stages + 1.1, 1.5; row-wise 0.25 stages + 1.3, 2.4)
-  // So large problems run on SM pairs, and problems of about a tile per SM on the narrow kernel, whose smaller tiles also
-  // spread a small output over more SMs.  Measured, us, narrow / wide / pair: row-wise 512 x 4096 x 2048 8.9 / 12.0 / 10.7,
-  // 500 x 8192 x 1024 10.2 / 10.0 / 8.6, 1024 x 8192 x 2048 23.8 / 21.1 / 16.5, 16384 x 1024 x 1024 28.6 / 29.7 / 19.3;
-  // MXFP8 3000 x 1000 x 5120 25.5 / 18.9 / 19.6; MXFP4 1000 x 4096 x 512 6.1 / 6.5 / 6.5, 4096 x 4096 x 256 13.6 / 14.7 / 12.3.
-  // Over 26 shapes in each of the three modes the kernel chosen took at most 6 % longer than the quickest (before: 53 %).
-  const int64_t m_tiles = ceil_div64(c.m, kBM);
-  const double stages = static_cast<double>(ceil_div64(c.k_bytes, kBK));
-  constexpr bool kRow = MODE == kRowwise;
-  auto rounds = [](int64_t tiles, int64_t slots) { return static_cast<double>(ceil_div64(tiles, slots)); };
-  const double wide = 4.2 + rounds(m_tiles * ceil_div64(c.n, 256), dev.sm_count) * std::max(0.36 * stages + 1.9, kRow ? 4.6 : 2.6);
-  const double narrow =
-      3.2 + rounds(m_tiles * ceil_div64(c.n, 128), dev.sm_count) * std::max(0.25 * stages + (kRow ? 1.3 : 1.1), kRow ? 2.4 : 1.5);
-  int dev_id = 0, max_clusters = 0;
+  const int64_t stages = ceil_div64(c.k_bytes, kBK);
+  int dev_id = 0, pair_clusters = 0, split_clusters = 0;
   DTQ_CUDA_TRY(cudaGetDevice(&dev_id));
-  if (int e = pair_cluster_capacity<MODE>(dev_id, &max_clusters)) return e;
-  const double pair = max_clusters > 0 ? 5.6 + rounds(ceil_div64(c.m, 256) * ceil_div64(c.n, 256), max_clusters) *
-                                                   std::max(0.333 * stages + 0.6, kRow ? 2.2 : 1.8)
-                                       : 1e30;
-  if (kernel == DTQ_GEMM_PAIR && max_clusters <= 0) return DTQ_ERR_CUDA_BASE + static_cast<int>(cudaErrorNotSupported);
-  // Few tiles and a long K: the split kernel, once it gets four CTAs per tile, or two where a tile is only 32 tokens wide or,
-  // with 32 stages of K or more, 64.  Measured split against the best of the others, us: four CTAs, row-wise 64 x 8192 x 4096
-  // 9.9 / 12.1, 128 x 4096 x 4096 10.3 / 12.4, 300 x 2048 x 8192 14.3 / 19.4, MXFP4 512 x 1024 x 8192 10.3 / 12.0; two CTAs,
-  // 16 x 16384 x 8192 24.0 / 27.0, 64 x 16384 x 8192 25.8 / 28.7, MXFP4 16 x 8192 x 4096 6.7 / 9.2, but 512 x 4096 x 4096
-  // 14.3 / 13.4 and MXFP4 64 x 8192 x 4096 8.1 / 8.0; one CTA, 32 x 1024 x 1024 6.1 / 4.9.
-  const int splits = split_count(ceil_div64(c.n, 128) * ceil_div64(c.m, split_tokens(c.m)), ceil_div64(c.k_bytes, kBK), dev);
-  if (kernel == DTQ_GEMM_AUTO) {
-    const bool two_pay = c.m <= 32 || (c.m <= 64 && stages >= 32);
-    if (splits >= (two_pay ? 2 : 4)) kernel = DTQ_GEMM_SPLIT;
-  }
+  if (int e = pair_cluster_capacity<MODE>(dev_id, &pair_clusters)) return e;
+  const int splits = kernel == DTQ_GEMM_SPLIT  ? split_count(c.m, c.n, stages, dev.sm_count)
+                     : kernel == DTQ_GEMM_AUTO ? split_worthwhile(c.m, c.n, stages, dev.sm_count)
+                                               : 1;
+  if (splits > 1)
+    if (int e = split_cluster_capacity<MODE>(dev_id, c.m, splits, &split_clusters)) return e;
   if (kernel == DTQ_GEMM_AUTO)
-    kernel = (pair < wide && pair < narrow) ? DTQ_GEMM_PAIR : (narrow <= wide ? DTQ_GEMM_NARROW : DTQ_GEMM_WIDE);
+    kernel = choose_kernel(MODE == kRowwise, c.m, c.n, c.k_bytes, dev.sm_count, pair_clusters, split_clusters);
   if (kernel == DTQ_GEMM_SPLIT) {
     if (splits < 2) return DTQ_ERR_SHAPE;  // named, but too many tiles or too little of K to split anything
+    if (split_clusters <= 0) return DTQ_ERR_CUDA_BASE + static_cast<int>(cudaErrorNotSupported);
     switch (split_tokens(c.m)) {
-      case 32: return launch_split<32, 5, MODE>(c, dev);
-      case 64: return launch_split<64, 4, MODE>(c, dev);
-      default: return launch_split<128, 3, MODE>(c, dev);
+      case 32: return launch_split<32, MODE>(c, splits);
+      case 64: return launch_split<64, MODE>(c, splits);
+      default: return launch_split<128, MODE>(c, splits);
     }
   }
-  if (kernel == DTQ_GEMM_PAIR) return launch_pair<MODE>(c, max_clusters);
+  if (kernel == DTQ_GEMM_PAIR && pair_clusters <= 0) return DTQ_ERR_CUDA_BASE + static_cast<int>(cudaErrorNotSupported);
+  if (kernel == DTQ_GEMM_PAIR) return launch_pair<MODE>(c, pair_clusters);
   if (kernel == DTQ_GEMM_NARROW) return launch_shape<NarrowShape, MODE>(c, dev);
   return launch_shape<WideShape, MODE>(c, dev);
 }
 
 }  // namespace
 }  // namespace dtq
+
+extern "C" int dtq_gemm_kernel_for(int row_wise, int64_t m, int64_t n, int64_t k_bytes, int sm_count, int pair_clusters,
+                                   int split_clusters) {
+  if (m <= 0 || n <= 0 || k_bytes <= 0 || sm_count <= 0) return DTQ_GEMM_AUTO;
+  return dtq::choose_kernel(row_wise != 0, m, n, k_bytes, sm_count, pair_clusters, split_clusters);
+}
 
 extern "C" size_t dtq_mx_gemm_scale_bytes(int64_t rows, int64_t k) {
   if (rows <= 0 || k <= 0) return 0;

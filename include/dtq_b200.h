@@ -377,6 +377,12 @@ int dtq_mx_fp4_bf16(const void *a, const void *b, const void *a_scales_blocked, 
 int dtq_mx_gemm_bf16(const void *a, const void *b, const void *a_scales_blocked, const void *b_scales_blocked,
                      void *out_bf16, int64_t m, int64_t n, int64_t k, int elem_format, int kernel, void *workspace,
                      size_t workspace_bytes, void *stream);
+/*
+ * The kernel (one of the above) that DTQ_GEMM_AUTO takes on a device with `sm_count` SMs that can hold `pair_clusters`
+ * clusters of PAIR and `split_clusters` of SPLIT at once (0: cannot launch any; the choice then falls to the others).
+ * k_bytes = bytes per operand row; row_wise != 0: dtq_rowwise_fp8_bf16.  Touches no device.  DTQ_GEMM_AUTO for a size <= 0.
+ */
+int dtq_gemm_kernel_for(int row_wise, int64_t m, int64_t n, int64_t k_bytes, int sm_count, int pair_clusters, int split_clusters);
 
 /*
  * Row-wise scaled fp8 GEMM, the consumer of dtq_dynamic_scaled_quant_rowwise's scales:

@@ -509,3 +509,37 @@ def test_split_kernel_on_special_values(tokens, n, kb, mode):
     finite = split.isfinite()
     assert finite.any() and not finite.all()
     assert ((split.double() - want).abs() <= bound)[finite].all()
+
+
+# ---- the default choice (no device needed) -------------------------------------------------------------------------
+
+def _choice(row_wise, m, n, k_bytes, sms=148, pairs=74, splits=1):
+    from driss_torch_b200 import _cabi
+
+    names = {code: name for name, code in _cabi.GEMM_KERNELS.items()}
+    return names[_cabi.load().dtq_gemm_kernel_for(row_wise, m, n, k_bytes, sms, pairs, splits)]
+
+
+@pytest.mark.parametrize("row_wise", [0, 1])
+@pytest.mark.parametrize("tokens,n,kb", _SPLIT_SHAPES)
+def test_choice_gives_way_where_clusters_cannot_be_launched(tokens, n, kb, row_wise):
+    assert _choice(row_wise, tokens, n, kb) == "split"
+    assert _choice(row_wise, tokens, n, kb, splits=0) in ("pair", "wide", "narrow")
+    assert _choice(row_wise, tokens, n, kb, pairs=0, splits=0) in ("wide", "narrow")
+
+
+def test_choice_at_the_edges_of_the_split_rule():
+    for row_wise in (0, 1):
+        # up to 32 tokens from the sixteenth stage of 128 bytes, up to 64 and above from the thirty-second
+        for tokens, last_without in [(1, 1920), (32, 1920), (33, 3968), (64, 3968), (65, 3968), (300, 3968)]:
+            assert _choice(row_wise, tokens, 1024, last_without) != "split", (tokens, last_without)
+            assert _choice(row_wise, tokens, 1024, last_without + 1) == "split", (tokens, last_without)
+        # two CTAs per tile (75 to 148 tiles) pay for 64 tokens, not for 128
+        assert _choice(row_wise, 64, 148 * 128, 8192) == "split" and _choice(row_wise, 64, 149 * 128, 8192) != "split"
+        assert _choice(row_wise, 128, 74 * 128, 8192) == "split" and _choice(row_wise, 128, 75 * 128, 8192) != "split"
+
+
+def test_choice_leaves_the_reference_sizes_on_the_straight_sum():
+    for m, k, n in REFERENCE_SIZES + [(4096, 4096, 4096), (2048, 1024, 8192)]:
+        for k_bytes in (k, k // 2):
+            assert _choice(0, m, n, k_bytes) != "split"
