@@ -42,7 +42,8 @@ mx_stream_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, ui
       return;
     }
   }
-  for (int64_t tile = blockIdx.x - (BLOCKED ? pad_blocks : 0); tile * kTile < nchunks; tile += gridDim.x) {
+  const TileWalk walk = tile_walk(blockIdx.x, gridDim.x, BLOCKED ? pad_blocks : 0);
+  for (int64_t tile = walk.first; tile * kTile < nchunks; tile += walk.step) {
     const int64_t warp_first = tile * kTile + int64_t(warp) * (32 * kUnroll);
     uint4 v[kUnroll];
 #pragma unroll

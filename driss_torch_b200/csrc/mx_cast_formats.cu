@@ -167,7 +167,8 @@ mx_formats_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, u
   // in the blocked layout (a division) ran four times as often, and 64 bits wide it was most of the kernel.
   // Measured, bf16 -> MXFP4 with blocked scales: 8192 x 8192 38.0 -> 26.9 us (row-major scales 24.7), 16384 x 8192
   // 73.1 -> 53.2 (50.2); from fp32 129 -> 91.
-  for (int64_t tile = blockIdx.x - pad_blocks; tile * kTile < nchunks; tile += gridDim.x) {
+  const TileWalk walk = tile_walk(blockIdx.x, gridDim.x, pad_blocks);
+  for (int64_t tile = walk.first; tile * kTile < nchunks; tile += walk.step) {
     const int64_t first = tile * kTile + int64_t(warp) * (32 * kUnrollF) + lane;
     uint4 v[kUnrollF];
     int my_scale = 0;

@@ -118,6 +118,28 @@ __device__ __forceinline__ void zero_scale_padding(uint8_t *scales, int64_t rows
       for (int c = live; c < 4; ++c) p[c] = 0;
     }
 }
+// The tiles of block `block` of a grid whose first `pad_blocks` blocks write padding instead: its first, and the step to its
+// next (the number of blocks that take tiles).
+struct TileWalk {
+  int64_t first, step;
+};
+__host__ __device__ constexpr TileWalk tile_walk(unsigned block, unsigned grid, unsigned pad_blocks) {
+  return {int64_t(block) - pad_blocks, int64_t(grid) - pad_blocks};
+}
+constexpr bool takes_every_tile_once(int64_t tiles, unsigned grid, unsigned pad_blocks) {
+  for (int64_t t = 0; t < tiles; ++t) {
+    int taken = 0;
+    for (unsigned b = pad_blocks; b < grid; ++b)
+      for (int64_t i = tile_walk(b, grid, pad_blocks).first; i < tiles; i += tile_walk(b, grid, pad_blocks).step) taken += i == t;
+    if (taken != 1) return false;
+  }
+  return true;
+}
+// as many blocks as tiles, as today's grids; blocks that take several, with and without padding
+static_assert(takes_every_tile_once(7, 9, 2) && takes_every_tile_once(7, 7, 0) && takes_every_tile_once(13, 5, 2) &&
+                  takes_every_tile_once(13, 3, 0) && takes_every_tile_once(1, 4, 3),
+              "blocks beside the padding share out the tiles");
+
 // Spare blocks of `threads` threads for it, about two items per thread.
 inline int64_t scale_padding_blocks(int64_t rows, int64_t kblocks, int threads) {
   const int64_t n = (scale_padding_items(rows, kblocks) + 2 * threads - 1) / (2 * threads);
