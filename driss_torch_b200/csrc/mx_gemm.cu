@@ -84,6 +84,15 @@ using WideShape = GemmShape<256, 4, 1>;
 using NarrowShape = GemmShape<128, 6, 2>;
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // a wait gives up after two seconds of wall time (Workspace::wait_limit_us)
 
+// Shared memory that a kernel asks for: its struct, and what aligning that to 1024 bytes may take.  A struct that outgrew
+// the limit would fail in cudaFuncSetAttribute, and for the cluster kernels look like a device without them.
+constexpr size_t kMaxDynamicSmem = 227 * 1024;
+template <typename SMEM>
+constexpr int smem_bytes() {
+  static_assert(sizeof(SMEM) + 1024 <= kMaxDynamicSmem, "more shared memory than a block can have");
+  return static_cast<int>(sizeof(SMEM) + 1024);
+}
+
 template <typename SH, int MODE>
 struct __align__(1024) GemmSmem {
   uint8_t a[SH::STAGES][kBM * kBK];        // 16 KB per stage, 1024-byte aligned (swizzle atom = 8 rows x 128 B)
@@ -616,10 +625,11 @@ template <int MODE>
 struct __align__(1024) PairSmem {
   uint8_t a[PairStages<MODE>][kBM * kBK];             // this CTA's 128 rows of A
   uint8_t b[PairStages<MODE>][kPairBN / 2 * kBK];     // this CTA's 128 of the tile's 256 rows of B
-  uint8_t sfa[PairStages<MODE>][Format<MODE>::kKAtoms * 512];      // scales of this CTA's 128 rows of A
-  uint8_t sfb[PairStages<MODE>][2 * Format<MODE>::kKAtoms * 512];  // scales of all 256 rows of B: [128 columns][atom along K]
-  uint8_t out[kEpilogueWarps][32 * 64];          // per epilogue warp 32 rows x 32 bf16 on their way out (64-byte swizzle)
-  float scales[MODE == kRowwise ? kEpilogueWarps : 1][2][128];  // per epilogue warp its columns' scales and biases
+  // scales of this CTA's 128 rows of A, and of all 256 rows of B ([128 columns][atom along K]); one dummy without block scales
+  uint8_t sfa[Format<MODE>::kScaled ? PairStages<MODE> : 1][Format<MODE>::kKAtoms * 512];
+  uint8_t sfb[Format<MODE>::kScaled ? PairStages<MODE> : 1][2 * Format<MODE>::kKAtoms * 512];
+  alignas(512) uint8_t out[kEpilogueWarps][32 * 64];  // per epilogue warp 32 rows x 32 bf16 on their way out (64-byte swizzle)
+  float scales[MODE == kRowwise ? kEpilogueWarps : 1][2][128];  // per epilogue warp its columns' scales and biases (row-wise)
   uint64_t full[PairStages<MODE>];               // used in the leader CTA only
   uint64_t empty[PairStages<MODE>];
   uint64_t tmem_full[2];                         // one per accumulator
@@ -1286,7 +1296,7 @@ int pair_cluster_capacity(int dev_id, int *max_clusters) {
     static std::mutex mutex;
     std::lock_guard<std::mutex> lock(mutex);
     if (!ready[dev_id].load(std::memory_order_relaxed)) {
-      const int smem = static_cast<int>(sizeof(PairSmem<MODE>)) + 1024;
+      constexpr int smem = smem_bytes<PairSmem<MODE>>();
       int n = 0;
       if (cudaFuncSetAttribute(mx_gemm_pair_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess) {
         cudaLaunchConfig_t cfg;
@@ -1344,7 +1354,7 @@ int launch_pair(const GemmCall &c, int max_clusters) {
   const int clusters = static_cast<int>(tiles < max_clusters ? tiles : max_clusters);
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
-  cluster_launch_config(&cfg, attr, 2 * clusters, kGemmThreads, 2, sizeof(PairSmem<MODE>) + 1024, c.st);
+  cluster_launch_config(&cfg, attr, 2 * clusters, kGemmThreads, 2, smem_bytes<PairSmem<MODE>>(), c.st);
   return cuda_status(cudaLaunchKernelEx(&cfg, mx_gemm_pair_kernel<MODE>, map_a, map_b, map_sfa, map_sfb, map_out, p));
 }
 
@@ -1355,7 +1365,7 @@ int launch_shape(const GemmCall &c, const DeviceInfo &dev) {
   int dev_id = 0;
   DTQ_CUDA_TRY(cudaGetDevice(&dev_id));
   if (dev_id < 0 || dev_id >= kMaxGemmDevices) return DTQ_ERR_INVALID_ARGUMENT;
-  const int smem = static_cast<int>(sizeof(GemmSmem<SH, MODE>)) + 1024;
+  constexpr int smem = smem_bytes<GemmSmem<SH, MODE>>();
   if (!configured[dev_id].load(std::memory_order_acquire)) {  // setting the attribute twice is harmless
     DTQ_CUDA_TRY(cudaFuncSetAttribute(mx_gemm_kernel<SH, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     configured[dev_id].store(1, std::memory_order_release);
@@ -1409,7 +1419,8 @@ int split_cluster_capacity(int dev_id, int splits, int *max_clusters) {
   if (dev_id < 0 || dev_id >= kMaxGemmDevices) return DTQ_ERR_INVALID_ARGUMENT;
   int value = known[dev_id][splits].load(std::memory_order_acquire);
   if (value == 0) {  // asking twice is harmless
-    const int smem = static_cast<int>(sizeof(SplitSmem<BN, SplitStages<BN>, MODE>)) + 1024;
+    constexpr int smem = smem_bytes<SplitSmem<BN, SplitStages<BN>, MODE>>();
+    static_assert(2 * (smem + 1024) <= 228 * 1024, "two CTAs per SM, with the kilobyte that each takes besides");
     int n = 0;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess) {
       cudaLaunchConfig_t cfg;
@@ -1437,7 +1448,7 @@ int split_cluster_capacity(int dev_id, int64_t m, int splits, int *max_clusters)
 // split_cluster_capacity has been asked for these sizes: it also sets the kernel's shared-memory attribute.
 template <int BN, int MODE>
 int launch_split(const GemmCall &c, int splits) {
-  const size_t smem = sizeof(SplitSmem<BN, SplitStages<BN>, MODE>) + 1024;
+  constexpr int smem = smem_bytes<SplitSmem<BN, SplitStages<BN>, MODE>>();
   CUtensorMap map_w, map_x, map_sfw, map_sfx;
   if (int e = make_operand_map(&map_w, c.b, c.n, c.k_bytes, kBM)) return e;
   if (int e = make_operand_map(&map_x, c.a, c.m, c.k_bytes, BN)) return e;
