@@ -235,12 +235,12 @@ def mx_fp8_quantize(x, payload=None, scales=None):
 
 @_on_device_of_first_tensor
 def mx_fp8_quantize_blocked(x, payload=None, scales=None):
-    """MX cast with the scales in the blocked layout of the consumer GEMM (zero-filled padding)."""
+    """MX cast with the scales in the blocked layout of the consumer GEMM (the cast writes zeros in the padding)."""
     rows, cols = x.shape
     payload = torch.empty(x.shape, dtype=torch.float8_e4m3fn, device=x.device) if payload is None else payload
     if scales is None:
         nbytes = load().dtq_mx_blocked_scale_bytes(rows, cols)
-        scales = torch.zeros(nbytes, dtype=torch.uint8, device=x.device).view(torch.float8_e8m0fnu)
+        scales = torch.empty(nbytes, dtype=torch.float8_e8m0fnu, device=x.device)
     check(load().dtq_mx_fp8_quantize_blocked(x.data_ptr(), payload.data_ptr(), scales.data_ptr(), rows, cols, _stream()),
           "dtq_mx_fp8_quantize_blocked")
     return payload, scales
@@ -268,9 +268,9 @@ def mx_fp8_quantize_dual(x, payload=None, scales=None, payload_t=None, scales_t=
     if blocked:
         L = load()
         if scales is None:
-            scales = torch.zeros(L.dtq_mx_blocked_scale_bytes(rows, cols), dtype=torch.uint8, device=x.device).view(e8m0)
+            scales = torch.empty(L.dtq_mx_blocked_scale_bytes(rows, cols), dtype=e8m0, device=x.device)
         if scales_t is None:
-            scales_t = torch.zeros(L.dtq_mx_blocked_scale_bytes(cols, rows), dtype=torch.uint8, device=x.device).view(e8m0)
+            scales_t = torch.empty(L.dtq_mx_blocked_scale_bytes(cols, rows), dtype=e8m0, device=x.device)
         check(L.dtq_mx_fp8_quantize_dual_blocked(x.data_ptr(), payload.data_ptr(), scales.data_ptr(), payload_t.data_ptr(),
                                                  scales_t.data_ptr(), rows, cols, _stream()), "dtq_mx_fp8_quantize_dual_blocked")
         return payload, scales, payload_t, scales_t
@@ -301,7 +301,7 @@ MX_FMT_CODE = {torch.float8_e4m3fn: 0, torch.float8_e5m2: 1, torch.float4_e2m1fn
 @_on_device_of_first_tensor
 def mx_quantize(x, elem, payload=None, scales=None, blocked=False):
     """MX block-32 cast of bf16 / fp16 / fp32 to e4m3 / e5m2 (payload [M, N]) or e2m1 (uint8 [M, N/2]);
-    ``blocked``: the scales in the MX GEMM's blocked layout (zero-filled padding)."""
+    ``blocked``: the scales in the MX GEMM's blocked layout (the cast writes zeros in the padding)."""
     rows, cols = x.shape
     fmt = MX_FMT_CODE[elem]
     if payload is None:
@@ -310,7 +310,7 @@ def mx_quantize(x, elem, payload=None, scales=None, blocked=False):
     if blocked:
         if scales is None:
             nbytes = load().dtq_mx_blocked_scale_bytes(rows, cols)
-            scales = torch.zeros(nbytes, dtype=torch.uint8, device=x.device).view(torch.float8_e8m0fnu)
+            scales = torch.empty(nbytes, dtype=torch.float8_e8m0fnu, device=x.device)
         check(load().dtq_mx_quantize_blocked(x.data_ptr(), payload.data_ptr(), scales.data_ptr(), rows, cols,
                                              MX_IN_CODE[x.dtype], fmt, _stream()), "dtq_mx_quantize_blocked")
         return payload, scales

@@ -503,3 +503,31 @@ def test_padding_of_blocked_scales_is_written(rows, cols, offset):
         _cabi.mx_fp8_quantize_dual(x, scales=s, scales_t=s_t, blocked=True)
         check(room, s, want, rows, cols)
         check(room_t, s_t, _cabi.mx_fp8_quantize(x.t().contiguous())[1], cols, rows)
+
+
+@pytest.mark.parametrize("rows,cols", [(32, 96), (160, 32), (288, 4128)])
+def test_blocked_wrappers_launch_no_fill(rows, cols, monkeypatch):
+    # the casts write the padding themselves, whatever the array held before
+    from driss_torch_b200 import _cabi
+
+    x = workloads.make_cfg3(rows=rows, cols=cols).cuda()
+    want, want_t = ((_cabi.mx_fp8_quantize(v)[1].cpu().view(torch.uint8), *v.shape) for v in (x, x.t().contiguous()))
+    want_fp4 = (_cabi.mx_quantize(x, "e2m1")[1].cpu().view(torch.uint8), rows, cols)
+    empty = torch.empty
+
+    def poisoned(*args, **kwargs):
+        t = empty(*args, **kwargs)
+        t.view(torch.uint8).fill_(0xAA)
+        return t
+
+    def unwanted(*args, **kwargs):
+        raise AssertionError("a fill in front of the cast")
+
+    monkeypatch.setattr(torch, "empty", poisoned)
+    monkeypatch.setattr(torch, "zeros", unwanted)
+    got = [(_cabi.mx_fp8_quantize_blocked(x)[1], want), (_cabi.mx_quantize(x, "e2m1", blocked=True)[1], want_fp4)]
+    dual = _cabi.mx_fp8_quantize_dual(x, blocked=True)
+    got += [(dual[1], want), (dual[3], want_t)]
+    monkeypatch.undo()
+    for scales, (row_major, r, c) in got:
+        assert torch.equal(as_bytes(scales), as_bytes(qo.to_blocked(row_major, r, c // 32)))
