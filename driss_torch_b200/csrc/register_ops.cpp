@@ -35,10 +35,14 @@ int out_code(at::ScalarType t) { return t == at::kFloat8_e4m3fn ? DTQ_E4M3 : DTQ
 
 // Outputs straight from the CUDA allocator: what at::empty / at::empty_like end in, without a second and third trip
 // through the dispatcher.  The smallest calls are bound by the host, and each at::empty was 0.4 us of their 5 to 9.
+// at::empty also fills what it returns under torch.use_deterministic_algorithms (unless told not to), so then it is asked.
 at::Tensor new_on_device_of(const at::Tensor &like, at::IntArrayRef sizes, at::ScalarType dtype) {
+  if (C10_UNLIKELY(at::globalContext().deterministicAlgorithms())) return at::empty(sizes, like.options().dtype(dtype));
   return at::Tensor(at::detail::empty_cuda(sizes, dtype, like.device(), std::nullopt));
 }
 at::Tensor new_same_layout(const at::Tensor &like, at::ScalarType dtype) {  // `like` is dense: its strides are kept as they are
+  if (C10_UNLIKELY(at::globalContext().deterministicAlgorithms()))
+    return at::empty_strided(like.sizes(), like.strides(), like.options().dtype(dtype));
   return at::Tensor(at::detail::empty_strided_cuda(like.sizes(), like.strides(), dtype, like.device()));
 }
 

@@ -345,3 +345,40 @@ def test_cast_with_amax_dual_on_the_tie_lattice_and_with_foreign_amax(fp8_dtype)
         p32, p32_t, _ = dt.cast_with_amax_dual(f32.cuda(), am.cuda(), fp8_dtype)
         assert_fp8_equal(p32, want32, fp8_dtype, "fp32 row-major")
         assert_fp8_equal(p32_t, want32.t().contiguous(), fp8_dtype, "fp32 transposed")
+
+
+def test_outputs_are_filled_under_deterministic_algorithms():
+    # torch.use_deterministic_algorithms promises that newly allocated outputs hold no stray bytes (torch.utils.deterministic.
+    # fill_uninitialized_memory); every kernel writes its whole output, so only the fills themselves can be seen
+    import driss_torch_b200 as dt
+
+    x = workloads.make_cfg2(rows=64, cols=128).cuda()
+    one = torch.ones(1, device="cuda")
+    calls = {
+        "saturated_cast": lambda: dt.saturated_cast(x, one, torch.float8_e4m3fn),
+        "amax": lambda: dt.amax(x),
+        "dynamic_scaled_quant_with_scale": lambda: dt.dynamic_scaled_quant_with_scale(x, torch.float8_e5m2),
+        "dynamic_scaled_quant_rowwise": lambda: dt.dynamic_scaled_quant_rowwise(x, torch.float8_e4m3fn),
+        "cast_with_amax_dual": lambda: dt.cast_with_amax_dual(x, one, torch.float8_e4m3fn),
+        "mx_fp8_quantize": lambda: dt.mx_fp8_quantize(x),
+        "mx_fp8_quantize_blocked": lambda: dt.mx_fp8_quantize_blocked(x),
+        "mx_fp4_quantize": lambda: dt.mx_fp4_quantize(x, blocked=True),
+        "mx_fp8_bf16": lambda: dt.mx_fp8_bf16(payload, payload.t(), scales, scales),
+    }
+    payload, scales = dt.mx_fp8_quantize_blocked(x)
+
+    def run(call):
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+            out = call()
+        out = out if isinstance(out, tuple) else (out,)
+        return [t.clone().view(torch.uint8) for t in out], sum(e.count for e in prof.key_averages() if e.key == "aten::fill_")
+
+    plain = {name: run(call) for name, call in calls.items()}
+    torch.use_deterministic_algorithms(True)
+    try:
+        filled = {name: run(call) for name, call in calls.items()}
+    finally:
+        torch.use_deterministic_algorithms(False)
+    for name, (outs, fills) in filled.items():
+        assert plain[name][1] == 0 and fills >= len(outs), f"{name}: {fills} fills of {len(outs)} outputs"
+        assert all(torch.equal(a, b) for a, b in zip(outs, plain[name][0])), name
