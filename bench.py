@@ -12,11 +12,12 @@ rows.  Total work is fixed as N grows (strong scaling).  ``value`` is algorithmi
 the whole job per second of device time (max over ranks): tensor-wise N*(2+1) compulsory
 bytes + MX N*(2+1+1/32).
 
-Rank 0 prints ONE JSON line.  Besides the contract keys it carries ``roofline`` (dominant
-kernel), ``kernels`` (every kernel of the step), ``ops`` (N == 1: the single-GPU
-configurations cfg1-cfg4, cold-L2, one line per op, with the reference CUDA kernel timed
-beside it when oracle/_ref is built), ``cpu_baseline`` and ``e2e`` (host buffers in, host
-buffers out, through driss_torch_b200.host_pipeline).
+Rank 0 prints ONE JSON line, short enough to survive whoever keeps only the end of an output.
+Besides the contract keys it carries ``roofline`` (dominant kernel), ``kernels`` (every kernel
+of the step), ``cpu_baseline`` and ``e2e`` (host buffers in, host buffers out, through
+driss_torch_b200.host_pipeline).  The per-op table (N == 1: the single-GPU configurations
+cfg1-cfg4, cold-L2, with the reference CUDA kernel timed beside each op when oracle/_ref is
+built, and the GEMMs) goes to stderr, one JSON line per op.
 
 ``--impl reference`` times the CPU restatement of the reference (oracle/, all host threads)
 on a bounded sample of the same workload; rank 0 alone works.
@@ -617,6 +618,12 @@ def run_reference_arm(args, rank: int):
 
 # ---- main ---------------------------------------------------------------------------------------------------
 
+def print_result(out: dict, ops: list | None):
+    """The result as one line of stdout; the per-op table, several times as long, before it on stderr."""
+    for op in ops or []:
+        print(json.dumps(op), file=sys.stderr, flush=True)
+    print(json.dumps(out), flush=True)
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -986,13 +993,11 @@ def main():
             out["config"]["exchange_note"] = exchange_note
         if e2e is not None:
             out["e2e"] = e2e
-        if ops is not None:
-            out["ops"] = ops
         if parity is not None:
             out["parity_checked"] = parity
         if cpu is not None:
             out["cpu_baseline"] = cpu
-        print(json.dumps(out), flush=True)
+        print_result(out, ops)
     if world > 1:
         dist.destroy_process_group()
 
