@@ -141,7 +141,7 @@ def mx_fp4_bf16(a: Tensor, b: Tensor, a_scale: Tensor, b_scale: Tensor) -> Tenso
     return ops.mx_fp4_bf16(a, b, a_scale, b_scale)
 
 
-# The north-star text calls the MX op "mx_cast"; the reference symbol is mx_fp8_quantize.
+# A second name for the MX op; the reference symbol is mx_fp8_quantize.
 mx_cast = mx_fp8_quantize
 
 

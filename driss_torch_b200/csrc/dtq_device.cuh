@@ -132,8 +132,9 @@ __device__ __forceinline__ float dsq_mul(double sd, float x) {
 //     maxima are 7 * 2^j) and |theta| <= 1e-12/amax + 2^-51 <= 2^-36.9.  If m divides 7n 2^i, Q has
 //     at most 11 significant bits, is an fp32 number, and P stays within 2^-36.9 of it; otherwise
 //     |Q - M| >= 2^-33 |Q| for every 25-bit midpoint M (the difference of the two fractions is a
-//     non-zero integer over m times a power of two).  Where t underflows, |P| < 2^-100 converts to a
-//     signed zero either way.  Both products have the sign of x, zeros included, because tail is not negative; it
+//     non-zero integer over m times a power of two).  Where t underflows (for an sd that is an fp32 number the tail
+//     is the 2^-126 below, and t does for every |x| < 1) it is off by at most 2^-149, which is below 2^-45 |P| from
+//     |P| = 2^-100 on; a smaller P converts to a signed zero either way.  Both products have the sign of x, zeros included, because tail is not negative; it
 //     is not zero either (at least 2^-126, less than 2^-70 sd), so an infinite x gives an infinity and not 0 * inf,
 //     and saturates as in the reference.  Two packed instructions per pair; the form with the rounding error of x*head
 //     taken separately took four and two sign copies, and the issue of instructions is what bounds these kernels as soon

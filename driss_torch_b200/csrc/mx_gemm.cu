@@ -21,12 +21,14 @@
 //     through the descriptor's scale-factor id; tcgen05.commit releases the stage (`empty`) and finally hands
 //     the accumulator (128 lanes x up to 256 fp32 columns of tensor memory) to the epilogue;
 //   * both of those warps walk their loops as whole warps with one elected lane issuing (see elect_one);
-//   * warps 2..9 are the epilogue: tcgen05.ld 2 x 32 columns at a time, fp32 -> bf16, 64-byte row segments
-//     straight to global memory; the accumulator is released as soon as it is in registers, so the next tile's
-//     MMAs overlap the stores.
+//   * warps 2..9 are the epilogue.  Single CTA: tcgen05.ld 2 x 32 columns at a time, fp32 -> bf16, 64-byte row segments
+//     straight to global memory; the accumulator is released as soon as it is in registers, so the next tile's MMAs
+//     overlap the stores.  The SM pair stages 32 x 32 boxes in shared memory for TMA stores; the split kernel's four
+//     warps leave partial sums in shared memory, which the cluster adds up.
 // No load is shared between CTAs: every CTA loads its own operands (A and B of an 8192^3 problem both fit in
 // L2).  Every wait is bounded: a wait that runs out records DTQ_ERR_TIMEOUT in the status word, raises the CTA's
-// abort flag, the roles drain what they have in flight, tensor memory is freed and the kernel returns.
+// abort flag, the roles drain what they have in flight, tensor memory is freed and the kernel returns.  (Roles wait as
+// whole warps, see mbar_wait_warp.)
 #include <cuda.h>
 
 #include <algorithm>
@@ -67,7 +69,7 @@ struct Format {
   // formats come with the call (e4m3 = 0 or e5m2 = 1 in bits 7-9 / 10-12)
   static constexpr uint32_t kFormatBits = MODE == kMxFp4 ? ((1u << 7) | (1u << 10) | (1u << 23)) : (MODE == kMxFp8 ? (1u << 23) : (1u << 4));
 };
-constexpr int kTmemCols = 512;             // allocation (power of two); columns 0..255 hold the accumulator(s)
+constexpr int kTmemCols = 512;             // allocation (power of two); one CTA: columns 0..255 hold the accumulator(s); pair: PairTmem
 
 // Two tile shapes.  Wide: 128 x 256, one accumulator of 256 columns, 4 stages -- least operand traffic per
 // output (every byte of B serves 128 rows, every byte of A 256 columns), the shape for large problems.
@@ -849,7 +851,8 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // A warp's 128 columns go 32 at a time, the next 32 on their way from tensor memory while these are converted and
     // staged in shared memory, from where a TMA store takes them (which also cuts off what lies past the edges).  With
     // stores from registers a lane owned a row, a warp's store touched 32 lines, and the epilogue took longer than the
-    // MMAs of 1024 bytes of K; see launch_pair for the figures.  The half that holds the shared columns starts with them: half 1 at its end (columns 255..224 of the first
+    // MMAs of 1024 bytes of K; see launch_pair for the figures.
+    // The half that holds the shared columns starts with them: half 1 at its end (columns 255..224 of the first
     // accumulator), half 0 at its beginning (columns 0..31 of the second, the same columns of tensor memory).
     const int quad = warp & 3, half = (warp - 2) >> 2;
     const uint32_t leader_empty[2] = {map_to_cta(smem_addr(&sm.tmem_empty[0]), 0), map_to_cta(smem_addr(&sm.tmem_empty[1]), 0)};
