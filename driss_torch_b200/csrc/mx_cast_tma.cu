@@ -119,8 +119,9 @@ mx_tma_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, uint8
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++k) {
     const int s = static_cast<int>(k % kStages);
     const unsigned round = static_cast<unsigned>(k / kStages);
-    if (*static_cast<volatile int *>(&sm.abort)) return;  // the producer drains its copies before the CTA ends
-    if (!mbar_wait(&sm.full[s], round & 1u)) {
+    // one answer for the warp each time: what follows (shuffles, the warp's arrival) needs all of its lanes
+    if (__any_sync(0xFFFFFFFFu, *static_cast<volatile int *>(&sm.abort) != 0)) return;  // the producer drains its copies before the CTA ends
+    if (!__all_sync(0xFFFFFFFFu, mbar_wait(&sm.full[s], round & 1u))) {
       // the copy never landed: nothing can be drained; after this status the outputs are not to be trusted
       if (lane == 0) {
         atomicExch(status, DTQ_ERR_TIMEOUT);

@@ -84,6 +84,10 @@ def test_argument_validation_before_any_device_work():
     assert lib.dtq_mx_fp8_quantize_amax_p2p(one, one, one, one, 4, 64, one, 1 << 20, ptrs, 0, 17, 1, 0, None) == 1  # world
     assert lib.dtq_dynamic_scaled_quant_rowwise(one, one, None, None, 0, 16, 0, 0, None) == 0
     assert lib.dtq_dynamic_scaled_quant_rowwise(one, one, None, None, 4, 16, 9, 0, None) == 2
+    for kernel in (-1, 5):  # no such kernel
+        assert lib.dtq_mx_gemm_bf16(one, one, one, one, one, 8, 8, 32, 0, kernel, one, 1 << 20, None) == 1
+        assert lib.dtq_rowwise_fp8_bf16(one, one, one, one, None, 0, one, 8, 8, 32, 0, kernel, one, 1 << 20, None) == 1
+    assert lib.dtq_gemm_kernel_for(0, 0, 8, 32, 148, 74, 1) == 0
     assert lib.dtq_workspace_init(None, 0, None) == 4
 
 

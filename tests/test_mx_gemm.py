@@ -367,6 +367,11 @@ def test_waits_of_the_gemm_roles_are_warp_wide():
     source = (Path(__file__).resolve().parents[1] / "driss_torch_b200" / "csrc" / "mx_gemm.cu").read_text()
     calls = re.findall(r"^.*\bmbar_wait\(.*$", source, flags=re.M)
     assert len(calls) == 3, calls  # its definition and the two wrappers
+    # the same for the consumers of the TMA-staged MX cast: flag and barrier are looked at by vote
+    staged = (Path(__file__).resolve().parents[1] / "driss_torch_b200" / "csrc" / "mx_cast_tma.cu").read_text()
+    consumers = staged[staged.index("// consumers"):]
+    assert "if (__any_sync(0xFFFFFFFFu, *static_cast<volatile int *>(&sm.abort) != 0)) return;" in consumers
+    assert "if (!__all_sync(0xFFFFFFFFu, mbar_wait(&sm.full[s], round & 1u)))" in consumers
     # and the barrier that the way out waits for is committed to by nobody else
     assert len(re.findall(r"umma_commit\(&sm\.drained\)", source)) == len(re.findall(r"mbar_drain\(&sm\.drained", source)) == 2
 
