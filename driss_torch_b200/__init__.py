@@ -15,14 +15,17 @@ from pathlib import Path
 from typing import Optional
 
 import torch
+from torch.compiler import is_dynamo_compiling
+from torch.jit import is_scripting
 
 _LIB_DIR = Path(__file__).resolve().parent / "lib"
 lib_path = _LIB_DIR / "libdriss_torch.so"
 kernels_lib_path = _LIB_DIR / "libdtq_b200.so"
+_direct_path = _LIB_DIR / "_direct.so"
 
-if not lib_path.exists() or not kernels_lib_path.exists():
+if not lib_path.exists() or not kernels_lib_path.exists() or not _direct_path.exists():
     raise ImportError(
-        f"{lib_path.name} / {kernels_lib_path.name} not found in {_LIB_DIR}: build them with "
+        f"{lib_path.name} / {kernels_lib_path.name} / {_direct_path.name} not found in {_LIB_DIR}: build them with "
         "`python driss_torch_b200/build.py` (needs nvcc with sm_100a support); there is no fallback path"
     )
 
@@ -31,6 +34,10 @@ torch.ops.import_module("driss_torch_b200.abstract_impls")
 
 ops = torch.ops.DrissTorch
 Tensor = torch.Tensor
+
+# The same operators as plain functions (csrc/direct_calls.cpp): what the wrappers below call in eager mode, 1.6 us cheaper
+# than torch.ops.  TorchScript and Dynamo look into the wrappers and know torch.ops only; both see which branch is theirs.
+from .lib import _direct as direct  # noqa: E402
 
 
 def saturated_cast(
@@ -50,29 +57,39 @@ def saturated_cast(
     reference kernel (src/saturated_cast.cu:66,81).
     """
     assert not transpose, "Transpose is not supported yet"
-    return ops.saturated_cast(x, scale, out_dtype, transpose)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.saturated_cast(x, scale, out_dtype, transpose)
+    return direct.saturated_cast(x, scale, out_dtype, transpose)
 
 
 def saturated_cast_transposed(x: Tensor, scale: Tensor, out_dtype: torch.dtype) -> Tensor:
     """``saturated_cast(x.t().contiguous(), scale, out_dtype)`` without the separate transpose:
     a contiguous ``[cols, rows]`` tensor.  (The reference declares ``transpose`` on
     ``saturated_cast`` but asserts it off, driss_torch/__init__.py:24-38.)"""
-    return ops.saturated_cast_transposed(x, scale, out_dtype)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.saturated_cast_transposed(x, scale, out_dtype)
+    return direct.saturated_cast_transposed(x, scale, out_dtype)
 
 
 def saturated_cast_dual(x: Tensor, scale: Tensor, out_dtype: torch.dtype) -> tuple[Tensor, Tensor]:
     """``(saturated_cast(x), saturated_cast(x.t().contiguous()))`` from a single read of ``x``."""
-    return ops.saturated_cast_dual(x, scale, out_dtype)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.saturated_cast_dual(x, scale, out_dtype)
+    return direct.saturated_cast_dual(x, scale, out_dtype)
 
 
 def amax(x: Tensor) -> Tensor:
     """``max(abs(x))`` as an fp32 tensor of shape [1]."""
-    return ops.amax(x)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.amax(x)
+    return direct.amax(x)
 
 
 def dynamic_scaled_quant(inpt: Tensor, dtype: torch.dtype) -> Tensor:
     """Tensor-wise amax -> scale -> fp8 cast in one launch; returns the fp8 tensor."""
-    return ops.dynamic_scaled_quant(inpt, dtype)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.dynamic_scaled_quant(inpt, dtype)
+    return direct.dynamic_scaled_quant(inpt, dtype)
 
 
 def mx_fp8_quantize(
@@ -93,7 +110,9 @@ def mx_fp8_quantize(
     -- payload [N, M], one scale per 32 rows of a column of ``input`` -- from one read of ``input``;
     ``axis=0`` returns the same bytes with the payload viewed as [M, N]; both together give the ordinary
     blocks with the payload viewed as [N, M]."""
-    return ops.mx_fp8_quantize(input, block_size, axis, transpose, ScalarType)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.mx_fp8_quantize(input, block_size, axis, transpose, ScalarType)
+    return direct.mx_fp8_quantize(input, block_size, axis, transpose, ScalarType)
 
 
 def mx_fp8_bf16(a: Tensor, b: Tensor, a_scale: Tensor, b_scale: Tensor) -> Tensor:
@@ -105,7 +124,9 @@ def mx_fp8_bf16(a: Tensor, b: Tensor, a_scale: Tensor, b_scale: Tensor) -> Tenso
     The bits are those of the straight sum over K, except for few rows and a long K, where K is split and the parts'
     fp32 sums are added in order: there a row's result may differ in the last bit from the same row's in a larger batch
     (``DTQ_GEMM_AUTO`` in ``include/dtq_b200.h`` has the rule, and the kernels that a C caller can name instead)."""
-    return ops.mx_fp8_bf16(a, b, a_scale, b_scale)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.mx_fp8_bf16(a, b, a_scale, b_scale)
+    return direct.mx_fp8_bf16(a, b, a_scale, b_scale)
 
 
 def sweep_mm(
@@ -128,7 +149,10 @@ def sweep_mm(
     ``bf16((acc * x_scale) * w_scale + bias)``.  The arguments after ``out_dtype`` tune the reference's Hopper
     kernels and have no effect here.  For few rows and a long K the last bit may depend on the number of rows, see
     ``mx_fp8_bf16``."""
-    return ops.sweep_mm(x, w, x_scale, w_scale, bias, out_dtype, use_fast_accum, cluster_shape_x, cluster_shape_y,
+    if is_scripting() or is_dynamo_compiling():
+        return ops.sweep_mm(x, w, x_scale, w_scale, bias, out_dtype, use_fast_accum, cluster_shape_x, cluster_shape_y,
+                        cluster_shape_z, transposed, swizzle)
+    return direct.sweep_mm(x, w, x_scale, w_scale, bias, out_dtype, use_fast_accum, cluster_shape_x, cluster_shape_y,
                         cluster_shape_z, transposed, swizzle)
 
 
@@ -138,7 +162,9 @@ def mx_fp4_bf16(a: Tensor, b: Tensor, a_scale: Tensor, b_scale: Tensor) -> Tenso
     bytes row-major, ``b`` [K/2, N] column-major (``w.t()`` of a row-major [N, K/2] payload); returns bf16 [M, N].
     ``mx_fp4_quantize(x, blocked=True)`` produces the payloads and the scales in that layout.  For few rows and a long K
     the last bit may depend on the number of rows, see ``mx_fp8_bf16``."""
-    return ops.mx_fp4_bf16(a, b, a_scale, b_scale)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.mx_fp4_bf16(a, b, a_scale, b_scale)
+    return direct.mx_fp4_bf16(a, b, a_scale, b_scale)
 
 
 # A second name for the MX op; the reference symbol is mx_fp8_quantize.
@@ -152,35 +178,47 @@ def dynamic_scaled_quant_with_scale(inpt: Tensor, dtype: torch.dtype) -> tuple[T
 
     The payload is computed from the double-precision scale, not from the returned fp32 one.
     """
-    return ops.dynamic_scaled_quant_with_scale(inpt, dtype)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.dynamic_scaled_quant_with_scale(inpt, dtype)
+    return direct.dynamic_scaled_quant_with_scale(inpt, dtype)
 
 
 def dynamic_scaled_quant_rowwise(inpt: Tensor, dtype: torch.dtype) -> tuple[Tensor, Tensor, Tensor]:
     """Per-row amax -> scale -> fp8 cast; returns (payload, amax [M,1], scale [M,1])."""
-    return ops.dynamic_scaled_quant_rowwise(inpt, dtype)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.dynamic_scaled_quant_rowwise(inpt, dtype)
+    return direct.dynamic_scaled_quant_rowwise(inpt, dtype)
 
 
 def cast_with_amax(inpt: Tensor, amax_value: Tensor, dtype: torch.dtype) -> tuple[Tensor, Tensor]:
     """The cast phase of ``dynamic_scaled_quant`` for a given device-resident amax; returns (payload, scale)."""
-    return ops.cast_with_amax(inpt, amax_value, dtype)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.cast_with_amax(inpt, amax_value, dtype)
+    return direct.cast_with_amax(inpt, amax_value, dtype)
 
 
 def cast_with_amax_dual(inpt: Tensor, amax_value: Tensor, dtype: torch.dtype) -> tuple[Tensor, Tensor, Tensor]:
     """``(payload, payload_t, scale)``: ``cast_with_amax`` of ``x`` and of ``x.t().contiguous()`` from one read."""
-    return ops.cast_with_amax_dual(inpt, amax_value, dtype)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.cast_with_amax_dual(inpt, amax_value, dtype)
+    return direct.cast_with_amax_dual(inpt, amax_value, dtype)
 
 
 def dynamic_scaled_quant_dual(inpt: Tensor, dtype: torch.dtype) -> tuple[Tensor, Tensor, Tensor, Tensor]:
     """``(payload, payload_t, amax, scale)`` with ``payload == dynamic_scaled_quant(x)`` and
     ``payload_t == dynamic_scaled_quant(x.t().contiguous())``: the two fp8 operands tensor-wise scaled
     training needs, in two reads of ``x`` (amax, then both casts at once)."""
-    return ops.dynamic_scaled_quant_dual(inpt, dtype)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.dynamic_scaled_quant_dual(inpt, dtype)
+    return direct.dynamic_scaled_quant_dual(inpt, dtype)
 
 
 def mx_fp8_quantize_with_amax(input: Tensor) -> tuple[Tensor, Tensor, Tensor]:
     """``mx_fp8_quantize(x)`` plus ``max(0, amax(x))`` (fp32 [1]) from the same read of ``x``: with
     ``cast_with_amax`` behind it, a tensor is quantised both tensor-wise and MX in two reads instead of three."""
-    return ops.mx_fp8_quantize_with_amax(input)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.mx_fp8_quantize_with_amax(input)
+    return direct.mx_fp8_quantize_with_amax(input)
 
 
 def mx_fp4_quantize(input: Tensor, blocked: bool = False) -> tuple[Tensor, Tensor]:
@@ -188,7 +226,9 @@ def mx_fp4_quantize(input: Tensor, blocked: bool = False) -> tuple[Tensor, Tenso
     lower index in the low nibble -- the operands of the reference's ``mx_fp4_bf16``, which has no
     producer kernel there.  Same scale rule as ``mx_fp8_quantize`` with e2m1's largest exponent 2.
     ``blocked``: the scales in the blocked layout ``mx_fp4_bf16`` takes (as ``mx_fp8_quantize_blocked``)."""
-    return ops.mx_fp4_quantize(input, blocked)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.mx_fp4_quantize(input, blocked)
+    return direct.mx_fp4_quantize(input, blocked)
 
 
 def mx_fp8_quantize_dual(input: Tensor, blocked: bool = False) -> tuple[Tensor, Tensor, Tensor, Tensor]:
@@ -196,13 +236,17 @@ def mx_fp8_quantize_dual(input: Tensor, blocked: bool = False) -> tuple[Tensor, 
     ``(p_t, s_t) == mx_fp8_quantize(x.t().contiguous())``, from a single read of ``x``
     (both dimensions multiples of 32).  ``blocked=True``: both scale tensors as
     ``mx_fp8_quantize_blocked`` lays them out, ready for the MX GEMM."""
-    return ops.mx_fp8_quantize_dual(input, blocked)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.mx_fp8_quantize_dual(input, blocked)
+    return direct.mx_fp8_quantize_dual(input, blocked)
 
 
 def mx_fp8_quantize_blocked(input: Tensor) -> tuple[Tensor, Tensor]:
     """``mx_fp8_quantize`` with the E8M0 scales already in the blocked (128x4-atom) layout that the MX
     GEMM ``mx_fp8_bf16`` expects, i.e. without the separate ``to_blocked`` pass; zero in the padding."""
-    return ops.mx_fp8_quantize_blocked(input)
+    if is_scripting() or is_dynamo_compiling():
+        return ops.mx_fp8_quantize_blocked(input)
+    return direct.mx_fp8_quantize_blocked(input)
 
 
 def check_device_status() -> None:

@@ -1,11 +1,13 @@
-"""In-tree build of the two shared libraries (no cmake, no JIT cache).
+"""In-tree build of the three shared libraries (no cmake, no JIT cache).
 
 * ``lib/libdtq_b200.so``   -- the torch-free CUDA kernels and their C ABI
   (``include/dtq_b200.h``), built with nvcc for sm_100a only.
 * ``lib/libdriss_torch.so`` -- ``register_ops.cpp``: the ``TORCH_LIBRARY(DrissTorch)``
   registration that binds the C ABI into the PyTorch dispatcher, built with g++.
+* ``lib/_direct.so`` -- ``direct_calls.cpp``: the operators as plain Python functions (an extension module),
+  built with g++.
 
-``python driss_torch_b200/build.py`` builds both; objects are rebuilt only when a
+``python driss_torch_b200/build.py`` builds all; objects are rebuilt only when a
 source or header is newer.  The reference builds one ``libdriss_torch.so`` through
 scikit-build/CMake with the same architecture flags (CMakeLists.txt:25-27).
 """
@@ -97,15 +99,13 @@ def build_kernels(force: bool = False, extra_flags=()) -> Path:
     return so
 
 
-def build_torch_binding(force: bool = False) -> Path:
+def _build_torch_library(source: str, target: str, libs, force: bool) -> Path:
     import torch
     from torch.utils.cpp_extension import include_paths
 
     LIB.mkdir(exist_ok=True)
-    OBJ.mkdir(exist_ok=True)
-    src = CSRC / "register_ops.cpp"
-    so = LIB / "libdriss_torch.so"
-    kernels = LIB / "libdtq_b200.so"
+    src = CSRC / source
+    so = LIB / target
     dep_time = max(src.stat().st_mtime, _newest(list(INCLUDE.glob("*.h"))))
     if not (force or not so.exists() or so.stat().st_mtime < dep_time):
         return so
@@ -115,12 +115,19 @@ def build_torch_binding(force: bool = False) -> Path:
     cmd = [
         "g++", "-std=c++17", "-O2", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={abi}", *incs, str(src),
         "-o", str(so),
-        f"-L{LIB}", "-ldtq_b200", f"-L{torch_lib}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
+        f"-L{LIB}", f"-L{torch_lib}", *libs,
         f"-L{CUDA_HOME / 'lib64'}", "-lcudart",
         "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}", f"-Wl,-rpath,{CUDA_HOME / 'lib64'}",
     ]
-    assert kernels.exists(), "build the kernel library first"
     _run(cmd)
+    return so
+
+
+def build_torch_binding(force: bool = False) -> Path:
+    assert (LIB / "libdtq_b200.so").exists(), "build the kernel library first"
+    so = _build_torch_library("register_ops.cpp", "libdriss_torch.so",
+                              ["-ldtq_b200", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"], force)
+    _build_torch_library("direct_calls.cpp", "_direct.so", ["-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10"], force)
     return so
 
 
