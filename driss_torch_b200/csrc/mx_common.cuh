@@ -95,6 +95,8 @@ __device__ __forceinline__ int64_t scale_offset(int64_t blk, int64_t kblocks, in
 // `thread` of `threads` in all takes its share.  One item is the four bytes that a row of the last row band has in one of
 // its atoms (32 x 16 bytes: byte group q of chunk l is row 32 q + l; a thread takes a chunk), or the tail of one row.
 // No divisions: 64-bit ones made these few bytes take longer than the cast (2016 x 4096: 4.8 us without padding, 8.5 with).
+// And no single bytes where the array allows it: the scales of 8 or 16 rows are nearly all padding, and with four byte stores
+// per group the padding blocks were still at it 2 us after the cast itself (16 x 4096: 3.2 us of a decode step's chain).
 __host__ __device__ inline int64_t scale_padding_items(int64_t rows, int64_t kblocks) {
   return (rows % 128 ? (kblocks + 3) / 4 * 32 : 0) + (kblocks % 4 ? rows : 0);
 }
@@ -103,11 +105,20 @@ __device__ __forceinline__ void zero_scale_padding(uint8_t *scales, int64_t rows
   const int used = int(rows & 127);  // rows of the last band that exist
   if (used) {
     uint8_t *band = scales + (rows >> 7) * katoms * 512;
-    for (int64_t i = thread; i < katoms * 32; i += threads) {
+    const bool wide = (reinterpret_cast<uintptr_t>(scales) & 15) == 0;
+    for (int64_t i = thread; i < katoms * 32; i += threads) {  // atom i / 32, chunk i % 32
+      const int l = int(i & 31);
+      if (wide && l >= used) {
+        *reinterpret_cast<uint4 *>(band + i * 16) = make_uint4(0, 0, 0, 0);
+        continue;
+      }
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        uint8_t *p = band + i * 16 + q * 4;  // atom i / 32, chunk i % 32
-        if (32 * q + int(i & 31) >= used) p[0] = p[1] = p[2] = p[3] = 0;
+        uint8_t *p = band + i * 16 + q * 4;
+        if (32 * q + l >= used) {
+          if (wide) *reinterpret_cast<uint32_t *>(p) = 0;
+          else p[0] = p[1] = p[2] = p[3] = 0;
+        }
       }
     }
   }
@@ -140,9 +151,9 @@ static_assert(takes_every_tile_once(7, 9, 2) && takes_every_tile_once(7, 7, 0) &
                   takes_every_tile_once(13, 3, 0) && takes_every_tile_once(1, 4, 3),
               "blocks beside the padding share out the tiles");
 
-// Spare blocks of `threads` threads for it, about two items per thread.
+// Spare blocks of `threads` threads for it, about one item per thread.
 inline int64_t scale_padding_blocks(int64_t rows, int64_t kblocks, int threads) {
-  const int64_t n = (scale_padding_items(rows, kblocks) + 2 * threads - 1) / (2 * threads);
+  const int64_t n = (scale_padding_items(rows, kblocks) + threads - 1) / threads;
   return n < 1024 ? n : 1024;
 }
 
