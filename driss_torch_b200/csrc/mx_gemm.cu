@@ -955,13 +955,18 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 //     partials of its share of the tokens through distributed shared memory, in the order of K;
 //   * while the kernel before this one drains, the first stages of weights are already asked into L2: that is where this
 //     GPU's memory is coherent, so it does not matter whether that kernel still writes them.
-// Measured (B200, back to back, weights not in L2; 128 x 128 kernel -> this one; reading the weights alone at the measured
-// copy rate): 8 x 8192 x 8192 MXFP8 27.9 -> 13.6 us (10.3), 16 x 8192 x 4096 row-wise 15.4 -> 8.5 (5.1),
+// Measured (B200, products back to back, weights not in L2, 8 stages prefetched; 128 x 128 kernel -> this one; reading the weights
+// alone at the measured copy rate): 8 x 8192 x 8192 MXFP8 27.9 -> 13.6 us (10.3), 16 x 8192 x 4096 row-wise 15.4 -> 8.5 (5.1),
 // 16 x 256 x 8192 16.5 -> 5.0, 300 x 2048 x 8192 19.4 -> 14.3.
 constexpr int kSplitThreads = 192;   // producer warp, MMA warp, 4 warps that empty tensor memory; all six add up and store
 constexpr int kSplitWarps = kSplitThreads / 32;
 constexpr int kMaxSplits = 8;        // portable cluster size
-constexpr int kSplitPrefetch = 8;    // stages of weights asked into L2 ahead of the dependency
+// Stages of weights asked into L2 ahead of the dependency.  Few: the kernel that the dependency waits for (the cast of the
+// tokens) reads through the same memory, and it is what everybody waits for.  Cast and product, us, with 0 / 2 / 4 / 8 stages:
+// MXFP8 8 x 8192 x 8192 16.7 / 16.4 / 16.6 / 17.0, 100 x 4096 x 8192 16.2 / 15.6 / 15.9 / 16.8, row-wise 16 x 8192 x 4096
+// 11.6 / 11.2 / 11.5 / 12.1, 60 x 8192 x 4096 13.2 / 12.9 / 13.2 / 13.7, MXFP4 16 x 8192 x 8192 12.1 / 11.7 / 11.8 / 12.6; where two
+// CTAs share a tile of 64 stages (8 x 16384 x 8192) 27.0 / 26.4 / 26.1 / 26.4.
+constexpr int kSplitPrefetch = 2;
 
 template <int BN, int STAGES, int MODE>
 struct __align__(1024) SplitSmem {
