@@ -382,3 +382,36 @@ def test_outputs_are_filled_under_deterministic_algorithms():
     for name, (outs, fills) in filled.items():
         assert plain[name][1] == 0 and fills >= len(outs), f"{name}: {fills} fills of {len(outs)} outputs"
         assert all(torch.equal(a, b) for a, b in zip(outs, plain[name][0])), name
+
+
+# ---- inputs of up to 1 MiB take one cluster, larger ones (and the exchanging entry point) the grid ------------------------
+
+@pytest.mark.parametrize("fp8_dtype", FP8_DTYPES)
+@pytest.mark.parametrize("in_dtype", IN_DTYPES)
+@pytest.mark.parametrize("special", [False, True])
+def test_one_cluster_equals_the_grid(in_dtype, fp8_dtype, special):
+    from driss_torch_b200 import _cabi
+
+    slots = torch.zeros(_cabi.load().dtq_p2p_exchange_bytes() // 8, dtype=torch.int64, device="cuda")
+    per_chunk = 16 // torch.empty(0, dtype=in_dtype).element_size()
+    # 16-byte chunks: where the CTAs of the cluster and the chunks per thread change, and elements past the last whole chunk
+    sizes = [(0, 1), (0, per_chunk - 1), (1, 0), (511, 1), (512, 0), (512, 3), (1025, 0), (2048, 1), (4096, 0), (4097, 2), (8192, 0),
+             (8193, 1), (32768, 0), (32769, 0), (65535, per_chunk - 1), (65536, 0), (65536, 1)]
+    g = torch.Generator().manual_seed(5)
+    for epoch, (chunks, extra) in enumerate(sizes, 1):
+        n = chunks * per_chunk + extra
+        x = torch.randn(n, 1, generator=g) * 10.0 ** (epoch % 7 - 3)
+        if special:
+            x[-1] = float("nan")  # a NaN is no maximum
+            if epoch % 3 == 0:
+                x[n // 2] = float("-inf")
+            if epoch % 3 == 1:
+                x.mul_(0.0)
+        x = x.to(in_dtype).cuda()
+        room = torch.full((n + 64,), 0xAA, dtype=torch.uint8, device="cuda")
+        amax, scale, want_amax, want_scale = (torch.full((1,), -1.0, device="cuda") for _ in range(4))
+        got = _cabi.dynamic_scaled_quant(x, fp8_dtype, out=room[32:32 + n].view(fp8_dtype).view(n, 1), amax_out=amax, scale_out=scale)
+        want = _cabi.dynamic_scaled_quant_p2p(x, fp8_dtype, [slots.data_ptr()], 0, epoch, amax_out=want_amax, scale_out=want_scale)
+        assert torch.equal(got.view(torch.uint8), want.view(torch.uint8)), (chunks, extra)
+        assert _bits(amax) == _bits(want_amax) and _bits(scale) == _bits(want_scale), (chunks, extra)
+        assert (room[:32] == 0xAA).all() and (room[32 + n:] == 0xAA).all()
