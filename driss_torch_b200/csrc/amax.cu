@@ -93,12 +93,11 @@ amax_kernel(const void *__restrict__ in, float *__restrict__ out, int64_t numel,
   // harmless whatever the predecessor still writes (see l2_prefetch_bulk).  What it hides is the start of the stream, which a
   // launch of one or two tiles per block consists of.  Measured, amax then both casts of bf16 (amax alone back to back), us, without
   // / with: 3500 x 4096 17.2 / 15.8 (7.8 / 6.6), 5003 x 4096 23.0 / 21.2 (10.6 / 9.9), 3570 x 6416 25.4 / 23.6 (11.0 / 10.2), 8192 x 8192
-  // 66.9 / 66.3 (22.6 / 20.1), up to 2048 x 4096 the same; with the second tile too 5003 x 4096 20.8, 8192 x 8192 67.0 (22.1).
+  // 66.9 / 66.3 (22.6 / 20.1), up to 2048 x 4096 the same, 16384 x 8192 131.0 / 132.4, so not beyond 128 MiB; with the second tile
+  // too 5003 x 4096 20.8, 8192 x 8192 67.0 (22.1).
   constexpr int64_t kTile = int64_t(kAmaxThreads) * UNROLL;
-  if (threadIdx.x == 0 && blockIdx.x * kTile < nchunks) {
-    const int64_t left = nchunks - blockIdx.x * kTile;
-    l2_prefetch_bulk(body + blockIdx.x * kTile, unsigned((left < kTile ? left : kTile) * sizeof(uint4)));
-  }
+  if (threadIdx.x == 0 && nchunks * int64_t(sizeof(uint4)) <= kPrefetchToBytes)
+    prefetch_first_tile(body, blockIdx.x * kTile, kTile, nchunks);
   pdl_wait();
   const float identity = -INFINITY;
   AbsMax<IN> acc(identity);

@@ -69,6 +69,13 @@ inline cudaError_t launch_after_dependency(void (*kernel)(KArgs...), dim3 grid, 
 
 inline bool aligned_to(const void *p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 
+// Blocks of a stream kernel that call prefetch_first_tile (dtq_device.cuh, with the figures): none for inputs outside the range
+// in which it pays.
+constexpr int64_t kPrefetchFromBytes = int64_t(16) << 20, kPrefetchToBytes = int64_t(128) << 20;
+inline unsigned prefetch_blocks(int64_t input_bytes, unsigned blocks, int64_t to_bytes = kPrefetchToBytes) {
+  return input_bytes >= kPrefetchFromBytes && input_bytes <= to_bytes ? blocks : 0;
+}
+
 inline int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // Grid for a persistent kernel that walks `tiles` tiles grid-stride: at most `max_grid` blocks,

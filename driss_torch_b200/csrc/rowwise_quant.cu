@@ -20,6 +20,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
+constexpr unsigned kPrefetchers = 148 * 8;  // see prefetch_first_tile
 
 template <int IN>
 struct RowIn;
@@ -79,7 +80,9 @@ struct RowIn<DTQ_F32> {
 // independent warps, one row each, and never synchronises.  TEAM_WARPS > 1: the CTA is the team
 // (one row per CTA), so short rows get small CTAs, many of which are resident per SM and drift
 // out of phase -- some loading while others convert -- which keeps HBM busy.
-template <int IN, int OUT, int CHUNKS, int TEAM_WARPS>
+// PREFETCH: the first blocks ask for their rows ahead of the dependency (an instantiation of its own: with the test for it at run
+// time the compiler orders the rest differently, and 1024 x 4096 bf16 took 3.9 us instead of 3.5).
+template <int IN, int OUT, int CHUNKS, int TEAM_WARPS, bool PREFETCH>
 __global__ void __launch_bounds__(TEAM_WARPS == 1 ? kThreads : 32 * TEAM_WARPS)
 rowwise_regs_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float *__restrict__ amax_out,
                     float *__restrict__ scale_out, int64_t rows, int chunks_per_row) {
@@ -89,6 +92,11 @@ rowwise_regs_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, flo
   // programmatic dependent launch, both ways (see dtq_device.cuh): blocks may become resident under the tail of the
   // kernel before this one, and what is queued behind this one under its own tail
   pdl_launch_dependents();
+  if constexpr (PREFETCH) {
+    constexpr int64_t kBlockRows = TEAM_WARPS == 1 ? kWarps : 1;
+    if (threadIdx.x == 0 && blockIdx.x < kPrefetchers)
+      prefetch_first_tile(in, blockIdx.x * kBlockRows * chunks_per_row, kBlockRows * chunks_per_row, rows * chunks_per_row);
+  }
   pdl_wait();
   int64_t row;
   int t;
@@ -185,9 +193,10 @@ int launch_regs(const void *in, void *out, float *amax_out, float *scale_out, in
                 cudaStream_t st) {
   const unsigned grid = static_cast<unsigned>(TEAM_WARPS == 1 ? ceil_div64(rows, kWarps) : rows);
   const int threads = TEAM_WARPS == 1 ? kThreads : 32 * TEAM_WARPS;
-  return cuda_status(launch_after_dependency(rowwise_regs_kernel<IN, OUT, CHUNKS, TEAM_WARPS>, dim3(grid), dim3(threads), 0, st,
-                                             static_cast<const uint4 *>(in), static_cast<uint8_t *>(out), amax_out, scale_out,
-                                             rows, chunks_per_row));
+  auto kernel = prefetch_blocks(rows * chunks_per_row * 16, kPrefetchers) ? rowwise_regs_kernel<IN, OUT, CHUNKS, TEAM_WARPS, true>
+                                                                          : rowwise_regs_kernel<IN, OUT, CHUNKS, TEAM_WARPS, false>;
+  return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(threads), 0, st, static_cast<const uint4 *>(in),
+                                             static_cast<uint8_t *>(out), amax_out, scale_out, rows, chunks_per_row));
 }
 
 // Smallest team that keeps a thread at <= 4 chunks (64 bytes in flight); the largest team may

@@ -22,6 +22,7 @@ constexpr int kUnroll = 2;  // 128-bit loads in flight per thread: 8 KB tiles.  
 // then store burst).  The in-kernel loop then only matters beyond 2^31-1 tiles.
 constexpr int64_t kBlocksPerSmCap = 1 << 20;
 constexpr int kThreads = 256;
+constexpr unsigned kPrefetchers = 3 * 148 * 8;  // see prefetch_first_tile
 
 // One 16-byte input chunk -> its fp8 bytes, stored with one instruction.
 template <int IN, int OUT>
@@ -66,15 +67,16 @@ struct Chunk<DTQ_F32, OUT> {
 template <int IN, int OUT, int UNROLL>
 __global__ void __launch_bounds__(kThreads)
 saturated_cast_stream(const uint4 *__restrict__ in, uint8_t *__restrict__ out, const float *__restrict__ scale,
-                      int64_t numel) {
+                      int64_t numel, unsigned prefetchers) {
   using C = Chunk<IN, OUT>;
   // launched so that its blocks may become resident under the tail of the kernel before it on the stream
   // (launch latency and block ramp hidden); nothing is read before that kernel has completed
   pdl_launch_dependents();
-  pdl_wait();
-  const typename C::Scale s = C::load_scale(scale);
   const int64_t nchunks = numel / C::kElems;
   constexpr int64_t kTile = int64_t(kThreads) * UNROLL;
+  if (threadIdx.x == 0 && blockIdx.x < prefetchers) prefetch_first_tile(in, blockIdx.x * kTile, kTile, nchunks);
+  pdl_wait();
+  const typename C::Scale s = C::load_scale(scale);
 
   for (int64_t tile = blockIdx.x; tile * kTile < nchunks; tile += gridDim.x) {
     const int64_t first = tile * kTile + threadIdx.x;
@@ -119,7 +121,8 @@ int launch(const void *in, void *out, const float *scale, int64_t numel, const D
     const int64_t tiles = ceil_div64(numel / C::kElems, int64_t(kThreads) * kUnroll);
     const int grid = balanced_grid(tiles, max_grid);
     return cuda_status(launch_after_dependency(saturated_cast_stream<IN, OUT, kUnroll>, dim3(grid), dim3(kThreads), 0, st,
-                                               static_cast<const uint4 *>(in), static_cast<uint8_t *>(out), scale, numel));
+                                               static_cast<const uint4 *>(in), static_cast<uint8_t *>(out), scale, numel,
+                                               prefetch_blocks(numel * (16 / C::kElems), kPrefetchers)));
   } else {
     const int64_t blocks = ceil_div64(numel, kThreads);
     const int grid = static_cast<int>(blocks < max_grid ? blocks : max_grid);
