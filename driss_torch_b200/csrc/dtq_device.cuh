@@ -108,6 +108,10 @@ __device__ __forceinline__ void st_cluster_u32(uint32_t cluster_addr, uint32_t v
 // So it stops at 128 MiB, except in the MX cast.  1184 blocks are the first wave of 256-thread blocks; further ones pay in the
 // lightest of the kernels only.  Below 16 MiB the grid is not much more than what is resident at once, and the loads follow at the
 // prefetch's heels: 1300 x 4096 cast 2.7 / 2.9, row-wise 3.6 / 4.0.
+// Up to 512 KiB it is on again, for the tokens of a decode step: the product queued behind asks for its weights as soon as it is
+// resident, and the cast's reads would stand behind those.  Cast and product, us, without / with, both with two stages of
+// weights per CTA: row-wise 16 x 8192 x 4096 11.2 / 10.8, 60 x 8192 x 4096 12.9 / 12.7, MXFP8 17 x 2048 x 8192 8.6 / 8.4, 16 x 4096 x
+// 4096 8.1 / 8.0, 8 x 8192 x 8192 16.3 / 16.3, MXFP4 16 x 8192 x 8192 11.7 / 11.55.
 __device__ __forceinline__ void prefetch_first_tile(const uint4 *in, int64_t first, int64_t chunks, int64_t nchunks) {
   const int64_t left = nchunks - first;
   if (left > 0) l2_prefetch_bulk(in + first, unsigned((left < chunks ? left : chunks) * sizeof(uint4)));

@@ -72,8 +72,9 @@ inline bool aligned_to(const void *p, uintptr_t a) { return (reinterpret_cast<ui
 // Blocks of a stream kernel that call prefetch_first_tile (dtq_device.cuh, with the figures): none for inputs outside the range
 // in which it pays.
 constexpr int64_t kPrefetchFromBytes = int64_t(16) << 20, kPrefetchToBytes = int64_t(128) << 20;
+constexpr int64_t kPrefetchSmallBytes = int64_t(512) << 10;  // and none above: the tokens of a decode step
 inline unsigned prefetch_blocks(int64_t input_bytes, unsigned blocks, int64_t to_bytes = kPrefetchToBytes) {
-  return input_bytes >= kPrefetchFromBytes && input_bytes <= to_bytes ? blocks : 0;
+  return input_bytes <= kPrefetchSmallBytes || (input_bytes >= kPrefetchFromBytes && input_bytes <= to_bytes) ? blocks : 0;
 }
 
 inline int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }

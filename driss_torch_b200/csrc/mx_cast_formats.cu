@@ -142,22 +142,28 @@ __device__ __forceinline__ void convert_store(const float (&f)[N], float inv, ui
   }
 }
 
+// Few tokens only (see prefetch_first_tile): with the larger inputs that the other casts ask ahead for, 8192 x 8192 to e2m1 took
+// 27.8 us instead of 26.8.
+constexpr unsigned kPrefetchers = 148;
+
 // nchunks 16-byte chunks; a block of 32 elements is kLanes consecutive chunks (never split across warps).
 template <int IN, int FMT>
 __global__ void __launch_bounds__(kThreadsF, 2048 / kThreadsF)
 mx_formats_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, uint8_t *__restrict__ scales,
                   int64_t nchunks, int64_t kblocks,  // kblocks > 0: scales in the MX GEMM's blocked layout, that many per row
-                  int64_t rows, unsigned pad_blocks) {
+                  int64_t rows, unsigned pad_blocks, unsigned prefetchers) {
   // programmatic dependent launch, both ways (see dtq_device.cuh): blocks may become resident under the tail of the
   // kernel before this one, and what is queued behind this one under its own tail
   pdl_launch_dependents();
+  constexpr int64_t kTile = int64_t(kThreadsF) * kUnrollF;
+  const int64_t first_tile = int64_t(blockIdx.x) - pad_blocks;  // negative: this block writes padding
+  if (threadIdx.x == 0 && first_tile >= 0 && first_tile < prefetchers) prefetch_first_tile(in, first_tile * kTile, kTile, nchunks);
   pdl_wait();
   using I = MxIn<IN>;
   using O = MxOut<FMT>;
   constexpr int kLanes = 32 / I::kElems;                        // lanes per MX block
   constexpr int kChunkBytesOut = I::kElems * O::kBitsPerElem / 8;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int64_t kTile = int64_t(kThreadsF) * kUnrollF;
   if (blockIdx.x < pad_blocks) {  // the first blocks of the grid write the padding of blocked scales, if there is any
     zero_scale_padding(scales, rows, kblocks, int64_t(blockIdx.x) * kThreadsF + threadIdx.x, int64_t(pad_blocks) * kThreadsF);
     return;
@@ -213,7 +219,8 @@ int launch_formats(const void *in, void *payload, void *scales, int64_t numel, i
   return cuda_status(launch_after_dependency(mx_formats_kernel<IN, FMT>, dim3(grid), dim3(kThreadsF), 0, st,
                                              static_cast<const uint4 *>(in), static_cast<uint8_t *>(payload),
                                              static_cast<uint8_t *>(scales), nchunks, kblocks, rows,
-                                             static_cast<unsigned>(pad_blocks)));
+                                             static_cast<unsigned>(pad_blocks),
+                                             prefetch_blocks(nchunks * 16, kPrefetchers, 0)));
 }
 
 template <int IN>
