@@ -69,12 +69,13 @@ inline cudaError_t launch_after_dependency(void (*kernel)(KArgs...), dim3 grid, 
 
 inline bool aligned_to(const void *p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 
-// Blocks of a stream kernel that call prefetch_first_tile (dtq_device.cuh, with the figures): none for inputs outside the range
-// in which it pays.
+// Whether the first blocks of a stream kernel are to call prefetch_first_tile (dtq_device.cuh, with the figures).  The kernels have
+// an instantiation for either answer: with the question at run time the compiler orders the rest of them differently, and those
+// that do not ask ahead lost up to 2 %.
 constexpr int64_t kPrefetchFromBytes = int64_t(16) << 20, kPrefetchToBytes = int64_t(128) << 20;
 constexpr int64_t kPrefetchSmallBytes = int64_t(512) << 10;  // and none above: the tokens of a decode step
-inline unsigned prefetch_blocks(int64_t input_bytes, unsigned blocks, int64_t to_bytes = kPrefetchToBytes) {
-  return input_bytes <= kPrefetchSmallBytes || (input_bytes >= kPrefetchFromBytes && input_bytes <= to_bytes) ? blocks : 0;
+inline bool prefetch_pays(int64_t input_bytes, int64_t to_bytes = kPrefetchToBytes) {
+  return input_bytes <= kPrefetchSmallBytes || (input_bytes >= kPrefetchFromBytes && input_bytes <= to_bytes);
 }
 
 inline int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }

@@ -28,17 +28,18 @@ constexpr int kUnroll = 4;  // tied to the scale-byte mapping below: lane&3 pick
 
 // nchunks = numel / 8 is a multiple of 4.  A warp owns kUnroll consecutive 512-byte rows of
 // chunks; a CTA tile is kThreads * kUnroll chunks.
-template <bool BLOCKED>
+template <bool BLOCKED, bool PREFETCH>
 __global__ void __launch_bounds__(kThreads, 2048 / kThreads)
 mx_stream_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, uint8_t *__restrict__ scales,
-                 int64_t nchunks, int64_t kblocks, int64_t katoms, int64_t rows, unsigned pad_blocks,
-                 unsigned prefetchers) {
+                 int64_t nchunks, int64_t kblocks, int64_t katoms, int64_t rows, unsigned pad_blocks) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int64_t kTile = int64_t(kThreads) * kUnroll;
   // may have become resident under the tail of the kernel before it on the stream: wait for that kernel
   pdl_launch_dependents();
-  const int64_t first_tile = int64_t(blockIdx.x) - (BLOCKED ? pad_blocks : 0);  // negative: this block writes padding
-  if (threadIdx.x == 0 && first_tile >= 0 && first_tile < prefetchers) prefetch_first_tile(in, first_tile * kTile, kTile, nchunks);
+  if constexpr (PREFETCH) {
+    const int64_t first_tile = int64_t(blockIdx.x) - (BLOCKED ? pad_blocks : 0);  // negative: this block writes padding
+    if (threadIdx.x == 0 && first_tile >= 0 && first_tile < kPrefetchers) prefetch_first_tile(in, first_tile * kTile, kTile, nchunks);
+  }
   pdl_wait();
   if constexpr (BLOCKED) {  // the first blocks of the grid write the padding, if there is any
     if (blockIdx.x < pad_blocks) {
@@ -114,10 +115,11 @@ int launch_mx(const void *in_bf16, void *payload, void *scales_e8m0, int64_t row
     const int64_t tiles = ceil_div64(nchunks, int64_t(kThreads) * kUnroll);
     const int64_t pad_blocks = BLOCKED ? scale_padding_blocks(rows, kblocks, kThreads) : 0;
     const int grid = balanced_grid(tiles, max_grid) + static_cast<int>(pad_blocks);
-    return cuda_status(launch_after_dependency(mx_stream_kernel<BLOCKED>, dim3(grid), dim3(kThreads), 0, st,
+    auto kernel = prefetch_pays(numel * 2, INT64_MAX) ? mx_stream_kernel<BLOCKED, true> : mx_stream_kernel<BLOCKED, false>;
+    return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(kThreads), 0, st,
                                                static_cast<const uint4 *>(in_bf16), static_cast<uint8_t *>(payload),
                                                static_cast<uint8_t *>(scales_e8m0), nchunks, kblocks, katoms, rows,
-                                               static_cast<unsigned>(pad_blocks), prefetch_blocks(numel * 2, kPrefetchers, INT64_MAX)));
+                                               static_cast<unsigned>(pad_blocks)));
   } else {
     const int64_t blocks = ceil_div64(numel / 32, kThreads);
     const int grid = static_cast<int>(blocks < max_grid ? blocks : max_grid);

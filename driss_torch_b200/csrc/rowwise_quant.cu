@@ -80,8 +80,7 @@ struct RowIn<DTQ_F32> {
 // independent warps, one row each, and never synchronises.  TEAM_WARPS > 1: the CTA is the team
 // (one row per CTA), so short rows get small CTAs, many of which are resident per SM and drift
 // out of phase -- some loading while others convert -- which keeps HBM busy.
-// PREFETCH: the first blocks ask for their rows ahead of the dependency (an instantiation of its own: with the test for it at run
-// time the compiler orders the rest differently, and 1024 x 4096 bf16 took 3.9 us instead of 3.5).
+// PREFETCH: the first blocks ask for their rows ahead of the dependency.
 template <int IN, int OUT, int CHUNKS, int TEAM_WARPS, bool PREFETCH>
 __global__ void __launch_bounds__(TEAM_WARPS == 1 ? kThreads : 32 * TEAM_WARPS)
 rowwise_regs_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float *__restrict__ amax_out,
@@ -193,7 +192,7 @@ int launch_regs(const void *in, void *out, float *amax_out, float *scale_out, in
                 cudaStream_t st) {
   const unsigned grid = static_cast<unsigned>(TEAM_WARPS == 1 ? ceil_div64(rows, kWarps) : rows);
   const int threads = TEAM_WARPS == 1 ? kThreads : 32 * TEAM_WARPS;
-  auto kernel = prefetch_blocks(rows * chunks_per_row * 16, kPrefetchers) ? rowwise_regs_kernel<IN, OUT, CHUNKS, TEAM_WARPS, true>
+  auto kernel = prefetch_pays(rows * chunks_per_row * 16) ? rowwise_regs_kernel<IN, OUT, CHUNKS, TEAM_WARPS, true>
                                                                           : rowwise_regs_kernel<IN, OUT, CHUNKS, TEAM_WARPS, false>;
   return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(threads), 0, st, static_cast<const uint4 *>(in),
                                              static_cast<uint8_t *>(out), amax_out, scale_out, rows, chunks_per_row));

@@ -64,17 +64,19 @@ struct Chunk<DTQ_F32, OUT> {
   }
 };
 
-template <int IN, int OUT, int UNROLL>
+template <int IN, int OUT, int UNROLL, bool PREFETCH>
 __global__ void __launch_bounds__(kThreads)
 saturated_cast_stream(const uint4 *__restrict__ in, uint8_t *__restrict__ out, const float *__restrict__ scale,
-                      int64_t numel, unsigned prefetchers) {
+                      int64_t numel) {
   using C = Chunk<IN, OUT>;
   // launched so that its blocks may become resident under the tail of the kernel before it on the stream
   // (launch latency and block ramp hidden); nothing is read before that kernel has completed
   pdl_launch_dependents();
   const int64_t nchunks = numel / C::kElems;
   constexpr int64_t kTile = int64_t(kThreads) * UNROLL;
-  if (threadIdx.x == 0 && blockIdx.x < prefetchers) prefetch_first_tile(in, blockIdx.x * kTile, kTile, nchunks);
+  if constexpr (PREFETCH) {
+    if (threadIdx.x == 0 && blockIdx.x < kPrefetchers) prefetch_first_tile(in, blockIdx.x * kTile, kTile, nchunks);
+  }
   pdl_wait();
   const typename C::Scale s = C::load_scale(scale);
 
@@ -120,9 +122,10 @@ int launch(const void *in, void *out, const float *scale, int64_t numel, const D
   if (aligned_to(in, 16) && aligned_to(out, 8)) {
     const int64_t tiles = ceil_div64(numel / C::kElems, int64_t(kThreads) * kUnroll);
     const int grid = balanced_grid(tiles, max_grid);
-    return cuda_status(launch_after_dependency(saturated_cast_stream<IN, OUT, kUnroll>, dim3(grid), dim3(kThreads), 0, st,
-                                               static_cast<const uint4 *>(in), static_cast<uint8_t *>(out), scale, numel,
-                                               prefetch_blocks(numel * (16 / C::kElems), kPrefetchers)));
+    auto kernel = prefetch_pays(numel * (16 / C::kElems)) ? saturated_cast_stream<IN, OUT, kUnroll, true>
+                                                                          : saturated_cast_stream<IN, OUT, kUnroll, false>;
+    return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(kThreads), 0, st,
+                                               static_cast<const uint4 *>(in), static_cast<uint8_t *>(out), scale, numel));
   } else {
     const int64_t blocks = ceil_div64(numel, kThreads);
     const int grid = static_cast<int>(blocks < max_grid ? blocks : max_grid);
