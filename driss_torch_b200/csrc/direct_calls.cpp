@@ -86,28 +86,30 @@ PyObject *give(std::tuple<Ts...> &&v) {
   return t;
 }
 
-// The operator under its name in torch.ops, for the calls that are not taken here.
-PyObject *through_torch_ops(const char *name, PyObject *const *args, Py_ssize_t n) {
+// The operator under its name in torch.ops, for the calls that are not taken here.  Looked up once per operator and kept: a
+// program with a default device (torch.set_default_device, a torch-function mode) makes every call this way.
+PyObject *torch_ops_operator(const char *name) {
   PyObject *torch = PyImport_ImportModule("torch");
   PyObject *ops = torch ? PyObject_GetAttrString(torch, "ops") : nullptr;
   PyObject *ns = ops ? PyObject_GetAttrString(ops, "DrissTorch") : nullptr;
   PyObject *op = ns ? PyObject_GetAttrString(ns, name) : nullptr;
-  PyObject *result = op ? PyObject_Vectorcall(op, args, static_cast<size_t>(n), nullptr) : nullptr;
-  Py_XDECREF(op);
   Py_XDECREF(ns);
   Py_XDECREF(ops);
   Py_XDECREF(torch);
-  return result;
+  return op;
 }
 
 template <typename R, typename... Args>
 struct Operator {
   using Signature = R(Args...);
   template <typename Handle, size_t... I>
-  static PyObject *run(const char *name, const Handle &op, PyObject *const *args, Py_ssize_t n, std::index_sequence<I...>) {
+  static PyObject *run(const char *name, PyObject **in_torch_ops, const Handle &op, PyObject *const *args, Py_ssize_t n,
+                       std::index_sequence<I...>) {
     std::tuple<std::decay_t<Args>...> v{};
-    if (n != static_cast<Py_ssize_t>(sizeof...(Args)) || at::impl::torch_function_mode_enabled() || !(take(args[I], std::get<I>(v)) && ...))
-      return through_torch_ops(name, args, n);
+    if (n != static_cast<Py_ssize_t>(sizeof...(Args)) || at::impl::torch_function_mode_enabled() || !(take(args[I], std::get<I>(v)) && ...)) {
+      if (!*in_torch_ops) *in_torch_ops = torch_ops_operator(name);
+      return *in_torch_ops ? PyObject_Vectorcall(*in_torch_ops, args, static_cast<size_t>(n), nullptr) : nullptr;
+    }
     auto call = [&] {
       ReleaseGil no_gil;
       return op.call(std::get<I>(v)...);
@@ -119,9 +121,10 @@ struct Operator {
 #define DTQ_DIRECT(NAME, ...)                                                                                              \
   PyObject *NAME(PyObject *, PyObject *const *args, Py_ssize_t n) {                                                        \
     using Op = Operator<__VA_ARGS__>;                                                                                      \
+    static PyObject *in_torch_ops = nullptr;                                                                               \
     try {                                                                                                                  \
       static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("DrissTorch::" #NAME, "").typed<Op::Signature>(); \
-      return Op::run(#NAME, op, args, n, Arity<Op::Signature>{});                                                          \
+      return Op::run(#NAME, &in_torch_ops, op, args, n, Arity<Op::Signature>{});                                           \
     } catch (...) {                                                                                                        \
       torch::translate_exception_to_python(std::current_exception());                                                      \
       return nullptr;                                                                                                      \

@@ -95,6 +95,28 @@ def test_torch_function_subclasses_and_modes():
         assert dt.amax(X) == "mode"
 
 
+def test_calls_left_to_torch_ops_look_the_operator_up_once(monkeypatch):
+    # a default device is such a mode: a program that sets one makes every call this way
+    looked_up = []
+
+    class Ops:  # torch looks the operator up itself under a mode: the wrappers add nothing to that
+        def __getattr__(self, name):
+            looked_up.append(name)
+            return getattr(torch._ops.ops, name)
+
+    def lookups(functions):
+        looked_up.clear()
+        with torch.device("meta"):
+            shapes = [[o.shape for o in outputs(f(*args))] for f, (_, args) in zip(functions, calls("meta"))]
+        return shapes, list(looked_up)
+
+    names = [name for name, _ in calls("meta")]
+    operators, wrappers = [getattr(dt.ops, n) for n in names], [getattr(dt.direct, n) for n in names]
+    lookups(wrappers)
+    monkeypatch.setattr(torch, "ops", Ops())
+    assert lookups(wrappers) == lookups(operators)
+
+
 def test_dispatch_modes_see_the_operator():
     seen = []
 
