@@ -2,6 +2,7 @@
 // layout that kernels and launchers agree on.
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -65,6 +66,53 @@ inline cudaError_t launch_after_dependency(void (*kernel)(KArgs...), dim3 grid, 
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// ---- thread-block clusters: whether the device can place them ------------------------------------------------------
+// The runtime's word that there is no such thing on this device, as against a failure of the moment (no memory to load the
+// kernel, say).
+inline bool means_no_such_clusters(cudaError_t e) {
+  return e == cudaErrorNotSupported || e == cudaErrorInvalidClusterSize || e == cudaErrorInvalidConfiguration ||
+         e == cudaErrorInvalidDeviceFunction || e == cudaErrorInvalidValue;
+}
+// How many clusters of a kernel the device holds at once, 0 where it cannot place them.  `ask(&n)` puts the question, and
+// `known` (0: no answer yet, else the answer + 1) keeps the answer for the process.  A failure of the moment is 0 for this
+// call and is not kept.  An error that was pending before stays pending: it is the caller's.  Asking twice is harmless.
+template <typename Ask>
+int clusters_that_fit(std::atomic<int> &known, Ask ask) {
+  const int answer = known.load(std::memory_order_acquire);
+  if (answer) return answer - 1;
+  int n = 0;
+  const cudaError_t e = ask(&n);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();  // the question's own
+    n = 0;
+  }
+  if (e == cudaSuccess || means_no_such_clusters(e)) known.store(n + 1, std::memory_order_release);
+  return n;
+}
+// Whether a launch was turned down for what a cluster needs: the answer above is the device's, and the context may have
+// fewer SMs (a green context, a partition).
+inline bool turned_down_for_room(cudaError_t e) {
+  return e == cudaErrorLaunchOutOfResources || e == cudaErrorInvalidClusterSize || e == cudaErrorInvalidConfiguration ||
+         e == cudaErrorNotSupported;
+}
+
+// ---- tensor-wise quantization: which kernels -------------------------------------------------------------------------
+enum class Tensorwise { kCluster, kGrid, kTwoLaunches, kScalar };
+constexpr int64_t kClusterMaxBytes = int64_t(1) << 20;  // of input; figures at dsq_cluster_kernel
+// Inputs above this many bytes are quantised as amax kernel + cast kernel instead of the single
+// fused launch: what the chip can keep between the two looks (about 140 MB) no longer matters at
+// that size, and the two stream kernels run at higher occupancy than the persistent fused one
+// (measured, bf16, fused / two launches: 128 MiB 44.8 / 49.5 us, 256 MiB 94.3 / 100.8, 320 MiB 118.3 / 120.2; fp32 320 MiB
+// 105.7 / 104.9).
+constexpr int64_t kFusedMaxBytes = int64_t(320) << 20;
+// `aligned`: input and output allow 16-byte loads and whole stores.
+inline Tensorwise tensorwise_path(int64_t input_bytes, bool aligned, bool clusters, bool cooperative) {
+  if (!aligned) return Tensorwise::kScalar;
+  if (input_bytes > kFusedMaxBytes) return Tensorwise::kTwoLaunches;
+  if (input_bytes <= kClusterMaxBytes && clusters) return Tensorwise::kCluster;
+  return cooperative ? Tensorwise::kGrid : Tensorwise::kScalar;
 }
 
 inline bool aligned_to(const void *p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }

@@ -52,12 +52,6 @@ constexpr int kFusedSmemTiles = 3;
 // A block's first tile stays in registers across the barrier: one more tile kept on chip for
 // 4 * kUnroll registers per thread.
 constexpr int kFusedRegTiles = 1;
-// Inputs above this many bytes are quantised as amax kernel + cast kernel instead of the single
-// fused launch: what the chip can keep between the two looks (about 140 MB) no longer matters at
-// that size, and the two stream kernels run at higher occupancy than the persistent fused one
-// (measured, bf16, fused / two launches: 128 MiB 44.8 / 49.5 us, 256 MiB 94.3 / 100.8, 320 MiB 118.3 / 120.2; fp32 320 MiB
-// 105.7 / 104.9).
-constexpr int64_t kFusedMaxBytes = int64_t(320) << 20;
 // The stand-alone cast kernel: one tile per block (no grid cap), see saturated_cast.cu.
 constexpr int kThreads = 256;
 constexpr int64_t kCastBlocksPerSmCap = 1 << 20;
@@ -471,12 +465,11 @@ int launch_fused_kernel(const void *in, void *out, float *amax_out, float *scale
   return DTQ_OK;
 }
 
-// One cluster for inputs of up to kClusterMaxBytes; *taken is false where the device cannot place it.
-constexpr int64_t kClusterMaxBytes = int64_t(1) << 20;
+// One cluster for inputs of up to kClusterMaxBytes; *taken is false where it cannot be placed.
 template <int IN, int OUT, int CHUNKS>
 int launch_cluster_kernel(const void *in, void *out, float *amax_out, float *scale_out, int64_t numel, int ctas, cudaStream_t st,
                           bool *taken) {
-  static std::atomic<int> known[kMaxPlanDevices];  // 0: not asked yet, 1: the device cannot, 2: it can
+  static std::atomic<int> known[kMaxPlanDevices];  // see clusters_that_fit
   auto kernel = dsq_cluster_kernel<IN, OUT, CHUNKS>;
   int dev_id = 0;
   DTQ_CUDA_TRY(cudaGetDevice(&dev_id));
@@ -494,20 +487,18 @@ int launch_cluster_kernel(const void *in, void *out, float *amax_out, float *sca
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;  // the occupancy query wants the cluster shape only
-  int answer = known[dev_id].load(std::memory_order_acquire);
-  if (answer == 0) {  // asking twice is harmless
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) n = 0;
-    (void)cudaGetLastError();  // a device without such clusters is not an error of this call
-    answer = n > 0 ? 2 : 1;
-    known[dev_id].store(answer, std::memory_order_release);
-  }
-  *taken = answer == 2;
+  *taken = clusters_that_fit(known[dev_id], [&](int *n) { return cudaOccupancyMaxActiveClusters(n, kernel, &cfg); }) > 0;
   if (!*taken) return DTQ_OK;
   cfg.gridDim = dim3(ctas);
   attr[0].val.clusterDim.x = ctas;
   cfg.numAttrs = 2;
-  return cuda_status(cudaLaunchKernelEx(&cfg, kernel, static_cast<const uint4 *>(in), static_cast<uint8_t *>(out), amax_out, scale_out, numel));
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<const uint4 *>(in), static_cast<uint8_t *>(out), amax_out, scale_out, numel);
+  if (turned_down_for_room(e)) {
+    (void)cudaGetLastError();
+    *taken = false;
+    return DTQ_OK;
+  }
+  return cuda_status(e);
 }
 template <int IN, int OUT>
 int launch_cluster(const void *in, void *out, float *amax_out, float *scale_out, int64_t numel, cudaStream_t st, bool *taken) {
@@ -525,8 +516,16 @@ int launch_fused(const void *in, void *out, float *amax_out, float *scale_out, i
                  const DeviceInfo &dev, cudaStream_t st) {
   using C = DsqChunk<IN, OUT>;
   uint8_t *o = static_cast<uint8_t *>(out);
-  const bool vector_ok = aligned_to(in, 16) && aligned_to(out, C::kOutAlign);
-  if (vector_ok && numel * C::kElemBytes > kFusedMaxBytes) {
+  const bool aligned = aligned_to(in, 16) && aligned_to(out, C::kOutAlign);
+  const int64_t bytes = numel * C::kElemBytes;
+  Tensorwise path = tensorwise_path(bytes, aligned, true, dev.cooperative);
+  if (path == Tensorwise::kCluster) {
+    bool taken = false;
+    if (int e = launch_cluster<IN, OUT>(in, out, amax_out, scale_out, numel, st, &taken)) return e;
+    if (taken) return DTQ_OK;
+    path = tensorwise_path(bytes, aligned, false, dev.cooperative);
+  }
+  if (path == Tensorwise::kTwoLaunches) {
     if (int e = launch_amax(in, &ws->amax, numel, IN, ws, dev, st)) return e;
     const int64_t tiles = ceil_div64(numel / C::kElems, int64_t(kThreads) * kUnroll);
     const int grid = balanced_grid(tiles, int64_t(dev.sm_count) * kCastBlocksPerSmCap);
@@ -534,12 +533,7 @@ int launch_fused(const void *in, void *out, float *amax_out, float *scale_out, i
                                                0, st, static_cast<const uint4 *>(in), o, &ws->amax, scale_out, amax_out,
                                                numel));
   }
-  if (vector_ok && numel * C::kElemBytes <= kClusterMaxBytes) {
-    bool taken = false;
-    if (int e = launch_cluster<IN, OUT>(in, out, amax_out, scale_out, numel, st, &taken)) return e;
-    if (taken) return DTQ_OK;
-  }
-  if (vector_ok && dev.cooperative)
+  if (path == Tensorwise::kGrid)
     return launch_fused_kernel<IN, OUT, false>(in, out, amax_out, scale_out, numel, ws, dev, PeerExchange{}, st);
   const int64_t blocks = ceil_div64(numel, kThreads);
   const int64_t max_grid = int64_t(dev.sm_count) * 8;

@@ -33,7 +33,6 @@
 
 #include <algorithm>
 #include <atomic>
-#include <mutex>
 
 #include "dtq_device.cuh"
 #include "dtq_host.h"
@@ -1285,28 +1284,18 @@ void cluster_launch_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, i
 // *max_clusters (cached per device and format) is 0 where cluster launches of this kernel are not possible.
 template <int MODE>
 int pair_cluster_capacity(int dev_id, int *max_clusters) {
-  static std::atomic<int> ready[kMaxGemmDevices];
-  static int capacity[kMaxGemmDevices];
+  static std::atomic<int> known[kMaxGemmDevices];
   if (dev_id < 0 || dev_id >= kMaxGemmDevices) return DTQ_ERR_INVALID_ARGUMENT;
-  if (!ready[dev_id].load(std::memory_order_acquire)) {
-    static std::mutex mutex;
-    std::lock_guard<std::mutex> lock(mutex);
-    if (!ready[dev_id].load(std::memory_order_relaxed)) {
-      constexpr int smem = smem_bytes<PairSmem<MODE>>();
-      int n = 0;
-      if (cudaFuncSetAttribute(mx_gemm_pair_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess) {
-        cudaLaunchConfig_t cfg;
-        cudaLaunchAttribute attr[2];
-        cluster_launch_config(&cfg, attr, 2, kGemmThreads, 2, smem, nullptr);
-        cfg.numAttrs = 1;  // the occupancy query wants the cluster shape only
-        if (cudaOccupancyMaxActiveClusters(&n, mx_gemm_pair_kernel<MODE>, &cfg) != cudaSuccess) n = 0;
-      }
-      (void)cudaGetLastError();  // a device without cluster support is not an error of this call
-      capacity[dev_id] = n;
-      ready[dev_id].store(1, std::memory_order_release);
-    }
-  }
-  *max_clusters = capacity[dev_id];
+  *max_clusters = clusters_that_fit(known[dev_id], [](int *n) {
+    constexpr int smem = smem_bytes<PairSmem<MODE>>();
+    const cudaError_t e = cudaFuncSetAttribute(mx_gemm_pair_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    cluster_launch_config(&cfg, attr, 2, kGemmThreads, 2, smem, nullptr);
+    cfg.numAttrs = 1;  // the occupancy query wants the cluster shape only
+    return cudaOccupancyMaxActiveClusters(n, mx_gemm_pair_kernel<MODE>, &cfg);
+  });
   return DTQ_OK;
 }
 
@@ -1410,26 +1399,20 @@ int split_count(int64_t m, int64_t n, int64_t stages, int sm_count) {
 // where it cannot launch them.
 template <int BN, int MODE>
 int split_cluster_capacity(int dev_id, int splits, int *max_clusters) {
-  static std::atomic<int> known[kMaxGemmDevices][kMaxSplits + 1];  // 0: not asked yet, else the answer + 1
+  static std::atomic<int> known[kMaxGemmDevices][kMaxSplits + 1];
   auto kernel = mx_gemm_split_kernel<BN, SplitStages<BN>, MODE>;
   if (dev_id < 0 || dev_id >= kMaxGemmDevices) return DTQ_ERR_INVALID_ARGUMENT;
-  int value = known[dev_id][splits].load(std::memory_order_acquire);
-  if (value == 0) {  // asking twice is harmless
+  *max_clusters = clusters_that_fit(known[dev_id][splits], [=](int *n) {
     constexpr int smem = smem_bytes<SplitSmem<BN, SplitStages<BN>, MODE>>();
     static_assert(2 * (smem + 1024) <= 228 * 1024, "two CTAs per SM, with the kilobyte that each takes besides");
-    int n = 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess) {
-      cudaLaunchConfig_t cfg;
-      cudaLaunchAttribute attr[2];
-      cluster_launch_config(&cfg, attr, splits, kSplitThreads, splits, smem, nullptr);
-      cfg.numAttrs = 1;  // the occupancy query wants the cluster shape only
-      if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) n = 0;
-    }
-    (void)cudaGetLastError();  // a device without such clusters is not an error of this call
-    value = n + 1;
-    known[dev_id][splits].store(value, std::memory_order_release);
-  }
-  *max_clusters = value - 1;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    cluster_launch_config(&cfg, attr, splits, kSplitThreads, splits, smem, nullptr);
+    cfg.numAttrs = 1;  // the occupancy query wants the cluster shape only
+    return cudaOccupancyMaxActiveClusters(n, kernel, &cfg);
+  });
   return DTQ_OK;
 }
 template <int MODE>

@@ -1,0 +1,66 @@
+"""The host's choices between kernels, compiled for themselves: no GPU is asked."""
+import ctypes as C
+import os
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+MIB = 1 << 20
+OUT_OF_MEMORY, INVALID_CONFIGURATION, INVALID_DEVICE, OUT_OF_RESOURCES, NOT_SUPPORTED, INVALID_CLUSTER = 2, 9, 101, 701, 801, 912
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    so = tmp_path_factory.mktemp("rules") / "rules.so"
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic",  # its own stand-ins, not a CUDA runtime in this process
+                           f"-I{ROOT / 'driss_torch_b200' / 'csrc'}", f"-I{cuda}/include",
+                           str(ROOT / "tests" / "host_rules.cpp"), "-o", str(so)])
+    lib = C.CDLL(str(so))
+    lib.rule_tensorwise.argtypes = [C.c_longlong] + 3 * [C.c_int]
+    return lib
+
+
+@pytest.mark.parametrize("size, aligned, clusters, cooperative, path", [
+    (0, 1, 1, 1, "cluster"), (MIB, 1, 1, 1, "cluster"), (MIB + 16, 1, 1, 1, "grid"), (320 * MIB, 1, 1, 1, "grid"),
+    (320 * MIB + 16, 1, 1, 1, "two launches"), (320 * MIB + 16, 1, 0, 0, "two launches"),
+    (MIB, 1, 0, 1, "grid"), (MIB, 1, 0, 0, "scalar"), (MIB + 16, 1, 1, 0, "scalar"), (16, 0, 1, 1, "scalar"), (400 * MIB, 0, 1, 1, "scalar"),
+])
+def test_tensorwise_path(rules, size, aligned, clusters, cooperative, path):
+    names = ["cluster", "grid", "two launches", "scalar"]
+    assert names[rules.rule_tensorwise(size, aligned, clusters, cooperative)] == path
+
+
+def ask(rules, error=0, n=5, pending=0, forget=False):
+    after, asked = C.c_int(-1), C.c_int(-1)
+    return rules.rule_clusters(forget, error, n, pending, C.byref(after), C.byref(asked)), after.value, asked.value
+
+
+def test_an_answer_about_clusters_is_kept(rules):
+    assert ask(rules, n=5, forget=True) == (5, 0, 1)
+    assert ask(rules, n=7) == (5, 0, 1)
+    assert ask(rules, n=0, forget=True) == (0, 0, 1)
+    assert ask(rules, n=7) == (0, 0, 1)
+
+
+def test_a_pending_error_of_the_caller_stays(rules):
+    assert ask(rules, pending=INVALID_DEVICE, forget=True) == (5, INVALID_DEVICE, 1)
+
+
+@pytest.mark.parametrize("error", [NOT_SUPPORTED, INVALID_CLUSTER, INVALID_CONFIGURATION])
+def test_no_such_clusters_is_an_answer(rules, error):
+    assert ask(rules, error=error, forget=True) == (0, 0, 1)
+    assert ask(rules) == (0, 0, 1)
+
+
+def test_a_failure_of_the_moment_is_not(rules):
+    assert ask(rules, error=OUT_OF_MEMORY, forget=True) == (0, 0, 1)
+    assert ask(rules, error=OUT_OF_MEMORY) == (0, 0, 2)
+    assert ask(rules) == (5, 0, 3)
+
+
+def test_launches_turned_down_for_room_go_to_the_grid(rules):
+    assert all(rules.rule_turned_down(e) for e in (OUT_OF_RESOURCES, INVALID_CLUSTER, INVALID_CONFIGURATION, NOT_SUPPORTED))
+    assert not any(rules.rule_turned_down(e) for e in (0, 1, 700, 719))
