@@ -11,6 +11,7 @@ libraries have not been built (``python driss_torch_b200/build.py``) the import 
 """
 from __future__ import annotations
 
+from importlib.machinery import EXTENSION_SUFFIXES
 from pathlib import Path
 from typing import Optional
 
@@ -21,7 +22,7 @@ from torch.jit import is_scripting
 _LIB_DIR = Path(__file__).resolve().parent / "lib"
 lib_path = _LIB_DIR / "libdriss_torch.so"
 kernels_lib_path = _LIB_DIR / "libdtq_b200.so"
-_direct_path = _LIB_DIR / "_direct.so"
+_direct_path = _LIB_DIR / ("_direct" + EXTENSION_SUFFIXES[0])
 
 if not lib_path.exists() or not kernels_lib_path.exists() or not _direct_path.exists():
     raise ImportError(

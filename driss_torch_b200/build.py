@@ -4,15 +4,16 @@
   (``include/dtq_b200.h``), built with nvcc for sm_100a only.
 * ``lib/libdriss_torch.so`` -- ``register_ops.cpp``: the ``TORCH_LIBRARY(DrissTorch)``
   registration that binds the C ABI into the PyTorch dispatcher, built with g++.
-* ``lib/_direct.so`` -- ``direct_calls.cpp``: the operators as plain Python functions (an extension module),
-  built with g++.
+* ``lib/_direct.<python ABI>.so`` -- ``direct_calls.cpp``: the operators as plain Python functions (an extension
+  module), built with g++.
 
 ``python driss_torch_b200/build.py`` builds all; objects are rebuilt only when a
-source or header is newer.  The reference builds one ``libdriss_torch.so`` through
+source or header is newer, the two that are linked to torch also for another torch, Python or command.  The reference builds one ``libdriss_torch.so`` through
 scikit-build/CMake with the same architecture flags (CMakeLists.txt:25-27).
 """
 from __future__ import annotations
 
+import importlib.machinery
 import os
 import subprocess
 import sys
@@ -99,16 +100,27 @@ def build_kernels(force: bool = False, extra_flags=()) -> Path:
     return so
 
 
+def made_for(cmd) -> str:
+    """What a library linked to torch was made with: it has to be made again for any other."""
+    import torch
+
+    return "\n".join([f"torch {torch.__version__} {torch.version.git_version}", sysconfig.get_config_var("SOABI"), " ".join(map(str, cmd))])
+
+
+def out_of_date(target: Path, sources, stamp: Path, wanted: str) -> bool:
+    if not target.exists() or target.stat().st_mtime < _newest(sources):
+        return True
+    return not stamp.exists() or stamp.read_text() != wanted
+
+
 def _build_torch_library(source: str, target: str, libs, force: bool) -> Path:
     import torch
     from torch.utils.cpp_extension import include_paths
 
     LIB.mkdir(exist_ok=True)
+    OBJ.mkdir(exist_ok=True)
     src = CSRC / source
     so = LIB / target
-    dep_time = max(src.stat().st_mtime, _newest(list(INCLUDE.glob("*.h"))))
-    if not (force or not so.exists() or so.stat().st_mtime < dep_time):
-        return so
     torch_lib = Path(torch.__file__).parent / "lib"
     incs = [f"-I{p}" for p in include_paths("cuda")] + [f"-I{INCLUDE}", f"-I{sysconfig.get_paths()['include']}"]
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
@@ -116,18 +128,23 @@ def _build_torch_library(source: str, target: str, libs, force: bool) -> Path:
         "g++", "-std=c++17", "-O2", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={abi}", *incs, str(src),
         "-o", str(so),
         f"-L{LIB}", f"-L{torch_lib}", *libs,
-        f"-L{CUDA_HOME / 'lib64'}", "-lcudart",
         "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}", f"-Wl,-rpath,{CUDA_HOME / 'lib64'}",
     ]
-    _run(cmd)
+    stamp, wanted = OBJ / (target + ".stamp"), made_for(cmd)
+    if force or out_of_date(so, [src, *INCLUDE.glob("*.h")], stamp, wanted):
+        _run(cmd)
+        stamp.write_text(wanted)
     return so
 
 
 def build_torch_binding(force: bool = False) -> Path:
     assert (LIB / "libdtq_b200.so").exists(), "build the kernel library first"
     so = _build_torch_library("register_ops.cpp", "libdriss_torch.so",
-                              ["-ldtq_b200", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"], force)
-    _build_torch_library("direct_calls.cpp", "_direct.so", ["-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10"], force)
+                              ["-ldtq_b200", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", f"-L{CUDA_HOME / 'lib64'}", "-lcudart"],
+                              force)
+    (LIB / "_direct.so").unlink(missing_ok=True)  # its name once, which any Python would load
+    _build_torch_library("direct_calls.cpp", "_direct" + importlib.machinery.EXTENSION_SUFFIXES[0],
+                         ["-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10"], force)
     return so
 
 
