@@ -704,7 +704,6 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const Bounds bounds{&sm.abort, p.ws};
   const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
   const int total_tiles = p.m_pairs * p.n_tiles;
-  pdl_launch_dependents();  // as in the single-CTA kernel
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kPairStages; ++s) {
@@ -738,6 +737,15 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     for (int tile = cluster_id; tile < total_tiles && ok; tile += n_clusters) {
       int mp, nt;
       tile_coords(tile, p.m_pairs, p.n_tiles, &mp, &nt);
+      // What is queued behind this kernel may become resident once every CTA has come to its last tile, and not at once as in
+      // the other kernels: a cast that becomes resident asks for its first tiles (prefetch_first_tile), and at the start of a
+      // large product that took memory from the first operands, for lines that the product was about to write.  Measured, MXFP8
+      // product and an operation on its output, us, released at once / here: 2000 x 12288 x 4096 product alone 78.0 / 77.5, static
+      // cast 89.1 / 88.9, MX cast 90.8 / 90.0, amax 89.2 / 87.8, amax and both casts 106.5 / 104.1; 8192 x 4096 x 1024: 33.2 / 33.1, 47.0 / 46.7,
+      // 49.4 / 48.7, 45.0 / 43.4, 69.6 / 66.6; 3000 x 8192 x 2048: 44.2 / 43.9, 54.7 / 54.4, 56.1 / 55.3, 56.2 / 54.4, 80.4 / 77.7.  Later still, with
+      // eight stages of the last tile left, the operations gain up to 2 us more, but a product behind a product starts too late
+      // where the last round of tiles leaves SMs idle: 2000 x 12288 x 4096 80.1.
+      if (tile + n_clusters >= total_tiles) pdl_launch_dependents();
       for (int ks = 0; ks < p.k_stages; ++ks) {
         if (!first_pass && !mbar_wait_warp(&sm.empty[stage], phase ^ 1u, bounds)) {
           ok = false;
