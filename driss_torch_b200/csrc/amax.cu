@@ -79,9 +79,10 @@ __device__ __forceinline__ void absmax_stream(AbsMax<IN> &acc, const uint4 *__re
 
 // `in` may have any element alignment: up to `head` leading and `tail` trailing elements are
 // read one by one by block 0, the 16-byte aligned middle is streamed.
-template <int IN, int UNROLL>
+// PREFETCH: every block asks for the first `ask_chunks` chunks of its first tile ahead of the dependency.
+template <int IN, int UNROLL, bool PREFETCH>
 __global__ void __launch_bounds__(kAmaxThreads)
-amax_kernel(const void *__restrict__ in, float *__restrict__ out, int64_t numel, int64_t head, Workspace *ws) {
+amax_kernel(const void *__restrict__ in, float *__restrict__ out, int64_t numel, int64_t head, Workspace *ws, int ask_chunks) {
   __shared__ float smem32[32];
   __shared__ int flag;
   constexpr int kElems = 16 / AbsMax<IN>::kElemBytes;
@@ -89,15 +90,19 @@ amax_kernel(const void *__restrict__ in, float *__restrict__ out, int64_t numel,
   const char *base = static_cast<const char *>(in);
   const uint4 *body = reinterpret_cast<const uint4 *>(base + head * AbsMax<IN>::kElemBytes);
   const int64_t nchunks = (numel - head) / kElems;
-  // This launch itself may have started under the tail of its predecessor: the block's first tile is asked into L2 meanwhile,
-  // harmless whatever the predecessor still writes (see l2_prefetch_bulk).  What it hides is the start of the stream, which a
-  // launch of one or two tiles per block consists of.  Measured, amax then both casts of bf16 (amax alone back to back), us, without
-  // / with: 3500 x 4096 17.2 / 15.8 (7.8 / 6.6), 5003 x 4096 23.0 / 21.2 (10.6 / 9.9), 3570 x 6416 25.4 / 23.6 (11.0 / 10.2), 8192 x 8192
-  // 66.9 / 66.3 (22.6 / 20.1), up to 2048 x 4096 the same, 16384 x 8192 131.0 / 132.4, so not beyond 128 MiB; with the second tile
-  // too 5003 x 4096 20.8, 8192 x 8192 67.0 (22.1).
+  // This launch itself may have started under the tail of its predecessor: part of the block's first tile is asked into L2
+  // meanwhile, harmless whatever the predecessor still writes (see l2_prefetch_bulk).  What it hides is the start of the stream.
+  // 4 MiB in all, of inputs of up to 20 MiB (amax_ask_chunks).  Measured, us, bf16, nothing asked / this, inputs from memory
+  // (400 MB of them in turn): amax 8 MiB 5.3 / 4.9, 16 MiB 6.4 / 6.0; amax then both casts 10.0 / 9.6, 12.0 / 11.5; behind an MXFP8
+  // product that writes the input, 16 MiB, 17.5 / 17.4 and 22.7 / 22.5.  More of it gains more on inputs that stay in L2
+  // or where an amax follows an amax, and loses where the kernel before still reads and writes: with whole first tiles, up to 37 MiB,
+  // amax then both casts 39 MiB 22.0 / 24.6, 47 MiB 25.3 / 29.3, 64 MiB 32.7 / 36.4 (with three inputs in turn 21.2 / 23.2, 24.7 / 28.0, 32.4 /
+  // 35.7), behind a product 16 MiB 39.2 / 41.4; with 4 MiB asked 39 MiB still 22.0 / 23.5, 24 MiB 15.8 / 16.2.  Rows that are no
+  // multiple of 16 gain all the same (39 MiB 24.6 / 24.2, whole tiles 23.9), which the amax cannot see.
   constexpr int64_t kTile = int64_t(kAmaxThreads) * UNROLL;
-  if (threadIdx.x == 0 && nchunks * int64_t(sizeof(uint4)) <= kPrefetchToBytes)
-    prefetch_first_tile(body, blockIdx.x * kTile, kTile, nchunks);
+  if constexpr (PREFETCH) {
+    if (threadIdx.x == 0) prefetch_first_tile(body, blockIdx.x * kTile, ask_chunks, nchunks);
+  }
   pdl_wait();
   const float identity = -INFINITY;
   AbsMax<IN> acc(identity);
@@ -136,11 +141,11 @@ int launch_amax(const void *in, float *out, int64_t numel, int in_dtype, Workspa
   const int eb = in_dtype == DTQ_BF16 ? 2 : 4;
   const int grid = amax_grid(numel, eb, dev);
   const int64_t head = head_elems(in, eb, numel);
-  if (in_dtype == DTQ_BF16)
-    return cuda_status(launch_after_dependency(amax_kernel<DTQ_BF16, kAmaxUnroll>, dim3(grid), dim3(kAmaxThreads), 0, st, in,
-                                               out, numel, head, ws));
-  return cuda_status(launch_after_dependency(amax_kernel<DTQ_F32, kAmaxUnroll>, dim3(grid), dim3(kAmaxThreads), 0, st, in, out,
-                                             numel, head, ws));
+  const int ask_chunks = amax_ask_chunks(numel * eb, grid, kAmaxThreads * kAmaxUnroll);
+  const bool ask = ask_chunks > 0;
+  auto kernel = in_dtype == DTQ_BF16 ? (ask ? amax_kernel<DTQ_BF16, kAmaxUnroll, true> : amax_kernel<DTQ_BF16, kAmaxUnroll, false>)
+                                     : (ask ? amax_kernel<DTQ_F32, kAmaxUnroll, true> : amax_kernel<DTQ_F32, kAmaxUnroll, false>);
+  return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(kAmaxThreads), 0, st, in, out, numel, head, ws, ask_chunks));
 }
 
 }  // namespace dtq
@@ -219,8 +224,8 @@ extern "C" int dtq_amax_static_scratch(const void *in, float *out, int64_t numel
   const int grid = static_cast<int>(tiles < 1 ? 1 : tiles);  // <= kMaxGridBlocks by the size check
   const int64_t head = head_elems(in, eb, numel);
   if (in_dtype == DTQ_BF16)
-    amax_kernel<DTQ_BF16, kAmaxUnroll><<<grid, kAmaxThreads, 0, st>>>(in, out, numel, head, ws);
+    amax_kernel<DTQ_BF16, kAmaxUnroll, false><<<grid, kAmaxThreads, 0, st>>>(in, out, numel, head, ws, 0);
   else
-    amax_kernel<DTQ_F32, kAmaxUnroll><<<grid, kAmaxThreads, 0, st>>>(in, out, numel, head, ws);
+    amax_kernel<DTQ_F32, kAmaxUnroll, false><<<grid, kAmaxThreads, 0, st>>>(in, out, numel, head, ws, 0);
   return cuda_status(cudaGetLastError());
 }

@@ -126,6 +126,15 @@ inline bool prefetch_pays(int64_t input_bytes, int64_t to_bytes = kPrefetchToByt
   return input_bytes <= kPrefetchSmallBytes || (input_bytes >= kPrefetchFromBytes && input_bytes <= to_bytes);
 }
 
+// How much of its first tile, in 16-byte chunks, every block of the amax asks for ahead of its dependency; 0: nothing (figures in
+// amax.cu).
+constexpr int64_t kAmaxAskToBytes = int64_t(20) << 20, kAmaxAskBytes = int64_t(4) << 20;
+inline int amax_ask_chunks(int64_t input_bytes, int grid, int tile_chunks) {
+  if (input_bytes > kAmaxAskToBytes) return 0;
+  const int64_t share = kAmaxAskBytes / 16 / grid;
+  return static_cast<int>(share < tile_chunks ? share : tile_chunks);
+}
+
 inline int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // Grid for a persistent kernel that walks `tiles` tiles grid-stride: at most `max_grid` blocks,

@@ -17,6 +17,7 @@ cudaError_t cudaGetLastError() {
 int rule_tensorwise(long long bytes, int aligned, int clusters, int cooperative) {
   return static_cast<int>(dtq::tensorwise_path(bytes, aligned != 0, clusters != 0, cooperative != 0));
 }
+int rule_amax_asks(long long bytes, int grid, int tile_chunks) { return dtq::amax_ask_chunks(bytes, grid, tile_chunks); }
 int rule_turned_down(int error) { return dtq::turned_down_for_room(static_cast<cudaError_t>(error)); }
 
 // One question about clusters: the runtime answers `n`, or fails with `error` as its runtime would.
