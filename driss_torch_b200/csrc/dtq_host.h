@@ -117,13 +117,22 @@ inline Tensorwise tensorwise_path(int64_t input_bytes, bool aligned, bool cluste
 
 inline bool aligned_to(const void *p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 
-// Whether the first blocks of a stream kernel are to call prefetch_first_tile (dtq_device.cuh, with the figures).  The kernels have
-// an instantiation for either answer: with the question at run time the compiler orders the rest of them differently, and those
-// that do not ask ahead lost up to 2 %.
-constexpr int64_t kPrefetchFromBytes = int64_t(16) << 20, kPrefetchToBytes = int64_t(128) << 20;
-constexpr int64_t kPrefetchSmallBytes = int64_t(512) << 10;  // and none above: the tokens of a decode step
-inline bool prefetch_pays(int64_t input_bytes, int64_t to_bytes = kPrefetchToBytes) {
-  return input_bytes <= kPrefetchSmallBytes || (input_bytes >= kPrefetchFromBytes && input_bytes <= to_bytes);
+// Which stream kernels call prefetch_first_tile, by bytes of input (dtq_device.cuh has the figures).  They have an instantiation
+// for either answer: with the question at run time the compiler orders the rest of them differently, and those that do not
+// ask ahead lost up to 2 %.
+enum class Asks { kCastBf16, kCastF32, kMx, kMxBlocked, kMxFormats, kRowwise };
+constexpr int64_t kAskSmallBytes = int64_t(512) << 10;  // the tokens of a decode step
+inline bool asks_ahead(Asks kernel, int64_t input_bytes) {
+  if (input_bytes <= kAskSmallBytes) return true;
+  const auto mebibytes = [=](int64_t from, int64_t to) { return input_bytes >= from << 20 && input_bytes <= to << 20; };
+  switch (kernel) {
+    case Asks::kCastBf16: return mebibytes(16, 48) || mebibytes(80, 128);
+    case Asks::kCastF32: return mebibytes(28, 128);
+    case Asks::kMx: return input_bytes >= int64_t(16) << 20;
+    case Asks::kMxBlocked: return mebibytes(16, 128);
+    case Asks::kRowwise: return mebibytes(16, 128);
+    default: return false;
+  }
 }
 
 // How much of its first tile, in 16-byte chunks, every block of the amax asks for ahead of its dependency; 0: nothing (figures in

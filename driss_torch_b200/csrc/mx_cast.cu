@@ -23,7 +23,8 @@ namespace {
 // Grid cap in blocks per SM; the default is "no cap" (one tile per block), see saturated_cast.cu.
 constexpr int64_t kBlocksPerSmCap = 1 << 20;
 constexpr int kThreads = 256;
-constexpr unsigned kPrefetchers = 148 * 8;  // see prefetch_first_tile
+template <bool BLOCKED>
+constexpr unsigned kAskers = (BLOCKED ? 2 : 4) * kB200Sms;  // blocks that ask ahead, see prefetch_first_tile
 constexpr int kUnroll = 4;  // tied to the scale-byte mapping below: lane&3 picks the iteration
 
 // nchunks = numel / 8 is a multiple of 4.  A warp owns kUnroll consecutive 512-byte rows of
@@ -38,7 +39,8 @@ mx_stream_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, ui
   pdl_launch_dependents();
   if constexpr (PREFETCH) {
     const int64_t first_tile = int64_t(blockIdx.x) - (BLOCKED ? pad_blocks : 0);  // negative: this block writes padding
-    if (threadIdx.x == 0 && first_tile >= 0 && first_tile < kPrefetchers) prefetch_first_tile(in, first_tile * kTile, kTile, nchunks);
+    if (threadIdx.x == 0 && first_tile >= 0 && first_tile < kAskers<BLOCKED>)
+      prefetch_first_tile(in, first_tile * kTile, kTile, nchunks);
   }
   pdl_wait();
   if constexpr (BLOCKED) {  // the first blocks of the grid write the padding, if there is any
@@ -115,7 +117,7 @@ int launch_mx(const void *in_bf16, void *payload, void *scales_e8m0, int64_t row
     const int64_t tiles = ceil_div64(nchunks, int64_t(kThreads) * kUnroll);
     const int64_t pad_blocks = BLOCKED ? scale_padding_blocks(rows, kblocks, kThreads) : 0;
     const int grid = balanced_grid(tiles, max_grid) + static_cast<int>(pad_blocks);
-    auto kernel = prefetch_pays(numel * 2, INT64_MAX) ? mx_stream_kernel<BLOCKED, true> : mx_stream_kernel<BLOCKED, false>;
+    auto kernel = asks_ahead(BLOCKED ? Asks::kMxBlocked : Asks::kMx, numel * 2) ? mx_stream_kernel<BLOCKED, true> : mx_stream_kernel<BLOCKED, false>;
     return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(kThreads), 0, st,
                                                static_cast<const uint4 *>(in_bf16), static_cast<uint8_t *>(payload),
                                                static_cast<uint8_t *>(scales_e8m0), nchunks, kblocks, katoms, rows,

@@ -144,8 +144,6 @@ __device__ __forceinline__ void convert_store(const float (&f)[N], float inv, ui
 
 // Few tokens only (see prefetch_first_tile): with the larger inputs that the other casts ask ahead for, 8192 x 8192 to e2m1 took
 // 27.8 us instead of 26.8, and 0.6 of it stayed with the question at run time instead of an instantiation of its own.
-constexpr unsigned kPrefetchers = 148;
-
 // nchunks 16-byte chunks; a block of 32 elements is kLanes consecutive chunks (never split across warps).
 template <int IN, int FMT, bool PREFETCH>
 __global__ void __launch_bounds__(kThreadsF, 2048 / kThreadsF)
@@ -158,7 +156,7 @@ mx_formats_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, u
   constexpr int64_t kTile = int64_t(kThreadsF) * kUnrollF;
   if constexpr (PREFETCH) {
     const int64_t first_tile = int64_t(blockIdx.x) - pad_blocks;  // negative: this block writes padding
-    if (threadIdx.x == 0 && first_tile >= 0 && first_tile < kPrefetchers) prefetch_first_tile(in, first_tile * kTile, kTile, nchunks);
+    if (threadIdx.x == 0 && first_tile >= 0) prefetch_first_tile(in, first_tile * kTile, kTile, nchunks);
   }
   pdl_wait();
   using I = MxIn<IN>;
@@ -218,7 +216,7 @@ int launch_formats(const void *in, void *payload, void *scales, int64_t numel, i
   const int64_t tiles = ceil_div64(nchunks, int64_t(kThreadsF) * kUnrollF);
   const int64_t pad_blocks = kblocks > 0 ? scale_padding_blocks(rows, kblocks, kThreadsF) : 0;
   const int grid = balanced_grid(tiles, int64_t(dev.sm_count) * (1 << 20)) + static_cast<int>(pad_blocks);
-  auto kernel = prefetch_pays(nchunks * 16, 0) ? mx_formats_kernel<IN, FMT, true> : mx_formats_kernel<IN, FMT, false>;
+  auto kernel = asks_ahead(Asks::kMxFormats, nchunks * 16) ? mx_formats_kernel<IN, FMT, true> : mx_formats_kernel<IN, FMT, false>;
   return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(kThreadsF), 0, st,
                                              static_cast<const uint4 *>(in), static_cast<uint8_t *>(payload),
                                              static_cast<uint8_t *>(scales), nchunks, kblocks, rows,

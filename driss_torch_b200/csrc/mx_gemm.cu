@@ -956,7 +956,7 @@ constexpr int kMaxSplits = 8;        // portable cluster size
 // MXFP8 8 x 8192 x 8192 16.7 / 16.4 / 16.6 / 17.0, 100 x 4096 x 8192 16.2 / 15.6 / 15.9 / 16.8, row-wise 16 x 8192 x 4096
 // 11.6 / 11.2 / 11.5 / 12.1, 60 x 8192 x 4096 13.2 / 12.9 / 13.2 / 13.7, MXFP4 16 x 8192 x 8192 12.1 / 11.7 / 11.8 / 12.6; where two
 // CTAs share a tile of 64 stages (8 x 16384 x 8192) 27.0 / 26.4 / 26.1 / 26.4.
-// Since the casts ask for few tokens ahead of their own wait (prefetch_pays in dtq_host.h), 2 / 4 / 8 stages: row-wise 16 x 8192 x
+// Since the casts ask for few tokens ahead of their own wait (asks_ahead in dtq_host.h), 2 / 4 / 8 stages: row-wise 16 x 8192 x
 // 4096 10.8 / 10.5 / 10.8, 60 x 8192 x 4096 12.7 / 12.4 / 12.5, 8 x 16384 x 8192 26.5 / 26.1 / 26.3, MXFP4 16 x 8192 x 8192 11.6 / 11.1 /
 // 11.3, 4 x 12288 x 4096 9.9 / 9.8 / 9.8, but MXFP8 8 x 8192 x 8192 16.3 / 16.5 / 16.9, 100 x 4096 x 8192 15.7 / 15.9 / 16.8: its cast
 // also writes scales into whole atoms, and is the longest of the three.

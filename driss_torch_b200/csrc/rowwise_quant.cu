@@ -20,7 +20,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr unsigned kPrefetchers = 148 * 8;  // see prefetch_first_tile
+constexpr unsigned kAskers = 8 * kB200Sms;  // blocks that ask ahead, see prefetch_first_tile
 
 template <int IN>
 struct RowIn;
@@ -93,7 +93,7 @@ rowwise_regs_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, flo
   pdl_launch_dependents();
   if constexpr (PREFETCH) {
     constexpr int64_t kBlockRows = TEAM_WARPS == 1 ? kWarps : 1;
-    if (threadIdx.x == 0 && blockIdx.x < kPrefetchers)
+    if (threadIdx.x == 0 && blockIdx.x < kAskers)
       prefetch_first_tile(in, blockIdx.x * kBlockRows * chunks_per_row, kBlockRows * chunks_per_row, rows * chunks_per_row);
   }
   pdl_wait();
@@ -192,8 +192,8 @@ int launch_regs(const void *in, void *out, float *amax_out, float *scale_out, in
                 cudaStream_t st) {
   const unsigned grid = static_cast<unsigned>(TEAM_WARPS == 1 ? ceil_div64(rows, kWarps) : rows);
   const int threads = TEAM_WARPS == 1 ? kThreads : 32 * TEAM_WARPS;
-  auto kernel = prefetch_pays(rows * chunks_per_row * 16) ? rowwise_regs_kernel<IN, OUT, CHUNKS, TEAM_WARPS, true>
-                                                                          : rowwise_regs_kernel<IN, OUT, CHUNKS, TEAM_WARPS, false>;
+  auto kernel = asks_ahead(Asks::kRowwise, rows * chunks_per_row * 16) ? rowwise_regs_kernel<IN, OUT, CHUNKS, TEAM_WARPS, true>
+                                                                       : rowwise_regs_kernel<IN, OUT, CHUNKS, TEAM_WARPS, false>;
   return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(threads), 0, st, static_cast<const uint4 *>(in),
                                              static_cast<uint8_t *>(out), amax_out, scale_out, rows, chunks_per_row));
 }

@@ -22,7 +22,7 @@ constexpr int kUnroll = 2;  // 128-bit loads in flight per thread: 8 KB tiles.  
 // then store burst).  The in-kernel loop then only matters beyond 2^31-1 tiles.
 constexpr int64_t kBlocksPerSmCap = 1 << 20;
 constexpr int kThreads = 256;
-constexpr unsigned kPrefetchers = 3 * 148 * 8;  // see prefetch_first_tile
+constexpr unsigned kAskers = 16 * kB200Sms;  // blocks that ask ahead, see prefetch_first_tile
 
 // One 16-byte input chunk -> its fp8 bytes, stored with one instruction.
 template <int IN, int OUT>
@@ -75,7 +75,7 @@ saturated_cast_stream(const uint4 *__restrict__ in, uint8_t *__restrict__ out, c
   const int64_t nchunks = numel / C::kElems;
   constexpr int64_t kTile = int64_t(kThreads) * UNROLL;
   if constexpr (PREFETCH) {
-    if (threadIdx.x == 0 && blockIdx.x < kPrefetchers) prefetch_first_tile(in, blockIdx.x * kTile, kTile, nchunks);
+    if (threadIdx.x == 0 && blockIdx.x < kAskers) prefetch_first_tile(in, blockIdx.x * kTile, kTile, nchunks);
   }
   pdl_wait();
   const typename C::Scale s = C::load_scale(scale);
@@ -122,8 +122,9 @@ int launch(const void *in, void *out, const float *scale, int64_t numel, const D
   if (aligned_to(in, 16) && aligned_to(out, 8)) {
     const int64_t tiles = ceil_div64(numel / C::kElems, int64_t(kThreads) * kUnroll);
     const int grid = balanced_grid(tiles, max_grid);
-    auto kernel = prefetch_pays(numel * (16 / C::kElems)) ? saturated_cast_stream<IN, OUT, kUnroll, true>
-                                                                          : saturated_cast_stream<IN, OUT, kUnroll, false>;
+    constexpr Asks kAsks = IN == DTQ_BF16 ? Asks::kCastBf16 : Asks::kCastF32;
+    auto kernel = asks_ahead(kAsks, numel * (16 / C::kElems)) ? saturated_cast_stream<IN, OUT, kUnroll, true>
+                                                              : saturated_cast_stream<IN, OUT, kUnroll, false>;
     return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(kThreads), 0, st,
                                                static_cast<const uint4 *>(in), static_cast<uint8_t *>(out), scale, numel));
   } else {

@@ -17,6 +17,7 @@ cudaError_t cudaGetLastError() {
 int rule_tensorwise(long long bytes, int aligned, int clusters, int cooperative) {
   return static_cast<int>(dtq::tensorwise_path(bytes, aligned != 0, clusters != 0, cooperative != 0));
 }
+int rule_asks_ahead(int kernel, long long bytes) { return dtq::asks_ahead(static_cast<dtq::Asks>(kernel), bytes); }
 int rule_amax_asks(long long bytes, int grid, int tile_chunks) { return dtq::amax_ask_chunks(bytes, grid, tile_chunks); }
 int rule_turned_down(int error) { return dtq::turned_down_for_room(static_cast<cudaError_t>(error)); }
 
