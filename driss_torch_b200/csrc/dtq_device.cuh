@@ -139,10 +139,17 @@ constexpr int kB200Sms = 148;
 //      32 MiB   9.11  -8.7 -13.6 -15.1    9.28  -7.4 -11.6 -15.5                           27.9 -1.0 -1.0 -0.7
 //     128 MiB  30.9   -2.1  -3.0  -4.0   31.0   -2.8  -3.7  -4.7                           96.8 -0.4 -0.6 -0.8
 // Below 16 MiB the grid is not much more than what is resident at once, and the loads follow at the prefetch's heels.
-// Up to 512 KiB it is on again, for the tokens of a decode step: the product queued behind asks for its weights as soon as it is
-// resident, and the cast's reads would stand behind those.  Cast and product, us, without / with, both with two stages of
-// weights per CTA: row-wise 16 x 8192 x 4096 11.2 / 10.8, 60 x 8192 x 4096 12.9 / 12.7, MXFP8 17 x 2048 x 8192 8.6 / 8.4, 16 x 4096 x
-// 4096 8.1 / 8.0, 8 x 8192 x 8192 16.3 / 16.3, MXFP4 16 x 8192 x 8192 11.7 / 11.55.
+// Up to 2 MiB it is on again, for the tokens of a decode step: the product queued behind asks for its weights as soon as it is
+// resident, and the cast's reads would stand behind those.  Cast and product, weights from memory, us, without / with, two (MXFP8),
+// four (MXFP4) and three (row-wise) stages of weights asked for by the product:
+//   tokens of K = 8192, N = 8192    16 (0.25 MiB)    33 (0.5)         64 (1)           128 (2)
+//   MXFP8                           16.77 / 16.67    17.38 / 17.26    18.31 / 18.22    21.37 / 21.24
+//   MXFP4                           11.80 / 11.15    12.49 / 11.85    13.59 / 12.98    16.32 / 15.59
+//   row-wise                        16.53 / 16.46    17.35 / 17.19    18.46 / 18.25    21.12 / 20.93
+//   128 tokens of K = 4096 (1 MiB), N = 8192: 15.85 / 15.54, 11.43 / 11.25, 15.56 / 15.10; of K = 16384 (4), N = 4096: 23.37 / 23.37, 18.17 / 17.60,
+//   23.12 / 22.86
+// By themselves, from memory: static cast 1 MiB 1.76 / 1.57, 2 MiB 2.10 / 1.88; MX 2.04 / 1.89, 2.27 / 2.01; row-wise 2.20 / 2.08, 3.00 / 2.33; in L2 all
+// of them equal but the blocked MX cast, 1.95 / 2.00 and 2.09 / 2.20.
 __device__ __forceinline__ void prefetch_first_tile(const uint4 *in, int64_t first, int64_t chunks, int64_t nchunks) {
   const int64_t left = nchunks - first;
   if (left > 0) l2_prefetch_bulk(in + first, unsigned((left < chunks ? left : chunks) * sizeof(uint4)));

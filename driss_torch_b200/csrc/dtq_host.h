@@ -121,7 +121,7 @@ inline bool aligned_to(const void *p, uintptr_t a) { return (reinterpret_cast<ui
 // for either answer: with the question at run time the compiler orders the rest of them differently, and those that do not
 // ask ahead lost up to 2 %.
 enum class Asks { kCastBf16, kCastF32, kMx, kMxBlocked, kMxFormats, kRowwise };
-constexpr int64_t kAskSmallBytes = int64_t(512) << 10;  // the tokens of a decode step
+constexpr int64_t kAskSmallBytes = int64_t(2) << 20;  // the tokens of a decode step: 128 of K = 8192
 inline bool asks_ahead(Asks kernel, int64_t input_bytes) {
   if (input_bytes <= kAskSmallBytes) return true;
   const auto mebibytes = [=](int64_t from, int64_t to) { return input_bytes >= from << 20 && input_bytes <= to << 20; };

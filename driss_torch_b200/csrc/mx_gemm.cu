@@ -945,23 +945,27 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 //     partials of its share of the tokens through distributed shared memory, in the order of K;
 //   * while the kernel before this one drains, the first stages of weights are already asked into L2: that is where this
 //     GPU's memory is coherent, so it does not matter whether that kernel still writes them.
-// Measured (B200, products back to back, weights not in L2, 8 stages prefetched; 128 x 128 kernel -> this one; reading the weights
+// Measured (B200, products back to back, weights not in L2, 8 stages asked ahead at that time; 128 x 128 kernel -> this one; reading the weights
 // alone at the measured copy rate): 8 x 8192 x 8192 MXFP8 27.9 -> 13.6 us (10.3), 16 x 8192 x 4096 row-wise 15.4 -> 8.5 (5.1),
 // 16 x 256 x 8192 16.5 -> 5.0, 300 x 2048 x 8192 19.4 -> 14.3.
 constexpr int kSplitThreads = 192;   // producer warp, MMA warp, 4 warps that empty tensor memory; all six add up and store
 constexpr int kSplitWarps = kSplitThreads / 32;
 constexpr int kMaxSplits = 8;        // portable cluster size
 // Stages of weights asked into L2 ahead of the dependency.  Few: the kernel that the dependency waits for (the cast of the
-// tokens) reads through the same memory, and it is what everybody waits for.  Cast and product, us, with 0 / 2 / 4 / 8 stages:
-// MXFP8 8 x 8192 x 8192 16.7 / 16.4 / 16.6 / 17.0, 100 x 4096 x 8192 16.2 / 15.6 / 15.9 / 16.8, row-wise 16 x 8192 x 4096
-// 11.6 / 11.2 / 11.5 / 12.1, 60 x 8192 x 4096 13.2 / 12.9 / 13.2 / 13.7, MXFP4 16 x 8192 x 8192 12.1 / 11.7 / 11.8 / 12.6; where two
-// CTAs share a tile of 64 stages (8 x 16384 x 8192) 27.0 / 26.4 / 26.1 / 26.4.
-// Since the casts ask for few tokens ahead of their own wait (asks_ahead in dtq_host.h), 2 / 4 / 8 stages: row-wise 16 x 8192 x
-// 4096 10.8 / 10.5 / 10.8, 60 x 8192 x 4096 12.7 / 12.4 / 12.5, 8 x 16384 x 8192 26.5 / 26.1 / 26.3, MXFP4 16 x 8192 x 8192 11.6 / 11.1 /
-// 11.3, 4 x 12288 x 4096 9.9 / 9.8 / 9.8, but MXFP8 8 x 8192 x 8192 16.3 / 16.5 / 16.9, 100 x 4096 x 8192 15.7 / 15.9 / 16.8: its cast
-// also writes scales into whole atoms, and is the longest of the three.
+// tokens) reads through the same memory, and it is what everybody waits for; but that cast asks for its tokens ahead of its own
+// wait (asks_ahead in dtq_host.h).  Cast and product, us, with 2 / 3 / 4 stages:
+//   tokens x N x K        MXFP8                    MXFP4                    row-wise
+//    16 x 8192 x 4096     11.17 / 10.98 / 10.78     9.17 /  9.00 /  8.85    10.69 / 10.54 / 10.46
+//    64 x 8192 x 4096     12.79 / 12.68 / 12.64    10.11 / 10.13 / 10.13    12.70 / 12.56 / 12.52
+//    16 x 8192 x 8192     16.67 / 16.76 / 16.98    11.56 / 11.36 / 11.15    16.22 / 16.46 / 16.81
+//    64 x 8192 x 8192     18.22 / 18.25 / 18.62    13.15 / 13.03 / 12.98    18.12 / 18.25 / 18.53
+//   128 x 8192 x 8192     21.24 / 21.32 / 21.57    15.81 / 15.66 / 15.59    20.83 / 20.93 / 21.22
+//    16 x 16384 x 8192    27.44 / 27.36 / 27.21    17.12 / 17.04 / 17.13    26.90 / 26.70 / 26.65
+//    64 x 4096 x 16384    19.02 / 19.23 / 19.73    13.82 / 13.79 / 13.70    19.34 / 19.65 / 20.09
+// None / eight: MXFP8 8 x 8192 x 8192 16.9 / 17.2, row-wise 16 x 8192 x 4096 11.5 / 10.8.  Three for the row-wise product because
+// with four 64 x 8192 x 8192 was behind two without the cast's asking (18.53 against 18.37).
 template <int MODE>
-constexpr int kSplitPrefetch = MODE == kMxFp8 ? 2 : 4;
+constexpr int kSplitPrefetch = MODE == kMxFp8 ? 2 : (MODE == kRowwise ? 3 : 4);
 
 template <int BN, int STAGES, int MODE>
 struct __align__(1024) SplitSmem {

@@ -81,8 +81,8 @@ def test_amax_asks_for_four_mebibytes_of_small_inputs(rules, size, grid, chunks)
 def test_which_casts_ask_ahead(rules, kernel, ranges):
     # outside of these some use loses: a blocked MX cast of 512 MiB took 125.3 us with asking, 120.9 without
     code = ["cast bf16", "cast fp32", "mx", "mx blocked", "mx formats", "rowwise"].index(kernel)
-    small = 512 << 10
-    sizes = [0, small, small + 16] + [m * MIB + d for m in (1, 16, 28, 48, 64, 80, 128, 512, 4096) for d in (-16, 0, 16)]
+    small = 2 * MIB  # 128 tokens of K = 8192
+    sizes = [0, small, small + 16] + [m * MIB + d for m in (1, 4, 16, 28, 48, 64, 80, 128, 512, 4096) for d in (-16, 0, 16)]
     for size in sizes:
         want = size <= small or any(a * MIB <= size <= b * MIB for a, b in ranges)
         assert bool(rules.rule_asks_ahead(code, C.c_longlong(size))) == want, size
