@@ -92,13 +92,25 @@ amax_kernel(const void *__restrict__ in, float *__restrict__ out, int64_t numel,
   const int64_t nchunks = (numel - head) / kElems;
   // This launch itself may have started under the tail of its predecessor: part of the block's first tile is asked into L2
   // meanwhile, harmless whatever the predecessor still writes (see l2_prefetch_bulk).  What it hides is the start of the stream.
-  // 4 MiB in all, of inputs of up to 20 MiB (amax_ask_chunks).  Measured, us, bf16, nothing asked / this, inputs from memory
-  // (400 MB of them in turn): amax 8 MiB 5.3 / 4.9, 16 MiB 6.4 / 6.0; amax then both casts 10.0 / 9.6, 12.0 / 11.5; behind an MXFP8
-  // product that writes the input, 16 MiB, 17.5 / 17.4 and 22.7 / 22.5.  More of it gains more on inputs that stay in L2
-  // or where an amax follows an amax, and loses where the kernel before still reads and writes: with whole first tiles, up to 37 MiB,
-  // amax then both casts 39 MiB 22.0 / 24.6, 47 MiB 25.3 / 29.3, 64 MiB 32.7 / 36.4 (with three inputs in turn 21.2 / 23.2, 24.7 / 28.0, 32.4 /
-  // 35.7), behind a product 16 MiB 39.2 / 41.4; with 4 MiB asked 39 MiB still 22.0 / 23.5, 24 MiB 15.8 / 16.2.  Rows that are no
-  // multiple of 16 gain all the same (39 MiB 24.6 / 24.2, whole tiles 23.9), which the amax cannot see.
+  // 4 MiB in all of inputs of up to 20 MiB of bf16 and 22 MiB of fp32, 16 MiB of up to 40 MiB of fp32 (amax_ask_chunks).  Measured, us with
+  // nothing asked, and the change in percent with 4 / 8 / 16 MiB and with whole first tiles (up to 37 MiB); inputs from memory (400 MB of them
+  // in turn) and three inputs in turn:
+  //                         amax, from memory        amax, both casts, from memory   amax, both casts, three
+  //   bf16   8 MiB    5.3   -6.2 -10.8  -9.6  -9.8   10.0  -2.2 -2.5 -2.4  -1.9       9.1 -0.5  0.0  +0.1  -0.1
+  //         16 MiB    6.4   -4.4  -9.7  -7.6  -6.7   11.9  -3.2 -2.5 +0.2  +0.3      12.2 -3.9 -7.3 -11.4 -11.8
+  //         24 MiB    7.4   -2.4  -1.3  +3.2  +5.8   15.8  +2.8 +4.4 +7.4 +12.5      15.6 +2.7 +3.4  +2.9  +6.3
+  //         39 MiB    9.6   -2.5  +0.6  +5.9  +4.3   22.3  +5.2 +6.8 +9.2 +10.7      21.7 +4.9 +6.7  +9.1 +10.5
+  //         47 MiB   11.1   -0.5  -0.6  +0.1  +4.0   25.7  +7.8 +10.1 +11.8 +14.8    25.3 +5.3 +8.5 +10.5 +13.1
+  //         39 MiB, rows no multiple of 16           24.8  -1.5 -3.9 -4.5  -3.6      24.8 -1.4 -4.2  -5.1  -4.4
+  //   fp32  16 MiB    6.5   -7.0 -10.4 -10.2  -9.5   10.5  -4.6 -6.1 -4.3  -3.8       9.7 -2.4 -1.2  -2.3  -2.8
+  //         22 MiB    7.2   -1.5  -2.2  +2.1  +4.5   12.5  -3.7 -7.6 -8.8  -9.8      12.5 -3.7 -9.1 -11.9 -13.9
+  //         24 MiB    7.5   -3.5  -5.0  +0.3  +1.7   13.1  -4.8 -8.2 -7.3  -7.5      13.1 -4.2 -8.7 -13.1 -14.1
+  //         28 MiB    7.9   -5.8  -9.8  -4.2  -0.3   14.5  -5.9 -6.9 -8.0  -5.4      14.7 -4.8 -8.6 -15.0 -15.8
+  //         39 MiB   10.0   -7.0  -3.2  -0.9  -6.2   18.3  -5.3 -7.0 -6.0  -4.2      18.5 -2.3 -8.3 -11.3 -10.9
+  //         47 MiB   11.2   -1.6  -2.8  -1.7  +1.8   21.2  +1.6 +2.6 +5.0  +8.1      20.9 +0.5 +0.1  +1.0  +3.2
+  // It loses where the kernel before, the casts of the tensor before, still reads and writes as much as L2 holds; that ragged
+  // rows of bf16 gain all the same the amax cannot see.  Behind an MXFP8 product that writes the input, 16 MiB: 17.5 us / 17.4 with
+  // 4 MiB, with both casts 39.2 / 39.2 (whole tiles 41.4).
   constexpr int64_t kTile = int64_t(kAmaxThreads) * UNROLL;
   if constexpr (PREFETCH) {
     if (threadIdx.x == 0) prefetch_first_tile(body, blockIdx.x * kTile, ask_chunks, nchunks);
@@ -141,7 +153,7 @@ int launch_amax(const void *in, float *out, int64_t numel, int in_dtype, Workspa
   const int eb = in_dtype == DTQ_BF16 ? 2 : 4;
   const int grid = amax_grid(numel, eb, dev);
   const int64_t head = head_elems(in, eb, numel);
-  const int ask_chunks = amax_ask_chunks(numel * eb, grid, kAmaxThreads * kAmaxUnroll);
+  const int ask_chunks = amax_ask_chunks(numel * eb, in_dtype == DTQ_F32, grid, kAmaxThreads * kAmaxUnroll);
   const bool ask = ask_chunks > 0;
   auto kernel = in_dtype == DTQ_BF16 ? (ask ? amax_kernel<DTQ_BF16, kAmaxUnroll, true> : amax_kernel<DTQ_BF16, kAmaxUnroll, false>)
                                      : (ask ? amax_kernel<DTQ_F32, kAmaxUnroll, true> : amax_kernel<DTQ_F32, kAmaxUnroll, false>);

@@ -137,10 +137,10 @@ inline bool asks_ahead(Asks kernel, int64_t input_bytes) {
 
 // How much of its first tile, in 16-byte chunks, every block of the amax asks for ahead of its dependency; 0: nothing (figures in
 // amax.cu).
-constexpr int64_t kAmaxAskToBytes = int64_t(20) << 20, kAmaxAskBytes = int64_t(4) << 20;
-inline int amax_ask_chunks(int64_t input_bytes, int grid, int tile_chunks) {
-  if (input_bytes > kAmaxAskToBytes) return 0;
-  const int64_t share = kAmaxAskBytes / 16 / grid;
+inline int amax_ask_chunks(int64_t input_bytes, bool f32, int grid, int tile_chunks) {
+  if (input_bytes > int64_t(f32 ? 40 : 20) << 20) return 0;
+  const int64_t in_all = int64_t(f32 && input_bytes > int64_t(22) << 20 ? 16 : 4) << 20;
+  const int64_t share = in_all / 16 / grid;
   return static_cast<int>(share < tile_chunks ? share : tile_chunks);
 }
 

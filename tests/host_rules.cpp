@@ -18,7 +18,7 @@ int rule_tensorwise(long long bytes, int aligned, int clusters, int cooperative)
   return static_cast<int>(dtq::tensorwise_path(bytes, aligned != 0, clusters != 0, cooperative != 0));
 }
 int rule_asks_ahead(int kernel, long long bytes) { return dtq::asks_ahead(static_cast<dtq::Asks>(kernel), bytes); }
-int rule_amax_asks(long long bytes, int grid, int tile_chunks) { return dtq::amax_ask_chunks(bytes, grid, tile_chunks); }
+int rule_amax_asks(long long bytes, int f32, int grid, int tile_chunks) { return dtq::amax_ask_chunks(bytes, f32 != 0, grid, tile_chunks); }
 int rule_turned_down(int error) { return dtq::turned_down_for_room(static_cast<cudaError_t>(error)); }
 
 // One question about clusters: the runtime answers `n`, or fails with `error` as its runtime would.

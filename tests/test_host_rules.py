@@ -66,13 +66,14 @@ def test_launches_turned_down_for_room_go_to_the_grid(rules):
     assert not any(rules.rule_turned_down(e) for e in (0, 1, 700, 719))
 
 
-@pytest.mark.parametrize("size, grid, chunks", [
-    (0, 1, 4096), (64 * 1024, 1, 4096), (4 * MIB, 64, 4096), (8 * MIB, 128, 2048), (20 * MIB, 320, 819), (20 * MIB + 16, 321, 0), (64 * MIB, 512, 0),
-    (20 * MIB, 4096, 64), (1 << 40, 592, 0),
+@pytest.mark.parametrize("size, f32, grid, chunks", [
+    (0, 0, 1, 4096), (64 * 1024, 0, 1, 4096), (4 * MIB, 0, 64, 4096), (8 * MIB, 0, 128, 2048), (20 * MIB, 0, 320, 819), (20 * MIB + 16, 0, 321, 0),
+    (64 * MIB, 0, 512, 0), (20 * MIB, 0, 4096, 64), (1 << 40, 0, 592, 0), (0, 1, 1, 4096), (22 * MIB, 1, 352, 744), (22 * MIB + 16, 1, 353, 2970), (40 * MIB, 1, 320, 3276),
+    (40 * MIB + 16, 1, 321, 0),
 ])
-def test_amax_asks_for_four_mebibytes_of_small_inputs(rules, size, grid, chunks):
+def test_amax_asks_for_part_of_small_inputs(rules, size, f32, grid, chunks):
     # more of them, or of larger ones, takes memory from the kernel before: amax then both casts of 47 MiB 25.3 us -> 29.3
-    assert rules.rule_amax_asks(C.c_longlong(size), grid, 4096) == chunks
+    assert rules.rule_amax_asks(C.c_longlong(size), f32, grid, 4096) == chunks
 
 
 @pytest.mark.parametrize("kernel, ranges", [

@@ -35,7 +35,7 @@ def _rows_of(blocked, rows, kblocks):
 # Edges of asks_ahead and amax_ask_chunks (dtq_host.h); `ragged` lies just above the edge and has a partial last tile.
 @pytest.mark.parametrize("ragged", [0, 1])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("mib", [2, 16, 20, 28, 48, 80, 128])
+@pytest.mark.parametrize("mib", [2, 16, 20, 22, 28, 40, 48, 80, 128])
 def test_every_output_at_the_edges(mib, dtype, ragged):
     x = _input(mib * MIB, dtype, ragged, mib)
     cpu, scale = x.cpu(), torch.full((1,), SCALE, device="cuda")
