@@ -266,8 +266,8 @@ dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float 
 }
 
 // ---- small inputs: one cluster --------------------------------------------------------------------------
-// A few tens of kilobytes are bound by latency, and most of that was the cooperative launch and its grid barrier: 6.2 us
-// whatever the size, since such a launch cannot start under the tail of the kernel before it.  Here the CTAs of one cluster
+// A few tens of kilobytes are bound by latency, and most of that was the cooperative launch and its grid barrier: 4.1 to
+// 6.2 us, since such a launch cannot start under the tail of the kernel before it.  Here the CTAs of one cluster
 // (at most eight, which every device and partition that takes clusters can place) hold the whole input in registers, a thread up
 // to CHUNKS 16-byte chunks of it; every CTA sends its maximum into the others' shared memory and one cluster barrier later
 // converts.  No workspace, no wait that could run out, and a programmatic dependent like the stream kernels.

@@ -1,6 +1,6 @@
 // PyTorch operator boundary: TORCH_LIBRARY(DrissTorch) over the torch-free C ABI.
 //
-// This is the only translation unit that sees torch headers.  It keeps the reference's
+// This translation unit and direct_calls.cpp are the only ones that see torch headers.  It keeps the reference's
 // operator names and schema strings for the quantization path (src/register_ops.cpp:20-30,
 // :40-41), its argument checks and error behaviour (src/saturated_cast.cu:227-252,
 // src/amax.cu:106-119, src/dynamic_scaled_quant.cu:157-176, src/mx_cast.cu:168-246), CUDA-only
