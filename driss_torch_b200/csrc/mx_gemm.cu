@@ -100,6 +100,7 @@ struct __align__(1024) GemmSmem {
   uint8_t b[SH::STAGES][SH::BN * kBK];     // 16 or 32 KB per stage
   uint8_t sfa[SH::STAGES][Format<MODE>::kKAtoms * 512];                  // blocked atoms of 128 rows x 4 k-blocks
   uint8_t sfb[SH::STAGES][SH::BN / 128 * Format<MODE>::kKAtoms * 512];  // [128 tile columns][atom along K]
+  alignas(512) uint8_t out[kEpilogueWarps][32 * 64];  // per epilogue warp 32 rows x 32 bf16 on their way out (store_chunk)
   uint64_t full[SH::STAGES];
   uint64_t empty[SH::STAGES];
   uint64_t tmem_full[SH::ACC];
@@ -364,6 +365,34 @@ __device__ __forceinline__ void tmem_load_wait(uint32_t (&v)[32]) {
                : "memory");
 }
 
+// 32 columns of 32 rows of the output, a row per lane (16 bf16 pairs), to global memory through 2 KB of this warp's own
+// shared memory: read back, four lanes hold 64 consecutive bytes of a row, and a store touches 8 rows instead of 32.
+// With a row per lane and 16 bytes per store, every instruction sent a partial 32-byte sector to each of 32 lines, and these stores
+// bounded the single-CTA kernels wherever K is short.  Three outputs in turn, B200, us, wide / narrow, before -> now: row-wise 19879 x
+// 3072 x 640 89.4 / 93.3 -> 67.7 / 66.4, MXFP8 32768 x 4096 x 256 114.5 / 127.4 -> 74.7 / 82.5 (writing them alone: 72), 4096 x 4096 x 512 17.6 /
+// 17.1 -> 13.4 / 13.0, 1216 x 1280 x 3360 16.0 / 11.3 -> 14.7 / 10.7, 1632 x 736 x 2272 12.3 / 8.6 -> 10.8 / 7.9, 721 x 1784 x 672 7.4 / 5.1 ->
+// 6.6 / 4.7, row-wise 962 x 1392 x 944 11.4 / 7.4 -> 10.1 / 6.8.  The pair kernel stays with TMA stores: 32768 x 4096 x 256 76.9 / 84.8 this way,
+// row-wise 32768 x 4096 x 512 105 / 115.
+// `row0` / `col0`: the chunk's first row and column; N % 8 == 0, so 16 bytes are inside or outside as a whole.
+__device__ __forceinline__ void store_chunk(uint8_t *staging, const uint32_t (&packed)[16], uint16_t *out, int64_t row0, int64_t col0,
+                                            int M, int N, int lane) {
+  __syncwarp();  // the chunk before has been read
+#pragma unroll
+  for (int q = 0; q < 4; ++q)  // 16-byte groups XOR-swizzled by the row pair: both ways free of bank conflicts
+    *reinterpret_cast<uint4 *>(staging + lane * 64 + ((q ^ ((lane >> 1) & 3)) * 16)) =
+        make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
+  __syncwarp();
+  const int q = lane & 3, r = lane >> 2;
+  if (col0 + q * 8 >= N) return;
+  uint16_t *dst = out + (row0 + r) * N + col0 + q * 8;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = r + 8 * i;
+    const uint4 v = *reinterpret_cast<const uint4 *>(staging + row * 64 + ((q ^ ((row >> 1) & 3)) * 16));
+    if (row0 + row < M) stg_stream(dst + int64_t(8 * i) * N, v);  // streaming store: the output must not push the operands out of L2
+  }
+}
+
 struct GemmParams {
   RowwiseEpilogue rowwise;
   uint16_t *out;  // bf16 [M, N]
@@ -554,19 +583,9 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       tmem_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.tmem_empty[acc]);
-      if (row < p.M) {
-        uint16_t *dst = p.out + row * p.N + int64_t(nt) * kBN + half * kHalfCols;
-        const int64_t col0 = int64_t(nt) * kBN + half * kHalfCols;
+      const int64_t col0 = int64_t(nt) * kBN + half * kHalfCols;
 #pragma unroll
-        for (int c = 0; c < kChunks; ++c) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {  // 8 columns = 16 bytes per store; N % 8 == 0
-            if (col0 + c * 32 + q * 8 < p.N)
-              stg_stream(dst + c * 32 + q * 8,  // streaming store: the output must not push the operands out of L2
-                         make_uint4(packed[c][4 * q], packed[c][4 * q + 1], packed[c][4 * q + 2], packed[c][4 * q + 3]));
-          }
-        }
-      }
+      for (int c = 0; c < kChunks; ++c) store_chunk(sm.out[warp - 2], packed[c], p.out, row - lane, col0 + c * 32, p.M, p.N, lane);
     }
   }
 
