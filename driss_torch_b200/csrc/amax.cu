@@ -82,7 +82,8 @@ __device__ __forceinline__ void absmax_stream(AbsMax<IN> &acc, const uint4 *__re
 // PREFETCH: every block asks for the first `ask_chunks` chunks of its first tile ahead of the dependency.
 template <int IN, int UNROLL, bool PREFETCH>
 __global__ void __launch_bounds__(kAmaxThreads)
-amax_kernel(const void *__restrict__ in, float *__restrict__ out, int64_t numel, int64_t head, Workspace *ws, int ask_chunks) {
+amax_kernel(const void *__restrict__ in, float *__restrict__ out, int64_t numel, int64_t head, Workspace *ws, int ask_chunks,
+            LaunchPad<44>) {
   __shared__ float smem32[32];
   __shared__ int flag;
   constexpr int kElems = 16 / AbsMax<IN>::kElemBytes;
@@ -157,7 +158,8 @@ int launch_amax(const void *in, float *out, int64_t numel, int in_dtype, Workspa
   const bool ask = ask_chunks > 0;
   auto kernel = in_dtype == DTQ_BF16 ? (ask ? amax_kernel<DTQ_BF16, kAmaxUnroll, true> : amax_kernel<DTQ_BF16, kAmaxUnroll, false>)
                                      : (ask ? amax_kernel<DTQ_F32, kAmaxUnroll, true> : amax_kernel<DTQ_F32, kAmaxUnroll, false>);
-  return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(kAmaxThreads), 0, st, in, out, numel, head, ws, ask_chunks));
+  return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(kAmaxThreads), 0, st, in, out, numel, head, ws, ask_chunks,
+                                             LaunchPad<44>{}));
 }
 
 }  // namespace dtq
@@ -236,8 +238,8 @@ extern "C" int dtq_amax_static_scratch(const void *in, float *out, int64_t numel
   const int grid = static_cast<int>(tiles < 1 ? 1 : tiles);  // <= kMaxGridBlocks by the size check
   const int64_t head = head_elems(in, eb, numel);
   if (in_dtype == DTQ_BF16)
-    amax_kernel<DTQ_BF16, kAmaxUnroll, false><<<grid, kAmaxThreads, 0, st>>>(in, out, numel, head, ws, 0);
+    amax_kernel<DTQ_BF16, kAmaxUnroll, false><<<grid, kAmaxThreads, 0, st>>>(in, out, numel, head, ws, 0, {});
   else
-    amax_kernel<DTQ_F32, kAmaxUnroll, false><<<grid, kAmaxThreads, 0, st>>>(in, out, numel, head, ws, 0);
+    amax_kernel<DTQ_F32, kAmaxUnroll, false><<<grid, kAmaxThreads, 0, st>>>(in, out, numel, head, ws, 0, {});
   return cuda_status(cudaGetLastError());
 }

@@ -163,7 +163,8 @@ __device__ __forceinline__ void store_tile(const uint4 (&v)[UNROLL], const DsqSc
 template <int IN, int OUT, int UNROLL, bool P2P>
 __global__ void __launch_bounds__(kFusedThreads, kFusedBlocksPerSm)
 dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float *__restrict__ amax_out,
-                 float *__restrict__ scale_out, int64_t numel, Workspace *ws, int smem_tiles, PeerExchange px) {
+                 float *__restrict__ scale_out, int64_t numel, Workspace *ws, int smem_tiles, PeerExchange px,
+                 LaunchPad<56 + sizeof(PeerExchange)>) {
   using C = DsqChunk<IN, OUT>;
   extern __shared__ uint4 kept_smem[];  // [smem_tiles][UNROLL][kFusedThreads]
   __shared__ float smem32[32];
@@ -278,7 +279,7 @@ constexpr int kClusterCtas = 8;
 template <int IN, int OUT, int CHUNKS>
 __global__ void __launch_bounds__(kClusterThreads, 1)
 dsq_cluster_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float *__restrict__ amax_out,
-                   float *__restrict__ scale_out, int64_t numel) {
+                   float *__restrict__ scale_out, int64_t numel, LaunchPad<40>) {
   using C = DsqChunk<IN, OUT>;
   __shared__ float smem32[32];
   __shared__ float maxima[kClusterCtas];  // one from every CTA of the cluster
@@ -320,7 +321,7 @@ constexpr int kCastPrefetchTiles = 6;  // tiles per block asked of L2 while the 
 template <int IN, int OUT, int UNROLL>
 __global__ void __launch_bounds__(kThreads, 2048 / kThreads)
 cast_with_amax_stream(const uint4 *__restrict__ in, uint8_t *__restrict__ out, const float *__restrict__ amax_p,
-                      float *__restrict__ scale_out, float *__restrict__ amax_out, int64_t numel) {
+                      float *__restrict__ scale_out, float *__restrict__ amax_out, int64_t numel, LaunchPad<48>) {
   using C = DsqChunk<IN, OUT>;
   pdl_launch_dependents();
   const int64_t nchunks = numel / C::kElems;
@@ -454,14 +455,18 @@ int launch_fused_kernel(const void *in, void *out, float *amax_out, float *scale
   if (int e = fused_plan(kernel, dev, cache, ready, &plan)) return e;
   const int64_t tiles = ceil_div64(numel / C::kElems, int64_t(kFusedThreads) * kUnroll);
   const int grid = balanced_grid(tiles, plan.max_grid);
-  const uint4 *in4 = static_cast<const uint4 *>(in);
-  uint8_t *o = static_cast<uint8_t *>(out);
-  int smem_tiles = plan.smem_tiles;
-  PeerExchange exchange = px;
-  const size_t dyn = size_t(smem_tiles) * kFusedThreads * kUnroll * 16;
-  void *args[] = {&in4, &o, &amax_out, &scale_out, &numel, &ws, &smem_tiles, &exchange};
-  DTQ_CUDA_TRY(
-      cudaLaunchCooperativeKernel(reinterpret_cast<void *>(kernel), dim3(grid), dim3(kFusedThreads), args, dyn, st));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kFusedThreads);
+  cfg.dynamicSmemBytes = size_t(plan.smem_tiles) * kFusedThreads * kUnroll * 16;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  DTQ_CUDA_TRY(launch_quickly(cfg, kernel, static_cast<const uint4 *>(in), static_cast<uint8_t *>(out), amax_out, scale_out, numel, ws,
+                              plan.smem_tiles, px, LaunchPad<56 + sizeof(PeerExchange)>{}));
   return DTQ_OK;
 }
 
@@ -492,7 +497,8 @@ int launch_cluster_kernel(const void *in, void *out, float *amax_out, float *sca
   cfg.gridDim = dim3(ctas);
   attr[0].val.clusterDim.x = ctas;
   cfg.numAttrs = 2;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<const uint4 *>(in), static_cast<uint8_t *>(out), amax_out, scale_out, numel);
+  const cudaError_t e = launch_quickly(cfg, kernel, static_cast<const uint4 *>(in), static_cast<uint8_t *>(out), amax_out, scale_out, numel,
+                                       LaunchPad<40>{});
   if (turned_down_for_room(e)) {
     (void)cudaGetLastError();
     *taken = false;
@@ -531,7 +537,7 @@ int launch_fused(const void *in, void *out, float *amax_out, float *scale_out, i
     const int grid = balanced_grid(tiles, int64_t(dev.sm_count) * kCastBlocksPerSmCap);
     return cuda_status(launch_after_dependency(cast_with_amax_stream<IN, OUT, kUnroll>, dim3(grid), dim3(kThreads),
                                                0, st, static_cast<const uint4 *>(in), o, &ws->amax, scale_out, amax_out,
-                                               numel));
+                                               numel, LaunchPad<48>{}));
   }
   if (path == Tensorwise::kGrid)
     return launch_fused_kernel<IN, OUT, false>(in, out, amax_out, scale_out, numel, ws, dev, PeerExchange{}, st);
@@ -554,7 +560,7 @@ int launch_cast(const void *in, void *out, const float *amax, float *scale_out, 
     const int grid = balanced_grid(tiles, max_grid);
     return cuda_status(launch_after_dependency(cast_with_amax_stream<IN, OUT, kUnroll>, dim3(grid),
                                                dim3(kThreads), 0, st, static_cast<const uint4 *>(in), o, amax, scale_out,
-                                               static_cast<float *>(nullptr), numel));
+                                               static_cast<float *>(nullptr), numel, LaunchPad<48>{}));
   } else {
     const int64_t blocks = ceil_div64(numel, kThreads);
     const int grid = static_cast<int>(blocks < 1 ? 1 : (blocks < max_grid ? blocks : max_grid));

@@ -32,7 +32,7 @@ constexpr int kUnroll = 4;  // tied to the scale-byte mapping below: lane&3 pick
 template <bool BLOCKED, bool PREFETCH>
 __global__ void __launch_bounds__(kThreads, 2048 / kThreads)
 mx_stream_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, uint8_t *__restrict__ scales,
-                 int64_t nchunks, int64_t kblocks, int64_t katoms, int64_t rows, unsigned pad_blocks) {
+                 int64_t nchunks, int64_t kblocks, int64_t katoms, int64_t rows, unsigned pad_blocks, LaunchPad<60>) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int64_t kTile = int64_t(kThreads) * kUnroll;
   // may have become resident under the tail of the kernel before it on the stream: wait for that kernel
@@ -121,7 +121,7 @@ int launch_mx(const void *in_bf16, void *payload, void *scales_e8m0, int64_t row
     return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(kThreads), 0, st,
                                                static_cast<const uint4 *>(in_bf16), static_cast<uint8_t *>(payload),
                                                static_cast<uint8_t *>(scales_e8m0), nchunks, kblocks, katoms, rows,
-                                               static_cast<unsigned>(pad_blocks)));
+                                               static_cast<unsigned>(pad_blocks), LaunchPad<60>{}));
   } else {
     const int64_t blocks = ceil_div64(numel / 32, kThreads);
     const int grid = static_cast<int>(blocks < max_grid ? blocks : max_grid);

@@ -53,7 +53,7 @@ __device__ __forceinline__ unsigned int ld_relaxed_u32(const unsigned int *p) {
 
 __global__ void __launch_bounds__(kThreadsA, 2048 / kThreadsA)
 mx_amax_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, uint8_t *__restrict__ scales,
-               int64_t nchunks, Workspace *ws) {
+               int64_t nchunks, Workspace *ws, LaunchPad<40>) {
   __shared__ uint32_t warp_cand[kThreadsA / 32];
   pdl_launch_dependents();  // the finishing warp may become resident now; it waits for this grid to complete
   pdl_wait();               // and this grid itself may have become resident under the tail of the kernel before it
@@ -107,7 +107,7 @@ mx_amax_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, uint
 // exchanges with the peers if asked to, writes the result.
 template <bool P2P>
 __global__ void __launch_bounds__(32)
-mx_amax_finish_kernel(float *__restrict__ amax_out, Workspace *ws, PeerExchange px) {
+mx_amax_finish_kernel(float *__restrict__ amax_out, Workspace *ws, PeerExchange px, LaunchPad<16 + sizeof(PeerExchange)>) {
   const int lane = threadIdx.x;
   pdl_launch_dependents();  // a cast queued behind this launch may become resident while the maxima meet
   pdl_wait();               // every block of the MX kernel has folded its maximum
@@ -140,9 +140,10 @@ int launch_mx_amax(const void *in_bf16, void *payload, void *scales, float *amax
   Workspace *ws = static_cast<Workspace *>(workspace);
   if (numel > 0)
     DTQ_CUDA_TRY(launch_after_dependency(mx_amax_kernel, dim3(grid), dim3(kThreadsA), 0, st, static_cast<const uint4 *>(in_bf16),
-                                         static_cast<uint8_t *>(payload), static_cast<uint8_t *>(scales), nchunks, ws));
+                                         static_cast<uint8_t *>(payload), static_cast<uint8_t *>(scales), nchunks, ws, LaunchPad<40>{}));
   // an empty shard still takes part in the exchange
-  return cuda_status(launch_after_dependency(mx_amax_finish_kernel<P2P>, dim3(1), dim3(32), 0, st, amax_out, ws, px));
+  return cuda_status(launch_after_dependency(mx_amax_finish_kernel<P2P>, dim3(1), dim3(32), 0, st, amax_out, ws, px,
+                                             LaunchPad<16 + sizeof(PeerExchange)>{}));
 }
 
 }  // namespace

@@ -151,7 +151,7 @@ template <bool BLOCKED, bool ROW_OUT>
 __global__ void __launch_bounds__(kThreadsDual, kDualMinBlocks)
 mx_dual_kernel(const uint16_t *__restrict__ in, uint8_t *__restrict__ payload, uint8_t *__restrict__ scales,
                uint8_t *__restrict__ payload_t, uint8_t *__restrict__ scales_t, int64_t rows, int64_t cols,
-               int64_t row_tiles, int64_t col_tiles, bool atoms_aligned) {
+               int64_t row_tiles, int64_t col_tiles, bool atoms_aligned, LaunchPad<73>) {
   __shared__ __align__(16) uint32_t tile[kTile][kTileWords];
   __shared__ __align__(16) uint8_t atoms[2][512];  // blocked scales of the tile, of x and of x^T
   // programmatic dependent launch, both ways (see dtq_device.cuh): blocks may become resident under the tail of the
@@ -196,7 +196,7 @@ int launch_dual(const void *in_bf16, void *payload, void *scales_e8m0, void *pay
                                              static_cast<uint8_t *>(payload), static_cast<uint8_t *>(scales_e8m0),
                                              static_cast<uint8_t *>(payload_t), static_cast<uint8_t *>(scales_t_e8m0), rows, cols,
                                              row_tiles, col_tiles,
-                                             (!row_out || aligned_to(scales_e8m0, 16)) && aligned_to(scales_t_e8m0, 16)));
+                                             (!row_out || aligned_to(scales_e8m0, 16)) && aligned_to(scales_t_e8m0, 16), LaunchPad<73>{}));
 }
 }  // namespace
 }  // namespace dtq

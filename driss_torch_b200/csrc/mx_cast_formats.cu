@@ -149,7 +149,7 @@ template <int IN, int FMT, bool PREFETCH>
 __global__ void __launch_bounds__(kThreadsF, 2048 / kThreadsF)
 mx_formats_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, uint8_t *__restrict__ scales,
                   int64_t nchunks, int64_t kblocks,  // kblocks > 0: scales in the MX GEMM's blocked layout, that many per row
-                  int64_t rows, unsigned pad_blocks) {
+                  int64_t rows, unsigned pad_blocks, LaunchPad<52>) {
   // programmatic dependent launch, both ways (see dtq_device.cuh): blocks may become resident under the tail of the
   // kernel before this one, and what is queued behind this one under its own tail
   pdl_launch_dependents();
@@ -220,7 +220,7 @@ int launch_formats(const void *in, void *payload, void *scales, int64_t numel, i
   return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(kThreadsF), 0, st,
                                              static_cast<const uint4 *>(in), static_cast<uint8_t *>(payload),
                                              static_cast<uint8_t *>(scales), nchunks, kblocks, rows,
-                                             static_cast<unsigned>(pad_blocks)));
+                                             static_cast<unsigned>(pad_blocks), LaunchPad<52>{}));
 }
 
 template <int IN>

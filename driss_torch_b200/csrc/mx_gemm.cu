@@ -83,6 +83,8 @@ struct GemmShape {
 };
 using WideShape = GemmShape<256, 4, 1>;
 using NarrowShape = GemmShape<128, 6, 2>;
+template <int MAPS, typename PARAMS>
+constexpr size_t kGemmParameterBytes = MAPS * sizeof(CUtensorMap) + sizeof(PARAMS);  // all but the padding, see LaunchPad
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // a wait gives up after two seconds of wall time (Workspace::wait_limit_us)
 
 // Shared memory that a kernel asks for: its struct, and what aligning that to 1024 bytes may take.  A struct that outgrew
@@ -404,7 +406,8 @@ struct GemmParams {
 template <typename SH, int MODE>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-               const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb, GemmParams p) {
+               const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb, GemmParams p,
+               LaunchPad<kGemmParameterBytes<4, GemmParams>>) {
   constexpr int kBN = SH::BN, kStagesG = SH::STAGES, kAcc = SH::ACC, kAtomsB = SH::BN / 128;
   constexpr int kKAtoms = Format<MODE>::kKAtoms;
   extern __shared__ unsigned char smem_raw[];
@@ -712,7 +715,7 @@ template <int MODE>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb,
-                    const __grid_constant__ CUtensorMap map_out, PairParams p) {
+                    const __grid_constant__ CUtensorMap map_out, PairParams p, LaunchPad<kGemmParameterBytes<5, PairParams>>) {
   constexpr int kKAtoms = Format<MODE>::kKAtoms, kPairStages = PairStages<MODE>;
   extern __shared__ unsigned char smem_raw[];
   PairSmem<MODE> &sm = *reinterpret_cast<PairSmem<MODE> *>(smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u));
@@ -1026,7 +1029,8 @@ __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap *map, int x, i
 template <int BN, int STAGES, int MODE>
 __global__ void __launch_bounds__(kSplitThreads, 2)
 mx_gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                     const __grid_constant__ CUtensorMap map_sfw, const __grid_constant__ CUtensorMap map_sfx, SplitParams p) {
+                     const __grid_constant__ CUtensorMap map_sfw, const __grid_constant__ CUtensorMap map_sfx, SplitParams p,
+                     LaunchPad<kGemmParameterBytes<4, SplitParams>>) {
   using Smem = SplitSmem<BN, STAGES, MODE>;
   static_assert(BN * kBM * 4 <= STAGES * (kBM + BN) * kBK, "partial sums fit the stage buffers");
   constexpr int kKAtoms = Format<MODE>::kKAtoms;
@@ -1371,7 +1375,8 @@ int launch_pair(const GemmCall &c, int max_clusters) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
   cluster_launch_config(&cfg, attr, 2 * clusters, kGemmThreads, 2, smem_bytes<PairSmem<MODE>>(), c.st);
-  return cuda_status(cudaLaunchKernelEx(&cfg, mx_gemm_pair_kernel<MODE>, map_a, map_b, map_sfa, map_sfb, map_out, p));
+  return cuda_status(launch_quickly(cfg, mx_gemm_pair_kernel<MODE>, map_a, map_b, map_sfa, map_sfb, map_out, p,
+                                    LaunchPad<kGemmParameterBytes<5, PairParams>>{}));
 }
 
 // One CTA per tile, tile shape SH.
@@ -1409,7 +1414,7 @@ int launch_shape(const GemmCall &c, const DeviceInfo &dev) {
   const int64_t tiles = int64_t(p.m_tiles) * p.n_tiles;
   const int grid = static_cast<int>(tiles < dev.sm_count ? tiles : dev.sm_count);
   return cuda_status(launch_after_dependency(mx_gemm_kernel<SH, MODE>, dim3(grid), dim3(kGemmThreads), size_t(smem), c.st, map_a,
-                                             map_b, map_sfa, map_sfb, p));
+                                             map_b, map_sfa, map_sfb, p, LaunchPad<kGemmParameterBytes<4, GemmParams>>{}));
 }
 
 // Token rows per tile of the split kernel, and its stages.
@@ -1483,7 +1488,8 @@ int launch_split(const GemmCall &c, int splits) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
   cluster_launch_config(&cfg, attr, static_cast<int>(tiles * p.splits), kSplitThreads, p.splits, smem, c.st);
-  return cuda_status(cudaLaunchKernelEx(&cfg, mx_gemm_split_kernel<BN, SplitStages<BN>, MODE>, map_w, map_x, map_sfw, map_sfx, p));
+  return cuda_status(launch_quickly(cfg, mx_gemm_split_kernel<BN, SplitStages<BN>, MODE>, map_w, map_x, map_sfw, map_sfx, p,
+                                    LaunchPad<kGemmParameterBytes<4, SplitParams>>{}));
 }
 
 // The CTAs per tile that the split kernel gets in the choice below; 1: the call is not one for it.

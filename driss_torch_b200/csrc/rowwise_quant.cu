@@ -84,7 +84,7 @@ struct RowIn<DTQ_F32> {
 template <int IN, int OUT, int CHUNKS, int TEAM_WARPS, bool PREFETCH>
 __global__ void __launch_bounds__(TEAM_WARPS == 1 ? kThreads : 32 * TEAM_WARPS)
 rowwise_regs_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float *__restrict__ amax_out,
-                    float *__restrict__ scale_out, int64_t rows, int chunks_per_row) {
+                    float *__restrict__ scale_out, int64_t rows, int chunks_per_row, LaunchPad<44>) {
   using R = RowIn<IN>;
   constexpr int kTeam = 32 * TEAM_WARPS;
   __shared__ float smem32[32];
@@ -195,7 +195,7 @@ int launch_regs(const void *in, void *out, float *amax_out, float *scale_out, in
   auto kernel = asks_ahead(Asks::kRowwise, rows * chunks_per_row * 16) ? rowwise_regs_kernel<IN, OUT, CHUNKS, TEAM_WARPS, true>
                                                                        : rowwise_regs_kernel<IN, OUT, CHUNKS, TEAM_WARPS, false>;
   return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(threads), 0, st, static_cast<const uint4 *>(in),
-                                             static_cast<uint8_t *>(out), amax_out, scale_out, rows, chunks_per_row));
+                                             static_cast<uint8_t *>(out), amax_out, scale_out, rows, chunks_per_row, LaunchPad<44>{}));
 }
 
 // Smallest team that keeps a thread at <= 4 chunks (64 bytes in flight); the largest team may

@@ -217,7 +217,7 @@ template <typename C, bool BOTH, bool RAGGED>
 __global__ void __launch_bounds__(kThreadsT, kTransposedMinBlocks)
 cast_transposed_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, uint8_t *__restrict__ out_t,
                        const float *__restrict__ scale, float *__restrict__ scale_out, float *__restrict__ amax_out,
-                       int64_t rows, int64_t cols, int64_t col_tiles) {
+                       int64_t rows, int64_t cols, int64_t col_tiles, LaunchPad<72>) {
   __shared__ __align__(16) uint32_t buffer[kTileRows * (RAGGED ? kRaggedPitch : kTileWords)];
   uint32_t (&tile)[kTileRows][kTileWords] = *reinterpret_cast<uint32_t (*)[kTileRows][kTileWords]>(buffer);
   constexpr int kTileCols = 16 * C::kChunkElems;
@@ -243,7 +243,7 @@ template <typename C, bool BOTH>
 __global__ void __launch_bounds__(256)
 cast_transposed_generic(const void *__restrict__ in, uint8_t *__restrict__ out, uint8_t *__restrict__ out_t,
                         const float *__restrict__ scale, float *__restrict__ scale_out, float *__restrict__ amax_out,
-                        int64_t rows, int64_t cols, int64_t col_tiles) {
+                        int64_t rows, int64_t cols, int64_t col_tiles, LaunchPad<72>) {
   __shared__ uint8_t tile[32][33];
   pdl_launch_dependents();
   pdl_wait();
@@ -294,14 +294,14 @@ int launch_transposed(const void *in, void *out, void *out_t, const float *scale
     return cuda_status(launch_after_dependency(kernel, dim3(static_cast<unsigned>(row_tiles * col_tiles)),
                                                dim3(kThreadsT), 0, st, static_cast<const uint4 *>(in),
                                                static_cast<uint8_t *>(out), static_cast<uint8_t *>(out_t), scale, scale_out,
-                                               amax_out, rows, cols, col_tiles));
+                                               amax_out, rows, cols, col_tiles, LaunchPad<72>{}));
   } else {
     const int64_t row_tiles = ceil_div64(rows, 32), col_tiles = ceil_div64(cols, 32);
     if (row_tiles > 0x7FFFFFFFLL / col_tiles) return DTQ_ERR_TOO_LARGE;
     return cuda_status(launch_after_dependency(cast_transposed_generic<C, BOTH>, dim3(static_cast<unsigned>(row_tiles * col_tiles)),
                                                dim3(256), 0, st, in, static_cast<uint8_t *>(out),
                                                static_cast<uint8_t *>(out_t), scale, scale_out, amax_out, rows, cols,
-                                               col_tiles));
+                                               col_tiles, LaunchPad<72>{}));
   }
 }
 
