@@ -246,6 +246,11 @@ __device__ __forceinline__ void issue_mma(uint32_t d_tmem, uint64_t a_desc, uint
                  : "memory");
 #undef DTQ_MMA
 }
+// Instructions of 32 operand bytes that stage `ks` takes: four, but the last one only as many as K has, for what lies behind it
+// arrived as zeros.  Adding them cost as much as any others where the tensor cores are the limit (B200, us, three sets in turn): MXFP8
+// 8721 x 1072 x 1728 22.9 -> 21.8, 933 x 6320 x 1312 12.9 -> 12.5, row-wise 12511 x 272 x 2144 14.2 -> 13.5.
+__device__ __forceinline__ uint32_t live_k(int ks, int k_stages, int last_k) { return ks + 1 == k_stages ? uint32_t(last_k) : 4u; }
+
 // One scale atom, shared memory -> 4 tensor-memory columns (32 rows x 16 bytes, replicated to the four lane quadrants).
 template <bool PAIR>
 __device__ __forceinline__ void copy_scale_atom(uint32_t tmem_col_addr, uint32_t smem_atom_addr) {
@@ -398,7 +403,7 @@ __device__ __forceinline__ void store_chunk(uint8_t *staging, const uint32_t (&p
 struct GemmParams {
   RowwiseEpilogue rowwise;
   uint16_t *out;  // bf16 [M, N]
-  int M, N, K;
+  int M, N, last_k;  // last_k: see live_k
   int m_tiles, n_tiles, k_stages;
   Workspace *ws;
 };
@@ -523,8 +528,10 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
           }
           const uint32_t a_addr = smem_addr(sm.a[stage]), b_addr = smem_addr(sm.b[stage]);
+          const uint32_t live = live_k(ks, p.k_stages, p.last_k);
 #pragma unroll
           for (uint32_t k = 0; k < 4; ++k) {  // four instructions of 32 operand bytes inside the 128-byte swizzle span
+            if (k >= live) break;
             const uint32_t accumulate = (ks > 0 || k > 0) ? 1u : 0u;
             const uint32_t j = Format<MODE>::k_atom(k), id = Format<MODE>::sf_id(k);
             issue_mma<MODE, false>(d_tmem, operand_desc(a_addr + k * 32), operand_desc(b_addr + k * 32),
@@ -708,6 +715,7 @@ struct PairParams {
   RowwiseEpilogue rowwise;
   int M, N;
   int m_pairs, n_tiles, k_stages;  // 256-row tile rows, 256-column tile columns, 128-byte K stages
+  int last_k;                      // see live_k
   Workspace *ws;
 };
 
@@ -832,8 +840,10 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
               }
             }
             const uint32_t a_addr = smem_addr(sm.a[stage]), b_addr = smem_addr(sm.b[stage]);
+            const uint32_t live = live_k(ks, p.k_stages, p.last_k);
 #pragma unroll
             for (uint32_t k = 0; k < 4; ++k) {
+              if (k >= live) break;
               const uint32_t accumulate = (ks > 0 || k > 0) ? 1u : 0u;
               const uint32_t j = Format<MODE>::k_atom(k), id = Format<MODE>::sf_id(k);
               issue_mma<MODE, true>(d_tmem, operand_desc(a_addr + k * 32), operand_desc(b_addr + k * 32),
@@ -1008,6 +1018,7 @@ struct SplitParams {
   uint16_t *out;  // bf16 [M, N]
   int M, N;
   int n_tiles, k_stages, splits;  // 128-column tiles of the output, 128-byte K stages, CTAs per cluster
+  int last_k;                     // see live_k
   Workspace *ws;
 };
 
@@ -1120,8 +1131,10 @@ mx_gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
           }
         }
         const uint32_t w_addr = smem_addr(sm.w[stage]), x_addr = smem_addr(sm.x[stage]);
+        const uint32_t live = live_k(ks, p.k_stages, p.last_k);
 #pragma unroll
         for (uint32_t k = 0; k < 4; ++k) {
+          if (k >= live) break;
           const uint32_t accumulate = (ks > k0 || k > 0) ? 1u : 0u;
           const uint32_t j = Format<MODE>::k_atom(k), id = Format<MODE>::sf_id(k);
           issue_mma<MODE, false>(tmem, operand_desc(w_addr + k * 32), operand_desc(x_addr + k * 32),
@@ -1297,6 +1310,9 @@ int make_scale_map(CUtensorMap *map, const void *base, int64_t atom_rows, int64_
 
 constexpr int kMaxGemmDevices = 64;
 
+// The instructions of 32 operand bytes in the last stage of K.
+int last_k(int64_t k_bytes) { return static_cast<int>(ceil_div64(k_bytes - (ceil_div64(k_bytes, kBK) - 1) * kBK, 32)); }
+
 // Clusters of `cluster` CTAs, launched as a programmatic dependent of what is before it on the stream (attr: room for two).
 void cluster_launch_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, int grid, int threads, int cluster, size_t smem,
                            cudaStream_t st) {
@@ -1369,6 +1385,7 @@ int launch_pair(const GemmCall &c, int max_clusters) {
   p.m_pairs = static_cast<int>(ceil_div64(c.m, 256));
   p.n_tiles = static_cast<int>(ceil_div64(c.n, kPairBN));
   p.k_stages = static_cast<int>(ceil_div64(c.k_bytes, kBK));
+  p.last_k = last_k(c.k_bytes);
   p.ws = c.ws;
   const int64_t tiles = int64_t(p.m_pairs) * p.n_tiles;
   const int clusters = static_cast<int>(tiles < max_clusters ? tiles : max_clusters);
@@ -1406,10 +1423,10 @@ int launch_shape(const GemmCall &c, const DeviceInfo &dev) {
   p.out = static_cast<uint16_t *>(c.out);
   p.M = static_cast<int>(c.m);
   p.N = static_cast<int>(c.n);
-  p.K = static_cast<int>(c.k_bytes);
   p.m_tiles = static_cast<int>(ceil_div64(c.m, kBM));
   p.n_tiles = static_cast<int>(ceil_div64(c.n, SH::BN));
   p.k_stages = static_cast<int>(ceil_div64(c.k_bytes, kBK));
+  p.last_k = last_k(c.k_bytes);
   p.ws = c.ws;
   const int64_t tiles = int64_t(p.m_tiles) * p.n_tiles;
   const int grid = static_cast<int>(tiles < dev.sm_count ? tiles : dev.sm_count);
@@ -1482,6 +1499,7 @@ int launch_split(const GemmCall &c, int splits) {
   p.N = static_cast<int>(c.n);
   p.n_tiles = static_cast<int>(ceil_div64(c.n, kBM));
   p.k_stages = static_cast<int>(ceil_div64(c.k_bytes, kBK));
+  p.last_k = last_k(c.k_bytes);
   p.ws = c.ws;
   const int64_t tiles = int64_t(p.n_tiles) * ceil_div64(c.m, BN);
   p.splits = splits;

@@ -356,6 +356,18 @@ def test_few_tiles_split_along_k(tokens, n, kb, mode):
                            a_dtype=torch.float8_e5m2 if tokens % 2 else E4M3, bias=[None, torch.float32, torch.bfloat16][tokens % 3])
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["mx8", "mx4", "rowwise"])
+@pytest.mark.parametrize("kernel", ["pair", "wide", "narrow"])
+@pytest.mark.parametrize("kb", [16, 32, 64, 80, 128, 144, 176, 224, 256, 2336])
+def test_last_stage_takes_only_the_instructions_that_k_has(mode, kernel, kb):
+    # bytes per operand row: one to four instructions of 32 in the last stage of 128, as the only stage and behind others;
+    # 137 x 264: a ragged last tile both ways, and stores that end inside a chunk of 32 columns
+    k = kb // 32 * 32 if mode == "mx8" else (kb * 2 if mode == "mx4" else kb)
+    if k:
+        _check_exact_on_device(mode, 137, 264, k, kernel, bias=torch.bfloat16 if kb % 64 else None)
+
+
 # ---- the way out of a wait that runs out ---------------------------------------------------------------------------
 
 def test_waits_of_the_gemm_roles_are_warp_wide():
