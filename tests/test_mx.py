@@ -422,6 +422,23 @@ def test_mx_with_amax_equals_mx_and_amax(shape):
     assert dt.amax(a.cuda()).item() == qo.amax(a).item()  # the plain amax kernel still finds the workspace clean
 
 
+@pytest.mark.parametrize("rows,cols", [(8, 1024), (9, 1024), (8192, 1024), (8193, 1024), (2731, 96)])
+def test_mx_with_amax_where_the_last_block_gives_way_to_the_finishing_launch(rows, cols):
+    # blocks of 8192 elements: one, one and a bit, 1024 (the most that finish by themselves), one more, a ragged last one
+    import driss_torch_b200 as dt
+
+    x = (torch.randn(rows, cols, generator=torch.Generator().manual_seed(rows)) * 3).to(torch.bfloat16).cuda()
+    for at in (0, rows * cols // 2, rows * cols - 1):  # the largest in the first block, in one between and in the last
+        y = x.clone()
+        y.view(-1)[at] = -300.0
+        for _ in range(2):  # twice: the workspace must be left clean
+            p, s, amax = dt.mx_fp8_quantize_with_amax(y)
+            assert amax.item() == 300.0
+        want_p, want_s = dt.mx_fp8_quantize(y)
+        assert torch.equal(p.view(torch.uint8), want_p.view(torch.uint8)) and torch.equal(s.view(torch.uint8), want_s.view(torch.uint8))
+    assert dt.amax(x).item() == x.float().abs().max().item()  # the plain amax kernel still finds the workspace clean
+
+
 def test_mx_with_amax_drops_nans_and_handles_empty_and_all_nan():
     import driss_torch_b200 as dt
     from driss_torch_b200 import _cabi
