@@ -35,6 +35,7 @@ SIGNATURES = {
     "dtq_amax": ([_vp, _vp, _i64, _i32, _vp, _sz, _vp], _i32),
     "dtq_amax_static_scratch": ([_vp, _vp, _i64, _i32, _vp], _i32),
     "dtq_dynamic_scaled_quant": ([_vp, _vp, _vp, _vp, _i64, _i32, _i32, _vp, _sz, _vp], _i32),
+    "dtq_dynamic_scaled_quant_blocks": ([_vp, _vp, _vp, _vp, _i64, _i32, _i32, _i32, _vp, _sz, _vp], _i32),
     "dtq_p2p_exchange_bytes": ([], _sz),
     "dtq_dynamic_scaled_quant_p2p": ([_vp, _vp, _vp, _vp, _i64, _i32, _i32, _vp, _sz, _vp, _i32, _i32, C.c_uint32,
                                       C.c_uint32, _vp], _i32),
@@ -181,6 +182,18 @@ def dynamic_scaled_quant(x, out_dtype, out=None, amax_out=None, scale_out=None, 
         "dtq_dynamic_scaled_quant",
     )
     return out
+
+
+@_on_device_of_first_tensor
+def dynamic_scaled_quant_blocks(x, out_dtype, blocks, ws=None):
+    """The persistent kernel with a grid of ``blocks``, whether the device holds them or not: (payload, amax, scale)."""
+    out = torch.empty(x.shape, dtype=out_dtype, device=x.device)
+    amax_out, scale_out = (torch.empty(1, dtype=torch.float32, device=x.device) for _ in range(2))
+    ws = workspace(x.device) if ws is None else ws
+    check(load().dtq_dynamic_scaled_quant_blocks(x.data_ptr(), out.data_ptr(), amax_out.data_ptr(), scale_out.data_ptr(), x.numel(),
+                                                 IN_CODE[x.dtype], OUT_CODE[out_dtype], blocks, ws.data_ptr(), ws.numel(), _stream()),
+          "dtq_dynamic_scaled_quant_blocks")
+    return out, amax_out, scale_out
 
 
 @_on_device_of_first_tensor

@@ -2,8 +2,8 @@
 //
 // Each block publishes one partial and takes a ticket; the block that draws the last ticket
 // reduces all partials.  No output has to be pre-initialised and the workspace is left ready for
-// the next launch.  Waiting (only the fused ops wait) is a bounded spin: if the generation word
-// does not move within the limit, the waiter records DTQ_ERR_TIMEOUT in the workspace and the
+// the next launch.  Waiting (only the fused ops wait) is a bounded spin: if what is waited for
+// does not come within the limit, the waiter records DTQ_ERR_TIMEOUT in the workspace and the
 // block returns, so a launch can never hang the device.
 #pragma once
 
@@ -48,48 +48,126 @@ __device__ __forceinline__ float reduce_partials(const Workspace *ws, float *sme
 
 constexpr unsigned int kSpinLimit = 1u << 20;  // polls, each an L2 round trip plus a short sleep: gives up after about a second
 
-// Grid barrier that also reduces a non-negative float maximum, for kernels whose blocks are all
-// co-resident.  `gen0` is the generation word as read by thread 0 BEFORE the block did anything
-// else; its parity picks the counter pair.  Thread 0 folds the block's value into the running
-// maximum, fences, takes a ticket; the last arriver clears the other parity's pair (the previous
-// launch is long over) and bumps the generation for the next launch.  Everybody then waits for
-// the count to reach gridDim.x (bounded spin) and reads the maximum.  Returns false on timeout
-// (status word set, nothing may be assumed about `*result`).
-__device__ __forceinline__ bool grid_max_barrier(Workspace *ws, unsigned int gen0, float block_value, int *flag,
-                                                 float *shared_result, float *result) {
-  if (threadIdx.x == 0) {
-    const unsigned int slot = gen0 & 1u;
-    atomicMax(&ws->bar_max[slot], __float_as_uint(block_value));
+// ---- a grid that meets without having to be resident as a whole -----------------------------------------------------
+// Every block of the fused kernel owns a share of the input, adds its share's maximum, and waits until all shares are in.  A
+// cooperative launch would make sure that all blocks are there; but in a stream of such launches it costs 2 to 3 us each
+// (dsq_fused_kernel has the figures).  Without it some blocks may not have started, because another stream's kernel holds
+// their SM, and it may hold it for as long as it likes, or wait in turn for an SM that this grid holds.  So nobody waits for a
+// block that has not started: a block claims its share when it starts, a block that has waited for some time takes over
+// shares that nobody has claimed, and a block that starts and finds its share taken leaves.  All who are waited for are running.
+//
+// A share's word: 0 nobody has come; +kOwnerCame by the owner when it starts; 0 -> kTaken by a block that takes the share over;
+// +kTakerDone when that has finished the share.  Whoever comes second, owner or taker, clears the word, and an owner whose share
+// was its own does once the shares are all in.  From then on a zero no longer means that nobody has come: a block that takes
+// one looks again whether all are in, and if so puts the zero back.  (A zero seen before that is true: the share of a word cleared
+// earlier would have to be in.)
+constexpr unsigned int kOwnerCame = 1, kTaken = 2, kTakerDone = 4;
+constexpr int kGaveUp = 0, kMet = 1, kImpatient = 2, kShareIsGone = 3;
+constexpr unsigned int kPatience = 64;  // polls, about 50 us, before a waiting block looks for shares to take over
+
+__device__ __forceinline__ void clear_share(unsigned int *word) { atomicExch(word, 0u); }
+// Thread 0 of the owner, first thing.  Whether the share is its own; if not, it has nothing left to do.
+__device__ __forceinline__ bool claim_own_share(Workspace *ws) {
+  const unsigned int before = atomicAdd(&ws->claims[blockIdx.x], kOwnerCame);
+  if (before == kTaken + kTakerDone) {
     __threadfence();
-    const unsigned int ticket = atomicAdd(&ws->bar_count[slot], 1u);
-    bool ok = true;
-    if (ticket == gridDim.x - 1) {
-      ws->bar_count[slot ^ 1u] = 0;
-      ws->bar_max[slot ^ 1u] = 0;
-      atomicAdd(&ws->generation, 1u);
-    } else {
-      unsigned int spins = 0;
-      while (ld_acquire(&ws->bar_count[slot]) != gridDim.x) {
-        if (++spins > kSpinLimit) {
-          ok = false;
-          atomicExch(&ws->status, DTQ_ERR_TIMEOUT);
-          break;
-        }
-        __nanosleep(20);
-      }
-    }
-    __threadfence();
-    *shared_result = __uint_as_float(ld_acquire(&ws->bar_max[slot]));
-    *flag = ok;
+    clear_share(&ws->claims[blockIdx.x]);
   }
-  __syncthreads();
-  *result = *shared_result;
-  const bool ok = *flag != 0;
-  __syncthreads();
-  return ok;
+  return before == 0;
+}
+// Thread 0: a share's maximum goes in.  `slot`: the parity of `generation` as read before, which picks the counter pair.  The last
+// one clears the other parity's pair (the previous launch is long over) and bumps the generation for the next launch.
+// Returns whether all shares are in.
+__device__ __forceinline__ bool add_share(Workspace *ws, unsigned int slot, float value) {
+  atomicMax(&ws->bar_max[slot], __float_as_uint(value));
+  __threadfence();
+  const unsigned int ticket = atomicAdd(&ws->bar_count[slot], 1u);
+  if (ticket != gridDim.x - 1) return false;
+  ws->bar_count[slot ^ 1u] = 0;
+  ws->bar_max[slot ^ 1u] = 0;
+  atomicAdd(&ws->generation, 1u);
+  return true;
+}
+// Thread 0: waits for all shares, for at most `polls`.
+__device__ __forceinline__ bool wait_for_shares(const Workspace *ws, unsigned int slot, unsigned int polls) {
+  for (unsigned int spins = 0; ld_acquire(&ws->bar_count[slot]) != gridDim.x;) {
+    if (++spins > polls) return false;
+    __nanosleep(20);
+  }
+  return true;
+}
+// Thread 0 of an owner, when all shares are in: the maximum.
+__device__ __forceinline__ float shares_are_in(Workspace *ws, unsigned int slot) {
+  __threadfence();  // whoever sees the word cleared also sees all shares in
+  clear_share(&ws->claims[blockIdx.x]);
+  return __uint_as_float(ld_acquire(&ws->bar_max[slot]));
 }
 
-// ---- the same barrier with an exchange across GPUs in its serial section -------------------------
+// What a block took over (shared memory; a bit per share).
+struct TakenShares {
+  int candidate;
+  int taken;
+  unsigned int bits[kMaxShares / 32];
+  template <typename F>
+  __device__ __forceinline__ void for_each(F f) const {
+    for (int w = 0; w < kMaxShares / 32; ++w)
+      for (unsigned int left = bits[w]; left; left &= left - 1) f(w * 32 + __ffs(int(left)) - 1);
+  }
+};
+// All threads of a block that has waited in vain: takes over shares until all are in.  share_max(share) is the share's
+// maximum as block_max_nonneg returns it.  kMet, or kGaveUp after kSpinLimit polls without a share to take.
+template <typename ShareMax>
+__device__ __forceinline__ int take_over_until_met(Workspace *ws, unsigned int slot, TakenShares &mine, ShareMax share_max) {
+  if (threadIdx.x < kMaxShares / 32) mine.bits[threadIdx.x] = 0;
+  unsigned int spins = 0;
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) mine.candidate = -1;
+    __syncthreads();
+    // of the shares that nobody has come for, the one farthest behind this block's own: blocks spread out
+    int best = -1;
+    for (unsigned int j = threadIdx.x; j < gridDim.x; j += blockDim.x)
+      if (ld_acquire(&ws->claims[j]) == 0) best = max(best, int((j + gridDim.x - blockIdx.x) % gridDim.x));
+    if (best >= 0) atomicMax(&mine.candidate, best);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      mine.taken = -1;
+      if (mine.candidate >= 0) {
+        const unsigned int j = (mine.candidate + blockIdx.x) % gridDim.x;
+        if (atomicCAS(&ws->claims[j], 0u, kTaken) == 0u) {
+          __threadfence();
+          if (ld_acquire(&ws->bar_count[slot]) == gridDim.x) clear_share(&ws->claims[j]);
+          else mine.taken = int(j);
+        }
+      }
+    }
+    __syncthreads();
+    const int j = mine.taken;
+    if (j >= 0) {
+      const float value = share_max(j);
+      if (threadIdx.x == 0) {
+        mine.bits[j / 32] |= 1u << (j & 31);
+        add_share(ws, slot, value);
+      }
+    }
+    // (after a share taken: only a look)
+    const bool wait = j < 0;
+    if (threadIdx.x == 0) mine.candidate = wait_for_shares(ws, slot, wait ? kPatience : 0) ? kMet : kImpatient;
+    __syncthreads();
+    if (mine.candidate == kMet) return kMet;
+    if (wait && (spins += kPatience) > kSpinLimit) {
+      if (threadIdx.x == 0) atomicExch(&ws->status, DTQ_ERR_TIMEOUT);
+      return kGaveUp;
+    }
+  }
+}
+// Thread 0, for every share that it took over, when all of them are finished.
+__device__ __forceinline__ void taken_share_is_done(Workspace *ws, int share) {
+  unsigned int *word = &ws->claims[share];
+  if (atomicAdd(word, kTakerDone) == kTaken + kOwnerCame) clear_share(word);
+}
+
+// ---- a grid barrier with an exchange across GPUs in its serial section -------------------------
 // Every rank (one process per GPU, same launch on each) owns a small exchange buffer that all
 // peers can address over NVLink: kPeerParities x kMaxPeers 64-bit slots.  The last block to arrive
 // at the local barrier stores {epoch, local maximum} into its slot of EVERY rank's buffer
@@ -155,7 +233,9 @@ __device__ __forceinline__ unsigned int peer_exchange_max(const PeerExchange &px
   return __reduce_max_sync(0xFFFFFFFFu, value);
 }
 
-// As grid_max_barrier, but the value every block leaves with is the maximum over all ranks.
+// For a grid whose blocks are all resident (a cooperative launch): the maximum over all blocks of all ranks.  `gen0` is the generation word as
+// read by thread 0 BEFORE the block did anything else.  Returns false on timeout (status word set, nothing may be assumed about
+// `*result`).
 // Waiting blocks watch the local count reach gridDim.x + 1: the last arriver adds the extra one
 // after the exchange, when ws->amax holds the global value.
 __device__ __forceinline__ bool grid_max_barrier_exchange(Workspace *ws, unsigned int gen0, float block_value,

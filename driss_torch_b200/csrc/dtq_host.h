@@ -11,6 +11,7 @@
 namespace dtq {
 
 constexpr int kMaxGridBlocks = 4096;  // upper bound on any persistent grid (148 SMs x 16 CTAs fits)
+constexpr int kMaxShares = 1024;      // upper bound on the grid of the fused kernel
 
 // Scratch shared by the single-launch reductions.  Zero-filled once by dtq_workspace_init;
 // every kernel leaves `arrivals` at zero again and only ever advances `generation`.
@@ -31,6 +32,8 @@ struct alignas(256) Workspace {
   unsigned int wait_limit_us;
   unsigned int pad[23];
   float partials[kMaxGridBlocks];
+  // The fused kernel's shares of the input, one word each (see dtq_grid.cuh); zero between launches.
+  unsigned int claims[kMaxShares];
 };
 
 struct DeviceInfo {

@@ -6,13 +6,15 @@
 // which is the arithmetic of the reference's cooperative kernel
 // (src/dynamic_scaled_quant.cu:83-118), restated for bf16 and fp32 inputs.
 //
-// dtq_dynamic_scaled_quant is one cooperative launch of a persistent grid (block b owns tiles
-// b, b+G, b+2G, ...).  The tensor-wise dependency forces a second look at every element; the
+// dtq_dynamic_scaled_quant is one launch of a persistent grid (block b owns tiles
+// b, b+G, b+2G, ...), an ordinary programmatic dependent whose blocks meet without having to be
+// resident together (dtq_grid.cuh).  The tensor-wise dependency forces a second look at every element; the
 // kernel makes as little of that second look as possible come from HBM:
 //   phase 1  each block keeps its FIRST tile in registers and its next few tiles in shared
 //            memory (filled through the registers the max is taken from), then streams the rest;
 //   finish   every block folds its maximum into one word with an atomic max and takes a ticket;
-//            all wait, with a bounded spin, until the ticket count reaches the grid size;
+//            all wait until the ticket count reaches the grid size, and who waits for long takes over the
+//            tiles of blocks that have not started;
 //   phase 2  each block converts its streamed tiles newest-first, so the re-read starts with
 //            what L2 still holds (about 50 MB on B200, measured), with the next tile's loads in
 //            flight while the current one is converted and stored; then the tiles it kept in
@@ -106,6 +108,10 @@ struct DsqChunk<DTQ_F32, OUT> {
 };
 
 // ---- fused single launch -------------------------------------------------------------------------
+// As a cooperative launch, or any that is not a programmatic dependent, it waited in a stream for whole multiples of about 2.05 us from
+// kernel to kernel, which a CUDA graph did not show.  Us in a stream, three inputs in turn, cooperative -> now (and in a graph): bf16 2 MiB 6.4 -> 5.5
+// (the host), 8.4 MiB 6.6 -> 5.5 (5.3 -> 5.2), 16 MiB 10.2 -> 7.8 (7.3 -> 7.1), 24 MiB 12.2 -> 10.0 (9.5 -> 9.3), 32 MiB 13.9 -> 11.9 (12.0 -> 11.9),
+// 64 MiB 20.5 -> 18.1 (18.3 -> 17.9), 128 MiB 45.0 -> 43.4 (43.0), 320 MiB 121.2 -> 119.6 (119.5).
 // Requires `in` 16-byte aligned and `out` aligned for the packed store; numel may be anything
 // (block 0 handles the elements past the last whole chunk).  Dynamic shared memory holds
 // `smem_tiles` tiles.
@@ -158,7 +164,45 @@ __device__ __forceinline__ void store_tile(const uint4 (&v)[UNROLL], const DsqSc
   }
 }
 
-// P2P: the tensor is row-sharded over several GPUs running this same launch; the barrier between
+// A share that its own block has not come for, taken over by another (dtq_grid.cuh): the tiles of block `share`, nothing kept.
+template <typename C, int UNROLL>
+__device__ __noinline__ float share_max(const uint4 *__restrict__ in, int64_t numel, int share) {
+  __shared__ float smem32[32];
+  const int64_t nchunks = numel / C::kElems, tail0 = nchunks * C::kElems;
+  constexpr int64_t kTile = int64_t(kFusedThreads) * UNROLL;
+  typename C::Acc acc0 = 0, acc1 = 0;
+  for (int64_t tile = share; tile * kTile < nchunks; tile += gridDim.x) {
+    uint4 v[UNROLL];
+    load_tile<UNROLL>(v, in, tile, nchunks);
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) C::absmax(acc0, acc1, v[u]);
+  }
+  float a = C::finish(acc0, acc1);
+  if (share == 0 && tail0 + threadIdx.x < numel) a = fmaxf(a, fabsf(C::load_one(in, tail0 + threadIdx.x)));
+  __syncthreads();  // smem32 of the share before
+  return block_max_nonneg(a, smem32, 0.0f);
+}
+template <typename C, int OUT, int UNROLL>
+__device__ __noinline__ void share_cast(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float *amax_out, float *scale_out,
+                                        int64_t numel, float amax, int share) {
+  const DsqScale sd = make_dsq_scale<OUT>(amax);
+  const int64_t nchunks = numel / C::kElems, tail0 = nchunks * C::kElems;
+  constexpr int64_t kTile = int64_t(kFusedThreads) * UNROLL;
+  for (int64_t tile = share; tile * kTile < nchunks; tile += gridDim.x) {
+    uint4 v[UNROLL];
+    load_tile<UNROLL>(v, in, tile, nchunks);
+    store_tile<C, UNROLL>(v, sd, out, tile, nchunks);
+  }
+  if (share != 0) return;
+  if (tail0 + threadIdx.x < numel)
+    out[tail0 + threadIdx.x] = cvt_fp8<OUT>(dsq_mul(sd.sd, C::load_one(in, tail0 + threadIdx.x)));
+  if (threadIdx.x == 0) {
+    if (amax_out) *amax_out = amax;
+    if (scale_out) *scale_out = static_cast<float>(sd.sd);
+  }
+}
+
+// P2P: the tensor is row-sharded over several GPUs running this same (cooperative) launch; the barrier between
 // the phases also exchanges the per-GPU maxima through peer memory (see grid_max_barrier_exchange).
 template <int IN, int OUT, int UNROLL, bool P2P>
 __global__ void __launch_bounds__(kFusedThreads, kFusedBlocksPerSm)
@@ -167,10 +211,17 @@ dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float 
                  LaunchPad<56 + sizeof(PeerExchange)>) {
   using C = DsqChunk<IN, OUT>;
   extern __shared__ uint4 kept_smem[];  // [smem_tiles][UNROLL][kFusedThreads]
+  // Static shared memory stays small: with 2.3 KB of it two blocks took more than 196 KB of their SM, which left 28 KB of L1 instead of
+  // 60 to the loads in flight, and the kernel took 8 % longer (128 MiB 43.4 -> 47.2 us).
   __shared__ float smem32[32];
   __shared__ int flag;
-  unsigned int gen0 = 0;
-  if (threadIdx.x == 0) gen0 = ld_acquire(&ws->generation);
+  __shared__ unsigned int gen0;  // thread 0's: the generation before this launch, and whether the share is this block's own
+  __shared__ bool own;
+  if constexpr (P2P) {
+    if (threadIdx.x == 0) gen0 = ld_acquire(&ws->generation);
+  } else {
+    pdl_wait();  // may have become resident under the tail of the kernel before it
+  }
 
   const int64_t nchunks = numel / C::kElems;
   constexpr int64_t kTile = int64_t(kFusedThreads) * UNROLL;
@@ -194,9 +245,15 @@ dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float 
   for (int u = 0; u < UNROLL; ++u) first_tile[u] = make_uint4(0, 0, 0, 0);
   if (kRegTiles && count > 0) {
     load_tile<UNROLL>(first_tile, in, blockIdx.x, nchunks);
-#pragma unroll
-    for (int u = 0; u < UNROLL; ++u) C::absmax(acc0, acc1, first_tile[u]);
   }
+  if constexpr (!P2P) {
+    if (threadIdx.x == 0) {  // under the first tile's loads
+      gen0 = ld_acquire(&ws->generation);
+      own = claim_own_share(ws);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < UNROLL; ++u) C::absmax(acc0, acc1, first_tile[u]);  // zeros where the block has no tile
   for (int64_t k = kRegTiles; k < count; k += 2) {  // two tiles (2 * UNROLL loads) in flight
     uint4 v[UNROLL], w[UNROLL];
     const bool second = k + 1 < count;
@@ -230,11 +287,32 @@ dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float 
   // finish
   const float block_value = block_max_nonneg(a, smem32, 0.0f);
   __shared__ float amax_shared;
+  __shared__ TakenShares others;
   float amax;
-  bool met;
-  if constexpr (P2P) met = grid_max_barrier_exchange(ws, gen0, block_value, px, &flag, &amax_shared, &amax);
-  else met = grid_max_barrier(ws, gen0, block_value, &flag, &amax_shared, &amax);
-  if (!met) {  // a bounded wait gave up (the status word says so): no payload, and NaN where a maximum was expected
+  int met;
+  bool took_over = false;
+  if constexpr (P2P) {
+    met = grid_max_barrier_exchange(ws, gen0, block_value, px, &flag, &amax_shared, &amax) ? kMet : kGaveUp;
+  } else {
+    const unsigned int slot = gen0 & 1u;  // thread 0's
+    if (threadIdx.x == 0) {
+      flag = kShareIsGone;
+      if (own) flag = add_share(ws, slot, block_value) || wait_for_shares(ws, slot, kPatience) ? kMet : kImpatient;
+      if (flag == kMet) amax_shared = shares_are_in(ws, slot);
+    }
+    __syncthreads();
+    met = flag;
+    if (met == kShareIsGone) return;
+    if (met == kImpatient) {
+      took_over = true;
+      met = take_over_until_met(ws, slot, others, [&](int share) { return share_max<C, UNROLL>(in, numel, share); });
+      if (threadIdx.x == 0 && met == kMet) amax_shared = shares_are_in(ws, slot);
+      __syncthreads();
+    }
+    amax = amax_shared;
+    pdl_launch_dependents();
+  }
+  if (met == kGaveUp) {  // a bounded wait gave up (the status word says so): no payload, and NaN where a maximum was expected
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       if (amax_out) *amax_out = __uint_as_float(0x7FC00000u);
       if (scale_out) *scale_out = __uint_as_float(0x7FC00000u);
@@ -264,15 +342,21 @@ dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float 
   if (kRegTiles && count > 0) store_tile<C, UNROLL>(first_tile, sd, out, blockIdx.x, nchunks);
   if (blockIdx.x == 0 && tail0 + threadIdx.x < numel)
     out[tail0 + threadIdx.x] = cvt_fp8<OUT>(dsq_mul(sd.sd, C::load_one(in, tail0 + threadIdx.x)));
+  if constexpr (!P2P) {
+    if (took_over) {
+      others.for_each([&](int share) { share_cast<C, OUT, UNROLL>(in, out, amax_out, scale_out, numel, amax, share); });
+      if (threadIdx.x == 0) others.for_each([&](int share) { taken_share_is_done(ws, share); });
+    }
+  }
 }
 
 // ---- small inputs: one cluster --------------------------------------------------------------------------
-// A few tens of kilobytes are bound by latency, and most of that was the cooperative launch and its grid barrier: 4.1 to
-// 6.2 us, since such a launch cannot start under the tail of the kernel before it.  Here the CTAs of one cluster
+// A few tens of kilobytes are bound by latency, and most of that was a cooperative launch and its grid barrier: 4.1 to
+// 6.2 us (the grid kernel without that launch takes 4.4 us at 1.5 MiB).  Here the CTAs of one cluster
 // (at most eight, which every device and partition that takes clusters can place) hold the whole input in registers, a thread up
 // to CHUNKS 16-byte chunks of it; every CTA sends its maximum into the others' shared memory and one cluster barrier later
 // converts.  No workspace, no wait that could run out, and a programmatic dependent like the stream kernels.
-// Measured, us back to back, grid / cluster: bf16 4 KB 4.1 / 1.8, 64 KB 5.6 / 2.2, 256 KB 6.1 / 2.9, 512 KB 6.2 / 3.3, 768 KB 6.2 /
+// Measured, us back to back, grid (cooperative) / cluster: bf16 4 KB 4.1 / 1.8, 64 KB 5.6 / 2.2, 256 KB 6.1 / 2.9, 512 KB 6.2 / 3.3, 768 KB 6.2 /
 // 4.2, 1 MB 6.2 / 4.5 (fp32 6.2 / 4.0); a thread holds sixteen chunks there, and the eight SMs' share of L2 bandwidth is what grows.
 constexpr int kClusterThreads = 512;
 constexpr int kClusterCtas = 8;
@@ -403,7 +487,7 @@ amax_scalar_kernel(const void *__restrict__ in, int64_t numel, float *__restrict
 }
 
 // Per device and kernel instantiation: the shared memory the kernel may keep tiles in and the
-// largest grid a cooperative launch accepts with it (cached after the first call).
+// largest grid that the device holds at once with it (cached after the first call).
 constexpr int kMaxPlanDevices = 64;
 struct FusedPlan {
   int smem_tiles = 0;
@@ -433,7 +517,7 @@ int fused_plan(Kernel kernel, const DeviceInfo &dev, FusedPlan *cache, std::atom
       int per_sm = 0;
       DTQ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kFusedThreads, dyn));
       p.max_grid = per_sm * dev.sm_count;
-      if (p.max_grid > kMaxGridBlocks) p.max_grid = kMaxGridBlocks;
+      if (p.max_grid > kMaxShares) p.max_grid = kMaxShares;
       if (p.max_grid <= 0) return DTQ_ERR_CUDA_BASE + static_cast<int>(cudaErrorLaunchOutOfResources);
       cache[dev_id] = p;
       ready[dev_id].store(1, std::memory_order_release);
@@ -443,10 +527,11 @@ int fused_plan(Kernel kernel, const DeviceInfo &dev, FusedPlan *cache, std::atom
   return DTQ_OK;
 }
 
-// The single persistent launch (optionally with the cross-GPU exchange in its barrier).
+// The single persistent launch (optionally with the cross-GPU exchange in its barrier), of as many blocks as fit the device; P2P == false:
+// or of `blocks`, if that is not 0, whether they fit or not.
 template <int IN, int OUT, bool P2P>
 int launch_fused_kernel(const void *in, void *out, float *amax_out, float *scale_out, int64_t numel, Workspace *ws,
-                        const DeviceInfo &dev, const PeerExchange &px, cudaStream_t st) {
+                        const DeviceInfo &dev, const PeerExchange &px, cudaStream_t st, int blocks = 0) {
   using C = DsqChunk<IN, OUT>;
   static FusedPlan cache[kMaxPlanDevices];
   static std::atomic<int> ready[kMaxPlanDevices];
@@ -454,20 +539,25 @@ int launch_fused_kernel(const void *in, void *out, float *amax_out, float *scale
   FusedPlan plan;
   if (int e = fused_plan(kernel, dev, cache, ready, &plan)) return e;
   const int64_t tiles = ceil_div64(numel / C::kElems, int64_t(kFusedThreads) * kUnroll);
-  const int grid = balanced_grid(tiles, plan.max_grid);
+  const int grid = blocks ? blocks : balanced_grid(tiles, plan.max_grid);
+  const size_t dyn = size_t(plan.smem_tiles) * kFusedThreads * kUnroll * 16;
+  const uint4 *in4 = static_cast<const uint4 *>(in);
+  uint8_t *o = static_cast<uint8_t *>(out);
+  constexpr LaunchPad<56 + sizeof(PeerExchange)> pad{};
+  if constexpr (!P2P)
+    return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(kFusedThreads), dyn, st, in4, o, amax_out, scale_out, numel, ws,
+                                               plan.smem_tiles, px, pad));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kFusedThreads);
-  cfg.dynamicSmemBytes = size_t(plan.smem_tiles) * kFusedThreads * kUnroll * 16;
+  cfg.dynamicSmemBytes = dyn;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  DTQ_CUDA_TRY(launch_quickly(cfg, kernel, static_cast<const uint4 *>(in), static_cast<uint8_t *>(out), amax_out, scale_out, numel, ws,
-                              plan.smem_tiles, px, LaunchPad<56 + sizeof(PeerExchange)>{}));
-  return DTQ_OK;
+  return cuda_status(launch_quickly(cfg, kernel, in4, o, amax_out, scale_out, numel, ws, plan.smem_tiles, px, pad));
 }
 
 // One cluster for inputs of up to kClusterMaxBytes; *taken is false where it cannot be placed.
@@ -596,6 +686,27 @@ extern "C" int dtq_dynamic_scaled_quant(const void *in, void *out, float *amax_o
                : launch_fused<DTQ_BF16, DTQ_E5M2>(in, out, amax_out, scale_out, numel, ws, dev, st);
   return out_dtype == DTQ_E4M3 ? launch_fused<DTQ_F32, DTQ_E4M3>(in, out, amax_out, scale_out, numel, ws, dev, st)
                                : launch_fused<DTQ_F32, DTQ_E5M2>(in, out, amax_out, scale_out, numel, ws, dev, st);
+}
+
+extern "C" int dtq_dynamic_scaled_quant_blocks(const void *in, void *out, float *amax_out, float *scale_out, int64_t numel, int in_dtype,
+                                               int out_dtype, int blocks, void *workspace, size_t workspace_bytes, void *stream) {
+  using namespace dtq;
+  if (numel <= 0 || !in || !out || blocks < 1 || blocks > kMaxShares) return DTQ_ERR_INVALID_ARGUMENT;
+  if (int e = check_dtypes(in_dtype, out_dtype)) return e;
+  if (!workspace || workspace_bytes < sizeof(Workspace) || !aligned_to(workspace, 256)) return DTQ_ERR_WORKSPACE;
+  if (!aligned_to(in, 16) || !aligned_to(out, in_dtype == DTQ_BF16 ? 8 : 4)) return DTQ_ERR_INVALID_ARGUMENT;
+  DeviceInfo dev;
+  if (int e = current_device_info(&dev)) return e;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  Workspace *ws = static_cast<Workspace *>(workspace);
+  const PeerExchange none{};
+  if (in_dtype == DTQ_BF16)
+    return out_dtype == DTQ_E4M3
+               ? launch_fused_kernel<DTQ_BF16, DTQ_E4M3, false>(in, out, amax_out, scale_out, numel, ws, dev, none, st, blocks)
+               : launch_fused_kernel<DTQ_BF16, DTQ_E5M2, false>(in, out, amax_out, scale_out, numel, ws, dev, none, st, blocks);
+  return out_dtype == DTQ_E4M3
+             ? launch_fused_kernel<DTQ_F32, DTQ_E4M3, false>(in, out, amax_out, scale_out, numel, ws, dev, none, st, blocks)
+             : launch_fused_kernel<DTQ_F32, DTQ_E5M2, false>(in, out, amax_out, scale_out, numel, ws, dev, none, st, blocks);
 }
 
 extern "C" size_t dtq_p2p_exchange_bytes(void) { return sizeof(unsigned long long) * dtq::kPeerParities * dtq::kMaxPeers; }

@@ -164,6 +164,15 @@ int dtq_dynamic_scaled_quant(const void *in, void *out, float *amax_out, float *
                              size_t workspace_bytes, void *stream);
 
 /*
+ * The persistent kernel behind dtq_dynamic_scaled_quant with a grid of `blocks` (1 to 1024) instead of as many as the device
+ * holds: for a partition of a device, and to have more blocks than fit, so that the running ones take over the others' shares.
+ * numel > 0; `in` must be 16-byte and `out` 8-byte (bf16) / 4-byte (fp32) aligned.  Same bytes.
+ */
+int dtq_dynamic_scaled_quant_blocks(const void *in, void *out, float *amax_out, float *scale_out,
+                                    int64_t numel, int in_dtype, int out_dtype, int blocks, void *workspace,
+                                    size_t workspace_bytes, void *stream);
+
+/*
  * dtq_dynamic_scaled_quant for a tensor that is row-sharded over the GPUs of one node, one
  * process per GPU, every rank making this same call on its shard: ONE launch per GPU whose
  * grid barrier also exchanges the per-GPU maxima through peer-addressable memory (plain

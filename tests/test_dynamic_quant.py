@@ -415,3 +415,53 @@ def test_one_cluster_equals_the_grid(in_dtype, fp8_dtype, special):
         assert torch.equal(got.view(torch.uint8), want.view(torch.uint8)), (chunks, extra)
         assert _bits(amax) == _bits(want_amax) and _bits(scale) == _bits(want_scale), (chunks, extra)
         assert (room[:32] == 0xAA).all() and (room[32 + n:] == 0xAA).all()
+
+
+# ---- blocks of the grid that have not started: the running ones take over their shares ---------------------------------------
+
+def _words_between_launches(ws):
+    # everything behind the partials: the shares' words
+    return ws.view(torch.int32)[64 + 4096:]
+
+
+@pytest.mark.parametrize("fp8_dtype", FP8_DTYPES)
+@pytest.mark.parametrize("in_dtype", IN_DTYPES)
+@pytest.mark.parametrize("blocks", [1, 7, 296, 297, 700, 1024])
+def test_a_grid_larger_than_the_device_meets_all_the_same(blocks, in_dtype, fp8_dtype):
+    from driss_torch_b200 import _cabi
+
+    ws = torch.zeros(_cabi.load().dtq_workspace_bytes(), dtype=torch.uint8, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(blocks)
+    # tiles of 32 KB: fewer than blocks, some more, several each; whole, and with chunks and elements behind the last whole tile
+    for n in (5, 16384 * 3, 16384 * blocks + 4099, 16384 * min(2 * blocks, 800) + 3):
+        x = torch.randn(n, generator=g, device="cuda").to(in_dtype)
+        for at in (0, n // 2, n - 1):
+            y = x.clone()
+            y[at] = -777.0
+            got, amax, scale = _cabi.dynamic_scaled_quant_blocks(y, fp8_dtype, blocks, ws=ws)
+            want = _cabi.cast_with_amax(y, torch.full((1,), 777.0 if in_dtype == torch.float32 else 776.0, device="cuda"), fp8_dtype)
+            assert torch.equal(got.view(torch.uint8), want.view(torch.uint8)), (n, at)
+            assert amax.item() == (777.0 if in_dtype == torch.float32 else 776.0) and scale.item() > 0
+            assert (_words_between_launches(ws) == 0).all(), (n, at)
+    assert _cabi.workspace_status(ws) == 0
+
+
+def test_launches_that_compete_for_the_device_meet():
+    # four streams, a grid as large as the device on each: whichever blocks start, all launches finish, with their own bytes
+    from driss_torch_b200 import _cabi
+
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    xs = [(torch.randn(n, generator=torch.Generator().manual_seed(i)) * 10.0 ** i).to(torch.bfloat16).cuda()
+          for i, n in enumerate((1 << 20, 5_000_011, 20_000_003, 60_000_001))]
+    wants = [_cabi.cast_with_amax(x, x.float().abs().max().view(1), torch.float8_e4m3fn) for x in xs]
+    room = [torch.zeros(_cabi.load().dtq_workspace_bytes(), dtype=torch.uint8, device="cuda") for _ in xs]
+    torch.cuda.synchronize()
+    got = [[] for _ in xs]
+    for _ in range(12):
+        for i, stream in enumerate(streams):
+            with torch.cuda.stream(stream):
+                got[i].append(_cabi.dynamic_scaled_quant(xs[i], torch.float8_e4m3fn, ws=room[i]))
+    torch.cuda.synchronize()
+    for i, outs in enumerate(got):
+        assert all(torch.equal(o.view(torch.uint8), wants[i].view(torch.uint8)) for o in outs), i
+        assert _cabi.workspace_status(room[i]) == 0 and (_words_between_launches(room[i]) == 0).all()
