@@ -1526,24 +1526,27 @@ int split_worthwhile(int64_t m, int64_t n, int64_t stages, int sm_count) {
 // kernel (0: cannot launch them).  Estimated time, in microseconds as measured on a B200 = a fixed part (launch, set-up,
 // filling the pipeline, the last epilogue) plus, for every round of tiles on the busiest SM, the stages of 128 operand bytes
 // along K at the time of one, and what a tile costs besides; a tile never takes less than its epilogue.
-//   pair   256 x 256 tiles on SM pairs: 5.6 + rounds x max(0.333 stages + 0.6, 1.8; row-wise 2.2)
-//   wide   128 x 256 on one SM: 4.2 + rounds x max(0.36 stages + 1.9, 2.6; row-wise 4.6), its epilogue not overlapped
-//   narrow 128 x 128 on one SM: 3.2 + rounds x max(0.25 stages + 1.1, 1.5; row-wise 0.25 stages + 1.3, 2.4)
+//   pair   256 x 256 tiles on SM pairs: 5.8 + rounds x max(0.333 stages + 0.6, 3.1; row-wise 2.3)
+//   wide   128 x 256 on one SM: 4.2 + rounds x max(0.36 stages + 1.9, 3.2; row-wise 0.36 stages + 2.1, 4.6), its epilogue not overlapped
+//   narrow 128 x 128 on one SM: 3.2 + rounds x max(0.23 stages + 1.1, 1.9; row-wise 0.23 stages + 1.3, 2.4)
 // So large problems run on SM pairs, and problems of about a tile per SM on the narrow kernel, whose smaller tiles also
-// spread a small output over more SMs.  Measured, us, narrow / wide / pair: row-wise 512 x 4096 x 2048 8.9 / 12.0 / 10.7,
-// 500 x 8192 x 1024 10.2 / 10.0 / 8.6, 1024 x 8192 x 2048 23.8 / 21.1 / 16.5, 16384 x 1024 x 1024 28.6 / 29.7 / 19.3;
-// MXFP8 3000 x 1000 x 5120 25.5 / 18.9 / 19.6; MXFP4 1000 x 4096 x 512 6.1 / 6.5 / 6.5, 4096 x 4096 x 256 13.6 / 14.7 / 12.3.
-// Over 26 shapes in each of the three modes the kernel chosen took at most 6 % longer than the quickest (before: 53 %).
+// spread a small output over more SMs.  The constants were fitted to 230 random shapes (a mode, K of 256 to 8192, 256 to 16384 outputs,
+// up to 32768 tokens; three sets in turn) since the single-CTA kernels store through shared memory: two thirds to fit, one third to check.
+// The kernel chosen takes 0.8 % longer than the quickest on average, at most 33 % (4 x 10280 x 1056, 7.9 instead of 5.9 us); with the constants
+// before 1.7 % and 38 %.  Measured, us, narrow / wide / pair: MXFP8 2544 x 1128 x 1344 9.0 / 8.3 / 11.4, 774 x 4280 x 1152 7.9 / 7.1 / 8.5, 3453 x
+// 5000 x 512 17.4 / 15.0 / 17.9, row-wise 316 x 6712 x 480 6.4 / 7.5 / 7.9, MXFP4 17078 x 1320 x 384 15.5 / 16.4 / 19.7; row-wise 500 x 8192 x 1024
+// 10.2 / 10.0 / 8.6.
 int choose_kernel(bool row_wise, int64_t m, int64_t n, int64_t k_bytes, int sm_count, int pair_clusters, int split_clusters) {
   const int64_t k_stages = ceil_div64(k_bytes, kBK), m_tiles = ceil_div64(m, kBM);
   if (split_clusters > 0 && split_worthwhile(m, n, k_stages, sm_count) > 1) return DTQ_GEMM_SPLIT;
   const double stages = static_cast<double>(k_stages);
   auto rounds = [](int64_t tiles, int64_t slots) { return static_cast<double>(ceil_div64(tiles, slots)); };
-  const double wide = 4.2 + rounds(m_tiles * ceil_div64(n, 256), sm_count) * std::max(0.36 * stages + 1.9, row_wise ? 4.6 : 2.6);
+  const double wide =
+      4.2 + rounds(m_tiles * ceil_div64(n, 256), sm_count) * std::max(0.36 * stages + (row_wise ? 2.1 : 1.9), row_wise ? 4.6 : 3.2);
   const double narrow =
-      3.2 + rounds(m_tiles * ceil_div64(n, 128), sm_count) * std::max(0.25 * stages + (row_wise ? 1.3 : 1.1), row_wise ? 2.4 : 1.5);
-  const double pair = pair_clusters > 0 ? 5.6 + rounds(ceil_div64(m, 256) * ceil_div64(n, 256), pair_clusters) *
-                                                    std::max(0.333 * stages + 0.6, row_wise ? 2.2 : 1.8)
+      3.2 + rounds(m_tiles * ceil_div64(n, 128), sm_count) * std::max(0.23 * stages + (row_wise ? 1.3 : 1.1), row_wise ? 2.4 : 1.9);
+  const double pair = pair_clusters > 0 ? 5.8 + rounds(ceil_div64(m, 256) * ceil_div64(n, 256), pair_clusters) *
+                                                    std::max(0.333 * stages + 0.6, row_wise ? 2.3 : 3.1)
                                         : 1e30;
   return (pair < wide && pair < narrow) ? DTQ_GEMM_PAIR : (narrow <= wide ? DTQ_GEMM_NARROW : DTQ_GEMM_WIDE);
 }
