@@ -10,8 +10,9 @@
 // Each op: check -> allocate outputs with the caching allocator -> one C-ABI call.  Nothing
 // here computes.
 #include <ATen/ATen.h>
-#include <ATen/cuda/EmptyTensor.h>
+#include <ATen/EmptyTensor.h>
 #include <c10/core/DispatchKey.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/library.h>
@@ -33,17 +34,30 @@ void check_status(int status, const char *what) {
 int in_code(at::ScalarType t) { return t == at::kBFloat16 ? DTQ_BF16 : DTQ_F32; }
 int out_code(at::ScalarType t) { return t == at::kFloat8_e4m3fn ? DTQ_E4M3 : DTQ_E5M2; }
 
-// Outputs straight from the CUDA allocator: what at::empty / at::empty_like end in, without a second and third trip
-// through the dispatcher.  The smallest calls are bound by the host, and each at::empty was 0.4 us of their 5 to 9.
+// The device of an operator's input, current from here on, and the current stream there.  Comes before the outputs: they are
+// allocated on the current device.
+struct OnDeviceOf {
+  c10::cuda::OptionalCUDAGuard guard;  // set only where another device was current
+  c10::cuda::CUDAStream stream;
+  explicit OnDeviceOf(const at::Tensor &t) : stream(c10::cuda::getCurrentCUDAStream(t.device().index())) {
+    if (C10_UNLIKELY(c10::cuda::current_device() != t.device().index())) guard.set_index(t.device().index());
+  }
+};
+
+// Outputs straight from the CUDA allocator: what at::empty / at::empty_like end in.  The smallest calls are bound by the host, and
+// each at::empty was 0.4 us of their 5 to 9; at::detail::empty_cuda, which makes the device current once more for each output, 0.51,
+// this 0.38 (0.29 of it the allocator's).
 // at::empty also fills what it returns under torch.use_deterministic_algorithms (unless told not to), so then it is asked.
-at::Tensor new_on_device_of(const at::Tensor &like, at::IntArrayRef sizes, at::ScalarType dtype) {
+at::Tensor new_here(const OnDeviceOf &, const at::Tensor &like, at::IntArrayRef sizes, at::ScalarType dtype) {
   if (C10_UNLIKELY(at::globalContext().deterministicAlgorithms())) return at::empty(sizes, like.options().dtype(dtype));
-  return at::Tensor(at::detail::empty_cuda(sizes, dtype, like.device(), std::nullopt));
+  return at::Tensor(at::detail::empty_generic(sizes, c10::cuda::CUDACachingAllocator::get(), c10::DispatchKeySet(c10::DispatchKey::CUDA),
+                                              dtype, std::nullopt));
 }
-at::Tensor new_same_layout(const at::Tensor &like, at::ScalarType dtype) {  // `like` is dense: its strides are kept as they are
+at::Tensor new_same_layout(const OnDeviceOf &, const at::Tensor &like, at::ScalarType dtype) {  // `like` is dense: its strides are kept as they are
   if (C10_UNLIKELY(at::globalContext().deterministicAlgorithms()))
     return at::empty_strided(like.sizes(), like.strides(), like.options().dtype(dtype));
-  return at::Tensor(at::detail::empty_strided_cuda(like.sizes(), like.strides(), dtype, like.device()));
+  return at::Tensor(at::detail::empty_strided_generic(like.sizes(), like.strides(), c10::cuda::CUDACachingAllocator::get(),
+                                                      c10::DispatchKeySet(c10::DispatchKey::CUDA), dtype));
 }
 
 void check_fp8(at::ScalarType dtype) {
@@ -111,11 +125,10 @@ at::Tensor saturated_cast(const at::Tensor &input, const at::Tensor &scale, at::
   const bool transposed = strides[0] == 1 && strides[1] == input.size(0);
   const bool as_is = (input.is_contiguous() || transposed) && input.storage_offset() == 0;
   const at::Tensor x = as_is ? input : input.contiguous();
-  at::Tensor out = new_same_layout(x, dtype);
-  c10::cuda::CUDAGuard guard(x.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
+  const OnDeviceOf here(x);
+  at::Tensor out = new_same_layout(here, x, dtype);
   check_status(dtq_saturated_cast(x.data_ptr(), out.data_ptr(), scale.data_ptr<float>(), x.numel(),
-                                  in_code(x.scalar_type()), out_code(dtype), stream.stream()),
+                                  in_code(x.scalar_type()), out_code(dtype), here.stream.stream()),
                "saturated_cast");
   return out;
 }
@@ -130,13 +143,12 @@ std::tuple<at::Tensor, at::Tensor> cast_transposed(const at::Tensor &input, cons
   TORCH_CHECK(scale.is_cuda() && scale.device() == input.device(), "Scale tensor must live on the input's device");
   const at::Tensor x = input.contiguous();
   const int64_t rows = x.size(0), cols = x.size(1);
-  at::Tensor out_t = new_on_device_of(x, {cols, rows}, dtype);
-  at::Tensor out = both ? new_on_device_of(x, {rows, cols}, dtype) : at::Tensor();
-  c10::cuda::CUDAGuard guard(x.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
+  const OnDeviceOf here(x);
+  at::Tensor out_t = new_here(here, x, {cols, rows}, dtype);
+  at::Tensor out = both ? new_here(here, x, {rows, cols}, dtype) : at::Tensor();
   check_status(dtq_saturated_cast_transposed(x.data_ptr(), both ? out.data_ptr() : nullptr, out_t.data_ptr(),
                                              scale.data_ptr<float>(), rows, cols, in_code(x.scalar_type()),
-                                             out_code(dtype), stream.stream()),
+                                             out_code(dtype), here.stream.stream()),
                what);
   return {out, out_t};
 }
@@ -160,18 +172,17 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> cast_with_amax_dual(const at::Ten
                   amax_value.device() == input.device(),
               "amax must be a one-element fp32 tensor on the input's device");
   const int64_t rows = input.size(0), cols = input.size(1);
-  at::Tensor out = new_on_device_of(input, {rows, cols}, dtype);
-  at::Tensor out_t = new_on_device_of(input, {cols, rows}, dtype);
-  at::Tensor scale = new_on_device_of(input, {1}, at::kFloat);
-  c10::cuda::CUDAGuard guard(input.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
+  const OnDeviceOf here(input);
+  at::Tensor out = new_here(here, input, {rows, cols}, dtype);
+  at::Tensor out_t = new_here(here, input, {cols, rows}, dtype);
+  at::Tensor scale = new_here(here, input, {1}, at::kFloat);
   if (input.numel() == 0) {  // nothing is launched: derive the scale like the cast kernels do
     scale.copy_((dtype == at::kFloat8_e4m3fn ? 448.0 : 57344.0) / (amax_value.clamp_min(0).to(at::kDouble) + 1e-12));
     return {out, out_t, scale};
   }
   check_status(dtq_cast_with_amax_transposed(input.data_ptr(), out.data_ptr(), out_t.data_ptr(),
                                              amax_value.data_ptr<float>(), scale.data_ptr<float>(), rows, cols,
-                                             in_code(input.scalar_type()), out_code(dtype), stream.stream()),
+                                             in_code(input.scalar_type()), out_code(dtype), here.stream.stream()),
                "cast_with_amax_dual");
   return {out, out_t, scale};
 }
@@ -184,21 +195,20 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> dynamic_scaled_quant_
   check_input(input);
   TORCH_CHECK(input.is_contiguous(), "Input tensor must be contiguous");
   const int64_t rows = input.size(0), cols = input.size(1);
-  at::Tensor out = new_on_device_of(input, {rows, cols}, dtype);
-  at::Tensor out_t = new_on_device_of(input, {cols, rows}, dtype);
+  const OnDeviceOf here(input);
+  at::Tensor out = new_here(here, input, {rows, cols}, dtype);
+  at::Tensor out_t = new_here(here, input, {cols, rows}, dtype);
   if (input.numel() == 0) {  // nothing is launched: the fused op's maximum starts at 0
     at::Tensor amax_value = at::zeros({1}, input.options().dtype(at::kFloat));
     at::Tensor scale = at::full({1}, (dtype == at::kFloat8_e4m3fn ? 448.0 : 57344.0) / 1e-12, input.options().dtype(at::kFloat));
     return {out, out_t, amax_value, scale};
   }
-  at::Tensor amax_value = new_on_device_of(input, {1}, at::kFloat);
-  at::Tensor scale = new_on_device_of(input, {1}, at::kFloat);
-  c10::cuda::CUDAGuard guard(input.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
+  at::Tensor amax_value = new_here(here, input, {1}, at::kFloat);
+  at::Tensor scale = new_here(here, input, {1}, at::kFloat);
   check_status(dtq_dynamic_scaled_quant_dual(input.data_ptr(), out.data_ptr(), out_t.data_ptr(), amax_value.data_ptr<float>(),
                                              scale.data_ptr<float>(), rows, cols, in_code(input.scalar_type()),
-                                             out_code(dtype), workspaces().get(stream), dtq_workspace_bytes(),
-                                             stream.stream()),
+                                             out_code(dtype), workspaces().get(here.stream), dtq_workspace_bytes(),
+                                             here.stream.stream()),
                "dynamic_scaled_quant_dual");
   return {out, out_t, amax_value, scale};
 }
@@ -207,11 +217,10 @@ at::Tensor amax(const at::Tensor &input) {
   check_input(input);
   // max is order independent, so any dense layout can be reduced over its storage.
   const at::Tensor x = input.is_non_overlapping_and_dense() ? input : input.contiguous();
-  at::Tensor out = new_on_device_of(x, {1}, at::kFloat);
-  c10::cuda::CUDAGuard guard(x.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
+  const OnDeviceOf here(x);
+  at::Tensor out = new_here(here, x, {1}, at::kFloat);
   check_status(dtq_amax(x.data_ptr(), out.data_ptr<float>(), x.numel(), in_code(x.scalar_type()),
-                        workspaces().get(stream), dtq_workspace_bytes(), stream.stream()),
+                        workspaces().get(here.stream), dtq_workspace_bytes(), here.stream.stream()),
                "amax");
   return out;
 }
@@ -221,15 +230,14 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> dynamic_scaled_quant_with_scale(c
   check_fp8(dtype);
   check_input(input);
   TORCH_CHECK(input.is_contiguous(), "Input tensor must be contiguous");
-  at::Tensor out = new_same_layout(input, dtype);
-  at::Tensor amax_value = new_on_device_of(input, {1}, at::kFloat);
-  at::Tensor scale = new_on_device_of(input, {1}, at::kFloat);
-  c10::cuda::CUDAGuard guard(input.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
+  const OnDeviceOf here(input);
+  at::Tensor out = new_same_layout(here, input, dtype);
+  at::Tensor amax_value = new_here(here, input, {1}, at::kFloat);
+  at::Tensor scale = new_here(here, input, {1}, at::kFloat);
   check_status(dtq_dynamic_scaled_quant(input.data_ptr(), out.data_ptr(), amax_value.data_ptr<float>(),
                                         scale.data_ptr<float>(), input.numel(),
-                                        in_code(input.scalar_type()), out_code(dtype), workspaces().get(stream),
-                                        dtq_workspace_bytes(), stream.stream()),
+                                        in_code(input.scalar_type()), out_code(dtype), workspaces().get(here.stream),
+                                        dtq_workspace_bytes(), here.stream.stream()),
                "dynamic_scaled_quant");
   return {out, amax_value, scale};
 }
@@ -238,12 +246,11 @@ at::Tensor dynamic_scaled_quant(const at::Tensor &input, at::ScalarType dtype) {
   check_fp8(dtype);
   check_input(input);
   TORCH_CHECK(input.is_contiguous(), "Input tensor must be contiguous");
-  at::Tensor out = new_same_layout(input, dtype);
-  c10::cuda::CUDAGuard guard(input.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
+  const OnDeviceOf here(input);
+  at::Tensor out = new_same_layout(here, input, dtype);
   check_status(dtq_dynamic_scaled_quant(input.data_ptr(), out.data_ptr(), nullptr, nullptr, input.numel(),
-                                        in_code(input.scalar_type()), out_code(dtype), workspaces().get(stream),
-                                        dtq_workspace_bytes(), stream.stream()),
+                                        in_code(input.scalar_type()), out_code(dtype), workspaces().get(here.stream),
+                                        dtq_workspace_bytes(), here.stream.stream()),
                "dynamic_scaled_quant");
   return out;
 }
@@ -272,30 +279,27 @@ std::tuple<at::Tensor, at::Tensor> mx_fp8_quantize(at::Tensor input, int64_t blo
   // two alone means blocks along the input's dimension 0, produced by the transposing kernel in one read
   // (payload_t [n, m] contiguous, one scale per 32 rows of a column): `transpose` returns payload_t itself,
   // axis = 0 returns it viewed as [m, n].  Both together cancel: the ordinary blocks, payload viewed as [n, m].
+  const OnDeviceOf here(input);
   if (along_rows != transpose) {
     TORCH_CHECK(in_type == at::kBFloat16 && fp8_type == at::kFloat8_e4m3fn,
                 "axis=0 / transpose=True need a bfloat16 input and an e4m3 payload");
     TORCH_CHECK(m % 32 == 0 && n % 32 == 0, "Both dimensions must be multiples of the block size 32, but got ", m, " x ", n);
-    at::Tensor out_t = new_on_device_of(input, {n, m}, fp8_type);
-    at::Tensor scale_t = new_on_device_of(input, {n * (m / 32)}, at::kFloat8_e8m0fnu);
-    c10::cuda::CUDAGuard guard(input.device());
-    auto stream = c10::cuda::getCurrentCUDAStream();
+    at::Tensor out_t = new_here(here, input, {n, m}, fp8_type);
+    at::Tensor scale_t = new_here(here, input, {n * (m / 32)}, at::kFloat8_e8m0fnu);
     check_status(dtq_mx_fp8_quantize_dual(input.data_ptr(), nullptr, nullptr, out_t.data_ptr(), scale_t.data_ptr(), m, n,
-                                          stream.stream()),
+                                          here.stream.stream()),
                  "mx_fp8_quantize");
     return {transpose ? out_t : out_t.t(), scale_t};
   }
   TORCH_CHECK(n % 32 == 0, "The last dimension must be a multiple of the block size 32, but got ", n);
-  at::Tensor out = new_same_layout(input, fp8_type);
-  at::Tensor scale = new_on_device_of(input, {m * (n / 32)}, at::kFloat8_e8m0fnu);
-  c10::cuda::CUDAGuard guard(input.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
+  at::Tensor out = new_same_layout(here, input, fp8_type);
+  at::Tensor scale = new_here(here, input, {m * (n / 32)}, at::kFloat8_e8m0fnu);
   if (in_type == at::kBFloat16 && fp8_type == at::kFloat8_e4m3fn) {
-    check_status(dtq_mx_fp8_quantize(input.data_ptr(), out.data_ptr(), scale.data_ptr(), m, n, stream.stream()),
+    check_status(dtq_mx_fp8_quantize(input.data_ptr(), out.data_ptr(), scale.data_ptr(), m, n, here.stream.stream()),
                  "mx_fp8_quantize");
   } else {
     check_status(dtq_mx_quantize(input.data_ptr(), out.data_ptr(), scale.data_ptr(), m, n, mx_in_code(in_type),
-                                 out_code(fp8_type), stream.stream()),
+                                 out_code(fp8_type), here.stream.stream()),
                  "mx_fp8_quantize");
   }
   return {transpose ? out.t() : out, scale};
@@ -312,13 +316,12 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> mx_fp8_quantize_with_amax(at::Ten
   TORCH_CHECK(input.scalar_type() == at::kBFloat16, "Input tensor must be bfloat16, but got ", input.dtype());
   const int64_t m = input.size(0), n = input.size(1);
   TORCH_CHECK(n % 32 == 0, "The last dimension must be a multiple of the block size 32, but got ", n);
-  at::Tensor out = new_same_layout(input, at::kFloat8_e4m3fn);
-  at::Tensor scale = new_on_device_of(input, {m * (n / 32)}, at::kFloat8_e8m0fnu);
-  at::Tensor amax = new_on_device_of(input, {1}, at::kFloat);
-  c10::cuda::CUDAGuard guard(input.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
+  const OnDeviceOf here(input);
+  at::Tensor out = new_same_layout(here, input, at::kFloat8_e4m3fn);
+  at::Tensor scale = new_here(here, input, {m * (n / 32)}, at::kFloat8_e8m0fnu);
+  at::Tensor amax = new_here(here, input, {1}, at::kFloat);
   check_status(dtq_mx_fp8_quantize_amax(input.data_ptr(), out.data_ptr(), scale.data_ptr(), amax.data_ptr<float>(), m, n,
-                                        workspaces().get(stream), dtq_workspace_bytes(), stream.stream()),
+                                        workspaces().get(here.stream), dtq_workspace_bytes(), here.stream.stream()),
                "mx_fp8_quantize_with_amax");
   return {out, scale, amax};
 }
@@ -334,19 +337,18 @@ std::tuple<at::Tensor, at::Tensor> mx_fp4_quantize(at::Tensor input, bool blocke
               "Input tensor must be bfloat16, float16 or float32, but got ", input.dtype());
   const int64_t m = input.size(0), n = input.size(1);
   TORCH_CHECK(n % 32 == 0, "The last dimension must be a multiple of the block size 32, but got ", n);
-  at::Tensor out = new_on_device_of(input, {m, n / 2}, at::kByte);
-  c10::cuda::CUDAGuard guard(input.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
+  const OnDeviceOf here(input);
+  at::Tensor out = new_here(here, input, {m, n / 2}, at::kByte);
   if (blocked) {  // scales in the layout mx_fp4_bf16 takes, zero in the padding
-    at::Tensor scale = new_on_device_of(input, {static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, at::kFloat8_e8m0fnu);
+    at::Tensor scale = new_here(here, input, {static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, at::kFloat8_e8m0fnu);
     check_status(dtq_mx_quantize_blocked(input.data_ptr(), out.data_ptr(), scale.data_ptr(), m, n, mx_in_code(in_type),
-                                         DTQ_E2M1, stream.stream()),
+                                         DTQ_E2M1, here.stream.stream()),
                  "mx_fp4_quantize");
     return {out, scale};
   }
-  at::Tensor scale = new_on_device_of(input, {m * (n / 32)}, at::kFloat8_e8m0fnu);
+  at::Tensor scale = new_here(here, input, {m * (n / 32)}, at::kFloat8_e8m0fnu);
   check_status(dtq_mx_quantize(input.data_ptr(), out.data_ptr(), scale.data_ptr(), m, n, mx_in_code(in_type), DTQ_E2M1,
-                               stream.stream()),
+                               here.stream.stream()),
                "mx_fp4_quantize");
   return {out, scale};
 }
@@ -360,20 +362,19 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> mx_fp8_quantize_dual(
   TORCH_CHECK(input.scalar_type() == at::kBFloat16, "Input tensor must be bfloat16, but got ", input.dtype());
   const int64_t m = input.size(0), n = input.size(1);
   TORCH_CHECK(m % 32 == 0 && n % 32 == 0, "Both dimensions must be multiples of the block size 32, but got ", m, " x ", n);
-  at::Tensor out = new_on_device_of(input, {m, n}, at::kFloat8_e4m3fn), out_t = new_on_device_of(input, {n, m}, at::kFloat8_e4m3fn);
+  const OnDeviceOf here(input);
+  at::Tensor out = new_here(here, input, {m, n}, at::kFloat8_e4m3fn), out_t = new_here(here, input, {n, m}, at::kFloat8_e4m3fn);
   at::Tensor scale, scale_t;
   if (blocked) {
-    scale = new_on_device_of(input, {static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, at::kFloat8_e8m0fnu);
-    scale_t = new_on_device_of(input, {static_cast<int64_t>(dtq_mx_blocked_scale_bytes(n, m))}, at::kFloat8_e8m0fnu);
+    scale = new_here(here, input, {static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, at::kFloat8_e8m0fnu);
+    scale_t = new_here(here, input, {static_cast<int64_t>(dtq_mx_blocked_scale_bytes(n, m))}, at::kFloat8_e8m0fnu);
   } else {
-    scale = new_on_device_of(input, {m * (n / 32)}, at::kFloat8_e8m0fnu);
-    scale_t = new_on_device_of(input, {n * (m / 32)}, at::kFloat8_e8m0fnu);
+    scale = new_here(here, input, {m * (n / 32)}, at::kFloat8_e8m0fnu);
+    scale_t = new_here(here, input, {n * (m / 32)}, at::kFloat8_e8m0fnu);
   }
-  c10::cuda::CUDAGuard guard(input.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
   auto fn = blocked ? dtq_mx_fp8_quantize_dual_blocked : dtq_mx_fp8_quantize_dual;
   check_status(fn(input.data_ptr(), out.data_ptr(), scale.data_ptr(), out_t.data_ptr(), scale_t.data_ptr(), m, n,
-                  stream.stream()),
+                  here.stream.stream()),
                "mx_fp8_quantize_dual");
   return {out, scale, out_t, scale_t};
 }
@@ -387,11 +388,10 @@ std::tuple<at::Tensor, at::Tensor> mx_fp8_quantize_blocked(at::Tensor input) {
   TORCH_CHECK(input.scalar_type() == at::kBFloat16, "Input tensor must be bfloat16, but got ", input.dtype());
   const int64_t m = input.size(0), n = input.size(1);
   TORCH_CHECK(n % 32 == 0, "The last dimension must be a multiple of the block size 32, but got ", n);
-  at::Tensor out = new_same_layout(input, at::kFloat8_e4m3fn);
-  at::Tensor scale = new_on_device_of(input, {static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, at::kFloat8_e8m0fnu);
-  c10::cuda::CUDAGuard guard(input.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
-  check_status(dtq_mx_fp8_quantize_blocked(input.data_ptr(), out.data_ptr(), scale.data_ptr(), m, n, stream.stream()),
+  const OnDeviceOf here(input);
+  at::Tensor out = new_same_layout(here, input, at::kFloat8_e4m3fn);
+  at::Tensor scale = new_here(here, input, {static_cast<int64_t>(dtq_mx_blocked_scale_bytes(m, n))}, at::kFloat8_e8m0fnu);
+  check_status(dtq_mx_fp8_quantize_blocked(input.data_ptr(), out.data_ptr(), scale.data_ptr(), m, n, here.stream.stream()),
                "mx_fp8_quantize_blocked");
   return {out, scale};
 }
@@ -403,14 +403,13 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> dynamic_scaled_quant_rowwise(cons
   TORCH_CHECK(input.is_contiguous(), "Input tensor must be contiguous");
   const int64_t m = input.size(0), n = input.size(1);
   TORCH_CHECK(m == 0 || n > 0, "Rows must not be empty");
-  at::Tensor out = new_same_layout(input, dtype);
-  at::Tensor amax_rows = new_on_device_of(input, {m, 1}, at::kFloat);
-  at::Tensor scale_rows = new_on_device_of(input, {m, 1}, at::kFloat);
-  c10::cuda::CUDAGuard guard(input.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
+  const OnDeviceOf here(input);
+  at::Tensor out = new_same_layout(here, input, dtype);
+  at::Tensor amax_rows = new_here(here, input, {m, 1}, at::kFloat);
+  at::Tensor scale_rows = new_here(here, input, {m, 1}, at::kFloat);
   check_status(dtq_dynamic_scaled_quant_rowwise(input.data_ptr(), out.data_ptr(), amax_rows.data_ptr<float>(),
                                                 scale_rows.data_ptr<float>(), m, n, in_code(input.scalar_type()),
-                                                out_code(dtype), stream.stream()),
+                                                out_code(dtype), here.stream.stream()),
                "dynamic_scaled_quant_rowwise");
   return {out, amax_rows, scale_rows};
 }
@@ -423,13 +422,12 @@ std::tuple<at::Tensor, at::Tensor> cast_with_amax(const at::Tensor &input, const
   TORCH_CHECK(amax_value.scalar_type() == at::kFloat && amax_value.numel() == 1 && amax_value.is_cuda() &&
                   amax_value.device() == input.device(),
               "amax must be one fp32 value on the input's device");
-  at::Tensor out = new_same_layout(input, dtype);
-  at::Tensor scale = new_on_device_of(input, {1}, at::kFloat);
-  c10::cuda::CUDAGuard guard(input.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
+  const OnDeviceOf here(input);
+  at::Tensor out = new_same_layout(here, input, dtype);
+  at::Tensor scale = new_here(here, input, {1}, at::kFloat);
   check_status(dtq_cast_with_amax(input.data_ptr(), out.data_ptr(), amax_value.data_ptr<float>(),
                                   scale.data_ptr<float>(), input.numel(), in_code(input.scalar_type()),
-                                  out_code(dtype), stream.stream()),
+                                  out_code(dtype), here.stream.stream()),
                "cast_with_amax");
   return {out, scale};
 }
@@ -462,11 +460,10 @@ at::Tensor mx_fp8_bf16(at::Tensor a, at::Tensor b, at::Tensor a_scale, at::Tenso
   TORCH_CHECK(a_scale.is_contiguous() && b_scale.is_contiguous(), "scale tensors must be contiguous");
   TORCH_CHECK(a.stride(1) == 1 && a.stride(0) == K, "Input tensor 'a' must be contiguous in the K dimension (row-major)");
   TORCH_CHECK(b.stride(0) == 1 && b.stride(1) == K, "Input tensor 'b' must be contiguous in the K dimension (column-major)");
-  at::Tensor out = new_on_device_of(a, {M, N}, at::kBFloat16);
-  c10::cuda::CUDAGuard guard(a.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
+  const OnDeviceOf here(a);
+  at::Tensor out = new_here(here, a, {M, N}, at::kBFloat16);
   check_status(dtq_mx_fp8_bf16(a.data_ptr(), b.data_ptr(), a_scale.data_ptr(), b_scale.data_ptr(), out.data_ptr(), M, N, K,
-                               workspaces().get(stream), dtq_workspace_bytes(), stream.stream()),
+                               workspaces().get(here.stream), dtq_workspace_bytes(), here.stream.stream()),
                "mx_fp8_bf16");
   return out;
 }
@@ -494,11 +491,10 @@ at::Tensor mx_fp4_bf16(at::Tensor a, at::Tensor b, at::Tensor a_scale, at::Tenso
   TORCH_CHECK(a_scale.is_contiguous() && b_scale.is_contiguous(), "scale tensors must be contiguous");
   TORCH_CHECK(a.stride(1) == 1 && a.stride(0) == Kb, "Input tensor 'a' must be contiguous in the K dimension (row-major)");
   TORCH_CHECK(b.stride(0) == 1 && b.stride(1) == Kb, "Input tensor 'b' must be contiguous in the K dimension (column-major)");
-  at::Tensor out = new_on_device_of(a, {M, N}, at::kBFloat16);
-  c10::cuda::CUDAGuard guard(a.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
+  const OnDeviceOf here(a);
+  at::Tensor out = new_here(here, a, {M, N}, at::kBFloat16);
   check_status(dtq_mx_fp4_bf16(a.data_ptr(), b.data_ptr(), a_scale.data_ptr(), b_scale.data_ptr(), out.data_ptr(), M, N, K,
-                               workspaces().get(stream), dtq_workspace_bytes(), stream.stream()),
+                               workspaces().get(here.stream), dtq_workspace_bytes(), here.stream.stream()),
                "mx_fp4_bf16");
   return out;
 }
@@ -533,12 +529,11 @@ at::Tensor sweep_mm(at::Tensor XQ, at::Tensor WQ, at::Tensor x_scale, at::Tensor
     bias_ptr = bias->data_ptr();
     bias_code = bias->scalar_type() == at::kBFloat16 ? DTQ_BF16 : DTQ_F32;
   }
-  at::Tensor out = new_on_device_of(XQ, {M, N}, out_dtype);
-  c10::cuda::CUDAGuard guard(XQ.device());
-  auto stream = c10::cuda::getCurrentCUDAStream();
+  const OnDeviceOf here(XQ);
+  at::Tensor out = new_here(here, XQ, {M, N}, out_dtype);
   check_status(dtq_rowwise_fp8_bf16(XQ.data_ptr(), WQ.data_ptr(), x_scale.data_ptr<float>(), w_scale.data_ptr<float>(), bias_ptr,
                                     bias_code, out.data_ptr(), M, N, K, out_code(XQ.scalar_type()), DTQ_GEMM_AUTO,
-                                    workspaces().get(stream), dtq_workspace_bytes(), stream.stream()),
+                                    workspaces().get(here.stream), dtq_workspace_bytes(), here.stream.stream()),
                "sweep_mm");
   return out;
 }

@@ -12,6 +12,7 @@ The reference has no multi-GPU path; the per-shard arithmetic is its kernels'
 """
 from __future__ import annotations
 
+import sys
 from typing import Optional, Sequence, Tuple
 
 import torch
@@ -34,15 +35,6 @@ def shard_rows(rows: int, world_size: int, rank: int, multiple: int = 1) -> Tupl
 
 class ExchangeTimeout(RuntimeError):
     """A bounded device-side wait for a peer's value gave up."""
-
-
-class _CudaKernels:
-    """The product kernels; resolved lazily so that importing this module needs no GPU."""
-
-    def __getattr__(self, name):
-        import driss_torch_b200 as pkg
-
-        return getattr(pkg, name)
 
 
 class ShardedQuantizer:
@@ -74,7 +66,7 @@ class ShardedQuantizer:
         going through ``torch.distributed`` symmetric memory: entry r is rank r's buffer
         (``dtq_p2p_exchange_bytes()`` zero-filled bytes) as addressable from this device."""
         self.group = group
-        self.kernels = _CudaKernels() if kernels is None else kernels
+        self.kernels = sys.modules[__package__] if kernels is None else kernels
         self.spin_limit = self.DEFAULT_SPIN_LIMIT if spin_limit is None else int(spin_limit)
         self._exchange = None
         self._rank = rank
