@@ -22,7 +22,8 @@
 // Any other number of rows (or alignment of out_t): the rows of out_t start at every byte offset, so no 16-byte store
 // fits as it is.  The transposed tile goes through shared memory once more, and a warp writes four row segments of out_t
 // (up to 128 bytes) at a time: eight lanes each, one aligned 16 bytes per lane, cut out of five words of shared memory by
-// funnel shifts, and single bytes for the ends.  launch_transposed has the figures.
+// funnel shifts, and single bytes for the ends (many tiles of bf16: none but at the ends of whole columns, see Rows).
+// launch_transposed has the figures.
 // Rows of input that are not 16-byte aligned, or few tiles of ragged rows: a 32 x 32 byte-tile kernel, one element per thread.
 #include "dtq_device.cuh"
 #include "dtq_host.h"
@@ -37,7 +38,17 @@ namespace {
 
 constexpr int kTileRows = 128;
 constexpr int kTileWords = 32;  // 32-bit words of fp8 bytes per shared-memory row (fp32 input uses 16 of them)
-constexpr int kRaggedPitch = 36;  // words between byte columns of the transposed tile when its rows start at any byte
+// How the rows of the transposed output lie, and how they are written.  kEnds and kWhole: they start at any byte.  With kEnds a tile
+// writes its 128 rows of a column as the aligned 16 bytes inside and single bytes at either end; with kWhole it reads 16 rows more and
+// writes the eight aligned 16 bytes that begin in its rows, so that only the ends of a whole column are single bytes.
+// Fewer partial sectors against an eighth more to read, convert and transpose: measured, both orientations behind an amax, us, kEnds / kWhole,
+// bf16 16383 x 8192 159.3 / 145.0, 9999 x 4096 43.2 / 41.7, 5003 x 4096 (1280 tiles) 22.6 / 21.0, 2001 x 4096 (512) 13.0 / 14.1, 333 x 8192 (192) 9.1 /
+// 11.6; fp32, where reading weighs twice, 9999 x 4096 67.4 / 68.4, 5003 x 4096 32.7 / 32.6, 2001 x 4096 14.9 / 15.7.
+enum Rows { kAligned, kEnds, kWhole };
+constexpr int kWholeMinTiles = 5 * kB200Sms;  // more than the device holds at once; bf16 only
+constexpr int kWholeRows = kTileRows + 16;
+constexpr int kRaggedPitch = kWholeRows / 4;  // words between byte columns of the transposed tile
+static_assert(kRaggedPitch % 4 == 0, "16-byte stores to its columns");
 constexpr int kThreadsT = 256;
 constexpr int kRowPasses = kTileRows / 16;  // a pass of 8 warps covers 16 rows (2 per warp)
 
@@ -114,52 +125,12 @@ struct DynCast<DTQ_F32, OUT> {
   }
 };
 
-// FULL: the tile lies inside the matrix, no access is predicated.  BOTH: also write the row-major output.
-// RAGGED: rows of out_t start at any byte.
-template <typename C, bool BOTH, bool RAGGED, bool FULL>
-__device__ __forceinline__ void transposed_tile(uint32_t (&tile)[kTileRows][kTileWords], const uint4 *__restrict__ in,
-                                                uint8_t *__restrict__ out, uint8_t *__restrict__ out_t,
-                                                const typename C::Scale &s, int64_t rows, int64_t cols,
-                                                int64_t row0, int64_t col0) {
-  constexpr int kE = C::kChunkElems;      // columns per chunk
-  constexpr int kChunkWords = kE / 4;     // words of fp8 bytes per chunk
-  constexpr int kRowWords = 16 * kChunkWords;  // words of fp8 bytes per tile row: 32 (bf16) or 16 (fp32)
-  // fp32 input fills only half of a shared-memory row: odd rows use the other half, so that the two rows a
-  // warp parks at once fall on different banks
-  constexpr int kSkew = kRowWords == 16 ? 16 : 0;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t row_chunks = cols / kE;
-
-  // ---- rows: in pass p warp w owns tile rows 16p + 2w and + 1; lane l the 16-byte input chunk l & 15 of the row
-  const int chunk = lane & 15;
-  const int64_t c = col0 + chunk * kE;  // first column of the chunk; cols is a multiple of a chunk
-  const bool col_live = FULL || c < cols;
-  uint4 v[kRowPasses];
-#pragma unroll
-  for (int p = 0; p < kRowPasses; ++p) {
-    const int64_t r = row0 + p * 16 + warp * 2 + (lane >> 4);
-    v[p] = (FULL || (col_live && r < rows)) ? ldg_stream(in + r * row_chunks + c / kE) : make_uint4(0, 0, 0, 0);
-  }
-#pragma unroll
-  for (int p = 0; p < kRowPasses; ++p) {
-    const int rt = p * 16 + warp * 2 + (lane >> 4);  // rt >> 4 == p: the 16-row group of this row
-    const typename C::Bytes b = C::convert(v[p], s);
-    park(&tile[rt][(chunk * kChunkWords) ^ (p << 2) ^ ((rt & 1) * kSkew)], b);
-    if (BOTH && (FULL || (col_live && row0 + rt < rows))) stg_stream(out + (row0 + rt) * cols + c, b);
-  }
-  __syncthreads();
-
-  // ---- columns: lane = 8 * q + g: 16-row group g of the tile, word column 4 * warp + q (four byte columns)
-  const int g = lane & 7, q = lane >> 3;
-  const int word = warp * 4 + q;
-  if (!RAGGED && word >= kRowWords) return;  // fp32 input: half as many byte columns per tile
-  const int64_t r_first = row0 + g * 16;
-  const int64_t col = col0 + word * 4;
+// 4 x 4 byte transposes of 16 words, one per row: word k of column j's sixteen bytes from rows 4k .. 4k+3.
+template <typename Row>
+__device__ __forceinline__ void transpose_group(uint32_t (&t)[4][4], Row row) {
   uint32_t w[16];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) w[i] = tile[g * 16 + i][word ^ (g << 2) ^ ((i & 1) * kSkew)];
-  // 4 x 4 byte transposes: rows 4k .. 4k+3 of byte column j -> word k of column j's sixteen bytes
-  uint32_t t[4][4];
+  for (int i = 0; i < 16; ++i) w[i] = row(i);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const uint32_t a0 = __byte_perm(w[4 * k], w[4 * k + 1], 0x5140), a1 = __byte_perm(w[4 * k], w[4 * k + 1], 0x7362);
@@ -169,35 +140,98 @@ __device__ __forceinline__ void transposed_tile(uint32_t (&tile)[kTileRows][kTil
     t[2][k] = __byte_perm(a1, b1, 0x5410);
     t[3][k] = __byte_perm(a1, b1, 0x7632);
   }
+}
+
+// FULL: the tile (with the rows behind it, kWhole) lies inside the matrix, no access is predicated.  BOTH: also write the row-major output.
+template <typename C, bool BOTH, Rows ROWS, bool FULL>
+__device__ __forceinline__ void transposed_tile(uint32_t (*tile)[kTileWords], const uint4 *__restrict__ in,
+                                                uint8_t *__restrict__ out, uint8_t *__restrict__ out_t,
+                                                const typename C::Scale &s, int64_t rows, int64_t cols,
+                                                int64_t row0, int64_t col0) {
+  constexpr int kE = C::kChunkElems;      // columns per chunk
+  constexpr int kChunkWords = kE / 4;     // words of fp8 bytes per chunk
+  constexpr int kRowWords = 16 * kChunkWords;  // words of fp8 bytes per tile row: 32 (bf16) or 16 (fp32)
+  // fp32 input fills only half of a shared-memory row: odd rows use the other half, so that the two rows a
+  // warp parks at once fall on different banks
+  constexpr int kSkew = kRowWords == 16 ? 16 : 0;
+  constexpr bool RAGGED = ROWS != kAligned, WHOLE = ROWS == kWhole;
+  constexpr int kPasses = kRowPasses + (WHOLE ? 1 : 0);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t row_chunks = cols / kE;
+
+  // ---- rows: in pass p warp w owns tile rows 16p + 2w and + 1; lane l the 16-byte input chunk l & 15 of the row
+  const int chunk = lane & 15;
+  const int64_t c = col0 + chunk * kE;  // first column of the chunk; cols is a multiple of a chunk
+  const bool col_live = FULL || c < cols;
+  uint4 v[kPasses];
+#pragma unroll
+  for (int p = 0; p < kPasses; ++p) {
+    const int64_t r = row0 + p * 16 + warp * 2 + (lane >> 4);
+    v[p] = (FULL || (col_live && r < rows)) ? ldg_stream(in + r * row_chunks + c / kE) : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int p = 0; p < kPasses; ++p) {
+    const int rt = p * 16 + warp * 2 + (lane >> 4);  // rt >> 4 == p: the 16-row group of this row
+    const typename C::Bytes b = C::convert(v[p], s);
+    park(&tile[rt][(chunk * kChunkWords) ^ ((p & 7) << 2) ^ ((rt & 1) * kSkew)], b);
+    if (BOTH && p < kRowPasses && (FULL || (col_live && row0 + rt < rows))) stg_stream(out + (row0 + rt) * cols + c, b);
+  }
+  __syncthreads();
+
+  // ---- columns: lane = 8 * q + g: 16-row group g of the tile, word column 4 * warp + q (four byte columns)
+  const int g = lane & 7, q = lane >> 3;
+  const int word = warp * 4 + q;
+  if (!RAGGED && word >= kRowWords) return;  // fp32 input: half as many byte columns per tile
+  const int64_t r_first = row0 + g * 16;
+  const int64_t col = col0 + word * 4;
+  uint32_t t[4][4];
+  transpose_group(t, [&](int i) { return tile[g * 16 + i][word ^ (g << 2) ^ ((i & 1) * kSkew)]; });
   if constexpr (RAGGED) {
-    // the tile again, now as [byte column][row]: 32 words of rows per column, 36 words apart
+    uint32_t behind[4][4];  // the rows behind the tile: one warp, a word column per lane
+    const bool mine = WHOLE && warp == 0 && lane < kRowWords;
+    if (mine) transpose_group(behind, [&](int i) { return tile[kTileRows + i][lane ^ ((i & 1) * kSkew)]; });
+    // the tile again, now as [byte column][row]
     uint32_t *tile_t = &tile[0][0];
     __syncthreads();
-    if (word < kRowWords) {
+    auto put = [&](int word_column, int group, const uint32_t (&b)[4][4]) {
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        *reinterpret_cast<uint4 *>(tile_t + (word * 4 + j) * kRaggedPitch + g * 4) = make_uint4(t[j][0], t[j][1], t[j][2], t[j][3]);
-    }
+        *reinterpret_cast<uint4 *>(tile_t + (word_column * 4 + j) * kRaggedPitch + group * 4) = make_uint4(b[j][0], b[j][1], b[j][2], b[j][3]);
+    };
+    if (word < kRowWords) put(word, g, t);
+    if (mine) put(lane, kTileRows / 16, behind);
     __syncthreads();
-    const int len = FULL ? kTileRows : static_cast<int>(min(rows - row0, int64_t(kTileRows)));
+    constexpr int kRows = WHOLE ? kWholeRows : kTileRows;
+    const int len = FULL ? kRows : static_cast<int>(min(rows - row0, int64_t(kRows)));
     const int ncols = FULL ? 4 * kRowWords : static_cast<int>(min(cols - col0, int64_t(4 * kRowWords)));
     // a warp takes four columns at a time, eight lanes each: lane l an aligned 16 bytes of the segment
     const int l = lane & 7;
     for (int cc = warp * 4 + (lane >> 3); cc < ncols; cc += kThreadsT / 8) {
       uint8_t *dst = out_t + (col0 + cc) * rows + row0;
       const uint32_t *src = tile_t + cc * kRaggedPitch;
+      const uint8_t *src_bytes = reinterpret_cast<const uint8_t *>(src);
       const int head = min(static_cast<int>(-reinterpret_cast<uintptr_t>(dst) & 15), len);  // bytes before the first aligned 16
-      const int vectors = (len - head) >> 4;
-      if (l < vectors) {
-        const int first = head + 16 * l, shift = 8 * (first & 3);
+      const int first = head + 16 * l;
+      const bool whole = (WHOLE && FULL) || first + 16 <= len;
+      if (whole) {
+        const int shift = 8 * (first & 3);
         const uint32_t *p = src + (first >> 2);  // five words, the fifth only looked at when shift > 0
         const uint32_t w0 = p[0], w1 = p[1], w2 = p[2], w3 = p[3], w4 = p[4];
         *reinterpret_cast<uint4 *>(dst + first) = make_uint4(__funnelshift_r(w0, w1, shift), __funnelshift_r(w1, w2, shift),
                                                              __funnelshift_r(w2, w3, shift), __funnelshift_r(w3, w4, shift));
       }
-      for (int i = l; i < len - 16 * vectors; i += 8) {  // the ends
-        const int b = i < head ? i : i + 16 * vectors;
-        dst[b] = reinterpret_cast<const uint8_t *>(src)[b];
+      if constexpr (WHOLE) {
+        // what begins before the first aligned 16 bytes is the tile's above, in the first tile the end of the column before
+        if (!whole)
+          for (int i = first; i < len; ++i) dst[i] = src_bytes[i];
+        if (row0 == 0)
+          for (int i = l; i < head; i += 8) dst[i] = src_bytes[i];
+      } else {
+        const int vectors = (len - head) >> 4;
+        for (int i = l; i < len - 16 * vectors; i += 8) {  // the ends
+          const int b = i < head ? i : i + 16 * vectors;
+          dst[b] = src_bytes[b];
+        }
       }
     }
     return;
@@ -213,13 +247,14 @@ __device__ __forceinline__ void transposed_tile(uint32_t (&tile)[kTileRows][kTil
 // `scale` points to the scale (Cast) or to the amax (DynCast); scale_out, if given, receives the fp32 scale
 // a DynCast derived from the amax, amax_out the amax it used (the given one, clamped at zero).
 constexpr int kTransposedMinBlocks = 4;
-template <typename C, bool BOTH, bool RAGGED>
+template <typename C, bool BOTH, Rows ROWS>
 __global__ void __launch_bounds__(kThreadsT, kTransposedMinBlocks)
 cast_transposed_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, uint8_t *__restrict__ out_t,
                        const float *__restrict__ scale, float *__restrict__ scale_out, float *__restrict__ amax_out,
                        int64_t rows, int64_t cols, int64_t col_tiles, LaunchPad<72>) {
-  __shared__ __align__(16) uint32_t buffer[kTileRows * (RAGGED ? kRaggedPitch : kTileWords)];
-  uint32_t (&tile)[kTileRows][kTileWords] = *reinterpret_cast<uint32_t (*)[kTileRows][kTileWords]>(buffer);
+  // as [row][word], and unless aligned then as [byte column][row]
+  static_assert(kWholeRows * kTileWords == 4 * kTileWords * kRaggedPitch, "the two take the same room");
+  __shared__ __align__(16) uint32_t tile[ROWS == kAligned ? kTileRows : kWholeRows][kTileWords];
   constexpr int kTileCols = 16 * C::kChunkElems;
   pdl_launch_dependents();
   pdl_wait();  // may have become resident under the tail of the kernel that delivers *scale
@@ -232,10 +267,10 @@ cast_transposed_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, 
   const int64_t t = int64_t(gridDim.x) - 1 - blockIdx.x;
   const int64_t row0 = (t / col_tiles) * kTileRows;
   const int64_t col0 = (t % col_tiles) * kTileCols;
-  if (row0 + kTileRows <= rows && col0 + kTileCols <= cols)
-    transposed_tile<C, BOTH, RAGGED, true>(tile, in, out, out_t, s, rows, cols, row0, col0);
+  if (row0 + (ROWS == kWhole ? kWholeRows : kTileRows) <= rows && col0 + kTileCols <= cols)
+    transposed_tile<C, BOTH, ROWS, true>(tile, in, out, out_t, s, rows, cols, row0, col0);
   else
-    transposed_tile<C, BOTH, RAGGED, false>(tile, in, out, out_t, s, rows, cols, row0, col0);
+    transposed_tile<C, BOTH, ROWS, false>(tile, in, out, out_t, s, rows, cols, row0, col0);
 }
 
 // Any shape and alignment: 32 x 32 tiles of fp8 bytes, block (32, 8), one element per thread per step.
@@ -286,8 +321,11 @@ int launch_transposed(const void *in, void *out, void *out_t, const float *scale
   const bool aligned_rows = rows % 16 == 0 && aligned_to(out_t, 16);
   DeviceInfo dev;
   if (int e = current_device_info(&dev)) return e;
-  const bool tiles = readable && (aligned_rows || ceil_div64(rows, kTileRows) * ceil_div64(cols, kTileCols) >= dev.sm_count);
-  auto kernel = aligned_rows ? cast_transposed_kernel<C, BOTH, false> : cast_transposed_kernel<C, BOTH, true>;
+  const int64_t tile_count = ceil_div64(rows, kTileRows) * ceil_div64(cols, kTileCols);
+  const bool tiles = readable && (aligned_rows || tile_count >= dev.sm_count);
+  auto kernel = aligned_rows ? cast_transposed_kernel<C, BOTH, kAligned> : cast_transposed_kernel<C, BOTH, kEnds>;
+  if constexpr (C::kChunkElems == 8)  // bf16
+    if (!aligned_rows && tile_count > kWholeMinTiles) kernel = cast_transposed_kernel<C, BOTH, kWhole>;
   if (tiles) {
     const int64_t row_tiles = ceil_div64(rows, kTileRows), col_tiles = ceil_div64(cols, kTileCols);
     if (row_tiles > 0x7FFFFFFFLL / col_tiles) return DTQ_ERR_TOO_LARGE;

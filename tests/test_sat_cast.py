@@ -254,3 +254,24 @@ def test_transposed_rows_at_any_byte(rows, cols, in_dtype, offset):
             assert_fp8_equal(got[0], want, fp8_dtype, "row-major")
         edge = torch.cat([room[:16 + offset], room[16 + offset + rows * cols:]])
         assert (edge == 0x55).all(), "bytes outside the output were written"
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 95400), (15, 95400), (17, 95400), (127, 95400), (129, 47720), (143, 47720), (145, 47720),
+                                       (271, 32000), (1537, 8200), (1551, 8200), (1553, 8200), (1663, 8200)])
+@pytest.mark.parametrize("offset", [0, 1, 15])  # byte offset of the transposed output
+def test_transposed_rows_at_any_byte_of_more_tiles_than_fit_at_once(rows, cols, offset):
+    # whole aligned 16 bytes from tiles that read 16 rows more: one row tile, a last one of 1 to 127 rows, one that ends inside the rows
+    # behind the tile above it, a ragged last column tile
+    from driss_torch_b200 import _cabi
+
+    x = (torch.randn(rows, cols, generator=torch.Generator(device="cuda").manual_seed(rows), device="cuda") * 100).to(torch.bfloat16)
+    scale = torch.tensor([0.7], device="cuda")
+    want = _cabi.saturated_cast(x, scale, torch.float8_e4m3fn).view(torch.uint8)
+    for both in (False, True):
+        room = torch.full((rows * cols + 64,), 0x55, dtype=torch.uint8, device="cuda")
+        out_t = room[16 + offset:16 + offset + rows * cols].view(torch.float8_e4m3fn).view(cols, rows)
+        got = _cabi.saturated_cast_transposed(x, scale, torch.float8_e4m3fn, out_t=out_t, both=both)
+        assert torch.equal(out_t.view(torch.uint8), want.t())
+        assert not both or torch.equal(got[0].view(torch.uint8), want)
+        edge = torch.cat([room[:16 + offset], room[16 + offset + rows * cols:]])
+        assert (edge == 0x55).all(), "bytes outside the output were written"
