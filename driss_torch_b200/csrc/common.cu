@@ -21,6 +21,7 @@ int current_device_info(DeviceInfo *info) {
     std::lock_guard<std::mutex> lock(g_mutex);
     if (!g_ready[dev].load(std::memory_order_relaxed)) {
       DeviceInfo d;
+      d.id = dev;
       DTQ_CUDA_TRY(cudaDeviceGetAttribute(&d.sm_count, cudaDevAttrMultiProcessorCount, dev));
       DTQ_CUDA_TRY(cudaDeviceGetAttribute(&d.cooperative, cudaDevAttrCooperativeLaunch, dev));
       g_info[dev] = d;

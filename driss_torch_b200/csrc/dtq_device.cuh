@@ -107,7 +107,8 @@ constexpr int kB200Sms = 148;
 // Measured, bf16 [rows, 4096], outputs that stay; us with nothing asked, and the change in percent with 8 / 16 / 24 (static cast)
 // or 2 / 4 / 8 blocks per SM (the others).  From memory: inputs of 400 MB in turn; three: three inputs in turn, as much of them in
 // L2 as fits; amax: behind an amax of the input, the two together; product: behind an MXFP8 product of K = 1024 that
-// wrote the input, the two together.  Products and amaxes release their dependents early, so that their lines are asked for in vain.
+// wrote the input, the two together.  The products, and at the time of these figures the amax, release their dependents early, so that their
+// lines are asked for in vain.
 //   static cast      from memory             three                   amax, from memory       product
 //      16 MiB   4.66  -6.9  -6.7  -6.7    3.96  -0.4  -4.3  -4.6    9.9 +0.9 +2.1 +2.8    16.1 -0.4 +0.3 +0.2
 //      32 MiB   7.92 -11.8 -12.3 -10.7    8.63 -13.1 -21.2 -24.0   15.5 -1.7 -3.4 -0.9    26.5 +0.5 +1.2 +1.7

@@ -107,7 +107,7 @@ mx_amax_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, uint
 // maximum is published before its outputs are stored, so that the fence has none of them to wait for and the ticket is on its way meanwhile.
 // What it saves is the host's: with cast_with_amax behind it, us per pass / on the device alone, finishing launch -> last block: 1 MiB
 // 12.0 / 4.5 -> 10.8 / 4.8, 4 MiB 12.0 / 7.5 -> 10.7 / 7.6, 16 MiB 12.0 / 9.4 -> 10.8 / 9.5; 24 MiB 12.0 / 11.9 -> 13.5 / 13.1, so not beyond
-// kSmallTiles.  With the ticket taken behind the stores 4 MiB took 8.4 on the device, with the last block's first warp collecting the
+// kSmallTiles.  It releases the cast behind when it ends: 8 MiB 8.3 -> 7.4 on the device.  With the ticket taken behind the stores 4 MiB took 8.4 on the device, with the last block's first warp collecting the
 // maxima ahead of its own stores 8.2.
 constexpr int64_t kSmallTiles = 1024;  // 16 MiB of input
 static_assert(kSmallTiles <= kMaxGridBlocks, "a partial per block");
@@ -116,7 +116,6 @@ mx_amax_small_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload
                      int64_t nchunks, float *__restrict__ amax_out, Workspace *ws, LaunchPad<48>) {
   __shared__ float smem32[32];
   __shared__ int last;
-  pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t keep_policy = l2_policy_evict_last();  // all of the input stays in L2 for the cast behind

@@ -191,7 +191,10 @@ int launch_dual(const void *in_bf16, void *payload, void *scales_e8m0, void *pay
   const int64_t row_tiles = ceil_div64(rows, kTile), col_tiles = ceil_div64(cols, kTile);
   if (row_tiles > 0x7FFFFFFFLL / col_tiles) return DTQ_ERR_TOO_LARGE;  // grid.x
   auto kernel = row_out ? mx_dual_kernel<BLOCKED, true> : mx_dual_kernel<BLOCKED, false>;
-  return cuda_status(launch_after_dependency(kernel, dim3(static_cast<unsigned>(row_tiles * col_tiles)), dim3(kThreadsDual), 0,
+  DeviceInfo dev;
+  if (int e = current_device_info(&dev)) return e;
+  constexpr size_t kStaticSmem = sizeof(uint32_t) * kTile * kTileWords + 2 * 512;
+  return cuda_status(launch_spread(kernel, static_cast<unsigned>(row_tiles * col_tiles), kThreadsDual, kStaticSmem, kDualMinBlocks, dev,
                                              static_cast<cudaStream_t>(stream), static_cast<const uint16_t *>(in_bf16),
                                              static_cast<uint8_t *>(payload), static_cast<uint8_t *>(scales_e8m0),
                                              static_cast<uint8_t *>(payload_t), static_cast<uint8_t *>(scales_t_e8m0), rows, cols,

@@ -256,7 +256,10 @@ cast_transposed_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, 
   static_assert(kWholeRows * kTileWords == 4 * kTileWords * kRaggedPitch, "the two take the same room");
   __shared__ __align__(16) uint32_t tile[ROWS == kAligned ? kTileRows : kWholeRows][kTileWords];
   constexpr int kTileCols = 16 * C::kChunkElems;
-  pdl_launch_dependents();
+  // A grid of less than a wave releases what is behind it when it ends: the blocks of an amax that settle beside this kernel's settle
+  // unevenly.  Amax and both casts, us, at the start -> at the end: bf16 3001 x 1024 11.5 -> 7.6, 333 x 8192 11.7 -> 7.6, 1001 x 4096 11.4 -> 8.3, fp32
+  // 1001 x 4096 10.9 -> 9.8; of a wave and more 1127 x 4992 of fp32 12.4 -> 13.0, bf16 2000 x 4096 equal.
+  if (gridDim.x >= kTransposedMinBlocks * kB200Sms) pdl_launch_dependents();
   pdl_wait();  // may have become resident under the tail of the kernel that delivers *scale
   const typename C::Scale s = C::load_scale(scale);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
