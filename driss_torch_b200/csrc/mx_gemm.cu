@@ -878,7 +878,11 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // accumulator), half 0 at its beginning (columns 0..31 of the second, the same columns of tensor memory).
     const int quad = warp & 3, half = (warp - 2) >> 2;
     const uint32_t leader_empty[2] = {map_to_cta(smem_addr(&sm.tmem_empty[0]), 0), map_to_cta(smem_addr(&sm.tmem_empty[1]), 0)};
-    uint8_t *staging = sm.out[warp - 2];
+    // The last tile's 32 columns each have a buffer of their own: the operands' stages are free by then.  A tile before takes
+    // one buffer four times, and waits each time until the store before has read it, behind the loads of the next tile.  Us, one buffer ->
+    // four: MXFP8 2048^3 10.3 -> 9.9, 3000 x 2000 x 1504 13.3 -> 12.9, 8192^3 429 -> 428; row-wise, whose conversion takes longer, within 1 %.
+    uint8_t *const last_staging = sm.a[0] + (warp - 2) * (4 * 32 * 64);
+    static_assert(kEpilogueWarps * 4 * 32 * 64 <= PairStages<MODE> * kBM * kBK, "the operands of A have the room");
     const uint64_t stream_policy = l2_policy_evict_first();  // the output must not push the operands out of L2
     int local_tile = 0;
     for (int tile = cluster_id; tile < total_tiles; tile += n_clusters, ++local_tile) {
@@ -887,6 +891,7 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const int64_t row = int64_t(mp) * 256 + int64_t(rank) * kBM + quad * 32 + lane;
       const int64_t col0 = int64_t(nt) * kPairBN + half * 128;
       const int acc = local_tile & 1;
+      const bool last = tile + n_clusters >= total_tiles;
       float xs = 0.0f;
       if constexpr (MODE == kRowwise) {
         // before the wait: the row's scale, and the columns' scales and biases to shared memory, read there by all lanes
@@ -933,8 +938,11 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         uint32_t packed[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) packed[j] = pack_bf16(v[i & 1][2 * j], v[i & 1][2 * j + 1]);
-        if (lane == 0) tma_store_wait_read();  // the staging buffer has been read
-        __syncwarp();
+        uint8_t *const staging = last ? last_staging + i * (32 * 64) : sm.out[warp - 2];
+        if (!last) {
+          if (lane == 0) tma_store_wait_read();  // the staging buffer has been read
+          __syncwarp();
+        }
 #pragma unroll
         for (int q = 0; q < 4; ++q)
           *reinterpret_cast<uint4 *>(staging + lane * 64 + ((q ^ ((lane >> 1) & 3)) * 16)) =
@@ -1526,14 +1534,14 @@ int split_worthwhile(int64_t m, int64_t n, int64_t stages, int sm_count) {
 // kernel (0: cannot launch them).  Estimated time, in microseconds as measured on a B200 = a fixed part (launch, set-up,
 // filling the pipeline, the last epilogue) plus, for every round of tiles on the busiest SM, the stages of 128 operand bytes
 // along K at the time of one, and what a tile costs besides; a tile never takes less than its epilogue.
-//   pair   256 x 256 tiles on SM pairs: 5.8 + rounds x max(0.333 stages + 0.6, 3.1; row-wise 2.3)
+//   pair   256 x 256 tiles on SM pairs: 5.4 + rounds x max(0.333 stages + 0.6, 3.1; row-wise 2.3)
 //   wide   128 x 256 on one SM: 4.2 + rounds x max(0.36 stages + 1.9, 3.2; row-wise 0.36 stages + 2.1, 4.6), its epilogue not overlapped
 //   narrow 128 x 128 on one SM: 3.2 + rounds x max(0.23 stages + 1.1, 1.9; row-wise 0.23 stages + 1.3, 2.4)
 // So large problems run on SM pairs, and problems of about a tile per SM on the narrow kernel, whose smaller tiles also
 // spread a small output over more SMs.  The constants were fitted to 230 random shapes (a mode, K of 256 to 8192, 256 to 16384 outputs,
 // up to 32768 tokens; three sets in turn) since the single-CTA kernels store through shared memory: two thirds to fit, one third to check.
 // The kernel chosen takes 0.8 % longer than the quickest on average, at most 33 % (4 x 10280 x 1056, 7.9 instead of 5.9 us); with the constants
-// before 1.7 % and 38 %.  Measured, us, narrow / wide / pair: MXFP8 2544 x 1128 x 1344 9.0 / 8.3 / 11.4, 774 x 4280 x 1152 7.9 / 7.1 / 8.5, 3453 x
+// before 1.7 % and 38 %.  (Pair is 0.4 quicker since than in those measurements, by its last tile's stores.)  Measured, us, narrow / wide / pair: MXFP8 2544 x 1128 x 1344 9.0 / 8.3 / 11.4, 774 x 4280 x 1152 7.9 / 7.1 / 8.5, 3453 x
 // 5000 x 512 17.4 / 15.0 / 17.9, row-wise 316 x 6712 x 480 6.4 / 7.5 / 7.9, MXFP4 17078 x 1320 x 384 15.5 / 16.4 / 19.7; row-wise 500 x 8192 x 1024
 // 10.2 / 10.0 / 8.6.
 int choose_kernel(bool row_wise, int64_t m, int64_t n, int64_t k_bytes, int sm_count, int pair_clusters, int split_clusters) {
@@ -1545,7 +1553,7 @@ int choose_kernel(bool row_wise, int64_t m, int64_t n, int64_t k_bytes, int sm_c
       4.2 + rounds(m_tiles * ceil_div64(n, 256), sm_count) * std::max(0.36 * stages + (row_wise ? 2.1 : 1.9), row_wise ? 4.6 : 3.2);
   const double narrow =
       3.2 + rounds(m_tiles * ceil_div64(n, 128), sm_count) * std::max(0.23 * stages + (row_wise ? 1.3 : 1.1), row_wise ? 2.4 : 1.9);
-  const double pair = pair_clusters > 0 ? 5.8 + rounds(ceil_div64(m, 256) * ceil_div64(n, 256), pair_clusters) *
+  const double pair = pair_clusters > 0 ? 5.4 + rounds(ceil_div64(m, 256) * ceil_div64(n, 256), pair_clusters) *
                                                     std::max(0.333 * stages + 0.6, row_wise ? 2.3 : 3.1)
                                         : 1e30;
   return (pair < wide && pair < narrow) ? DTQ_GEMM_PAIR : (narrow <= wide ? DTQ_GEMM_NARROW : DTQ_GEMM_WIDE);
