@@ -41,9 +41,11 @@ constexpr int kTileWords = 32;  // 32-bit words of fp8 bytes per shared-memory r
 // How the rows of the transposed output lie, and how they are written.  kEnds and kWhole: they start at any byte.  With kEnds a tile
 // writes its 128 rows of a column as the aligned 16 bytes inside and single bytes at either end; with kWhole it reads 16 rows more and
 // writes the eight aligned 16 bytes that begin in its rows, so that only the ends of a whole column are single bytes.
-// Fewer partial sectors against an eighth more to read, convert and transpose: measured, both orientations behind an amax, us, kEnds / kWhole,
-// bf16 16383 x 8192 159.3 / 145.0, 9999 x 4096 43.2 / 41.7, 5003 x 4096 (1280 tiles) 22.6 / 21.0, 2001 x 4096 (512) 13.0 / 14.1, 333 x 8192 (192) 9.1 /
-// 11.6; fp32, where reading weighs twice, 9999 x 4096 67.4 / 68.4, 5003 x 4096 32.7 / 32.6, 2001 x 4096 14.9 / 15.7.
+// Fewer partial sectors, and streaming stores, against an eighth more to read, convert and transpose.  Measured, both orientations behind an
+// amax, outputs that stay for a pass, us, kEnds / kWhole / kWhole with plain stores: bf16 16383 x 8192 161.1 / 137.6 / 143.7, 9999 x 4096 44.8 / 45.4 /
+// 45.4, 5003 x 4096 (1280 tiles) 24.3 / 22.6 / 23.8, 1500 x 8200 16.7 / 16.5 / 16.5, 1537 x 8192 (832) 17.3 / 16.6 / 16.6; kEnds / kWhole where outputs
+// are dropped at once 2001 x 4096 (512 tiles) 13.0 / 14.1, 333 x 8192 (192) 9.1 / 11.6; fp32, where reading weighs twice, 9999 x 4096 67.4 / 68.4,
+// 2001 x 4096 14.9 / 15.7.
 enum Rows { kAligned, kEnds, kWhole };
 constexpr int kWholeMinTiles = 5 * kB200Sms;  // more than the device holds at once; bf16 only
 constexpr int kWholeRows = kTileRows + 16;
@@ -217,8 +219,10 @@ __device__ __forceinline__ void transposed_tile(uint32_t (*tile)[kTileWords], co
         const int shift = 8 * (first & 3);
         const uint32_t *p = src + (first >> 2);  // five words, the fifth only looked at when shift > 0
         const uint32_t w0 = p[0], w1 = p[1], w2 = p[2], w3 = p[3], w4 = p[4];
-        *reinterpret_cast<uint4 *>(dst + first) = make_uint4(__funnelshift_r(w0, w1, shift), __funnelshift_r(w1, w2, shift),
-                                                             __funnelshift_r(w2, w3, shift), __funnelshift_r(w3, w4, shift));
+        const uint4 v16 = make_uint4(__funnelshift_r(w0, w1, shift), __funnelshift_r(w1, w2, shift), __funnelshift_r(w2, w3, shift),
+                                     __funnelshift_r(w3, w4, shift));
+        if constexpr (WHOLE) stg_stream(dst + first, v16);
+        else *reinterpret_cast<uint4 *>(dst + first) = v16;  // its sectors are completed by single bytes, from here and from other tiles
       }
       if constexpr (WHOLE) {
         // what begins before the first aligned 16 bytes is the tile's above, in the first tile the end of the column before
