@@ -313,7 +313,7 @@ dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float 
     pdl_launch_dependents();
   }
   if (met == kGaveUp) {  // a bounded wait gave up (the status word says so): no payload, and NaN where a maximum was expected
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if ((!P2P || blockIdx.x == 0) && threadIdx.x == 0) {  // block 0 may have found its share taken and be gone
       if (amax_out) *amax_out = __uint_as_float(0x7FC00000u);
       if (scale_out) *scale_out = __uint_as_float(0x7FC00000u);
     }
