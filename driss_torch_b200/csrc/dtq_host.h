@@ -120,7 +120,7 @@ inline size_t spread_bytes(int64_t grid, int sm_count, size_t static_smem, int m
   return (room < kSmemMost ? room : kSmemMost) - static_smem;
 }
 // Lets `kernel` have that much on the current device: asked of the runtime once per kernel and device (again, harmlessly, should the
-// table ever be full).
+// table ever be full).  Until then a launch may have 48 KB, static and dynamic together, so any spread launch asks.
 inline cudaError_t allow_spread(const void *kernel, int dev_id, size_t static_smem) {
   constexpr unsigned kSlots = 1024;
   static std::atomic<uintptr_t> seen[kSlots];
@@ -137,16 +137,18 @@ inline cudaError_t allow_spread(const void *kernel, int dev_id, size_t static_sm
   }
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMost - static_smem));
 }
-// launch_after_dependency with the blocks spread.
+// launch_after_dependency with the blocks spread.  Where the runtime does not grant the memory (the answer above was another context's,
+// say, or one from before the device was reset), the kernel is launched without: it runs as well.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_spread(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t static_smem, int most, const DeviceInfo &dev,
                                  cudaStream_t st, Args... args) {
-  size_t bytes = spread_bytes(grid, dev.sm_count, static_smem, most);
-  if (bytes > 48 * 1024 && allow_spread(reinterpret_cast<const void *>(kernel), dev.id, static_smem) != cudaSuccess) {
-    (void)cudaGetLastError();  // the question's own; the kernel runs as well without
-    bytes = 0;
+  const size_t bytes = spread_bytes(grid, dev.sm_count, static_smem, most);
+  if (bytes && allow_spread(reinterpret_cast<const void *>(kernel), dev.id, static_smem) == cudaSuccess) {
+    const cudaError_t e = launch_after_dependency(kernel, dim3(grid), dim3(block), bytes, st, args...);
+    if (e != cudaErrorInvalidValue && e != cudaErrorLaunchOutOfResources) return e;
   }
-  return launch_after_dependency(kernel, dim3(grid), dim3(block), bytes, st, args...);
+  if (bytes) (void)cudaGetLastError();  // the question's own, or the refused launch's
+  return launch_after_dependency(kernel, dim3(grid), dim3(block), 0, st, args...);
 }
 
 // ---- thread-block clusters: whether the device can place them ------------------------------------------------------
