@@ -56,51 +56,75 @@ constexpr unsigned int kSpinLimit = 1u << 20;  // polls, each an L2 round trip p
 // block that has not started: a block claims its share when it starts, a block that has waited for some time takes over
 // shares that nobody has claimed, and a block that starts and finds its share taken leaves.  All who are waited for are running.
 //
-// A share's word: 0 nobody has come; +kOwnerCame by the owner when it starts; 0 -> kTaken by a block that takes the share over;
-// +kTakerDone when that has finished the share.  Whoever comes second, owner or taker, clears the word, and an owner whose share
-// was its own does once the shares are all in.  From then on a zero no longer means that nobody has come: a block that takes
-// one looks again whether all are in, and if so puts the zero back.  (A zero seen before that is true: the share of a word cleared
-// earlier would have to be in.)
-constexpr unsigned int kOwnerCame = 1, kTaken = 2, kTakerDone = 4;
+// A share's word counts, in twos, the launches that its owner has come to; the lowest bit says that another block has taken the share over
+// in the launch that the owner has not come to yet, and goes when the owner comes.  Every launch counts on in all kMaxShares words,
+// so a block knows from its own which launch this is, and of another share's whether its owner has come: nothing is cleared between
+// launches, and a block that is late or gives up leaves nothing behind.
+//
+// A share that was claimed goes in, sooner or later, also when the waiting of others has run out, so the count of shares is
+// complete when the launch is over.  Who gives up notes it in the same word, unless the count is complete by then: all who see it complete
+// know whether all have met.
+constexpr unsigned int kTakenOver = 1, kLaunch = 2;
+constexpr unsigned int kOneGaveUp = 1u << 16;  // in shares_in, above the count
+static_assert(kMaxShares < kOneGaveUp && int64_t(kMaxShares) * kOneGaveUp <= 0xFFFFFFFFll - kMaxShares, "the halves of shares_in");
 constexpr int kGaveUp = 0, kMet = 1, kImpatient = 2, kShareIsGone = 3;
 constexpr unsigned int kPatience = 64;  // polls, about 50 us, before a waiting block looks for shares to take over
 
-__device__ __forceinline__ void clear_share(unsigned int *word) { atomicExch(word, 0u); }
-// Thread 0 of the owner, first thing.  Whether the share is its own; if not, it has nothing left to do.
-__device__ __forceinline__ bool claim_own_share(Workspace *ws) {
-  const unsigned int before = atomicAdd(&ws->claims[blockIdx.x], kOwnerCame);
-  if (before == kTaken + kTakerDone) {
-    __threadfence();
-    clear_share(&ws->claims[blockIdx.x]);
-  }
-  return before == 0;
+// Thread 0 of the owner, first thing.  The launch, in twos; with kTakenOver: the share is another block's by now, nothing is left to do.
+__device__ __forceinline__ unsigned int come_for_own_share(Workspace *ws) {
+  const unsigned int before = atomicAdd(&ws->shares[blockIdx.x], kLaunch);
+  if (before & kTakenOver) atomicSub(&ws->shares[blockIdx.x], kTakenOver);
+  return before;
 }
-// Thread 0: a share's maximum goes in.  `slot`: the parity of `generation` as read before, which picks the counter pair.  The last
-// one clears the other parity's pair (the previous launch is long over) and bumps the generation for the next launch.
-// Returns whether all shares are in.
-__device__ __forceinline__ bool add_share(Workspace *ws, unsigned int slot, float value) {
-  atomicMax(&ws->bar_max[slot], __float_as_uint(value));
+// All threads: this launch in the words that are no block's.
+__device__ __forceinline__ void count_unused_shares(Workspace *ws) {
+  for (unsigned int j = blockIdx.x + (threadIdx.x + 1) * gridDim.x; j < kMaxShares; j += blockDim.x * gridDim.x)
+    atomicAdd(&ws->shares[j], kLaunch);
+}
+__device__ __forceinline__ unsigned int parity_of(unsigned int launch) { return launch / kLaunch & 1u; }
+__device__ __forceinline__ bool all_in(unsigned int shares_in) { return (shares_in & (kOneGaveUp - 1)) == gridDim.x; }
+// What a block knows of the launch from shares_in.
+__device__ __forceinline__ int meeting(unsigned int shares_in) {
+  return !all_in(shares_in) ? kImpatient : shares_in == gridDim.x ? kMet : kGaveUp;
+}
+// Thread 0: a share's maximum goes in.  The last one clears the other parity's pair (the previous launch is long over).
+__device__ __forceinline__ int add_share(Workspace *ws, unsigned int launch, float value) {
+  const unsigned int slot = parity_of(launch);
+  atomicMax(&ws->shares_max[slot], __float_as_uint(value));
   __threadfence();
-  const unsigned int ticket = atomicAdd(&ws->bar_count[slot], 1u);
-  if (ticket != gridDim.x - 1) return false;
-  ws->bar_count[slot ^ 1u] = 0;
-  ws->bar_max[slot ^ 1u] = 0;
-  atomicAdd(&ws->generation, 1u);
-  return true;
+  const unsigned int in = atomicAdd(&ws->shares_in[slot], 1u) + 1u;
+  if (!all_in(in)) return kImpatient;
+  ws->shares_in[slot ^ 1u] = 0;
+  ws->shares_max[slot ^ 1u] = 0;
+  __threadfence();  // as the acquiring load of those who wait
+  return meeting(in);
 }
 // Thread 0: waits for all shares, for at most `polls`.
-__device__ __forceinline__ bool wait_for_shares(const Workspace *ws, unsigned int slot, unsigned int polls) {
-  for (unsigned int spins = 0; ld_acquire(&ws->bar_count[slot]) != gridDim.x;) {
-    if (++spins > polls) return false;
+__device__ __forceinline__ int wait_for_shares(const Workspace *ws, unsigned int launch, unsigned int polls) {
+  const unsigned int *word = &ws->shares_in[parity_of(launch)];
+  int met;
+  for (unsigned int spins = 0; (met = meeting(ld_acquire(word))) == kImpatient;) {
+    if (++spins > polls) break;
     __nanosleep(20);
   }
-  return true;
+  return met;
 }
-// Thread 0 of an owner, when all shares are in: the maximum.
-__device__ __forceinline__ float shares_are_in(Workspace *ws, unsigned int slot) {
-  __threadfence();  // whoever sees the word cleared also sees all shares in
-  clear_share(&ws->claims[blockIdx.x]);
-  return __uint_as_float(ld_acquire(&ws->bar_max[slot]));
+// Thread 0, when it has waited long enough.
+__device__ __forceinline__ int give_up_shares(Workspace *ws, unsigned int launch) {
+  unsigned int *word = &ws->shares_in[parity_of(launch)];
+  for (unsigned int before = ld_acquire(word); !all_in(before);) {  // the word changes at most twice for each block
+    const unsigned int now = atomicCAS(word, before, before + kOneGaveUp);
+    if (now == before) {
+      atomicExch(&ws->status, DTQ_ERR_TIMEOUT);
+      return kGaveUp;
+    }
+    before = now;
+  }
+  return wait_for_shares(ws, launch, 0);
+}
+// Thread 0, when all have met: the maximum.
+__device__ __forceinline__ float shares_maximum(const Workspace *ws, unsigned int launch) {
+  return __uint_as_float(ld_acquire(&ws->shares_max[parity_of(launch)]));
 }
 
 // What a block took over (shared memory; a bit per share).
@@ -115,10 +139,12 @@ struct TakenShares {
   }
 };
 // All threads of a block that has waited in vain: takes over shares until all are in.  share_max(share) is the share's
-// maximum as block_max_nonneg returns it.  kMet, or kGaveUp after kSpinLimit polls without a share to take.
+// maximum as block_max_nonneg returns it.  kMet, or kGaveUp: after kSpinLimit polls without a share to take, or where another gave up.
 template <typename ShareMax>
-__device__ __forceinline__ int take_over_until_met(Workspace *ws, unsigned int slot, TakenShares &mine, ShareMax share_max) {
+__device__ __forceinline__ int take_over_until_met(Workspace *ws, unsigned int launch, TakenShares &mine, ShareMax share_max) {
   if (threadIdx.x < kMaxShares / 32) mine.bits[threadIdx.x] = 0;
+  const unsigned int shortened = *const_cast<const volatile unsigned int *>(&ws->wait_limit_us);
+  const unsigned int limit = shortened ? shortened : kSpinLimit;  // a poll takes about a microsecond
   unsigned int spins = 0;
   for (;;) {
     __syncthreads();
@@ -127,18 +153,14 @@ __device__ __forceinline__ int take_over_until_met(Workspace *ws, unsigned int s
     // of the shares that nobody has come for, the one farthest behind this block's own: blocks spread out
     int best = -1;
     for (unsigned int j = threadIdx.x; j < gridDim.x; j += blockDim.x)
-      if (ld_acquire(&ws->claims[j]) == 0) best = max(best, int((j + gridDim.x - blockIdx.x) % gridDim.x));
+      if (ld_acquire(&ws->shares[j]) == launch) best = max(best, int((j + gridDim.x - blockIdx.x) % gridDim.x));
     if (best >= 0) atomicMax(&mine.candidate, best);
     __syncthreads();
     if (threadIdx.x == 0) {
       mine.taken = -1;
       if (mine.candidate >= 0) {
         const unsigned int j = (mine.candidate + blockIdx.x) % gridDim.x;
-        if (atomicCAS(&ws->claims[j], 0u, kTaken) == 0u) {
-          __threadfence();
-          if (ld_acquire(&ws->bar_count[slot]) == gridDim.x) clear_share(&ws->claims[j]);
-          else mine.taken = int(j);
-        }
+        if (atomicCAS(&ws->shares[j], launch, launch + kTakenOver) == launch) mine.taken = int(j);
       }
     }
     __syncthreads();
@@ -147,24 +169,20 @@ __device__ __forceinline__ int take_over_until_met(Workspace *ws, unsigned int s
       const float value = share_max(j);
       if (threadIdx.x == 0) {
         mine.bits[j / 32] |= 1u << (j & 31);
-        add_share(ws, slot, value);
+        add_share(ws, launch, value);
       }
     }
-    // (after a share taken: only a look)
-    const bool wait = j < 0;
-    if (threadIdx.x == 0) mine.candidate = wait_for_shares(ws, slot, wait ? kPatience : 0) ? kMet : kImpatient;
-    __syncthreads();
-    if (mine.candidate == kMet) return kMet;
-    if (wait && (spins += kPatience) > kSpinLimit) {
-      if (threadIdx.x == 0) atomicExch(&ws->status, DTQ_ERR_TIMEOUT);
-      return kGaveUp;
+    const bool wait = j < 0;  // (after a share taken: only a look)
+    if (wait) spins += kPatience;
+    if (threadIdx.x == 0) {
+      int met = wait_for_shares(ws, launch, wait ? kPatience : 0);
+      if (met == kImpatient && wait && spins > limit) met = give_up_shares(ws, launch);
+      mine.candidate = met;
     }
+    __syncthreads();
+    const int met = mine.candidate;
+    if (met != kImpatient) return met;
   }
-}
-// Thread 0, for every share that it took over, when all of them are finished.
-__device__ __forceinline__ void taken_share_is_done(Workspace *ws, int share) {
-  unsigned int *word = &ws->claims[share];
-  if (atomicAdd(word, kTakerDone) == kTaken + kOwnerCame) clear_share(word);
 }
 
 // ---- a grid barrier with an exchange across GPUs in its serial section -------------------------

@@ -20,20 +20,25 @@ struct alignas(256) Workspace {
   unsigned int generation;  // bumped by the last-arriving block; waiters spin on it (bounded)
   int status;               // sticky: DTQ_ERR_TIMEOUT if a bounded wait ever gave up
   float amax;               // the reduced value of the current launch, valid after the bump
-  // The fused kernel's grid barrier: arrival count and running maximum (as float bits), one pair
-  // per parity of `generation`; a launch uses the pair of its parity and clears the other.
+  // The grid barrier of the fused kernel that exchanges with other GPUs: arrival count and running maximum (as float bits), one
+  // pair per parity of `generation`; a launch uses the pair of its parity and clears the other.
   unsigned int bar_count[2];
   unsigned int bar_max[2];
   // Running maxima of kernels whose blocks fold their value into a few words (atomicMax, block b
   // into word b % 32) instead of publishing partials; a one-warp finishing launch takes them and
   // leaves zeros behind.
   unsigned int slot_max[32];
-  // Limit of a wait in the GEMMs, in microseconds; 0, as initialised, is two seconds.  Tests shorten it to see one run out.
+  // Limit of a wait in the GEMMs and in the fused kernel, in microseconds; 0, as initialised, is a second or two.  Tests shorten it
+  // to see one run out.
   unsigned int wait_limit_us;
-  unsigned int pad[23];
+  // The fused kernel on one GPU (see dtq_grid.cuh): the shares that are in and their maximum (as float bits), one pair per parity of
+  // the launch; a launch clears the other.
+  unsigned int shares_in[2];
+  unsigned int shares_max[2];
+  unsigned int pad[19];
+  // Its shares of the input, one word each: twice the launches so far, between launches the same in all.
+  unsigned int shares[kMaxShares];
   float partials[kMaxGridBlocks];
-  // The fused kernel's shares of the input, one word each (see dtq_grid.cuh); zero between launches.
-  unsigned int claims[kMaxShares];
 };
 
 struct DeviceInfo {

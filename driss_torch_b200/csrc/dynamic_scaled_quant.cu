@@ -215,10 +215,9 @@ dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float 
   // 60 to the loads in flight, and the kernel took 8 % longer (128 MiB 43.4 -> 47.2 us).
   __shared__ float smem32[32];
   __shared__ int flag;
-  __shared__ unsigned int gen0;  // thread 0's: the generation before this launch, and whether the share is this block's own
-  __shared__ bool own;
+  __shared__ unsigned int start;  // thread 0's: P2P: the generation before this launch; else the launch and whether the share is this block's own
   if constexpr (P2P) {
-    if (threadIdx.x == 0) gen0 = ld_acquire(&ws->generation);
+    if (threadIdx.x == 0) start = ld_acquire(&ws->generation);
   } else {
     pdl_wait();  // may have become resident under the tail of the kernel before it
   }
@@ -247,10 +246,8 @@ dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float 
     load_tile<UNROLL>(first_tile, in, blockIdx.x, nchunks);
   }
   if constexpr (!P2P) {
-    if (threadIdx.x == 0) {  // under the first tile's loads
-      gen0 = ld_acquire(&ws->generation);
-      own = claim_own_share(ws);
-    }
+    if (threadIdx.x == 0) start = come_for_own_share(ws);  // under the first tile's loads
+    count_unused_shares(ws);
   }
 #pragma unroll
   for (int u = 0; u < UNROLL; ++u) C::absmax(acc0, acc1, first_tile[u]);  // zeros where the block has no tile
@@ -292,28 +289,32 @@ dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float 
   int met;
   bool took_over = false;
   if constexpr (P2P) {
-    met = grid_max_barrier_exchange(ws, gen0, block_value, px, &flag, &amax_shared, &amax) ? kMet : kGaveUp;
+    met = grid_max_barrier_exchange(ws, start, block_value, px, &flag, &amax_shared, &amax) ? kMet : kGaveUp;
   } else {
-    const unsigned int slot = gen0 & 1u;  // thread 0's
     if (threadIdx.x == 0) {
       flag = kShareIsGone;
-      if (own) flag = add_share(ws, slot, block_value) || wait_for_shares(ws, slot, kPatience) ? kMet : kImpatient;
-      if (flag == kMet) amax_shared = shares_are_in(ws, slot);
+      if (!(start & kTakenOver)) {
+        flag = add_share(ws, start, block_value);
+        if (flag == kImpatient) flag = wait_for_shares(ws, start, kPatience);
+      }
+      if (flag == kMet) amax_shared = shares_maximum(ws, start);
     }
     __syncthreads();
     met = flag;
     if (met == kShareIsGone) return;
     if (met == kImpatient) {
       took_over = true;
-      met = take_over_until_met(ws, slot, others, [&](int share) { return share_max<C, UNROLL>(in, numel, share); });
-      if (threadIdx.x == 0 && met == kMet) amax_shared = shares_are_in(ws, slot);
+      met = take_over_until_met(ws, start, others, [&](int share) { return share_max<C, UNROLL>(in, numel, share); });
+      if (threadIdx.x == 0 && met == kMet) amax_shared = shares_maximum(ws, start);
       __syncthreads();
     }
     amax = amax_shared;
     pdl_launch_dependents();
   }
-  if (met == kGaveUp) {  // a bounded wait gave up (the status word says so): no payload, and NaN where a maximum was expected
-    if ((!P2P || blockIdx.x == 0) && threadIdx.x == 0) {  // block 0 may have found its share taken and be gone
+  // A bounded wait gave up (the status word says so): no payload from the blocks that know, and NaN where a maximum was expected.  P2P: block 0
+  // knows; else all know that would write a maximum, and block 0 may have found its share taken and be gone.
+  if (met == kGaveUp) {
+    if ((!P2P || blockIdx.x == 0) && threadIdx.x == 0) {
       if (amax_out) *amax_out = __uint_as_float(0x7FC00000u);
       if (scale_out) *scale_out = __uint_as_float(0x7FC00000u);
     }
@@ -343,10 +344,8 @@ dsq_fused_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, float 
   if (blockIdx.x == 0 && tail0 + threadIdx.x < numel)
     out[tail0 + threadIdx.x] = cvt_fp8<OUT>(dsq_mul(sd.sd, C::load_one(in, tail0 + threadIdx.x)));
   if constexpr (!P2P) {
-    if (took_over) {
+    if (took_over)
       others.for_each([&](int share) { share_cast<C, OUT, UNROLL>(in, out, amax_out, scale_out, numel, amax, share); });
-      if (threadIdx.x == 0) others.for_each([&](int share) { taken_share_is_done(ws, share); });
-    }
   }
 }
 

@@ -155,7 +155,9 @@ int dtq_amax_static_scratch(const void *in, float *out, int64_t numel, int in_dt
  *   amax = max |in| (>= 0);  scale_d = fp8_max / ((double)amax + 1e-12);
  *   out[i] = fp8_satfinite((float)(scale_d * (double)in[i])).
  * amax_out / scale_out (one fp32 each, nullable) receive amax and
- * (float)scale_d.  bf16 and fp32 inputs.
+ * (float)scale_d.  bf16 and fp32 inputs.  Should a bounded wait in it ever give up (DTQ_ERR_TIMEOUT in the
+ * workspace status word), amax_out / scale_out receive NaN and the payload is incomplete; the workspace
+ * stays usable (its sticky status aside) and the next call is right.
  * Replaces driss_torch::dynamic_scaled_quant and its cooperative kernel:
  * src/dynamic_scaled_quant.cu:83-118, :119-176.
  */

@@ -465,3 +465,51 @@ def test_launches_that_compete_for_the_device_meet():
     for i, outs in enumerate(got):
         assert all(torch.equal(o.view(torch.uint8), wants[i].view(torch.uint8)) for o in outs), i
         assert _cabi.workspace_status(room[i]) == 0 and (_words_between_launches(room[i]) == 0).all()
+
+
+# ---- a wait of the grid that gives up ------------------------------------------------------------------------------------------
+
+_STATUS_WORD, _WAIT_LIMIT_WORD = 2, 40  # of the workspace, csrc/dtq_host.h
+
+
+def test_a_wait_that_gives_up_spoils_that_call_only():
+    # 1024 shares of 4 MiB, a third of them left when the blocks that fit the device have done two each: some blocks then wait hundreds of
+    # microseconds for the others' last shares, under a limit of one (and the 100 or so that they wait before they look at it)
+    from driss_torch_b200 import _cabi
+
+    ws = torch.zeros(_cabi.load().dtq_workspace_bytes(), dtype=torch.uint8, device="cuda")
+    words = ws.view(torch.int32)
+    x = torch.empty(1 << 31, dtype=torch.bfloat16, device="cuda").normal_(generator=torch.Generator(device="cuda").manual_seed(1))
+    small = x[:5_000_003].clone()
+    want, want_small = (_cabi.cast_with_amax(v, v.abs().max().float().view(1), torch.float8_e4m3fn).view(torch.uint8) for v in (x, small))
+
+    def call(v, blocks):
+        got, amax, scale = _cabi.dynamic_scaled_quant_blocks(v, torch.float8_e4m3fn, blocks, ws=ws)
+        return got.view(torch.uint8), amax.item(), scale.isnan().item()
+
+    for _ in range(3):
+        words[_WAIT_LIMIT_WORD], words[_STATUS_WORD] = 1, 0
+        _, amax, no_scale = call(x, 1024)
+        assert _cabi.workspace_status(ws) == 5 and amax != amax and no_scale  # DTQ_ERR_TIMEOUT, whichever blocks met
+        words[_WAIT_LIMIT_WORD], words[_STATUS_WORD] = 0, 0
+        for v, blocks, right in ((small, 7, want_small), (small, 296, want_small), (small, 1024, want_small), (x, 1024, want)):
+            got, amax, no_scale = call(v, blocks)
+            assert torch.equal(got, right) and amax == v.abs().max().item() and not no_scale and _cabi.workspace_status(ws) == 0
+
+
+def test_one_workspace_for_grids_of_every_size():
+    # what one launch leaves for the next, whatever its grid and the next one's
+    from driss_torch_b200 import _cabi
+
+    ws = torch.zeros(_cabi.load().dtq_workspace_bytes(), dtype=torch.uint8, device="cuda")
+    x = torch.randn(3_000_017, generator=torch.Generator(device="cuda").manual_seed(2), device="cuda").to(torch.bfloat16)
+    order = torch.tensor([1, 2, 3, 147, 148, 295, 296, 297, 511, 512, 513, 800, 1023, 1024])
+    for seed in range(6):
+        for blocks in order[torch.randperm(len(order), generator=torch.Generator().manual_seed(seed))].tolist():
+            x[seed * 1000 + blocks] = 8.0 + seed + blocks / 2048  # a larger maximum than any before would do for a stale one
+            want = x.abs().max()
+            got, amax, _ = _cabi.dynamic_scaled_quant_blocks(x, torch.float8_e5m2, blocks, ws=ws)
+            assert amax.item() == want.item(), (seed, blocks)
+            assert torch.equal(got.view(torch.uint8), _cabi.cast_with_amax(x, want.float().view(1), torch.float8_e5m2).view(torch.uint8))
+            x[seed * 1000 + blocks] = 0.0
+    assert _cabi.workspace_status(ws) == 0
