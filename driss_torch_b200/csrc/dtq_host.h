@@ -109,11 +109,14 @@ inline cudaError_t launch_after_dependency(void (*kernel)(KArgs...), dim3 grid, 
 // A programmatic dependent becomes resident while the kernel before it drains.  Where that leaves some SMs free and others full (a
 // product with one CTA of 225 KB on each of 105 of the 148 SMs), the blocks of a small grid that follows all settle on the free
 // ones, as many as fit each, and stay there when the others come free.  So a grid of less than a full wave asks for as much shared
-// memory as leaves room for its even share of blocks per SM.  `most` is what fits without.  (Sixteen blocks or fewer: two per SM,
-// so that a product behind them finds room beside them; 8 blocks in front of 8 x 8192 x 8192: 16.3 us, with one per SM 16.5.)
-// Measured, us per pass, without -> with: MXFP8 training step 864 x 1920 x 1920 45.1 -> 36.9, 768 x 800 x 4576 53.3 -> 40.8, 2048^3 56.8 -> 48.5,
-// 4096 x 1024 x 4096 82.2 -> 79.6 (the two-orientation casts); layers: MXFP4 1024 x 4096 x 4096 16.3 -> 14.7, MXFP8 64 x 8192 x 4096 12.5 -> 11.9,
-// 128 x 8192 x 4096 15.3 -> 14.3, 1024 x 1024 x 4096 15.4 -> 14.5, row-wise 1024 x 2048 x 2048 16.1 -> 14.4.
+// memory as leaves room for its even share of blocks per SM (sixteen blocks or fewer: for two, which leaves room for a product behind
+// them).  `most` is what fits without.
+// Measured, us per pass, without -> with, the two-orientation MX casts in MXFP8 training steps: 864 x 1920 x 1920 45.1 -> 36.9, 768 x 800 x
+// 4576 53.3 -> 40.8, 2048^3 56.8 -> 48.5, 4096 x 1024 x 4096 82.2 -> 79.6.
+// Only for kernels whose own shared memory keeps them off an SM that a product holds anyway, like these.  The MX and row-wise casts have
+// none, and run beside a product on another stream: spread, they waited for it (64 x 8192 beside MXFP8 8192^3 15 -> 364 us, 1024 x 4096 beside 4096^3 15 ->
+// 64), which is more than their layers lose (row-wise 1024 x 2048 x 2048 12.1 -> 13.0, MXFP4 1024 x 4096 x 4096 13.5 -> 14.8, MXFP8 64 x 8192 x 4096 12.6 -> 12.7,
+// 1024 x 1024 x 4096 9.1 -> 10.6).
 // The amax and the elementwise two-orientation cast, whose kernels follow one another, release their dependents late instead: with an amax
 // in front of it spread, 5003 x 4096 took 25.7 instead of 22.0.  (So do the products gain for the casts, but a product behind a product
 // loses: MXFP8 300 x 2048 x 1024 5.8 -> 6.4, 1024 x 1024 x 4096 7.0 -> 7.2.)

@@ -118,7 +118,7 @@ int launch_mx(const void *in_bf16, void *payload, void *scales_e8m0, int64_t row
     const int64_t pad_blocks = BLOCKED ? scale_padding_blocks(rows, kblocks, kThreads) : 0;
     const int grid = balanced_grid(tiles, max_grid) + static_cast<int>(pad_blocks);
     auto kernel = asks_ahead(BLOCKED ? Asks::kMxBlocked : Asks::kMx, numel * 2) ? mx_stream_kernel<BLOCKED, true> : mx_stream_kernel<BLOCKED, false>;
-    return cuda_status(launch_spread(kernel, grid, kThreads, 0, 2048 / kThreads, dev, st,
+    return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(kThreads), 0, st,
                                                static_cast<const uint4 *>(in_bf16), static_cast<uint8_t *>(payload),
                                                static_cast<uint8_t *>(scales_e8m0), nchunks, kblocks, katoms, rows,
                                                static_cast<unsigned>(pad_blocks), LaunchPad<60>{}));

@@ -217,7 +217,7 @@ int launch_formats(const void *in, void *payload, void *scales, int64_t numel, i
   const int64_t pad_blocks = kblocks > 0 ? scale_padding_blocks(rows, kblocks, kThreadsF) : 0;
   const int grid = balanced_grid(tiles, int64_t(dev.sm_count) * (1 << 20)) + static_cast<int>(pad_blocks);
   auto kernel = asks_ahead(Asks::kMxFormats, nchunks * 16) ? mx_formats_kernel<IN, FMT, true> : mx_formats_kernel<IN, FMT, false>;
-  return cuda_status(launch_spread(kernel, grid, kThreadsF, 0, 2048 / kThreadsF, dev, st,
+  return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(kThreadsF), 0, st,
                                              static_cast<const uint4 *>(in), static_cast<uint8_t *>(payload),
                                              static_cast<uint8_t *>(scales), nchunks, kblocks, rows,
                                              static_cast<unsigned>(pad_blocks), LaunchPad<52>{}));

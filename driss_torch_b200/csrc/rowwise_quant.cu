@@ -190,14 +190,11 @@ rowwise_looped_kernel(const void *__restrict__ in, uint8_t *__restrict__ out, fl
 template <int IN, int OUT, int CHUNKS, int TEAM_WARPS>
 int launch_regs(const void *in, void *out, float *amax_out, float *scale_out, int64_t rows, int chunks_per_row,
                 cudaStream_t st) {
-  constexpr size_t kStaticSmem = 32 * sizeof(float);
   const unsigned grid = static_cast<unsigned>(TEAM_WARPS == 1 ? ceil_div64(rows, kWarps) : rows);
   const int threads = TEAM_WARPS == 1 ? kThreads : 32 * TEAM_WARPS;
   auto kernel = asks_ahead(Asks::kRowwise, rows * chunks_per_row * 16) ? rowwise_regs_kernel<IN, OUT, CHUNKS, TEAM_WARPS, true>
                                                                        : rowwise_regs_kernel<IN, OUT, CHUNKS, TEAM_WARPS, false>;
-  DeviceInfo dev;
-  if (int e = current_device_info(&dev)) return e;
-  return cuda_status(launch_spread(kernel, grid, threads, kStaticSmem, 2048 / threads < 32 ? 2048 / threads : 32, dev, st, static_cast<const uint4 *>(in),
+  return cuda_status(launch_after_dependency(kernel, dim3(grid), dim3(threads), 0, st, static_cast<const uint4 *>(in),
                                              static_cast<uint8_t *>(out), amax_out, scale_out, rows, chunks_per_row, LaunchPad<44>{}));
 }
 

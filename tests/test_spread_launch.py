@@ -11,7 +11,7 @@ import pytest
 
 ROOT = Path(__file__).resolve().parents[1]
 SMS = 148
-# (static bytes, blocks per SM without more) of the kernels that spread: MX casts, row-wise quantization, two-orientation MX cast
+# (static bytes, blocks per SM without more): the two-orientation MX cast's, and others
 KERNELS = [(0, 8), (128, 8), (128, 32), (33792, 5)]
 GRIDS = sorted({1, 16, 17} | {k * SMS + d for k in range(1, 9) for d in (0, 1)})
 
