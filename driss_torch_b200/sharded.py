@@ -78,6 +78,15 @@ class ShardedQuantizer:
         elif fused_exchange:
             self._setup_exchange(device)
 
+    # A copy or a pickle names the package's own ops by None: a module can be neither.
+    def __getstate__(self):
+        return {**self.__dict__, "kernels": None if self.kernels is sys.modules[__package__] else self.kernels}
+
+    def __setstate__(self, state):
+        self.__dict__.update(state)
+        if self.kernels is None:
+            self.kernels = sys.modules[__package__]
+
     def _setup_exchange(self, device) -> None:
         import torch.distributed._symmetric_memory as symm_mem
 

@@ -3,7 +3,9 @@ the single max all-reduce, per-shard launches -- is the product's ``ShardedQuant
 per-shard arithmetic is injected from the CPU oracle, since the product kernels are CUDA only.
 The sharded result must equal the single-process result on the concatenated matrix, byte for
 byte."""
+import copy
 import os
+import pickle
 import socket
 import tempfile
 
@@ -93,6 +95,18 @@ def test_sharded_equals_single_process(world, empty_last):
     assert torch.equal(torch.cat([p["rw_payload"] for p in parts]), want_rw.view(torch.uint8))
     assert torch.equal(torch.cat([p["rw_amax"] for p in parts]), want_rw_amax)
     assert torch.equal(torch.cat([p["rw_scale"] for p in parts]), want_rw_scale)
+
+
+@pytest.mark.parametrize("duplicate", [copy.copy, copy.deepcopy, lambda q: pickle.loads(pickle.dumps(q))], ids=["copy", "deepcopy", "pickle"])
+@pytest.mark.parametrize("kernels", [None, OracleKernels()], ids=["own", "given"])
+def test_a_quantizer_can_be_copied_and_pickled(duplicate, kernels):
+    import driss_torch_b200
+
+    q = ShardedQuantizer(kernels=kernels, spin_limit=7)
+    same = duplicate(q)
+    assert same is not q and same.spin_limit == 7 and same.world_size == 1
+    assert same.kernels is driss_torch_b200 if kernels is None else type(same.kernels) is type(kernels)
+    assert q.kernels is (driss_torch_b200 if kernels is None else kernels)
 
 
 def test_single_process_without_process_group():
