@@ -1,5 +1,6 @@
 // launch_spread of dtq_host.h against a stand-in for the runtime's rule on shared memory: a kernel may have 48 KB, static and dynamic
 // together, until it has been allowed more on that device, at most 227 KB.  No GPU, no CUDA library.
+#include <cuda.h>
 #include <map>
 #include <utility>
 
@@ -13,6 +14,7 @@ size_t static_bytes = 0;  // of the kernel being launched
 bool grants = true;
 cudaError_t pending = cudaSuccess;
 int launches = 0;
+bool in_green_context = false;
 size_t launched_with = 0;
 
 cudaError_t answer(cudaError_t e) {
@@ -44,6 +46,16 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *cfg, const void *kerne
   return cudaSuccess;
 }
 
+CUresult stand_in_for_the_query(CUstream, CUgreenCtx *ctx) {
+  *ctx = reinterpret_cast<CUgreenCtx>(in_green_context ? &in_green_context : nullptr);
+  return CUDA_SUCCESS;
+}
+cudaError_t cudaGetDriverEntryPoint(const char *, void **f, unsigned long long, cudaDriverEntryPointQueryResult *found) {
+  *f = reinterpret_cast<void *>(stand_in_for_the_query);
+  *found = cudaDriverEntryPointSuccess;
+  return cudaSuccess;
+}
+
 // The launch of kernel `which` (0 to 63) on device `dev` of 148 SMs.  Returns the runtime's error; *bytes: what it was launched with.
 int spread_launch(int which, int dev, unsigned grid, long long statically, int most, int granted, long long *bytes, int *times, int *error_left) {
   device = dev;
@@ -60,5 +72,6 @@ int spread_launch(int which, int dev, unsigned grid, long long statically, int m
   *error_left = pending;
   return e;
 }
+void move_to_green_context(int green) { in_green_context = green != 0; }
 void forget_what_was_allowed() { allowed.clear(); }  // as a device reset does
 }

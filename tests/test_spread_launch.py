@@ -31,7 +31,7 @@ def spread(tmp_path_factory):
         e = lib.spread_launch(which, dev, C.c_uint(grid), C.c_longlong(static), most, granted, C.byref(size), C.byref(times), C.byref(left))
         return e, size.value, times.value, left.value, (which, dev)
 
-    call.forget = lib.forget_what_was_allowed
+    call.forget, call.move_to_green_context = lib.forget_what_was_allowed, lib.move_to_green_context
     return call
 
 
@@ -60,6 +60,16 @@ def test_a_grant_that_no_longer_holds_is_done_without(spread, static, most):
     assert spread(1, static, most, on=on)[:4] == (0, 0, 1, 0)
 
 
+@pytest.mark.parametrize("static, most", KERNELS)
+def test_part_of_a_device_is_not_spread_over(spread, static, most):
+    spread.move_to_green_context(1)
+    try:
+        for grid in GRIDS:
+            assert spread(grid, static, most)[:4] == (0, 0, 1, 0), grid
+    finally:
+        spread.move_to_green_context(0)
+
+
 _FIRST_CALL = """
 import torch
 import driss_torch_b200 as dt
@@ -84,3 +94,21 @@ print("right")
 def test_two_orientation_mx_cast_first_in_a_process(call, tiles):
     run = subprocess.run([sys.executable, "-c", _FIRST_CALL.format(tiles=tiles, call=call)], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert run.returncode == 0 and "right" in run.stdout, run.stderr[-2000:]
+
+
+@pytest.mark.gpu
+def test_two_orientation_mx_cast_in_a_green_context():
+    import torch
+    import driss_torch_b200 as dt
+    from torch.cuda import green_contexts
+
+    if not green_contexts.SUPPORTED:
+        pytest.skip("torch without green contexts")
+    x = torch.randn(1024, 2048, device="cuda").bfloat16()
+    want = dt.mx_fp8_quantize_dual(x)
+    torch.cuda.synchronize()
+    part = green_contexts.GreenContext.create(32, torch.cuda.current_device())
+    with torch.cuda.stream(part.Stream()):
+        got = dt.mx_fp8_quantize_dual(x)
+        torch.cuda.current_stream().synchronize()
+    assert all(torch.equal(g.view(torch.uint8), w.view(torch.uint8)) for g, w in zip(got, want))
