@@ -1534,16 +1534,17 @@ int split_worthwhile(int64_t m, int64_t n, int64_t stages, int sm_count) {
 // kernel (0: cannot launch them).  Estimated time, in microseconds as measured on a B200 = a fixed part (launch, set-up,
 // filling the pipeline, the last epilogue) plus, for every round of tiles on the busiest SM, the stages of 128 operand bytes
 // along K at the time of one, and what a tile costs besides; a tile never takes less than its epilogue.
-//   pair   256 x 256 tiles on SM pairs: 5.4 + rounds x max(0.333 stages + 0.6, 3.1; row-wise 2.3)
+//   pair   256 x 256 tiles on SM pairs: 5.4 + rounds x max(0.333 stages + 0.6, 3.4); row-wise 5.8 + rounds x max(0.333 stages + 0.6, 2.3)
 //   wide   128 x 256 on one SM: 4.2 + rounds x max(0.36 stages + 1.9, 3.2; row-wise 0.36 stages + 2.1, 4.6), its epilogue not overlapped
 //   narrow 128 x 128 on one SM: 3.2 + rounds x max(0.23 stages + 1.1, 1.9; row-wise 0.23 stages + 1.3, 2.4)
 // So large problems run on SM pairs, and problems of about a tile per SM on the narrow kernel, whose smaller tiles also
-// spread a small output over more SMs.  The constants were fitted to 230 random shapes (a mode, K of 256 to 8192, 256 to 16384 outputs,
-// up to 32768 tokens; three sets in turn) since the single-CTA kernels store through shared memory: two thirds to fit, one third to check.
-// The kernel chosen takes 0.8 % longer than the quickest on average, at most 33 % (4 x 10280 x 1056, 7.9 instead of 5.9 us); with the constants
-// before 1.7 % and 38 %.  (Pair is 0.4 quicker since than in those measurements, by its last tile's stores.)  Measured, us, narrow / wide / pair: MXFP8 2544 x 1128 x 1344 9.0 / 8.3 / 11.4, 774 x 4280 x 1152 7.9 / 7.1 / 8.5, 3453 x
-// 5000 x 512 17.4 / 15.0 / 17.9, row-wise 316 x 6712 x 480 6.4 / 7.5 / 7.9, MXFP4 17078 x 1320 x 384 15.5 / 16.4 / 19.7; row-wise 500 x 8192 x 1024
-// 10.2 / 10.0 / 8.6.
+// spread a small output over more SMs.  The constants were fitted to random shapes (K of 256 to 8192, 256 to 16384 outputs, up to 32768
+// tokens; three sets in turn); pair's, whose last tile's stores came later, to 255 others of them, and checked on 180 with K up to 2048.
+// Over those 435 the kernel chosen takes longer than the quickest, on average and at most: MXFP8 0.5 % and 11 % (3815 x 12712 x 576, 48.1 instead of 43.3 us), MXFP4
+// 0.45 % and 9 %, row-wise 1.4 % and 39 % (512 x 536 x 416, where the host is what is measured; 3518 x 2584 x 4656 36 %).  With 5.4 and 3.1 for
+// pair in MXFP8 and MXFP4 1.0 % and 24 %, 0.9 % and 22 %; 5.4 for row-wise 1.4 % and 39 %.
+// Measured, us, narrow / wide / pair: MXFP8 7666 x 4840 x 512 29.3 / 26.8 / 33.1, 6311 x 8264 x 320 37.7 / 36.6 / 45.4, MXFP4 25579 x 2912 x 384 38.7 / 36.4 /
+// 44.5, 677 x 6608 x 2144 15.5 / 16.3 / 13.5.
 int choose_kernel(bool row_wise, int64_t m, int64_t n, int64_t k_bytes, int sm_count, int pair_clusters, int split_clusters) {
   const int64_t k_stages = ceil_div64(k_bytes, kBK), m_tiles = ceil_div64(m, kBM);
   if (split_clusters > 0 && split_worthwhile(m, n, k_stages, sm_count) > 1) return DTQ_GEMM_SPLIT;
@@ -1553,8 +1554,8 @@ int choose_kernel(bool row_wise, int64_t m, int64_t n, int64_t k_bytes, int sm_c
       4.2 + rounds(m_tiles * ceil_div64(n, 256), sm_count) * std::max(0.36 * stages + (row_wise ? 2.1 : 1.9), row_wise ? 4.6 : 3.2);
   const double narrow =
       3.2 + rounds(m_tiles * ceil_div64(n, 128), sm_count) * std::max(0.23 * stages + (row_wise ? 1.3 : 1.1), row_wise ? 2.4 : 1.9);
-  const double pair = pair_clusters > 0 ? 5.4 + rounds(ceil_div64(m, 256) * ceil_div64(n, 256), pair_clusters) *
-                                                    std::max(0.333 * stages + 0.6, row_wise ? 2.3 : 3.1)
+  const double pair = pair_clusters > 0 ? (row_wise ? 5.8 : 5.4) + rounds(ceil_div64(m, 256) * ceil_div64(n, 256), pair_clusters) *
+                                                    std::max(0.333 * stages + 0.6, row_wise ? 2.3 : 3.4)
                                         : 1e30;
   return (pair < wide && pair < narrow) ? DTQ_GEMM_PAIR : (narrow <= wide ? DTQ_GEMM_NARROW : DTQ_GEMM_WIDE);
 }
