@@ -110,8 +110,10 @@ inline cudaError_t launch_after_dependency(void (*kernel)(KArgs...), dim3 grid, 
 // A programmatic dependent becomes resident while the kernel before it drains.  Where that leaves some SMs free and others full (a
 // product with one CTA of 225 KB on each of 105 of the 148 SMs), the blocks of a small grid that follows all settle on the free
 // ones, as many as fit each, and stay there when the others come free.  So a grid of less than a full wave asks for as much shared
-// memory as leaves room for its even share of blocks per SM (sixteen blocks or fewer: for two, which leaves room for a product behind
-// them).  `most` is what fits without.
+// memory as keeps more than its even share of blocks off an SM (sixteen blocks or fewer: more than two).  `most` is what fits without.
+// Not for more: all that leaves room for the share kept the blocks off every SM on which another kernel has any; us on a stream beside
+// other work, with all -> with the least: 1024 x 4096 beside a row-wise quantization 270 -> 234, beside an amax 64 -> 18, beside an elementwise
+// two-orientation cast 378 -> 339.
 // Measured, us per pass, without -> with, the two-orientation MX casts in MXFP8 training steps: 864 x 1920 x 1920 45.1 -> 36.9, 768 x 800 x
 // 4576 53.3 -> 40.8, 2048^3 56.8 -> 48.5, 4096 x 1024 x 4096 82.2 -> 79.6.
 // Only for kernels whose own shared memory keeps them off an SM that a product holds anyway, like these.  The MX and row-wise casts have
@@ -121,12 +123,12 @@ inline cudaError_t launch_after_dependency(void (*kernel)(KArgs...), dim3 grid, 
 // The amax and the elementwise two-orientation cast, whose kernels follow one another, release their dependents late instead: with an amax
 // in front of it spread, 5003 x 4096 took 25.7 instead of 22.0.  (So do the products gain for the casts, but a product behind a product
 // loses: MXFP8 300 x 2048 x 1024 5.8 -> 6.4, 1024 x 1024 x 4096 7.0 -> 7.2.)
-constexpr size_t kSmemPerSm = 228 * 1024, kSmemReserved = 1024, kSmemMost = 226 * 1024;
+constexpr size_t kSmemPerSm = 228 * 1024, kSmemReserved = 1024, kSmemUnit = 128;  // of an SM; taken by each block besides its own
+constexpr size_t least_for_share(int64_t per_sm) { return (kSmemPerSm / kSmemUnit / (per_sm + 1) + 1) * kSmemUnit - kSmemReserved; }
 inline size_t spread_bytes(int64_t grid, int sm_count, size_t static_smem, int most) {
   const int64_t per_sm = grid <= 16 ? 2 : (grid + sm_count - 1) / sm_count;
   if (per_sm >= most) return 0;
-  const size_t room = (kSmemPerSm / per_sm - kSmemReserved) / 128 * 128;
-  return (room < kSmemMost ? room : kSmemMost) - static_smem;
+  return least_for_share(per_sm) > static_smem ? least_for_share(per_sm) - static_smem : 0;
 }
 // Lets `kernel` have that much on the current device: asked of the runtime once per kernel and device (again, harmlessly, should the
 // table ever be full).  Until then a launch may have 48 KB, static and dynamic together, so any spread launch asks.
@@ -139,12 +141,12 @@ inline cudaError_t allow_spread(const void *kernel, int dev_id, size_t static_sm
     const uintptr_t there = seen[slot].load(std::memory_order_acquire);
     if (there == key) return cudaSuccess;
     if (there) continue;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMost - static_smem));
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(least_for_share(1) - static_smem));
     uintptr_t empty = 0;
     if (e == cudaSuccess) seen[slot].compare_exchange_strong(empty, key, std::memory_order_acq_rel);
     return e;
   }
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMost - static_smem));
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(least_for_share(1) - static_smem));
 }
 // Whether work on `st` has the whole device, as against the SMs of a green context.  What the driver cannot tell is a yes.
 inline bool has_whole_device(cudaStream_t st) {

@@ -47,6 +47,15 @@ def test_the_first_launch_of_every_grid_is_taken(spread, static, most):
 
 
 @pytest.mark.parametrize("static, most", KERNELS)
+def test_no_more_is_asked_for_than_keeps_others_of_the_grid_off(spread, static, most):
+    # what is left of an SM is for other kernels' blocks
+    for grid in GRIDS:
+        size, per_sm = spread(grid, static, most)[1], 2 if grid <= 16 else -(-grid // SMS)
+        if size:
+            assert (per_sm + 1) * (static + size + 1024 - 128) <= 228 * 1024 < (per_sm + 1) * (static + size + 1024), grid
+
+
+@pytest.mark.parametrize("static, most", KERNELS)
 def test_memory_that_is_not_granted_is_left_out(spread, static, most):
     for grid in GRIDS:
         assert spread(grid, static, most, granted=0)[:4] == (0, 0, 1, 0), grid
