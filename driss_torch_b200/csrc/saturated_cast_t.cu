@@ -42,12 +42,14 @@ constexpr int kTileWords = 32;  // 32-bit words of fp8 bytes per shared-memory r
 // writes its 128 rows of a column as the aligned 16 bytes inside and single bytes at either end; with kWhole it reads 16 rows more and
 // writes the eight aligned 16 bytes that begin in its rows, so that only the ends of a whole column are single bytes.
 // Fewer partial sectors, and streaming stores, against an eighth more to read, convert and transpose.  Measured, both orientations behind an
-// amax, outputs that stay for a pass, us, kEnds / kWhole / kWhole with plain stores: bf16 16383 x 8192 161.1 / 137.6 / 143.7, 9999 x 4096 44.8 / 45.4 /
-// 45.4, 5003 x 4096 (1280 tiles) 24.3 / 22.6 / 23.8, 1500 x 8200 16.7 / 16.5 / 16.5, 1537 x 8192 (832) 17.3 / 16.6 / 16.6; kEnds / kWhole where outputs
-// are dropped at once 2001 x 4096 (512 tiles) 13.0 / 14.1, 333 x 8192 (192) 9.1 / 11.6; fp32, where reading weighs twice, 9999 x 4096 67.4 / 68.4,
-// 2001 x 4096 14.9 / 15.7.
+// amax, bf16, three inputs in turn in a graph, us, kEnds / kWhole, outputs that stay, and dropped at once so that the next pass writes where the last did:
+// 333 x 8192 (192 tiles) 8.2 / 8.8, 7.5 / 8.2; 2001 x 4096 (512) 13.2 / 12.8, 11.5 / 10.3; 3001 x 4096 (768) 18.3 / 17.0, 15.4 / 14.0; 5003 x 4096 (1280) 27.0 / 24.4,
+// 21.9 / 20.8; 8195 x 4096 42.5 / 37.6, 33.4 / 33.5; 9999 x 4096 50.6 / 45.3, 41.1 / 42.3; 12001 x 4096 59.7 / 53.0, 48.0 / 49.9; 16383 x 8192 159.6 / 139.7,
+// 158.0 / 135.6.  By themselves, dropped at once in a stream, 6147 x 4096 17.0 / 20.0 and 9999 x 4096 29.7 / 31.1; kept 22.2 / 20.0 and 35.6 / 31.2.  Plain
+// stores with kWhole, 5003 x 4096 23.8 for 22.6, 16383 x 8192 143.7 for 137.6.  fp32, where reading weighs twice, 9999 x 4096 67.4 / 68.4, 2001 x 4096
+// 14.9 / 15.7.
 enum Rows { kAligned, kEnds, kWhole };
-constexpr int kWholeMinTiles = 5 * kB200Sms;  // more than the device holds at once; bf16 only
+constexpr int kWholeMinTilesPerSm = 5;  // more than the device holds at once; bf16 only
 constexpr int kWholeRows = kTileRows + 16;
 constexpr int kRaggedPitch = kWholeRows / 4;  // words between byte columns of the transposed tile
 static_assert(kRaggedPitch % 4 == 0, "16-byte stores to its columns");
@@ -332,7 +334,7 @@ int launch_transposed(const void *in, void *out, void *out_t, const float *scale
   const bool tiles = readable && (aligned_rows || tile_count >= dev.sm_count);
   auto kernel = aligned_rows ? cast_transposed_kernel<C, BOTH, kAligned> : cast_transposed_kernel<C, BOTH, kEnds>;
   if constexpr (C::kChunkElems == 8)  // bf16
-    if (!aligned_rows && tile_count > kWholeMinTiles) kernel = cast_transposed_kernel<C, BOTH, kWhole>;
+    if (!aligned_rows && tile_count > int64_t(kWholeMinTilesPerSm) * dev.sm_count) kernel = cast_transposed_kernel<C, BOTH, kWhole>;
   if (tiles) {
     const int64_t row_tiles = ceil_div64(rows, kTileRows), col_tiles = ceil_div64(cols, kTileCols);
     if (row_tiles > 0x7FFFFFFFLL / col_tiles) return DTQ_ERR_TOO_LARGE;
