@@ -95,25 +95,23 @@ amax_kernel(const void *__restrict__ in, float *__restrict__ out, int64_t numel,
   const int64_t nchunks = (numel - head) / kElems;
   // This launch itself may have started under the tail of its predecessor: part of the block's first tile is asked into L2
   // meanwhile, harmless whatever the predecessor still writes (see l2_prefetch_bulk).  What it hides is the start of the stream.
-  // 4 MiB in all of inputs of up to 20 MiB of bf16 and 22 MiB of fp32, 16 MiB of up to 40 MiB of fp32 (amax_ask_chunks).  Measured, us with
-  // nothing asked, and the change in percent with 4 / 8 / 16 MiB and with whole first tiles (up to 37 MiB); inputs from memory (400 MB of them
-  // in turn) and three inputs in turn:
-  //                         amax, from memory        amax, both casts, from memory   amax, both casts, three
-  //   bf16   8 MiB    5.3   -6.2 -10.8  -9.6  -9.8   10.0  -2.2 -2.5 -2.4  -1.9       9.1 -0.5  0.0  +0.1  -0.1
-  //         16 MiB    6.4   -4.4  -9.7  -7.6  -6.7   11.9  -3.2 -2.5 +0.2  +0.3      12.2 -3.9 -7.3 -11.4 -11.8
-  //         24 MiB    7.4   -2.4  -1.3  +3.2  +5.8   15.8  +2.8 +4.4 +7.4 +12.5      15.6 +2.7 +3.4  +2.9  +6.3
-  //         39 MiB    9.6   -2.5  +0.6  +5.9  +4.3   22.3  +5.2 +6.8 +9.2 +10.7      21.7 +4.9 +6.7  +9.1 +10.5
-  //         47 MiB   11.1   -0.5  -0.6  +0.1  +4.0   25.7  +7.8 +10.1 +11.8 +14.8    25.3 +5.3 +8.5 +10.5 +13.1
-  //         39 MiB, rows no multiple of 16           24.8  -1.5 -3.9 -4.5  -3.6      24.8 -1.4 -4.2  -5.1  -4.4
-  //   fp32  16 MiB    6.5   -7.0 -10.4 -10.2  -9.5   10.5  -4.6 -6.1 -4.3  -3.8       9.7 -2.4 -1.2  -2.3  -2.8
-  //         22 MiB    7.2   -1.5  -2.2  +2.1  +4.5   12.5  -3.7 -7.6 -8.8  -9.8      12.5 -3.7 -9.1 -11.9 -13.9
-  //         24 MiB    7.5   -3.5  -5.0  +0.3  +1.7   13.1  -4.8 -8.2 -7.3  -7.5      13.1 -4.2 -8.7 -13.1 -14.1
-  //         28 MiB    7.9   -5.8  -9.8  -4.2  -0.3   14.5  -5.9 -6.9 -8.0  -5.4      14.7 -4.8 -8.6 -15.0 -15.8
-  //         39 MiB   10.0   -7.0  -3.2  -0.9  -6.2   18.3  -5.3 -7.0 -6.0  -4.2      18.5 -2.3 -8.3 -11.3 -10.9
-  //         47 MiB   11.2   -1.6  -2.8  -1.7  +1.8   21.2  +1.6 +2.6 +5.0  +8.1      20.9 +0.5 +0.1  +1.0  +3.2
-  // It loses where the kernel before, the casts of the tensor before, still reads and writes as much as L2 holds; that ragged
-  // rows of bf16 gain all the same the amax cannot see.  Behind an MXFP8 product that writes the input, 16 MiB: 17.5 us / 17.4 with
-  // 4 MiB, with both casts 39.2 / 39.2 (whole tiles 41.4).
+  // 4 MiB in all of inputs of up to 20 MiB of bf16 and 22 MiB of fp32, 16 MiB of up to 40 MiB of fp32 (amax_ask_chunks).  Measured in a
+  // graph, outputs that stay, us with nothing asked, and the change in percent with 4 / 8 / 16 / 32 MiB; inputs from memory (400 MB of them in
+  // turn), the last column three inputs in turn:
+  //                 amax                          amax, static cast             amax, both casts              amax, both casts, three
+  //   bf16   8 MiB   4.6  -8.4 -11.7 -11.5 -11.5   7.1  -3.5  -6.4  -6.8  -6.1   8.2  +5.1  +6.8  +6.7  +6.8   7.5 +4.5  +7.4  +8.0  +7.6
+  //         16 MiB   5.5  -6.5  -8.2  -1.8  -1.6  10.3  -7.0 -10.1  -8.0  -7.8  11.8  +3.6  +5.5  +6.4  +6.7  11.2 +4.5  +5.2  +6.4  +7.1
+  //         20 MiB   6.1  -5.1  -8.4  -2.8  -3.0  11.7  -4.4  -7.9  -8.1  -5.9  12.9 +11.1 +10.6 +15.1 +17.5  13.0 +8.1  +7.5  +9.8 +11.8
+  //         24 MiB   6.6  -5.3  -8.3  -2.3  +0.3  13.2  -3.8  -6.0  -8.8  -6.8  14.5 +11.9 +13.3 +15.3 +20.4  14.4 +8.6 +10.0  +9.8 +13.0
+  //         40 MiB   8.9  -3.7  -6.3  -6.2  -5.0  19.1  -2.4  -3.9  -4.0  -2.9  21.0 +13.2 +13.0 +15.3 +17.0  21.3 +9.1  +9.7 +10.5 +11.4
+  //         20 MiB, rows no multiple of 16                                      16.4  -1.3  -4.3  -3.5  -2.2  16.4 -1.9  -5.1  -5.3  -3.9
+  //   fp32   8 MiB   4.5  -7.9 -12.1 -12.1 -12.3   7.0  +0.1  -1.0  -1.0  -1.0   7.3  -1.2  +1.8  +1.5  +1.5   6.2 -3.9  -3.1  -3.2  -2.8
+  //         16 MiB   5.5  -5.6  -7.1  -2.0  -0.9   9.2  -2.0  -3.7  -0.7  -0.7   9.7  -0.2  +2.1  +1.8  +2.2   8.7 +1.8  +4.8  +4.9  +3.7
+  //         24 MiB   6.6  -4.4  -7.3  -2.0  +1.4  11.5  +0.3  +0.6  +1.4  +4.5  12.3  +3.6  +1.1  +1.1  +4.6  12.1 +3.6  -0.7  -1.5  -1.6
+  //         32 MiB   7.7  -3.1  -5.7  -6.6  +0.4  14.9  -3.0  -3.1  -5.0  -2.6  15.1  +4.9  +2.5  -0.6  +5.8  15.0 +2.4  +0.8  -4.9  -3.2
+  //         40 MiB   8.8  -3.5  -5.3  -5.8  -1.7  17.5  -2.5  -3.4  -2.5  -1.5  17.7  +5.2  +3.4  +5.2  +7.7  17.7 +3.2  +1.9  +2.0  +2.7
+  // An amax alone or with a static cast gains; with both casts aligned rows of bf16 lose, and more beyond 20 MiB, where it stops.  Which will follow
+  // the amax cannot see.
   constexpr int64_t kTile = int64_t(kAmaxThreads) * UNROLL;
   if constexpr (PREFETCH) {
     if (threadIdx.x == 0) prefetch_first_tile(body, blockIdx.x * kTile, ask_chunks, nchunks);

@@ -106,39 +106,39 @@ constexpr int kB200Sms = 148;
 // still writes, see l2_prefetch_bulk).  What it hides is the start of the stream.  asks_ahead (dtq_host.h) has the sizes.
 // Measured, bf16 [rows, 4096], outputs that stay; us with nothing asked, and the change in percent with 8 / 16 / 24 (static cast)
 // or 2 / 4 / 8 blocks per SM (the others).  From memory: inputs of 400 MB in turn; three: three inputs in turn, as much of them in
-// L2 as fits; amax: behind an amax of the input, the two together; product: behind an MXFP8 product of K = 1024 that
-// wrote the input, the two together.  The products, and at the time of these figures the amax, release their dependents early, so that their
-// lines are asked for in vain.
-//   static cast      from memory             three                   amax, from memory       product
-//      16 MiB   4.66  -6.9  -6.7  -6.7    3.96  -0.4  -4.3  -4.6    9.9 +0.9 +2.1 +2.8    16.1 -0.4 +0.3 +0.2
-//      32 MiB   7.92 -11.8 -12.3 -10.7    8.63 -13.1 -21.2 -24.0   15.5 -1.7 -3.4 -0.9    26.5 +0.5 +1.2 +1.7
-//      47 MiB  12.10  -5.6  -6.7  -6.2   12.17  -5.7  -9.4 -10.9   20.7 +1.9 +3.9 +5.1    36.9 +0.5 +0.9 +1.5
-//      64 MiB  16.09  -3.4  -3.7  -3.2   15.98  -3.5  -6.0  -6.0   27.1 +4.0 +5.4 +5.7    45.6 +0.6 +0.9 +1.1
-//      80 MiB  19.53  -2.3  -2.6  -2.0   19.46  -2.4  -4.2  -4.0   34.3 +1.4 +0.7 +0.4    59.4 -0.4 -0.7 -0.9
-//     128 MiB  29.82  -1.0  -1.4  -0.8   30.02  -0.7  -1.7  -1.5   53.8 -0.3 -0.9 -2.1    96.1 -0.7 -0.7 -0.8
+// L2 as fits; amax: behind an amax of the input from memory, the two together in a graph, with as many blocks as ask; product: behind an MXFP8
+// product of K = 1024 that wrote the input, the two together.  The products release their dependents early, so that their lines are asked for in
+// vain; the amax when it ends, and then the lines stand behind the end of its own.
+//   static cast      from memory             three                   amax            product
+//      16 MiB   4.66  -6.9  -6.7  -6.7    3.96  -0.4  -4.3  -4.6     9.1  +6.0       16.1 -0.4 +0.3 +0.2
+//      32 MiB   7.92 -11.8 -12.3 -10.7    8.63 -13.1 -21.2 -24.0   15.0  +5.7       26.5 +0.5 +1.2 +1.7
+//      47 MiB  12.10  -5.6  -6.7  -6.2   12.17  -5.7  -9.4 -10.9   19.5 +10.6       36.9 +0.5 +0.9 +1.5
+//      64 MiB  16.09  -3.4  -3.7  -3.2   15.98  -3.5  -6.0  -6.0   25.9  +8.0       45.6 +0.6 +0.9 +1.1
+//      80 MiB  19.53  -2.3  -2.6  -2.0   19.46  -2.4  -4.2  -4.0   32.9  +3.1       59.4 -0.4 -0.7 -0.9
+//     128 MiB  29.82  -1.0  -1.4  -0.8   30.02  -0.7  -1.7  -1.5   52.7  -0.9       96.1 -0.7 -0.7 -0.8
 //     256 MiB  57.26  +0.5  +0.7  +0.8
-//   fp32  16   4.51  -3.5  -5.4  -5.5    3.69  +4.8  +3.6  +3.8    9.8 +1.2 +1.7 +2.9
-//         28   6.58  -5.5  -6.0  -6.9    6.82  -6.6 -10.1 -12.4   13.4 +1.8 +0.4 +1.7
-//         64  13.28  -7.8 -11.8 -10.1   13.68  -4.8 -10.7 -13.5   25.4  0.0 -0.6 -1.1
-//        128  25.68  -0.5  -1.7  -2.0   25.66   0.0  -1.7  -2.7   48.8 +0.7 +0.3 -0.4
-//   Two waves of blocks (16 per SM), not between 48 and 80 MiB: there input and output of the pair just fill L2, and what is
-//   asked for pushes out what the cast behind the amax would have found.
+//   fp32  16   4.51  -3.5  -5.4  -5.5    3.69  +4.8  +3.6  +3.8     8.9  +2.8
+//         28   6.58  -5.5  -6.0  -6.9    6.82  -6.6 -10.1 -12.4   12.6  -0.6
+//         64  13.28  -7.8 -11.8 -10.1   13.68  -4.8 -10.7 -13.5   24.5  +4.5
+//        128  25.68  -0.5  -1.7  -2.0   25.66   0.0  -1.7  -2.7   47.7  +0.8
+//   Two waves of blocks (16 per SM), not of bf16 between 48 and 80 MiB: there input and output of the pair just fill L2, and what is
+//   asked for pushes out what the cast behind the amax would have found.  That holds below as well, where the cast alone gains more.
 //   MX cast (4 blocks per SM)
-//      16 MiB   5.00  -9.2  -4.2  -6.4    4.44  -5.0  -4.7  -4.5   10.8 -4.1 -3.3 -2.2    17.2  0.0 +0.1 +0.5
-//      32 MiB   8.65 -13.2 -12.6 -11.9    9.04  -8.6 -13.8 -16.9   16.1 -5.3 -6.3 -4.3    27.1 -0.3 +0.1 +0.4
-//      64 MiB  16.8   -1.4  -3.3  -2.0   16.8   -1.6  -3.4  -5.4   27.9 +3.2 +3.7 +2.7    47.6 +0.6 +1.1 +1.0
-//     128 MiB  31.4   -0.7  -1.2  -0.6   31.4   -0.7  -0.9  -0.4   55.2 -1.4 -1.6 -2.4    98.5 -0.4 -0.5 -0.9
+//      16 MiB   5.00  -9.2  -4.2  -6.4    4.44  -5.0  -4.7  -4.5   10.3  -9.1       17.2  0.0 +0.1 +0.5
+//      32 MiB   8.65 -13.2 -12.6 -11.9    9.04  -8.6 -13.8 -16.9   15.8  +3.2       27.1 -0.3 +0.1 +0.4
+//      64 MiB  16.8   -1.4  -3.3  -2.0   16.8   -1.6  -3.4  -5.4   29.5  -1.8       47.6 +0.6 +1.1 +1.0
+//     128 MiB  31.4   -0.7  -1.2  -0.6   31.4   -0.7  -0.9  -0.4   54.6  -1.5       98.5 -0.4 -0.5 -0.9
 //     512 MiB 120.1   -0.2  -0.3   0.0
 //   MX cast, blocked scales (2 blocks per SM)
-//      16 MiB   5.33  -6.4  -1.9  -5.1    4.97  +0.2  +1.6  -2.6                           17.6 +0.1 +0.1 +0.1
-//      32 MiB   8.99  -9.8  -8.1  -6.7    9.31  -6.4  -8.7 -11.1                           27.7 +0.5 +0.6 +0.6
-//      64 MiB  16.95  -1.7  -2.4  -1.2   17.0   -1.4  -2.8  -2.8                           48.3 +0.6 +0.9 +1.3
-//     128 MiB  31.5   -0.5  -0.5  +0.9   31.5   -0.5  -0.5  +0.9                           98.8 -0.2 -0.1 -0.4
+//      16 MiB   5.33  -6.4  -1.9  -5.1    4.97  +0.2  +1.6  -2.6                   17.6 +0.1 +0.1 +0.1
+//      32 MiB   8.99  -9.8  -8.1  -6.7    9.31  -6.4  -8.7 -11.1                   27.7 +0.5 +0.6 +0.6
+//      64 MiB  16.95  -1.7  -2.4  -1.2   17.0   -1.4  -2.8  -2.8                   48.3 +0.6 +0.9 +1.3
+//     128 MiB  31.5   -0.5  -0.5  +0.9   31.5   -0.5  -0.5  +0.9                   98.8 -0.2 -0.1 -0.4
 //     512 MiB 120.9   +0.5  +1.5  +3.6   so not beyond 128 MiB
 //   row-wise (8 blocks per SM)
-//      16 MiB   5.59  -7.2 -11.8 -12.0    5.17  -3.9  -5.2  -6.6                           17.3 -0.5 -0.1 -0.1
-//      32 MiB   9.11  -8.7 -13.6 -15.1    9.28  -7.4 -11.6 -15.5                           27.9 -1.0 -1.0 -0.7
-//     128 MiB  30.9   -2.1  -3.0  -4.0   31.0   -2.8  -3.7  -4.7                           96.8 -0.4 -0.6 -0.8
+//      16 MiB   5.59  -7.2 -11.8 -12.0    5.17  -3.9  -5.2  -6.6                   17.3 -0.5 -0.1 -0.1
+//      32 MiB   9.11  -8.7 -13.6 -15.1    9.28  -7.4 -11.6 -15.5                   27.9 -1.0 -1.0 -0.7
+//     128 MiB  30.9   -2.1  -3.0  -4.0   31.0   -2.8  -3.7  -4.7                   96.8 -0.4 -0.6 -0.8
 // Below 16 MiB the grid is not much more than what is resident at once, and the loads follow at the prefetch's heels.
 // Up to 2 MiB it is on again, for the tokens of a decode step: the product queued behind asks for its weights as soon as it is
 // resident, and the cast's reads would stand behind those.  Cast and product, weights from memory, us, without / with, two (MXFP8),

@@ -70,7 +70,9 @@ static_assert(kMaxShares < kOneGaveUp && int64_t(kMaxShares) * kOneGaveUp <= 0xF
 constexpr int kGaveUp = 0, kMet = 1, kImpatient = 2, kShareIsGone = 3;
 constexpr unsigned int kPatience = 64;  // polls, about 50 us, before a waiting block looks for shares to take over
 
-// Thread 0 of the owner, first thing.  The launch, in twos; with kTakenOver: the share is another block's by now, nothing is left to do.
+// Thread 0 of the owner, first thing.  The launch, in twos; with kTakenOver: the share is another block's by now, nothing is left to do.  (The
+// block reads it all the same before it looks: a barrier in front of the second tile cost inputs of 16 to 32 MiB 2 to 5 %, and saved 9 % of
+// 1 GiB in 1024 blocks, of which 296 fit.)
 __device__ __forceinline__ unsigned int come_for_own_share(Workspace *ws) {
   const unsigned int before = atomicAdd(&ws->shares[blockIdx.x], kLaunch);
   if (before & kTakenOver) atomicSub(&ws->shares[blockIdx.x], kTakenOver);

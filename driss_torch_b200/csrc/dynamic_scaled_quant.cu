@@ -109,9 +109,9 @@ struct DsqChunk<DTQ_F32, OUT> {
 
 // ---- fused single launch -------------------------------------------------------------------------
 // As a cooperative launch, or any that is not a programmatic dependent, it waited in a stream for whole multiples of about 2.05 us from
-// kernel to kernel, which a CUDA graph did not show.  Us in a stream, three inputs in turn, cooperative -> now (and in a graph): bf16 2 MiB 6.4 -> 5.5
-// (the host), 8.4 MiB 6.6 -> 5.5 (5.3 -> 5.2), 16 MiB 10.2 -> 7.8 (7.3 -> 7.1), 24 MiB 12.2 -> 10.0 (9.5 -> 9.3), 32 MiB 13.9 -> 11.9 (12.0 -> 11.9),
-// 64 MiB 20.5 -> 18.1 (18.3 -> 17.9), 128 MiB 45.0 -> 43.4 (43.0), 320 MiB 121.2 -> 119.6 (119.5).
+// kernel to kernel, which a CUDA graph did not show.  Us, three inputs in turn, cooperative -> now, in a stream with outputs dropped at once (and in a
+// graph with outputs that stay): bf16 4 MiB 6.2 -> 4.6 (4.6 -> 4.6), 8 MiB 7.2 -> 5.1 (5.8 -> 5.4), 16 MiB 10.3 -> 7.7 (9.2 -> 8.5), 32 MiB 14.3 -> 11.6
+// (13.7 -> 13.1), 64 MiB 22.5 -> 20.2 (21.6 -> 20.7), 128 MiB 45.0 -> 42.7 (43.1 -> 42.4), 320 MiB 120.4 -> 118.6 (118.5 -> 118.2).
 // Requires `in` 16-byte aligned and `out` aligned for the packed store; numel may be anything
 // (block 0 handles the elements past the last whole chunk).  Dynamic shared memory holds
 // `smem_tiles` tiles.
@@ -400,7 +400,9 @@ dsq_cluster_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ out, floa
 }
 
 // ---- cast phase alone ---------------------------------------------------------------------------------
-constexpr int kCastPrefetchTiles = 6;  // tiles per block asked of L2 while the block waits for the amax
+// Tiles per block asked of L2 while the block waits for the amax.  An amax kernel lets the cast in only when it ends, which leaves 352 MiB to
+// 1 GiB within 0.3 % of what they took when it did at its start.
+constexpr int kCastPrefetchTiles = 6;
 template <int IN, int OUT, int UNROLL>
 __global__ void __launch_bounds__(kThreads, 2048 / kThreads)
 cast_with_amax_stream(const uint4 *__restrict__ in, uint8_t *__restrict__ out, const float *__restrict__ amax_p,

@@ -107,8 +107,8 @@ mx_amax_kernel(const uint4 *__restrict__ in, uint8_t *__restrict__ payload, uint
 // maximum is published before its outputs are stored, so that the fence has none of them to wait for and the ticket is on its way meanwhile.
 // What it saves is the host's: with cast_with_amax behind it, us per pass / on the device alone, finishing launch -> last block: 1 MiB
 // 12.0 / 4.5 -> 10.8 / 4.8, 4 MiB 12.0 / 7.5 -> 10.7 / 7.6, 16 MiB 12.0 / 9.4 -> 10.8 / 9.5; 24 MiB 12.0 / 11.9 -> 13.5 / 13.1, so not beyond
-// kSmallTiles.  It releases the cast behind when it ends: 8 MiB 8.3 -> 7.4 on the device.  With the ticket taken behind the stores 4 MiB took 8.4 on the device, with the last block's first warp collecting the
-// maxima ahead of its own stores 8.2.
+// kSmallTiles.  It releases the cast behind when it ends: 8 MiB 8.3 -> 7.4 on the device.  With the ticket taken behind the stores 4 MiB took
+// 8.4 on the device, with the last block's first warp collecting the maxima ahead of its own stores 8.2.
 constexpr int64_t kSmallTiles = 1024;  // 16 MiB of input
 static_assert(kSmallTiles <= kMaxGridBlocks, "a partial per block");
 __global__ void __launch_bounds__(kThreadsA, 2048 / kThreadsA)
